@@ -348,6 +348,17 @@ int scene_consts(const pbf_scene* s, float dt, StepConsts& C) {
         }
         C.cut = std::max(C.h2, g);
     }
+    {
+        // Largest float g with sqrtf(g) <= 1e-7f: r_sq > g is |r| > 1e-7.
+        float g = 1e-7f * 1e-7f;
+        while (std::sqrt(g) > 1e-7f) g = std::nextafter(g, 0.0f);
+        while (std::sqrt(std::nextafter(g, 1.0f)) <= 1e-7f) g = std::nextafter(g, 1.0f);
+        C.r2_min = g;
+    }
+    C.one = 1.0f;
+    // Radii whose squares, kernel values and quotients all stay far from the
+    // ends of float's exponent range (the kernels scale with h^-9).
+    C.paired = h >= 1e-3f && h <= 100.0f ? 1 : 0;
     C.inv_cell = 1.0f / h;
     C.mass = s->mass;
     C.rho0 = st.rest_density;
@@ -363,6 +374,7 @@ int scene_consts(const pbf_scene* s, float dt, StepConsts& C) {
     }
     const float delta_q = st.corr_delta_q * h;
     C.w_dq = host_poly6(delta_q * delta_q, h);
+    C.inv_w_dq = 1.0f / C.w_dq;
     C.neg_corr_k = -st.corr_k;
     C.corr_n4 = st.corr_n == 4 ? 1 : 0;
     C.scorr_on = C.w_dq > 1e-10f ? 1 : 0;

@@ -13,6 +13,9 @@
 #include <cstdint>
 #include <type_traits>
 
+#include <cuda_fp16.h>
+
+#include "exact_pair.cuh"
 #include "exact_repeat.h"
 #include "pbf_types.cuh"
 #include "radix_sort.cuh"
@@ -28,16 +31,12 @@ namespace pbf {
 namespace PBF_NS {
 
 constexpr int kBlock = 128;
-// A single scene of at least this many particles runs its neighbour passes
-// with the warp-cooperative walk (and its one-thread fallback with the row
-// loop unrolled by 8).  Smaller scenes and batches keep one thread per
-// particle and the 4-way loop: many small scenes stepped side by side on their
-// own streams run several kernels per SM at once, and there the larger code
-// and shared memory measured up to 40 % slower.
+// Single scenes of at least this many particles look for runs of identical
+// particles (k_segments).
 constexpr int kBigScene = 1 << 17;
-// The fewest candidates a row of the cooperative walk must hold before the
-// walk looks for runs of identical candidates in it (rows of ordinary fluid
-// hold a few hundred).
+// The fewest candidates a row or bucket must hold before a walk looks for
+// runs of identical candidates in it (rows of ordinary fluid hold a few
+// hundred).
 constexpr uint32_t kRunRow = 1024;
 constexpr uint32_t kNoBucket = 0xffffffffu;
 constexpr uint32_t kImpureBit = 0x80000000u;
@@ -109,26 +108,10 @@ __device__ __forceinline__ float spiky_coeff(float r_sq, const StepConsts& C) {
 #endif
 }
 
-// Adding a term to a running sum once (One) or m times in a row (a run of
-// identical candidates in the cooperative walk): acc(s, t, m) is the float
-// that m single additions of t leave, bit for bit.  (rep_add is inlined: as
-// a call, the calling convention's saved registers cost the walk's hot
-// loops spills.)
-struct One {};
-__device__ __forceinline__ float acc(float s, float t, One) { return s + t; }
-__device__ __forceinline__ float acc(float s, float t, uint32_t m) { return rep_add(s, t, m); }
-// The same as a call (the constraint passes' one-thread walks, where the
-// inlined loop cost the density pass's hot loops registers).
-struct Many {
-    uint32_t n;
-};
+// Adding a term to a running sum m times in a row (a run of identical
+// candidates): the float that m single additions of t leave, bit for bit.  A
+// call: inlined, its loop cost the neighbour passes' hot loops registers.
 __device__ __noinline__ float rep_add_call(float s, float t, uint32_t m) { return rep_add(s, t, m); }
-__device__ __forceinline__ float acc(float s, float t, Many m) { return rep_add_call(s, t, m.n); }
-
-__device__ __forceinline__ bool bits_equal(const float4 a, const float4 b) {
-    return __float_as_uint(a.x) == __float_as_uint(b.x) && __float_as_uint(a.y) == __float_as_uint(b.y) &&
-           __float_as_uint(a.z) == __float_as_uint(b.z) && __float_as_uint(a.w) == __float_as_uint(b.w);
-}
 
 // ---------------------------------------------------------------------------
 // Grid helpers
@@ -592,15 +575,15 @@ struct Grid {
 // kRunRow candidates, a run's first particle q calls fr(q, L) for the run's L
 // particles, which come next in the candidate order (the run lies in one
 // cell, in cell order), and the walk goes on after them.
-template <int U, bool kRuns, class F, class FR>
+template <bool kRuns, class F, class FR>
 __device__ __forceinline__ void for_each_candidate_runs(const int4 cell, const Grid& G,
                                                         const StepConsts& C, F&& f, FR&& fr) {
     if constexpr (!kRuns) {
-        for_each_candidate<U>(cell, G.off, G.kpos, G.bend, G.btab, C, f);
+        for_each_candidate(cell, G.off, G.kpos, G.bend, G.btab, C, f);
         return;
     }
     if (!G.segend) {
-        for_each_candidate<U>(cell, G.off, G.kpos, G.bend, G.btab, C, f);
+        for_each_candidate(cell, G.off, G.kpos, G.bend, G.btab, C, f);
         return;
     }
     const GridDesc& Gd = C.grid;
@@ -611,7 +594,7 @@ __device__ __forceinline__ void for_each_candidate_runs(const int4 cell, const G
         if (q1 - q >= kRunRow)
             for (int d = 0; d < k; ++d) any |= (__ldg(G.slot_alias + s + d) & kRunSlot) != 0;
         if (!any) {
-#pragma unroll U
+#pragma unroll 4
             for (; q < q1; ++q) f(q);
             return;
         }
@@ -709,144 +692,199 @@ __device__ __forceinline__ T ld_step(const T* p) {
 }
 
 // ---------------------------------------------------------------------------
-// Warp-cooperative candidate walk (single scenes).
+// The neighbour walks: a pass's sums over the candidates of each particle.
 //
-// The 32 particles of a warp usually sit in one cell, or in two or three
-// cells next to each other along x.  When every lane is clean (no merged
-// reference bucket near it) and the lanes' cells share one (y, z) row and
-// span at most three cells in x, the lanes' candidate sequences are
-// sub-sequences of one sequence: the 9 rows (dz, dy) of cells
+// Particles next to each other in cell order usually sit in one cell, or in
+// a few cells next to each other along x.  Those of one (y, z) row of cells
+// within three cells in x form a group: their candidate sequences are
+// sub-sequences of one sequence, the 9 rows (dz, dy) of cells
 // [xmin - 1, xmax + 1], each in slot order, which is the reference's order
-// (cells in (dz, dy, dx) order, ascending particle index inside a cell).  A
-// lane's own sequence is that one restricted to the cells within one of its
-// own in x.  The warp walks it in two phases:
+// (cells in (dz, dy, dx) order, ascending particle index inside a cell).
+// Particles of one cell whose reference buckets are merged (dirty) form a
+// group too: their sequence is the cell's 27 buckets.  A walk takes its
+// groups one after another, each in two phases:
 //
-//  1. listing, chunk by chunk: each lane loads one candidate per round of 32
-//     (coalesced); a candidate farther from the bounding box of the warp's
-//     positions than the kernel support adds an exact zero to every lane and
-//     is dropped, the rest are staged in shared memory in order (x, y and z
-//     in separate arrays), up to CH per chunk, and their positions appended
-//     to the warp's survivor list.  Each lane then tests the chunk's
-//     candidates two at a time (paired f32x2 operations) and sets a bit in
-//     its own mask over the survivor list for each one that may be in its
-//     support and lies in its own 27 cells.  The test is conservative: it
-//     fuses the squares and sums (a few ulps from the exact r^2) and compares
-//     against the support radius widened by 1e-6, so it keeps every
-//     in-support candidate, and every term re-tests the exact r^2 itself;
-//  2. evaluation, once the list holds up to CAP survivors or the walk ends:
-//     each lane evaluates the terms of its set bits in order, loading each
-//     candidate by its position one term ahead.
+//  1. listing: the sequence is cut into words of up to 32 candidates, each a
+//     contiguous range of one row or bucket.  A warp stages four words in
+//     shared memory as fp16 rows, and the tensor core computes
+//     r^2 - support^2 of all pairs of the 128 candidates and the group's
+//     particles (see Rows below); the signs of the accumulators are the
+//     words' masks, one bit per candidate and particle.  The test is
+//     conservative, so it keeps every in-support candidate; every term
+//     re-tests the exact r^2 itself;
+//  2. evaluation, once enough is listed or the sequence ends: each
+//     particle's terms, two at a time, in list order.
 //
-// Every lane thus adds exactly the nonzero terms of the one-thread walk, in
-// the same order, so the sums are bit-identical.  The terms (two IEEE
-// divisions and a square root in the exact build) run with the lanes of a
-// step busy instead of waiting on the few in-support lanes of each
-// candidate, and the distance test runs on the surviving candidates only.
-// The list spans the whole walk rather than one chunk because the candidate
-// order is spatially coherent: a chunk covers a few rows, which lie in the
-// support of some lanes and not of others, so evaluating chunk by chunk
-// leaves many lanes of each term step idle.  Only single scenes of at least
-// kBigScene particles walk cooperatively (see CoopBlock).
+// Every sum thus sees exactly the nonzero terms of the one-thread walk, in
+// the same order, so it is bit-identical.
+//
+// Why: the exact terms (an IEEE square root and division each) should only
+// run for candidates in support, with all lanes busy, and the distance test,
+// which runs for every candidate (1,600 per particle at h = 4 r for about
+// 250 terms), should cost little.  Lane by lane a test costs about seven
+// instructions per candidate and particle; here 32 candidates x 32 particles
+// cost two fragment loads, eight mma and 32 shifts, about one instruction
+// and a quarter per candidate of a warp.
+//
+// Two forms:
+//  * the warp walk (walk_group): a warp has 32 particles, one a lane, and a
+//    lane adds its particle's terms itself.  The cheapest per particle;
+//  * the team walk (team_walk): four warps share TP = 8 or 16 particles.
+//    The warps list different words, then 128 / TP lanes evaluate each
+//    particle's terms side by side and pass them through shared memory to
+//    the lanes that add them in order.  For scenes whose particles would
+//    leave most of the chip idle, or its warps waiting on one chain each,
+//    with one lane per particle (team_size).
 
-// Candidates staged per chunk, and survivors listed before an evaluation:
-// shared memory is CH * 17 + CAP * 8 bytes per warp (6.98 KB), eight blocks
-// of four warps per SM (each block also takes 1 KB of the SM's 228 KB).  (128-candidate chunks pad less but fit seven
-// blocks per SM, and measured slower.)
-constexpr int coop_chunk(int) { return 64; }
-constexpr int kCoopCap = 736;
+// Words listed before an evaluation, in a warp walk and in a team walk.
+constexpr int kWalkWords = 32;
+constexpr int kTeamWords = 64;
+// Terms a team lists per particle before an evaluation: room for a round of
+// its four warps (16 words of 32 candidates).
+constexpr int kTeamTerms = 512;
+constexpr int kTeamWarps = 4;
+// Warps with more groups than this take the one-thread walk (sparse spray: a
+// group's listing costs a warp about as much as a few dozen candidates of a
+// one-thread walk).
+constexpr int kMaxGroups = 6;
 
-template <int CH, bool kExtra>
-struct CoopSmem {
-    static constexpr int kCap = CH > 1 ? kCoopCap : 1;
-    alignas(16) float sx[CH];          // staged x* of the chunk, by component; slots past
-    alignas(16) float sy[CH];          // the last staged one up to a multiple of 32
-    alignas(16) float sz[CH];          // hold +inf (never in support)
-    alignas(16) float sw[CH];          // staged x*.w (lambda in the delta pass)
-    unsigned char c[CH];               // cell of the candidate among [xmin - 1, xmax + 1]
-    uint32_t q[kCap];                  // candidate position of each listed survivor
-    uint32_t mask[(kCap + 31) / 32][32];  // mask[w][lane] bit b: survivor 32 w + b is a term of the lane
+// Shared memory of a warp walk.
+struct WalkSmem {
+    // One fp16 row of eight per candidate: x, y, z, |u|^2 (high, low), 1, 1, 0.
+    alignas(16) uint32_t stage[128 * 4];
+    uint32_t base[kWalkWords];  // first candidate (cell order, or key order in buckets)
+    uint32_t info[kWalkWords];  // candidates | row << 8 | kLastLeads
+    uint32_t mask[kWalkWords * 32];
+    // The mask of word w and particle p.  The exclusive-or spreads the four
+    // words that a store instruction touches over the banks.
+    static __device__ __forceinline__ int at(int w, int p) { return w * 32 + (p ^ ((w & 3) << 3)); }
+};
+// In WalkSmem::info: the word's last candidate leads a run (k_segments).
+constexpr uint32_t kLastLeads = 1u << 16;
+
+// Shared memory of a team walk.  During an evaluation the stage holds the
+// terms on their way to the adding lanes, one row of float2 (two quantities)
+// per pair of quantities and, in the fast build, their factors; rows are 66
+// apart so that the lanes that add read without conflicts.
+template <int TP>
+struct TeamSmem {
+    static constexpr int kRow = 66;
+    static constexpr int kTermBytes = (PBF_FAST ? 6 : 3) * kRow * 8;
+    static constexpr int kWarpBytes = kTermBytes > 2048 ? kTermBytes : 2048;
+    static constexpr int kListRow = kTeamTerms + 2;
+    alignas(16) unsigned char warp[kTeamWarps][(kWarpBytes + 15) / 16 * 16];
+    uint32_t base[kTeamWords];
+    uint32_t info[kTeamWords];
+    uint32_t mask[kTeamWarps][4 * TP];
+    uint32_t count[kTeamWarps][TP];  // a round's terms of each warp's words
+    uint32_t total[TP];              // terms listed
+    int flag[TP];
+    alignas(4) unsigned short list[TP * kListRow];  // word << 5 | candidate
 };
 
-// Blocks per SM the neighbour-pass kernels are compiled for: 32 warps per SM
-// (64 registers a thread), which their shared memory also fits.
+// Blocks per SM the neighbour-pass kernels are compiled for: 24 warps per SM
+// (80 registers a thread).
 template <int BS>
-constexpr int kPassMinBlocks = 1024 / BS;
+constexpr int kPassMinBlocks = 768 / BS;
 
-// Shared memory of a kernel's warps: real for the kernels of a single large
-// scene (those with the 8-way row loop, see kBigScene), one byte otherwise.
-// Small scenes and batches keep the one-thread walk: the shared memory costs
-// them occupancy (a batch of 1,024 small scenes ran at 94 M particle-steps/s
-// with the cooperative walk against 108 M without), and many small scenes
-// side by side on their own streams measured slower with it too.
-template <class P, int BS, bool kExtra, int U>
-struct CoopBlock {
-    static constexpr bool kOn = std::is_same<P, OneScene>::value && U == 8;
-    using Smem = CoopSmem<kOn ? coop_chunk(BS) : 1, kExtra>;
-    static constexpr int kWarps = kOn ? BS / 32 : 1;
+// An index of points that a walk visits: cell-order offsets, and the
+// reference buckets of the dirty cells.
+struct WalkIndex {
+    const uint32_t* __restrict__ off;
+    const uint32_t* __restrict__ kpos;
+    const uint32_t* __restrict__ bend;
+    const uint32_t* __restrict__ btab;
 };
 
-// The warp's shared row: cells y = cy, z = cz, x in [xmin, xmin + W - 3];
-// wx0 = wrapped x slot of xmin - 1.
-struct CoopRow {
-    int cy, cz, xmin, W, wx0;
+// A group: the cells [cx, cx + W - 3] of row (cy, cz), or one dirty cell
+// (own: its bucket row + 1).  split: the row would wrap in x, so its cells
+// are visited one by one (W = 3 then).
+struct WalkGroup {
+    int cx, cy, cz, W;
+    uint32_t own;
+    bool split;
 };
 
-__device__ __forceinline__ uint32_t lanemask_lt() {
-    uint32_t m;
-    asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m));
-    return m;
+__device__ __forceinline__ uint32_t pack_half2(float a, float b) {
+    const __half2 h = __floats2half2_rn(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// Warp-collective (every lane of the warp must call it): whether the warp
-// walks cooperatively, and its row.  `cell` is the lane's step-start cell
-// with w = its owner row (0 = clean); `sid` its scene (0 for a single scene):
-// the lanes must share one scene, whose grid is Gd.
-__device__ __forceinline__ bool coop_row(bool active, const int4 cell, const GridDesc& Gd,
-                                         CoopRow& R, uint32_t sid) {
-    const unsigned full = 0xffffffffu;
-    if (!__all_sync(full, active)) return false;
-    if (!__all_sync(full, sid == __shfl_sync(full, sid, 0))) return false;
-    const int cy0 = __shfl_sync(full, cell.y, 0);
-    const int cz0 = __shfl_sync(full, cell.z, 0);
-    if (!__all_sync(full, cell.w == 0 && cell.y == cy0 && cell.z == cz0)) return false;
-    const int xmin = __reduce_min_sync(full, cell.x);
-    const int xmax = __reduce_max_sync(full, cell.x);
-    if ((long long)xmax - (long long)xmin > 2 || xmin <= -(1 << 30) || xmax >= (1 << 30))
-        return false;
-    const int W = xmax - xmin + 3;
-    const int wx0 = wrap(xmin - 1, Gd.ox, Gd.gx);
-    if (wx0 + W > Gd.gx) return false;  // the row range would wrap: one-thread walk
-    R = CoopRow{cy0, cz0, xmin, W, wx0};
-    return true;
+__device__ __forceinline__ uint32_t pack_half2(__half a, __half b) {
+    const __half2 h = __halves2half2(a, b);
+    return *reinterpret_cast<const uint32_t*>(&h);
 }
 
-// The cooperative walk (see above) of a warp for which coop_row held.  xi is
-// the lane's x*, ci its cell x; `cut` the support test r_sq < cut of the
-// pass.  extra(q) returns the per-candidate extras of candidate q (kExtra);
-// body(xj, ej) adds the term of one candidate, re-testing r_sq < cut;
-// rep(xj, ej, L) adds it L times in a row (exactly, see acc).
-// Lanes with `want` false list no candidates and do not widen the warp's
-// box (at least one lane must want).
-// kRuns: rows of at least kRunRow candidates collapse runs of identical
-// candidates (below).  The XSPH and vorticity passes compile it in; the
-// constraint passes do not (it cost their register allocation about 4 %
-// of their time on ordinary fluid).
-// kLam (the delta pass): a candidate whose lambda sum with the lane,
-// xi.w + xj.w, is zero adds an exact zero to the lane's sum (no s_corr
-// either, which needs a negative sum), and the sum, started at +0, never is
-// -0, so such candidates are not listed; when every lane's lambda is zero,
-// candidates with zero lambda are not staged at all.
-template <int CH, bool kExtra, bool kPersist, bool kLam, bool kRuns, class Extra, class Body,
-          class Rep>
-__device__ __forceinline__ void coop_walk(CoopSmem<CH, kExtra>& sm, const CoopRow& R, int ci,
-                                          const float4 xi, const float4* xin, float cut,
-                                          const GridDesc& Gd, const uint32_t* __restrict__ off,
-                                          Extra&& extra, Body&& body, Rep&& rep,
-                                          bool want = true) {
-    constexpr int CAP = CoopSmem<CH, kExtra>::kCap;
-    static_assert(CH % 32 == 0 && CAP % 32 == 0 && CAP >= 2 * CH, "coop walk sizes");
+// D = A B for one 16 x 8 tile, K = 8 (fp16 inputs, fp32 accumulators): lane
+// (g = lane / 4, t = lane % 4) holds rows g and g + 8 of A (columns 2t,
+// 2t + 1), column g of B (rows 2t, 2t + 1), and of D rows g (d0, d1) and
+// g + 8 (d2, d3) in columns 2t, 2t + 1.
+__device__ __forceinline__ void mma_16x8x8(float& d0, float& d1, float& d2, float& d3, uint32_t a0,
+                                           uint32_t a1, uint32_t b0) {
+    asm("mma.sync.aligned.m16n8k8.row.col.f32.f16.f16.f32 {%0, %1, %2, %3}, {%4, %5}, {%6}, "
+        "{%7, %7, %7, %7};"
+        : "=f"(d0), "=f"(d1), "=f"(d2), "=f"(d3)
+        : "r"(a0), "r"(a1), "r"(b0), "f"(0.0f));
+}
+
+// Rows.  With positions u relative to the group's centre in units of h and
+// rounded to fp16, r^2 - lim = |u_j|^2 - 2 u_i.u_j + (|u_i|^2 - lim) is a
+// dot product of length seven: the candidate's row
+//   (x, y, z, hi|u|^2, lo|u|^2, 1, 1, 0)
+// times the particle's column
+//   (-2x, -2y, -2z, 1, 1, hi(|u|^2 - lim), lo(|u|^2 - lim), 0),
+// with each square split into two halves.  For |u| <= U per component the
+// rounding of the positions moves a distance by at most
+// 2 sqrt(3) U 2^-11 < 0.0018 U, and the split squares and the accumulation
+// (fp32) move r^2 by less than 4e-5 U^2: lim = (1 + 0.0018 U)^2 + 4e-5 U^2 +
+// 1e-5 keeps every candidate within h of a particle.  U is half the extent
+// of the group's box plus one (a candidate farther out is in nobody's
+// support, so its test may say anything); a group wider than kWalkReach
+// lists every candidate instead.
+constexpr float kWalkReach = 64.0f;
+constexpr float kHalfFar = 60000.0f;  // |u|^2 of a row or column that is never in support
+
+__device__ __forceinline__ uint4 candidate_row(float ux, float uy, float uz) {
+    const __half2 xy = __floats2half2_rn(ux, uy);
+    const __half z = __float2half_rn(uz);
+    const float2 f = __half22float2(xy);
+    const float fz = __half2float(z);
+    const float n = fmaf(f.x, f.x, fmaf(f.y, f.y, fz * fz));
+    const __half nh = __float2half_rn(n);
+    const __half nl = __float2half_rn(n - __half2float(nh));
+    return make_uint4(*reinterpret_cast<const uint32_t*>(&xy), pack_half2(z, nh),
+                      pack_half2(nl, __float2half_rn(1.0f)),
+                      pack_half2(__float2half_rn(1.0f), __float2half_rn(0.0f)));
+}
+
+__device__ __forceinline__ uint4 particle_column(float ux, float uy, float uz, float lim) {
+    const __half2 xy = __floats2half2_rn(ux, uy);
+    const __half z = __float2half_rn(uz);
+    const float2 f = __half22float2(xy);
+    const float fz = __half2float(z);
+    const float m = fmaf(f.x, f.x, fmaf(f.y, f.y, fz * fz)) - lim;
+    const __half mh = __float2half_rn(m);
+    const __half ml = __float2half_rn(m - __half2float(mh));
+    return make_uint4(pack_half2(-2.0f * f.x, -2.0f * f.y),
+                      pack_half2(__float2half_rn(-2.0f * fz), __float2half_rn(1.0f)),
+                      pack_half2(__float2half_rn(1.0f), mh), pack_half2(ml, __float2half_rn(0.0f)));
+}
+
+// Bits [lo, hi) of a word, for 0 <= lo, hi <= 32.
+__device__ __forceinline__ uint32_t bit_range(uint32_t lo, uint32_t hi) {
+    if (lo >= hi) return 0u;
+    return (0xffffffffu >> (32u - (hi - lo))) << lo;
+}
+
+// The box of the wanting lanes' positions: its centre, the test's limit and
+// whether it is too wide for the test.
+struct WalkBox {
+    float ox, oy, oz, lim;
+    bool wide;
+};
+
+__device__ __forceinline__ WalkBox walk_box(bool want, const float4 xi, float inv_h) {
     const unsigned full = 0xffffffffu;
-    const int lane = threadIdx.x & 31;
     const float inf = __int_as_float(0x7f800000);
     float lx = want ? xi.x : inf, ly = want ? xi.y : inf, lz = want ? xi.z : inf;
     float hx = want ? xi.x : -inf, hy = want ? xi.y : -inf, hz = want ? xi.z : -inf;
@@ -859,262 +897,674 @@ __device__ __forceinline__ void coop_walk(CoopSmem<CH, kExtra>& sm, const CoopRo
         hy = fmaxf(hy, __shfl_xor_sync(full, hy, o));
         hz = fmaxf(hz, __shfl_xor_sync(full, hz, o));
     }
-    // A candidate in some lane's support is within sqrt(cut) of the box, and
-    // within the widened radius of the lane's fused r^2; the margins cover
-    // the rounding of both distance computations.
-    const float lim = cut * 1.001f;
-    const float lim2 = cut * 1.000001f;
-    const bool all_member = R.W == 3;  // one cell: every staged candidate is in it
-    const int myc = ci - R.xmin + 1;   // the lane's cell among the row's cells
-    const uint32_t lt = lanemask_lt();
-    const float2 m1 = make_float2(-1.0f, -1.0f);
-    const float2 px = make_float2(xi.x, xi.x), py = make_float2(xi.y, xi.y),
-                 pz = make_float2(xi.z, xi.z), pw = make_float2(xi.w, xi.w);
-    // Only candidates with a nonzero lambda can add to a lane whose own is zero.
-    const bool lam_filter = kLam && !__any_sync(full, xi.w != 0.0f);
-    int nst = 0;   // staged in the current chunk
-    int base = 0;  // survivors listed so far (a multiple of 32)
-    int cnt = 0;   // the lane's listed terms
+    WalkBox B;
+    B.ox = 0.5f * (lx + hx);
+    B.oy = 0.5f * (ly + hy);
+    B.oz = 0.5f * (lz + hz);
+    const float U = 0.5f * fmaxf(hx - lx, fmaxf(hy - ly, hz - lz)) * inv_h + 1.01f;
+    B.wide = !(U <= kWalkReach);
+    const float reach = 1.0f + 0.0018f * U;
+    B.lim = reach * reach + 4e-5f * U * U + 1e-5f;
+    return B;
+}
 
-    // Phase 2: every lane evaluates its listed terms in list order, loading
-    // the next term's candidate before adding the current one.
-    auto evaluate = [&]() {
-        const int most = (int)__reduce_max_sync(full, (unsigned)cnt);
-        int w = 0;
-        uint32_t bits = sm.mask[0][lane];
-        auto next_q = [&]() {
-            while (bits == 0) bits = sm.mask[++w][lane];
-            const int k = 32 * w + __ffs(bits) - 1;
-            bits &= bits - 1u;
-            return sm.q[k];
-        };
-        float4 xn = make_float4(0.0f, 0.0f, 0.0f, 0.0f), en = xn;
-        if (cnt > 0) {
-            const uint32_t q = next_q();
-            xn = ld_step<kPersist>(xin + q);
-            if constexpr (kExtra) en = extra(q);
-        }
-        for (int t = 0; t < most; ++t) {
-            const float4 xj = xn, ej = en;
-            if (t + 1 < cnt) {
-                const uint32_t q = next_q();
-                xn = ld_step<kPersist>(xin + q);
-                if constexpr (kExtra) en = extra(q);
+// The candidate sequence of a group, one range per lane: [start, start + len)
+// in cell order (key order for a dirty cell), the row's first slot, the
+// number of words before the lane's first one and in total, and with kRuns
+// whether the range holds runs (at least kRunRow candidates in slots with a
+// run's first particle).
+struct WalkRanges {
+    uint32_t start, len, slot;
+    int words, before, total;
+    bool runs;
+};
+
+template <bool kRuns>
+__device__ __forceinline__ WalkRanges walk_ranges(const WalkGroup& Gr, const WalkIndex& I,
+                                                  const GridDesc& Gd, const Grid& G) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    WalkRanges R;
+    R.start = R.len = R.slot = 0u;
+    R.runs = false;
+    if (Gr.own) {
+        if (lane < 27) {
+            const uint32_t b0 = __ldg(I.btab + (size_t)(Gr.own - 1u) * 27u + (uint32_t)lane);
+            if (b0 != kNoBucket) {
+                const uint32_t be = __ldg(I.bend + b0);
+                R.start = b0;
+                R.len = (be & ~kImpureBit) - b0;
+                if constexpr (kRuns) {
+                    if (G.segend && R.len >= kRunRow && !(be & kImpureBit)) {
+                        const int4 c = G.scell[__ldg(I.kpos + b0)];
+                        R.runs = (__ldg(G.slot_alias + slot_of(c.x, c.y, c.z, Gd)) & kRunSlot) != 0;
+                    }
+                }
             }
-            if (t < cnt) body(xj, ej);
         }
+    } else if (Gr.split ? lane < 27 : lane < 9) {
+        const int dx = Gr.split ? lane % 3 : 0;
+        const int yz = Gr.split ? lane / 3 : lane;
+        const int k = Gr.split ? 1 : Gr.W;
+        R.slot = slot_of(Gr.cx - 1 + dx, Gr.cy + yz % 3 - 1, Gr.cz + yz / 3 - 1, Gd);
+        R.start = __ldg(I.off + R.slot);
+        R.len = __ldg(I.off + R.slot + k) - R.start;
+        if constexpr (kRuns) {
+            if (G.segend && R.len >= kRunRow)
+                for (int d = 0; d < k; ++d) R.runs |= (__ldg(G.slot_alias + R.slot + d) & kRunSlot) != 0;
+        }
+    }
+    R.words = (int)((R.len + 31u) >> 5);
+    int sum = R.words;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int v = __shfl_up_sync(full, sum, o);
+        if (lane >= o) sum += v;
+    }
+    R.total = __shfl_sync(full, sum, 31);
+    R.before = sum - R.words;
+    return R;
+}
+
+// Lists words [done, done + room) of the sequence; returns how many there are.
+__device__ __forceinline__ int list_words(const WalkRanges& R, int done, int room, uint32_t* base,
+                                          uint32_t* info) {
+    for (int k = max(0, done - R.before); k < R.words && R.before + k < done + room; ++k) {
+        const int w = R.before + k - done;
+        base[w] = R.start + 32u * (uint32_t)k;
+        info[w] = min(32u, R.len - 32u * (uint32_t)k) | ((threadIdx.x & 31u) << 8);
+    }
+    return min(room, R.total - done);
+}
+
+// Stages four words of candidates and tests them against the 8 NT particles
+// whose columns the lanes hold (col): on return, half words of the masks, as
+// 16 bits for particles 8 c + 2 t4 (h0[c]) and 8 c + 2 t4 + 1 (h1[c]) in lane
+// (g, t4), for the candidates 16 g + [0, 16) of the 128.
+template <int NT>
+__device__ __forceinline__ void test_words(uint32_t* stage, const float4 (&xj)[4],
+                                           const uint32_t (&sel)[4], const WalkBox& B, float inv_h,
+                                           const uint32_t (&col)[NT], uint32_t (&h0)[NT],
+                                           uint32_t (&h1)[NT]) {
+    const int lane = threadIdx.x & 31;
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+        const bool in = (sel[j] >> lane) & 1u;
+        uint4 r = candidate_row((xj[j].x - B.ox) * inv_h, (xj[j].y - B.oy) * inv_h,
+                                (xj[j].z - B.oz) * inv_h);
+        if (!in)
+            r = make_uint4(0u, pack_half2(0.0f, kHalfFar), pack_half2(0.0f, 1.0f), pack_half2(1.0f, 0.0f));
+        // Candidate 16 gg + jj of the 128 (bit jj of group gg's half word) is
+        // row 8 jj + (gg ^ (jj & 7)): stores and fragment loads both touch
+        // every bank.
+        const int jj = lane & 15, gg = 2 * j + (lane >> 4);
+        reinterpret_cast<uint4*>(stage)[8 * jj + (gg ^ (jj & 7))] = r;
+    }
+    __syncwarp();
+#pragma unroll
+    for (int c = 0; c < NT; ++c) h0[c] = h1[c] = 0u;
+#pragma unroll
+    for (int k = 7; k >= 0; --k) {
+        const uint32_t a0 = stage[32 * (2 * k) + (lane ^ (((2 * k) & 7) << 2))];
+        const uint32_t a1 = stage[32 * (2 * k + 1) + (lane ^ (((2 * k + 1) & 7) << 2))];
+#pragma unroll
+        for (int c = 0; c < NT; ++c) {
+            float d0, d1, d2, d3;
+            mma_16x8x8(d0, d1, d2, d3, a0, a1, col[c]);
+            // Sign bits in from the right: candidate 2k ends at bit 2k.
+            h0[c] = __funnelshift_l(__float_as_uint(d2), h0[c], 1);
+            h1[c] = __funnelshift_l(__float_as_uint(d3), h1[c], 1);
+            h0[c] = __funnelshift_l(__float_as_uint(d0), h0[c], 1);
+            h1[c] = __funnelshift_l(__float_as_uint(d1), h1[c], 1);
+        }
+    }
+}
+
+// The candidates of word w of a row of more than three cells that lie in the
+// three cells around the particle's own (x coordinate ci); slot is the row's
+// first slot.
+__device__ __forceinline__ uint32_t own_cells(const WalkIndex& I, uint32_t slot, int dx, uint32_t bs) {
+    const uint32_t a = __ldg(I.off + slot + (uint32_t)dx), e = __ldg(I.off + slot + (uint32_t)dx + 3u);
+    return bit_range(a > bs ? min(a - bs, 32u) : 0u, e > bs ? min(e - bs, 32u) : 0u);
+}
+
+// The warp walk of one group (every lane of the warp calls it; at least one
+// lane wants).  xi is the lane's x*, ci the x of its cell; lanes with `want`
+// false list no candidates.  xin holds the candidates' positions in cell order
+// and inv_h = 1 / support radius.  kLam (the delta pass): a candidate whose
+// lambda sum with the lane, xi.w + xj.w, is zero adds an exact zero to the
+// lane's sums (no s_corr either, which needs a negative sum) and the sums,
+// started at +0, never are -0, so a lane whose lambda is zero lists
+// candidates with a nonzero one only.  kRuns: in ranges that hold runs of
+// identical particles (k_segments) a run is listed as its first particle,
+// whose term is added as many times as the run is long.
+template <bool kPersist, bool kLam, bool kRuns, class Sums>
+__device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bool want, int ci,
+                                           const float4 xi, const float4* xin, float inv_h,
+                                           const GridDesc& Gd, const WalkIndex& I, const Grid& G,
+                                           Sums& sums) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    const int g = lane >> 2, t4 = lane & 3;
+    const WalkBox B = walk_box(want, xi, inv_h);
+    uint32_t col[4];
+    {
+        uint4 c = particle_column((xi.x - B.ox) * inv_h, (xi.y - B.oy) * inv_h, (xi.z - B.oz) * inv_h, B.lim);
+        if (!want) c = make_uint4(0u, 0u, pack_half2(0.0f, kHalfFar), 0u);
+        reinterpret_cast<uint4*>(sm.stage)[lane] = c;
         __syncwarp();
-        cnt = 0;
-        base = 0;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) col[j] = sm.stage[(8 * j + g) * 4 + t4];
+        __syncwarp();
+    }
+    const bool key = Gr.own != 0u;
+    const bool multi = Gr.W > 3;
+    const WalkRanges R = walk_ranges<kRuns>(Gr, I, Gd, G);
+    const bool runs = kRuns && __any_sync(full, R.runs);
+    // Position of the listing with runs: range and candidate.
+    int at_r = 0;
+    uint32_t at_q = __shfl_sync(full, R.start, 0);
+    int done = 0;
+    // Lists the next words; returns how many.
+    auto fill = [&]() -> int {
+        if (!runs) {
+            const int nw = list_words(R, done, kWalkWords, sm.base, sm.info);
+            done += nw;
+            return nw;
+        }
+        int nw = 0;
+        const int nr = key || Gr.split ? 27 : 9;
+        while (nw < kWalkWords && at_r < nr) {
+            const uint32_t e = __shfl_sync(full, R.start + R.len, at_r);
+            if (at_q >= e) {
+                ++at_r;
+                at_q = __shfl_sync(full, R.start, at_r & 31);
+                continue;
+            }
+            uint32_t cnt = min(32u, e - at_q), lead = 0u, step = cnt;
+            if (__shfl_sync(full, R.runs ? 1 : 0, at_r)) {
+                // A range with runs: the word ends with a run's first
+                // particle, and the next one begins past the run.
+                uint32_t q = at_q + (uint32_t)lane;
+                const bool ok = (uint32_t)lane < cnt;
+                if (ok && key) q = __ldg(I.kpos + q);
+                const bool first = ok && ((uint32_t)__ldg(G.sown + q) & kLeadBit);
+                const uint32_t m = __ballot_sync(full, first);
+                if (m) {
+                    const int f = __ffs(m) - 1;
+                    uint32_t len = 0u;
+                    if (lane == f) len = __ldg(G.segend + q) - q;
+                    cnt = (uint32_t)f + 1u;
+                    step = (uint32_t)f + __shfl_sync(full, len, f);
+                    lead = kLastLeads;
+                }
+            }
+            if (lane == 0) {
+                sm.base[nw] = at_q;
+                sm.info[nw] = cnt | ((uint32_t)at_r << 8) | lead;
+            }
+            ++nw;
+            at_q += step;
+        }
+        return nw;
     };
 
-    // Phase 1b: the lane's support tests over the staged chunk, two
-    // candidates per paired operation, one mask word per 32 candidates.  Only
-    // whole words are tested until the walk ends: the last partial word's
-    // candidates move to the front of the stage (their list positions stay
-    // where they are, at base + k) and wait for the next chunk, so a tested
-    // word is padded only at the very end of the walk.
-    auto test_chunk = [&](bool last) {
-        const int words = last ? (nst + 31) >> 5 : nst >> 5;
-        if (last) {
-            // Pad the last word with candidates that are never in support.
-            for (int k = nst + lane; k < (words << 5); k += 32) {
-                sm.sx[k] = __int_as_float(0x7f800000);
-                sm.sy[k] = 0.0f;
-                sm.sz[k] = 0.0f;
-                sm.sw[k] = 0.0f;
-                sm.c[k] = 0;
+    const bool lam_zero = kLam && xi.w == 0.0f;
+    const bool all_zero = kLam && !__any_sync(full, want && xi.w != 0.0f);
+    for (;;) {
+        const int nw = fill();
+        if (nw <= 0) break;
+        __syncwarp();
+        int cnt = 0;          // the lane's listed terms
+        uint32_t filled = 0;  // words with any of them
+        // --- phase 1, four words at a time
+        for (int b = 0; b < nw; b += 4) {
+            uint32_t sel[4], nz[4];  // candidates of each word, and those with a nonzero lambda
+            uint32_t any_nz = 0u;
+            float4 xj[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t n = b + j < nw ? sm.info[b + j] & 63u : 0u;
+                sel[j] = bit_range(0u, n);
+                xj[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                if ((uint32_t)lane < n) {
+                    uint32_t q = sm.base[b + j] + (uint32_t)lane;
+                    if (key) q = __ldg(I.kpos + q);
+                    xj[j] = ld_step<kPersist>(xin + q);
+                }
+                if constexpr (kLam) {
+                    nz[j] = __ballot_sync(full, xj[j].w != 0.0f);
+                    any_nz |= nz[j];
+                }
+            }
+            const bool test = !B.wide && (!kLam || !all_zero || any_nz != 0u);
+            if (test) {
+                uint32_t h0[4], h1[4];
+                test_words<4>(sm.stage, xj, sel, B, inv_h, col, h0, h1);
+                unsigned short* const mh = reinterpret_cast<unsigned short*>(sm.mask);
+#pragma unroll
+                for (int c = 0; c < 4; ++c) {
+                    const int w = b + (g >> 1), p = 8 * c + 2 * t4;
+                    mh[2 * sm.at(w, p) + (g & 1)] = (unsigned short)h0[c];
+                    mh[2 * sm.at(w, p + 1) + (g & 1)] = (unsigned short)h1[c];
+                }
+                __syncwarp();
+            }
+            // The bits that count: the word's candidates, for a lane whose
+            // lambda is zero those with a nonzero one, and in a row of more
+            // than three cells those of the lane's own three.
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const int w = b + j;
+                uint32_t m = B.wide ? 0xffffffffu : (test ? sm.mask[sm.at(w, lane)] : 0u);
+                m &= sel[j];
+                if constexpr (kLam)
+                    if (lam_zero) m &= nz[j];
+                if (!want) m = 0u;
+                if (multi) {
+                    const uint32_t slot = __shfl_sync(full, R.slot, w < nw ? (sm.info[w] >> 8) & 31u : 0u);
+                    if (m) m &= own_cells(I, slot, ci - Gr.cx, sm.base[w]);
+                }
+                sm.mask[sm.at(w, lane)] = m;
+                cnt += __popc(m);
+                if (m) filled |= 1u << w;
             }
             __syncwarp();
         }
-        for (int wd = 0; wd < words; ++wd) {
-            const int k0 = wd << 5;
-            uint32_t allowed = full;
-            if (!all_member) {
-                // Candidates of the word in each of the row's cells (at most
-                // 5), then those in the lane's three.
-                const int cc = sm.c[k0 + lane];
-                allowed = 0u;
-#pragma unroll
-                for (int v = 0; v < 5; ++v) {
-                    const uint32_t mc = __ballot_sync(full, cc == v);
-                    if ((unsigned)(v - myc + 1) <= 2u) allowed |= mc;
-                }
+        // --- phase 2
+        const int most = (int)__reduce_max_sync(full, (unsigned)cnt);
+        uint32_t bits = 0u, bq = 0u;
+        int w = 0;
+        // The next listed candidate (there is one).
+        auto next_q = [&]() -> uint32_t {
+            if (bits == 0u) {
+                w = __ffs(filled) - 1;
+                filled &= filled - 1u;
+                bits = sm.mask[sm.at(w, lane)];
+                bq = sm.base[w];
             }
-            uint32_t bits = 0u;
-#pragma unroll
-            for (int b = 0; b < 32; b += 2) {
-                const float2 X = *reinterpret_cast<const float2*>(&sm.sx[k0 + b]);
-                const float2 Y = *reinterpret_cast<const float2*>(&sm.sy[k0 + b]);
-                const float2 Z = *reinterpret_cast<const float2*>(&sm.sz[k0 + b]);
-                const float2 dx = __ffma2_rn(X, m1, px);
-                const float2 dy = __ffma2_rn(Y, m1, py);
-                const float2 dz = __ffma2_rn(Z, m1, pz);
-                float2 r2 = __fmul2_rn(dx, dx);
-                r2 = __ffma2_rn(dy, dy, r2);
-                r2 = __ffma2_rn(dz, dz, r2);
-                if constexpr (kLam) {
-                    const float2 W = *reinterpret_cast<const float2*>(&sm.sw[k0 + b]);
-                    const float2 ls = __fadd2_rn(pw, W);
-                    if (r2.x < lim2 && ls.x != 0.0f) bits |= 1u << b;
-                    if (r2.y < lim2 && ls.y != 0.0f) bits |= 2u << b;
-                } else {
-                    if (r2.x < lim2) bits |= 1u << b;
-                    if (r2.y < lim2) bits |= 2u << b;
-                }
+            const uint32_t k = (uint32_t)__ffs(bits) - 1u;
+            bits &= bits - 1u;
+            return bq + k;
+        };
+        if (kRuns && runs) {
+            for (int t = 0; t < cnt; ++t) {
+                uint32_t q = next_q();
+                const uint32_t i = sm.info[w];
+                const bool lead = (i & kLastLeads) && q - bq == (i & 63u) - 1u;
+                if (key) q = __ldg(I.kpos + q);
+                float4 e{};
+                if constexpr (Sums::kExtra) e = sums.extra(q);
+                if (lead) sums.add_run(ld_step<kPersist>(xin + q), e, __ldg(G.segend + q) - q);
+                else sums.add(ld_step<kPersist>(xin + q), e);
             }
-            bits &= allowed;
-            if (!want) bits = 0u;
-            sm.mask[(base >> 5) + wd][lane] = bits;
-            cnt += __popc(bits);
-        }
-        // The untested rest (fewer than 32) moves to the front of the stage.
-        const int rest = last ? 0 : nst - (words << 5);
-        float kx = 0.0f, ky = 0.0f, kz = 0.0f, kw = 0.0f;
-        unsigned char kc = 0;
-        uint32_t kq = 0u;
-        if (lane < rest) {
-            const int k = (words << 5) + lane;
-            kx = sm.sx[k];
-            ky = sm.sy[k];
-            kz = sm.sz[k];
-            kw = sm.sw[k];
-            kc = sm.c[k];
-            kq = sm.q[base + k];
+        } else {
+            float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
+            auto load = [&](float4& x, float4& e) {
+                uint32_t q = next_q();
+                if (key) q = __ldg(I.kpos + q);
+                x = ld_step<kPersist>(xin + q);
+                if constexpr (Sums::kExtra) e = sums.extra(q);
+            };
+            if (cnt > 0) load(xa, ea);
+            if (cnt > 1) load(xb, eb);
+            for (int t = 0; t < most; t += 2) {
+                const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
+                if (t + 2 < cnt) load(xa, ea);
+                if (t + 3 < cnt) load(xb, eb);
+                sums.add2(x0, x1, e0, e1, t < cnt, t + 1 < cnt);
+            }
         }
         __syncwarp();
-        base += words << 5;
-        if (base > CAP - CH) evaluate();
-        if (lane < rest) {
-            sm.sx[lane] = kx;
-            sm.sy[lane] = ky;
-            sm.sz[lane] = kz;
-            sm.sw[lane] = kw;
-            sm.c[lane] = kc;
-            sm.q[base + lane] = kq;
-        }
-        nst = rest;
-        __syncwarp();
-    };
+    }
+}
 
-    for (int rr = 0; rr < 9; ++rr) {
-        const int dz = rr / 3 - 1;
-        const int dy = rr - (rr / 3) * 3 - 1;
-        const uint32_t row = Gd.base + (uint32_t)R.wx0 +
-                             (uint32_t)Gd.gx * ((uint32_t)wrap(R.cy + dy, Gd.oy, Gd.gy) +
-                                                (uint32_t)Gd.gy * (uint32_t)wrap(R.cz + dz, Gd.oz, Gd.gz));
-        const uint32_t q0 = __ldg(off + row);
-        const uint32_t q1 = __ldg(off + row + R.W);
-        // Cell boundaries inside the row (cells 1.. W-1 start here).
-        uint32_t b1 = q1, b2 = q1, b3 = q1, b4 = q1;
-        if (!all_member) {
-            b1 = __ldg(off + row + 1);
-            b2 = __ldg(off + row + 2);
-            b3 = __ldg(off + row + 3);
-            if (R.W > 4) b4 = __ldg(off + row + 4);
+// A pass's sums.  A quantity k of a particle is the sum over its candidates of
+// factor x value, each product rounded before it is added (or fused, in the
+// fast build, as the one-thread walk's expressions are).  The term D says:
+// kQuantities; kFactors and factor_of(k), the factor of quantity k (-1: none);
+// kTermFactor, whether the factors come with the term (else const_factor(k));
+// kExtra and extra(q), per-candidate data besides the position; eval, the
+// values and factors of one candidate and whether it is in support; and in the
+// exact build products, the products of two candidates at once.
+//
+// The sums of one lane (warp walk).
+template <class D>
+struct LaneSums {
+    static constexpr int kNq = D::kQuantities;
+    static constexpr bool kExtra = D::kExtra;
+    float sum[kNq];
+    const D d;
+    __device__ __forceinline__ explicit LaneSums(const D& def) : d(def) {
+#pragma unroll
+        for (int k = 0; k < kNq; ++k) sum[k] = 0.0f;
+    }
+    // Continues from sums that are there already.
+    __device__ __forceinline__ void start(const float* from) {
+#pragma unroll
+        for (int k = 0; k < kNq; ++k) sum[k] = from[k];
+    }
+    __device__ __forceinline__ float4 extra(uint32_t q) const { return d.extra(q); }
+    __device__ __forceinline__ void add(const float4& xj, const float4& ej) {
+        float v[kNq], f[D::kFactors];
+        if (d.eval(xj, ej, v, f)) {
+#pragma unroll
+            for (int k = 0; k < kNq; ++k) {
+                if (D::factor_of(k) < 0) sum[k] = sum[k] + v[k];
+                else sum[k] = sum[k] + f[D::factor_of(k) < 0 ? 0 : D::factor_of(k)] * v[k];
+            }
         }
-        // Stages the candidates q of the lanes with `ok` that pass the box.
-        auto stage = [&](uint32_t q, bool ok) {
-            bool pass = false;
-            float4 xj = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-            if (ok) {
-                xj = ld_step<kPersist>(xin + q);
-                const float ex = fmaxf(0.0f, fmaxf(lx - xj.x, xj.x - hx));
-                const float ey = fmaxf(0.0f, fmaxf(ly - xj.y, xj.y - hy));
-                const float ez = fmaxf(0.0f, fmaxf(lz - xj.z, xj.z - hz));
-                pass = ex * ex + (ey * ey + ez * ez) < lim;
-                if (lam_filter) pass = pass && xj.w != 0.0f;
+    }
+    // The term of a run of L identical candidates: added L times, exactly.
+    __device__ __forceinline__ void add_run(const float4& xj, const float4& ej, uint32_t L) {
+        float v[kNq], f[D::kFactors];
+        if (d.eval(xj, ej, v, f)) {
+#pragma unroll
+            for (int k = 0; k < kNq; ++k)
+                sum[k] = rep_add_call(sum[k],
+                                      D::factor_of(k) < 0
+                                          ? v[k]
+                                          : f[D::factor_of(k) < 0 ? 0 : D::factor_of(k)] * v[k],
+                                      L);
+        }
+    }
+    // The terms of two candidates, the first one first, where they are there.
+    __device__ __forceinline__ void add2(const float4& xa, const float4& xb, const float4& ea,
+                                         const float4& eb, bool has_a, bool has_b) {
+#if PBF_FAST
+        if (has_a) add(xa, ea);
+        if (has_b) add(xb, eb);
+#else
+        if (!d.C.paired) {
+            if (has_a) add(xa, ea);
+            if (has_b) add(xb, eb);
+            return;
+        }
+        float2 v[kNq];
+        bool in_a, in_b;
+        d.products(xa, xb, ea, eb, v, in_a, in_b);
+        if (has_a && in_a) {
+#pragma unroll
+            for (int k = 0; k < kNq; ++k) sum[k] = sum[k] + v[k].x;
+        }
+        if (has_b && in_b) {
+#pragma unroll
+            for (int k = 0; k < kNq; ++k) sum[k] = sum[k] + v[k].y;
+        }
+#endif
+    }
+    __device__ __forceinline__ float get(int k) const { return sum[k]; }
+};
+
+// The sums of a particle of a team: S lanes evaluate two candidates each, and
+// lane j < kPairs of the S adds quantities 2 j and 2 j + 1 in list order.
+template <class D, int S>
+struct TeamSums {
+    static constexpr int kNq = D::kQuantities;
+    static constexpr int kPairs = (kNq + 1) / 2;
+    static constexpr int kRow = 66;
+    static constexpr bool kExtra = D::kExtra;
+    static_assert(kPairs <= S, "a lane per pair of quantities");
+    float2 sum;
+    const D d;
+    __device__ __forceinline__ explicit TeamSums(const D& def) : sum(make_float2(0.0f, 0.0f)), d(def) {}
+    __device__ __forceinline__ void start(const float* from) {
+        const int s = (int)threadIdx.x & (S - 1);
+#pragma unroll
+        for (int k = 0; k < kNq; ++k) {
+            if (s == k / 2) {
+                if (k & 1) sum.y = from[k];
+                else sum.x = from[k];
             }
-            const uint32_t m = __ballot_sync(full, pass);
-            if (pass) {
-                const int k = nst + __popc(m & lt);
-                sm.sx[k] = xj.x;
-                sm.sy[k] = xj.y;
-                sm.sz[k] = xj.z;
-                sm.sw[k] = xj.w;
-                sm.q[base + k] = q;
-                sm.c[k] = (unsigned char)((q >= b1) + (q >= b2) + (q >= b3) + (q >= b4));
+        }
+    }
+    __device__ __forceinline__ float4 extra(uint32_t q) const { return d.extra(q); }
+    // The lane's two terms into the rows, zeros where there are none (a sum
+    // started at +0 never is -0, so adding +0 keeps its bits).
+    __device__ __forceinline__ void put(float2* rows, const float4& xa, const float4& xb, const float4& ea,
+                                        const float4& eb, bool has_a, bool has_b) const {
+        float4* const at = reinterpret_cast<float4*>(rows + 2 * ((int)threadIdx.x & 31));
+#if !PBF_FAST
+        if (d.C.paired) {
+            float2 v[kNq];
+            bool in_a, in_b;
+            d.products(xa, xb, ea, eb, v, in_a, in_b);
+            in_a = in_a && has_a;
+            in_b = in_b && has_b;
+#pragma unroll
+            for (int j = 0; j < kPairs; ++j) {
+                const float2 lo = v[2 * j];
+                const float2 hi = 2 * j + 1 < kNq ? v[2 * j + 1 < kNq ? 2 * j + 1 : 0] : make_float2(0.0f, 0.0f);
+                at[j * (kRow / 2)] = make_float4(in_a ? lo.x : 0.0f, in_a ? hi.x : 0.0f,
+                                                 in_b ? lo.y : 0.0f, in_b ? hi.y : 0.0f);
             }
-            nst += __popc(m);
-            if (nst >= 32) {
-                __syncwarp();
-                test_chunk(false);
+            return;
+        }
+#endif
+        float va[kNq], vb[kNq], fa[D::kFactors], fb[D::kFactors];
+        const bool in_a = has_a && d.eval(xa, ea, va, fa);
+        const bool in_b = has_b && d.eval(xb, eb, vb, fb);
+        // Value, or its product in the exact build, of quantity k; factor in
+        // the fast build, whose sums fuse the product and the addition.
+        auto value = [&](bool in, const float* v, const float* f, int k) {
+            if (k >= kNq || !in) return 0.0f;
+            const int c = D::factor_of(k);
+            return PBF_FAST || c < 0 ? v[k] : f[c < 0 ? 0 : c] * v[k];
+        };
+        auto factor = [&](bool in, const float* f, int k) {
+            const int c = k < kNq ? D::factor_of(k) : -1;
+            return c < 0 ? 1.0f : (in ? f[c < 0 ? 0 : c] : 0.0f);
+        };
+#pragma unroll
+        for (int j = 0; j < kPairs; ++j) {
+            const int k0 = 2 * j, k1 = 2 * j + 1;
+            at[j * (kRow / 2)] = make_float4(value(in_a, va, fa, k0), value(in_a, va, fa, k1),
+                                             value(in_b, vb, fb, k0), value(in_b, vb, fb, k1));
+            if (PBF_FAST)
+                at[(kPairs + j) * (kRow / 2)] =
+                    make_float4(factor(in_a, fa, k0), factor(in_a, fa, k1), factor(in_b, fb, k0),
+                                factor(in_b, fb, k1));
+        }
+    }
+    __device__ __forceinline__ void fold(const float2* rows) {
+        const int lane = (int)threadIdx.x & 31, s = lane & (S - 1);
+        if (s < kPairs) {
+            const float4* const v = reinterpret_cast<const float4*>(rows + s * kRow + 2 * (lane - s));
+#if PBF_FAST
+            const float4* const f =
+                reinterpret_cast<const float4*>(rows + (kPairs + s) * kRow + 2 * (lane - s));
+#endif
+#pragma unroll
+            for (int i = 0; i < S; ++i) {
+                const float4 t = v[i];
+#if PBF_FAST
+                const float4 c = f[i];
+                sum = make_float2(fmaf(c.x, t.x, sum.x), fmaf(c.y, t.y, sum.y));
+                sum = make_float2(fmaf(c.z, t.z, sum.x), fmaf(c.w, t.w, sum.y));
+#else
+                sum = __fadd2_rn(sum, make_float2(t.x, t.y));
+                sum = __fadd2_rn(sum, make_float2(t.z, t.w));
+#endif
+            }
+        }
+    }
+    // Sum k, in every lane of the particle (warp-collective).
+    __device__ __forceinline__ float get(int k) const {
+        return __shfl_sync(0xffffffffu, k & 1 ? sum.y : sum.x, ((int)threadIdx.x & (32 - S)) + k / 2);
+    }
+};
+
+// The team walk of one group (every lane of the team's four warps calls it).
+// In the listing, lane l of each warp stands for the team's particle
+// l / (32 / TP): xi, ci, want as in walk_group.  In the evaluation, thread t
+// stands for particle t / (128 / TP), which is the one that `sums` is about.
+template <int TP, bool kLam, class Sums>
+__device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr, bool want, int ci,
+                                           const float4 xi, const float4* __restrict__ xin, float inv_h,
+                                           const GridDesc& Gd, const WalkIndex& I, const Grid& G,
+                                           Sums& sums) {
+    constexpr int NT = TP / 8;
+    constexpr int LPP = 32 / TP;  // listing lanes per particle
+    constexpr int WPL = 4 / LPP;  // words of a batch that a lane settles
+    constexpr int S = 128 / TP;   // evaluating lanes per particle
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    const int g = lane >> 2, t4 = lane & 3;
+    const int pl = lane / LPP, j0 = (lane % LPP) * WPL;
+    uint32_t* const stage = reinterpret_cast<uint32_t*>(sm.warp[wid]);
+    const WalkBox B = walk_box(want, xi, inv_h);
+    uint32_t col[NT];
+    {
+        uint4 c = particle_column((xi.x - B.ox) * inv_h, (xi.y - B.oy) * inv_h, (xi.z - B.oz) * inv_h, B.lim);
+        if (!want) c = make_uint4(0u, 0u, pack_half2(0.0f, kHalfFar), 0u);
+        if (lane % LPP == 0) reinterpret_cast<uint4*>(stage)[pl] = c;
+        __syncwarp();
+#pragma unroll
+        for (int j = 0; j < NT; ++j) col[j] = stage[(8 * j + g) * 4 + t4];
+        __syncwarp();
+    }
+    const bool key = Gr.own != 0u;
+    const bool multi = Gr.W > 3;
+    const WalkRanges R = walk_ranges<false>(Gr, I, Gd, G);
+    const bool lam_zero = kLam && xi.w == 0.0f;
+    const bool all_zero = kLam && !__any_sync(full, want && xi.w != 0.0f);
+    uint32_t run = 0u;  // terms of particle pl listed so far
+
+    // Phase 2 of everything listed; every thread of the team calls it.
+    auto evaluate = [&]() {
+        if (wid == 0 && lane % LPP == 0) sm.total[pl] = run;
+        __syncthreads();
+        const int pe = threadIdx.x / S, s = threadIdx.x & (S - 1);
+        const int cnt = (int)sm.total[pe];
+        const int most = (int)__reduce_max_sync(full, (unsigned)cnt);
+        const unsigned short* const my = sm.list + pe * TeamSmem<TP>::kListRow;
+        float2* const rows = reinterpret_cast<float2*>(sm.warp[wid]);
+        float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
+        auto load = [&](int t) {
+            const uint32_t two = *reinterpret_cast<const uint32_t*>(my + t);
+            if (t < cnt) {
+                uint32_t q = sm.base[(two >> 5) & (kTeamWords - 1)] + (two & 31u);
+                if (key) q = __ldg(I.kpos + q);
+                xa = __ldg(xin + q);
+                if constexpr (Sums::kExtra) ea = sums.extra(q);
+            }
+            if (t + 1 < cnt) {
+                uint32_t q = sm.base[(two >> 21) & (kTeamWords - 1)] + ((two >> 16) & 31u);
+                if (key) q = __ldg(I.kpos + q);
+                xb = __ldg(xin + q);
+                if constexpr (Sums::kExtra) eb = sums.extra(q);
             }
         };
-        if (!kRuns || q1 - q0 < kRunRow) {
-            for (uint32_t qb = q0; qb < q1; qb += 32) stage(qb + (uint32_t)lane, qb + lane < q1);
-        } else {
-            // (kRuns) A row long enough to hold a run of identical
-            // candidates: the domain clamp piles fluid into a box corner, bit
-            // for bit, and such a cell holds tens of thousands.  Candidates with the same
-            // (xj, ej) in the same cell add the same term to a lane, so a
-            // run of whole 32-candidate chunks of them is not staged: the
-            // candidates before it are settled first, then each lane adds
-            // the run's term as many times as the run is long (rep, an exact
-            // repeated addition), then the walk goes on.  Shorter runs and
-            // run ends inside a chunk are staged as usual.
-            bool inrun = false;
-            float4 rx = make_float4(0.0f, 0.0f, 0.0f, 0.0f), re = rx;
-            uint32_t rn = 0;
-            int rc = 0;
-            auto apply = [&]() {
-                if (want && (all_member || (unsigned)(rc - myc + 1) <= 2u)) rep(rx, re, rn);
-                __syncwarp();
-                inrun = false;
-            };
-            for (uint32_t qb = q0; qb < q1; qb += 32) {
-                const uint32_t q = qb + (uint32_t)lane;
-                const bool ok = q < q1;
-                float4 xj = make_float4(0.0f, 0.0f, 0.0f, 0.0f), ej = xj;
-                if (ok) {
-                    xj = ld_step<kPersist>(xin + q);
-                    if constexpr (kExtra) ej = extra(q);
-                }
-                const int cq = (int)((q >= b1) + (q >= b2) + (q >= b3) + (q >= b4));
-                float4 ax = rx, ae = re;
-                int ac = rc;
-                if (!inrun) {
-                    ax = make_float4(__shfl_sync(full, xj.x, 0), __shfl_sync(full, xj.y, 0),
-                                     __shfl_sync(full, xj.z, 0), __shfl_sync(full, xj.w, 0));
-                    if constexpr (kExtra)
-                        ae = make_float4(__shfl_sync(full, ej.x, 0), __shfl_sync(full, ej.y, 0),
-                                         __shfl_sync(full, ej.z, 0), __shfl_sync(full, ej.w, 0));
-                    ac = __shfl_sync(full, cq, 0);
-                }
-                const bool same = ok && cq == ac && bits_equal(xj, ax) && (!kExtra || bits_equal(ej, ae));
-                const uint32_t sm_same = __ballot_sync(full, same);
-                if (inrun) {
-                    if (sm_same == full) {
-                        rn += 32;
-                        continue;
+        load(2 * s < cnt ? 2 * s : 0);
+        for (int t0 = 0; t0 < most; t0 += 2 * S) {
+            const int t = t0 + 2 * s;
+            const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
+            if (t + 2 * S < cnt) load(t + 2 * S);
+            sums.put(rows, x0, x1, e0, e1, t < cnt, t + 1 < cnt);
+            __syncwarp();
+            sums.fold(rows);
+            __syncwarp();
+        }
+        run = 0u;
+        __syncthreads();
+    };
+
+    for (int done = 0; done < R.total;) {
+        const int nw = min(kTeamWords, R.total - done);
+        if (wid == 0) list_words(R, done, kTeamWords, sm.base, sm.info);
+        done += nw;
+        __syncthreads();
+        for (int b0 = 0; b0 < nw; b0 += 4 * kTeamWarps) {
+            // --- phase 1: this warp's four words
+            const int b = b0 + 4 * wid;
+            uint32_t m[WPL];
+#pragma unroll
+            for (int i = 0; i < WPL; ++i) m[i] = 0u;
+            if (b < nw) {
+                uint32_t sel[4], nz[4];
+                uint32_t any_nz = 0u;
+                float4 xj[4];
+#pragma unroll
+                for (int j = 0; j < 4; ++j) {
+                    const uint32_t n = b + j < nw ? sm.info[b + j] & 63u : 0u;
+                    sel[j] = bit_range(0u, n);
+                    xj[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+                    if ((uint32_t)lane < n) {
+                        uint32_t q = sm.base[b + j] + (uint32_t)lane;
+                        if (key) q = __ldg(I.kpos + q);
+                        xj[j] = __ldg(xin + q);
                     }
-                    const int f = __ffs(~sm_same) - 1;  // the run ends before lane f
-                    rn += (uint32_t)f;
-                    apply();
-                    stage(q, ok && lane >= f);
-                } else if (sm_same == full) {
-                    if (nst > 0) {
-                        __syncwarp();
-                        test_chunk(true);
+                    if constexpr (kLam) {
+                        nz[j] = __ballot_sync(full, xj[j].w != 0.0f);
+                        any_nz |= nz[j];
                     }
-                    if (base > 0) evaluate();
-                    inrun = true;
-                    rx = ax;
-                    re = ae;
-                    rc = ac;
-                    rn = 32;
-                } else {
-                    stage(q, ok);
+                }
+                const bool test = !B.wide && (!kLam || !all_zero || any_nz != 0u);
+                if (test) {
+                    uint32_t h0[NT], h1[NT];
+                    test_words<NT>(stage, xj, sel, B, inv_h, col, h0, h1);
+                    unsigned short* const mh = reinterpret_cast<unsigned short*>(sm.mask[wid]);
+#pragma unroll
+                    for (int c = 0; c < NT; ++c) {
+                        const int at = (g >> 1) * TP + 8 * c + 2 * t4;
+                        mh[2 * at + (g & 1)] = (unsigned short)h0[c];
+                        mh[2 * at + 2 + (g & 1)] = (unsigned short)h1[c];
+                    }
+                    __syncwarp();
+                }
+#pragma unroll
+                for (int i = 0; i < WPL; ++i) {
+                    const int j = j0 + i;
+                    uint32_t in = 0u, innz = 0u;
+#pragma unroll
+                    for (int c = 0; c < 4; ++c) {
+                        if (c == j) in = sel[c];
+                        if (kLam && c == j) innz = nz[c];
+                    }
+                    uint32_t v = B.wide ? 0xffffffffu : (test ? sm.mask[wid][j * TP + pl] : 0u);
+                    v &= in;
+                    if (kLam && lam_zero) v &= innz;
+                    if (!want) v = 0u;
+                    if (multi) {
+                        const int w = b + j;
+                        const uint32_t slot = __shfl_sync(full, R.slot, w < nw ? (sm.info[w] >> 8) & 31u : 0u);
+                        if (v) v &= own_cells(I, slot, ci - Gr.cx, sm.base[w]);
+                    }
+                    m[i] = v;
                 }
             }
-            if (inrun) apply();
+            uint32_t mine = 0u;
+#pragma unroll
+            for (int i = 0; i < WPL; ++i) mine += (uint32_t)__popc(m[i]);
+            uint32_t upto = mine;  // this lane's and the particle's lanes before it
+#pragma unroll
+            for (int o = 1; o < LPP; o <<= 1) {
+                const uint32_t v = __shfl_up_sync(full, upto, o);
+                if (lane % LPP >= o) upto += v;
+            }
+            if (lane % LPP == LPP - 1) sm.count[wid][pl] = upto;
+            __syncthreads();
+            uint32_t before = 0u, round = 0u;
+#pragma unroll
+            for (int v = 0; v < kTeamWarps; ++v) {
+                const uint32_t c = sm.count[v][pl];
+                if (v < wid) before += c;
+                round += c;
+            }
+            if (__syncthreads_or(run + round > (uint32_t)kTeamTerms)) evaluate();
+            uint32_t at = (uint32_t)(pl * TeamSmem<TP>::kListRow) + run + before + upto - mine;
+#pragma unroll
+            for (int i = 0; i < WPL; ++i) {
+                uint32_t v = m[i];
+                while (v) {
+                    sm.list[at++] = (unsigned short)(((b + j0 + i) << 5) | (__ffs(v) - 1));
+                    v &= v - 1u;
+                }
+            }
+            run += round;
         }
+        evaluate();
     }
-    if (nst > 0) {
-        __syncwarp();
-        test_chunk(true);
-    }
-    if (base > 0) evaluate();
 }
 
 // Scene of sorted particle p (0 for a single scene).
@@ -1122,189 +1572,625 @@ __device__ __forceinline__ uint32_t scene_at(const Grid& G, uint32_t p) {
     return G.spid ? __ldg(G.spid + p) : 0u;
 }
 
+// The group of the first lane in `todo`, and whether the lane is in it
+// (warp-collective).  p, cell (w = bucket row + 1, 0 when clean): the lane's
+// particle and candidate cell; sid: its scene.
+template <class P>
+__device__ __forceinline__ WalkGroup next_group(uint32_t todo, const Grid& G, const P& prm, uint32_t p,
+                                                uint32_t sid, const int4 cell, bool& mem, float& inv_h,
+                                                GridDesc& Gd) {
+    const unsigned full = 0xffffffffu;
+    const int L = __ffs(todo) - 1;
+    WalkGroup Gr;
+    Gr.cx = __shfl_sync(full, cell.x, L);
+    Gr.cy = __shfl_sync(full, cell.y, L);
+    Gr.cz = __shfl_sync(full, cell.z, L);
+    Gr.own = (uint32_t)__shfl_sync(full, cell.w, L);
+    Gr.W = 3;
+    Gr.split = false;
+    mem = ((todo >> (threadIdx.x & 31)) & 1u) && cell.y == Gr.cy && cell.z == Gr.cz;
+    uint32_t pl = 0u;
+    if constexpr (!std::is_same<P, OneScene>::value) {
+        pl = __shfl_sync(full, p, L);
+        const uint32_t sl = __shfl_sync(full, sid, L);
+        mem = mem && sid == sl;
+    }
+    const StepConsts& C = prm.at(G.spid, pl);
+    Gd = C.grid;
+    inv_h = C.inv_cell;
+    if (Gr.own) {
+        mem = mem && cell.w != 0 && cell.x == Gr.cx;
+    } else {
+        const int wx0 = wrap(Gr.cx - 1, Gd.ox, Gd.gx);
+        const uint32_t d = (uint32_t)cell.x - (uint32_t)Gr.cx;
+        mem = mem && cell.w == 0 && d <= 2u;
+        const int far = (int)__reduce_max_sync(full, mem ? d : 0u);
+        if (wx0 + far + 3 > Gd.gx || Gr.cx <= -(1 << 30) || Gr.cx >= (1 << 30)) {
+            mem = mem && d == 0u;
+            Gr.split = wx0 + 3 > Gd.gx;
+        } else {
+            Gr.W = far + 3;
+        }
+    }
+    return Gr;
+}
+
+// The warp walk over the candidates, in index I with positions xin, of every
+// lane that wants (every lane of the warp calls it): the lane's particle has
+// sorted position p (any valid one where it does not want), candidate cell
+// `cell` (w = its bucket row + 1, 0 when clean) and x* xi.  Returns false,
+// with nothing summed, when the warp's particles sit in too many cells (the
+// caller walks lane by lane then).
+template <bool kPersist, bool kLam, bool kRuns, class P, class Sums>
+__device__ __forceinline__ bool warp_walk(WalkSmem& sm, const Grid& G, const WalkIndex& I, const P& prm,
+                                          uint32_t p, const int4 cell, bool want, const float4 xi,
+                                          const float4* xin, Sums& sums) {
+    const unsigned full = 0xffffffffu;
+    uint32_t todo = __ballot_sync(full, want);
+    if (!todo) return true;
+    const uint32_t sid = scene_at(G, p);
+    {
+        const uint32_t x = cell.w ? (uint32_t)cell.x * 3u + 1u : ((uint32_t)cell.x + 0x30000000u) / 3u * 3u;
+        const uint32_t k = (((uint32_t)cell.y * 73856093u) ^ ((uint32_t)cell.z * 19349663u) ^
+                            (sid * 2654435761u)) + x * 83492791u;
+        const uint32_t same = __match_any_sync(full, want ? k : 0u) & todo;
+        const bool first = want && (int)(threadIdx.x & 31) == __ffs(same) - 1;
+        if (__popc(__ballot_sync(full, first)) > kMaxGroups) return false;
+    }
+    while (todo) {
+        bool mem;
+        float inv_h;
+        GridDesc Gd;
+        const WalkGroup Gr = next_group(todo, G, prm, p, sid, cell, mem, inv_h, Gd);
+        todo &= ~__ballot_sync(full, mem);
+        walk_group<kPersist, kLam, kRuns>(sm, Gr, mem, cell.x, xi, xin, inv_h, Gd, I, G, sums);
+    }
+    return true;
+}
+
+// The team walk (every thread of the team calls it; p, cell, want and xi as
+// in warp_walk, of the listing's particle, the same in all four warps).
+template <int TP, bool kLam, class P, class Sums>
+__device__ __forceinline__ void team_walk(TeamSmem<TP>& sm, const Grid& G, const WalkIndex& I, const P& prm,
+                                          uint32_t p, const int4 cell, bool want, const float4 xi,
+                                          const float4* __restrict__ xin, Sums& sums) {
+    const unsigned full = 0xffffffffu;
+    uint32_t todo = __ballot_sync(full, want);
+    const uint32_t sid = scene_at(G, p);
+    while (todo) {
+        bool mem;
+        float inv_h;
+        GridDesc Gd;
+        const WalkGroup Gr = next_group(todo, G, prm, p, sid, cell, mem, inv_h, Gd);
+        todo &= ~__ballot_sync(full, mem);
+        team_group<TP, kLam>(sm, Gr, mem, cell.x, xi, xin, inv_h, Gd, I, G, sums);
+    }
+}
+
+__device__ __forceinline__ WalkIndex fluid_index(const Grid& G) {
+    return WalkIndex{G.off, G.kpos, G.bend, G.btab};
+}
+
+__device__ __forceinline__ WalkIndex boundary_index(const Grid& G) {
+    return WalkIndex{G.bg.off, G.bg.kpos, G.bg.bend, G.bg.btab};
+}
+
 // Whether a slot among the 27 around a clean particle's cell holds the stamp
 // `it`: with the moved stamps and it, whether a candidate moved in the delta
 // pass of Jacobi iteration it - 1 (when none did, the candidates all sit
 // where they sat for the previous density pass, so the particle's rho and
 // lambda would come out bit for bit the same); with the lambda stamps and
-// it + 1, whether a candidate has a nonzero lambda in iteration it.
+// it + 1, whether a candidate has a nonzero lambda in iteration it.  Only
+// the z planes [c0, c1) of the three are looked at.
 template <bool kPersist>
-__device__ __forceinline__ bool neighbourhood_moved(const int4 cell, const GridDesc& Gd,
-                                                    const uint32_t* moved, int it) {
-    // The 27 slots from 3 wrapped coordinates per axis; the loads are
-    // independent, so they overlap.
-    uint32_t wx[3], wy[3], wz[3];
+__device__ __forceinline__ bool neighbourhood_stamped(const int4 cell, const GridDesc& Gd,
+                                                      const uint32_t* stamps, uint32_t it, int c0, int c1) {
+    // The slots from wrapped coordinates per axis; the loads are independent,
+    // so they overlap.
+    uint32_t wx[3], wy[3];
 #pragma unroll
     for (int d = 0; d < 3; ++d) {
         wx[d] = (uint32_t)wrap(cell.x + d - 1, Gd.ox, Gd.gx);
         wy[d] = (uint32_t)wrap(cell.y + d - 1, Gd.oy, Gd.gy);
-        wz[d] = (uint32_t)wrap(cell.z + d - 1, Gd.oz, Gd.gz);
     }
     bool any = false;
 #pragma unroll
-    for (int c = 0; c < 3; ++c)
+    for (int c = 0; c < 3; ++c) {
+        if (c < c0 || c >= c1) continue;
+        const uint32_t wz = (uint32_t)wrap(cell.z + c - 1, Gd.oz, Gd.gz);
 #pragma unroll
         for (int b = 0; b < 3; ++b) {
-            const uint32_t row = Gd.base + (uint32_t)Gd.gx * (wy[b] + (uint32_t)Gd.gy * wz[c]);
+            const uint32_t row = Gd.base + (uint32_t)Gd.gx * (wy[b] + (uint32_t)Gd.gy * wz);
 #pragma unroll
-            for (int a = 0; a < 3; ++a)
-                any |= ld_step<kPersist>(moved + row + wx[a]) == (uint32_t)it;
+            for (int a = 0; a < 3; ++a) any |= ld_step<kPersist>(stamps + row + wx[a]) == it;
         }
+    }
     return any;
 }
 
-// compute_density + compute_lambda (pbf_solver.cpp:129-179) in one candidate
-// pass for sorted particle p.  Reads x* from xin, writes (x*, lambda) to xout
-// and rho to srho.  Scenes whose `iters` are done by iteration `it` are left
-// untouched.  Warp-collective: every lane of the warp calls it, with
-// `active` false past the last particle.
-template <bool kPersist, int U, class P, int CH>
-__device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const float4* xin,
-                                                  float4* xout, float* __restrict__ srho, int it,
-                                                  const Grid& G, const P& prm,
-                                                  CoopSmem<CH, false>& sm) {
-    constexpr bool kCoop = CoopBlock<P, 32, false, U>::kOn;
-    const uint32_t pa = active ? p : 0u;
-    const StepConsts& C = prm.at(G.spid, pa);
-    const int4 cell = cell_at(G, pa);
-    const uint32_t rf = run_flags(G, pa);
-    bool live = active && it < C.iters && !(rf & kCopyBit);
-    if (live && it > 0 && G.moved && cell.w == 0 &&
-        !neighbourhood_moved<kPersist>(cell, C.grid, G.moved, it)) {
-        // Nothing around moved since the last density pass: keep its rho
-        // (srho) and lambda (x*.w, which the delta pass carried through).
-        const float4 keep = xin[p];
-        xout[p] = keep;
-        for (uint32_t m = p + 1, e = run_end(G, p, rf); m < e; ++m) xout[m] = keep;
-        if (G.lamnz && keep.w != 0.0f)
-            G.lamnz[slot_of(cell.x, cell.y, cell.z, C.grid)] = (uint32_t)it + 1u;
-        live = false;
+// The same for a team: whether each listing lane's particle (asking ones)
+// has a stamped slot; three warps look at a plane each.
+template <int TP>
+__device__ __forceinline__ bool team_stamped(TeamSmem<TP>& sm, bool ask, const int4 cell, const GridDesc& Gd,
+                                             const uint32_t* stamps, uint32_t it) {
+    const int lane = threadIdx.x & 31, wid = threadIdx.x >> 5, pl = lane / (32 / TP);
+    if (threadIdx.x < TP) sm.flag[threadIdx.x] = 0;
+    __syncthreads();
+    if (ask && wid < 3 && neighbourhood_stamped<false>(cell, Gd, stamps, it, wid, wid + 1)) sm.flag[pl] = 1;
+    __syncthreads();
+    return ask && sm.flag[pl] != 0;
+}
+
+#if !PBF_FAST
+// r = x_i - x_j and r^2 of two candidates (xa, xb), as rel_sq's.
+struct PairRel {
+    float2 x, y, z, r2;
+    __device__ __forceinline__ PairRel(const float4& xi, const float4& xa, const float4& xb, float one) {
+        x = make_float2(xi.x - xa.x, xi.x - xb.x);
+        y = make_float2(xi.y - xa.y, xi.y - xb.y);
+        z = make_float2(xi.z - xa.z, xi.z - xb.z);
+        r2 = pbf::add2(mul2(x, x), pbf::add2(mul2(y, y), mul2(z, z), one), one);
     }
-    CoopRow R;
-    bool coop = false;
-    if constexpr (kCoop) coop = coop_row(live, cell, C.grid, R, scene_at(G, pa));
-    if (!live) return;
-    const float4 xi = xin[p];
-    float density = 0.0f, sum_grad_sq = 0.0f, gix = 0.0f, giy = 0.0f, giz = 0.0f;
-    float ci_first = 0.0f;  // C_i of a density-first walk (computed once)
-    bool have_ci = false;
-    // The term of candidate xj, added L times (One: once); density-first
-    // walks add the density alone (grads false) or the gradient sums alone.
-    auto part = [&](const float4& xj, auto L, bool dens, bool grads) {
+};
+
+__device__ __forceinline__ float2 not_below_zero(float2 a) {
+    return make_float2(fmaxf(a.x, 0.0f), fmaxf(a.y, 0.0f));
+}
+
+// poly6 of two squared distances below the support's.
+__device__ __forceinline__ float2 poly6_2(float2 r2, const StepConsts& C) {
+    const float2 d = not_below_zero(sub2(both(C.h2), r2));
+    return mul2(mul2(mul2(both(C.k_poly), d), d), d);
+}
+
+// spiky_coeff of two squared distances below C.cut (C.paired).
+__device__ __forceinline__ float2 spiky_coeff_2(float2 r2, const StepConsts& C) {
+    float2 len, inv;
+    root_and_inverse(r2, len, inv);
+    const float2 d = not_below_zero(sub2(both(C.h), len));
+    const float2 c = quotient(mul2(mul2(both(C.k_spiky), d), d), len, inv);
+    return make_float2(r2.x > C.r2_min ? c.x : 0.0f, r2.y > C.r2_min ? c.y : 0.0f);
+}
+#endif
+
+// compute_density + compute_lambda (pbf_solver.cpp:129-179): the density, the
+// gradient sum and the sum of the squared gradients in one candidate pass.
+struct DensityGradTerm {
+    static constexpr int kQuantities = 5, kFactors = 2;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int k) { return k == 0 ? 0 : (k < 4 ? 1 : -1); }
+    __device__ __forceinline__ bool eval(const float4& xj, const float4&, float* v, float* f) const {
         float rx, ry, rz;
         const float r_sq = rel_sq(xi, xj, rx, ry, rz);
-        if (r_sq < C.cut) {
-            if (dens) density = acc(density, C.mass * poly6(r_sq, C), L);
-            if (grads) {
-                const float c = spiky_coeff(r_sq, C);
-                const float gx = C.mr * (c * rx);
-                const float gy = C.mr * (c * ry);
-                const float gz = C.mr * (c * rz);
-                sum_grad_sq = acc(sum_grad_sq, sqn(gx, gy, gz), L);
-                gix = acc(gix, gx, L);
-                giy = acc(giy, gy, L);
-                giz = acc(giz, gz, L);
-            }
-        }
-    };
-    auto term = [&](const float4& xj, auto L) { part(xj, L, true, true); };
-    if constexpr (kCoop) {
-        if (coop) {
-            auto none = [](uint32_t) { return float4{}; };
-            // Density first: when C_i < 0 lambda_i is 0 whatever the gradient
-            // sums, so a warp can sum the densities alone (poly6 terms, no
-            // square root or division), then walk again, in the same
-            // candidate order, for the gradients of its lanes with
-            // C_i >= 0 only.  Each sum sees the same terms in the same order
-            // as the single walk: same bits.  It pays where most warps have
-            // no such lane; which way a warp goes follows the share of
-            // warps that needed gradients in the same iteration of the last
-            // step.
-            bool dfirst = false;
-            if (G.dhist && it < kWalkHist && !G.bg.spos) {
-                const uint32_t need = __ldg(G.dhist + it), ran = __ldg(G.dhist + kWalkHist + it);
-                dfirst = ran > 0 && 3u * need < ran;
-            }
-            auto once = [&](const float4& xj, const float4&) { term(xj, One{}); };
-            // (The walk is compiled without runs here, kRuns false, so `times`
-            // is never called; it states what a run would add.)
-            auto times = [&](const float4& xj, const float4&, uint32_t L) { term(xj, L); };
-            if (!dfirst) {
-                coop_walk<CH, false, kPersist, false, false>(sm, R, cell.x, xi, xin, C.cut, C.grid, G.off,
-                                                      none, once, times);
-            } else {
-                // Densities only, then gradients only for the lanes that want.
-                bool want = true, grads = false;
-                for (;;) {
-                    coop_walk<CH, false, kPersist, false, false>(
-                        sm, R, cell.x, xi, xin, C.cut, C.grid, G.off, none,
-                        [&](const float4& xj, const float4&) {
-                            float rx, ry, rz;
-                            const float r_sq = rel_sq(xi, xj, rx, ry, rz);
-                            if (r_sq < C.cut) {
-                                if (!grads) {
-                                    density += C.mass * poly6(r_sq, C);
-                                } else {
-                                    const float c = spiky_coeff(r_sq, C);
-                                    const float gx = C.mr * (c * rx);
-                                    const float gy = C.mr * (c * ry);
-                                    const float gz = C.mr * (c * rz);
-                                    sum_grad_sq += sqn(gx, gy, gz);
-                                    gix += gx;
-                                    giy += gy;
-                                    giz += gz;
-                                }
-                            }
-                        },
-                        [&](const float4& xj, const float4&, uint32_t L) {
-                            part(xj, L, !grads, grads);
-                        },
-                        want);
-                    if (grads) break;
-                    ci_first = density * C.inv_rho0 - 1.0f;
-                    have_ci = true;
-                    want = !(ci_first < 0.0f);
-                    if (!__any_sync(0xffffffffu, want)) break;
-                    grads = true;
-                }
-            }
-            if (G.dhist && it < kWalkHist && (threadIdx.x & 31) == 0) {
-                atomicAdd(G.dhist + 3 * kWalkHist + it, 1u);
-            }
-        }
+        if (!(r_sq < C.cut)) return false;
+        v[0] = poly6(r_sq, C);
+        const float c = spiky_coeff(r_sq, C);
+        v[1] = c * rx;
+        v[2] = c * ry;
+        v[3] = c * rz;
+        v[4] = sqn(C.mr * v[1], C.mr * v[2], C.mr * v[3]);
+        f[0] = C.mass;
+        f[1] = C.mr;
+        return true;
     }
-    if (!coop)
-        for_each_candidate_runs<U, std::is_same<P, OneScene>::value>(
-            cell, G, C, [&](uint32_t q) { term(ld_step<kPersist>(xin + q), One{}); },
-            [&](uint32_t q, uint32_t L) { term(ld_step<kPersist>(xin + q), Many{L}); });
-    if (G.bg.spos) {
-        // Two-way coupling (no counterpart in the reference): after the fluid
-        // terms, the boundary's Akinci density rho0 psi_b W and its gradient
-        // psi_b grad W (= (rho0 psi_b / rho0) grad W) in the boundary index's
-        // bucket order.  The boundary does not move, so it adds nothing to
-        // the sum of the neighbours' squared gradients.
-        for_each_candidate<4>(boundary_cell(G, p, cell), G.bg.off, G.bg.kpos, G.bg.bend,
-                              G.bg.btab, C, [&](uint32_t q) {
-                                  const float4 b = __ldg(G.bg.spos + q);
-                                  const float rx = xi.x - b.x, ry = xi.y - b.y, rz = xi.z - b.z;
-                                  const float r_sq = sqn(rx, ry, rz);
-                                  if (r_sq < C.cut) {
-                                      density += C.rho0 * b.w * poly6(r_sq, C);
-                                      const float c = spiky_coeff(r_sq, C);
-                                      gix += b.w * (c * rx);
-                                      giy += b.w * (c * ry);
-                                      giz += b.w * (c * rz);
-                                  }
-                              });
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&,
+                                             const float4&, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.cut;
+        in_b = r.r2.y < C.cut;
+        v[0] = mul2(both(C.mass), poly6_2(r.r2, C));
+        const float2 c = spiky_coeff_2(r.r2, C), mr = both(C.mr);
+        v[1] = mul2(mr, mul2(c, r.x));
+        v[2] = mul2(mr, mul2(c, r.y));
+        v[3] = mul2(mr, mul2(c, r.z));
+        v[4] = pbf::add2(mul2(v[1], v[1]), pbf::add2(mul2(v[2], v[2]), mul2(v[3], v[3]), C.one), C.one);
     }
+#endif
+};
+
+// The density alone, and the gradient sums alone (density-first walks).
+struct DensityTerm {
+    static constexpr int kQuantities = 1, kFactors = 1;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    __device__ __forceinline__ bool eval(const float4& xj, const float4&, float* v, float* f) const {
+        float rx, ry, rz;
+        const float r_sq = rel_sq(xi, xj, rx, ry, rz);
+        if (!(r_sq < C.cut)) return false;
+        v[0] = poly6(r_sq, C);
+        f[0] = C.mass;
+        return true;
+    }
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&,
+                                             const float4&, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.cut;
+        in_b = r.r2.y < C.cut;
+        v[0] = mul2(both(C.mass), poly6_2(r.r2, C));
+    }
+#endif
+};
+
+struct GradTerm {
+    static constexpr int kQuantities = 4, kFactors = 1;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int k) { return k < 3 ? 0 : -1; }
+    __device__ __forceinline__ bool eval(const float4& xj, const float4&, float* v, float* f) const {
+        float rx, ry, rz;
+        const float r_sq = rel_sq(xi, xj, rx, ry, rz);
+        if (!(r_sq < C.cut)) return false;
+        const float c = spiky_coeff(r_sq, C);
+        v[0] = c * rx;
+        v[1] = c * ry;
+        v[2] = c * rz;
+        v[3] = sqn(C.mr * v[0], C.mr * v[1], C.mr * v[2]);
+        f[0] = C.mr;
+        return true;
+    }
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&,
+                                             const float4&, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.cut;
+        in_b = r.r2.y < C.cut;
+        const float2 c = spiky_coeff_2(r.r2, C), mr = both(C.mr);
+        v[0] = mul2(mr, mul2(c, r.x));
+        v[1] = mul2(mr, mul2(c, r.y));
+        v[2] = mul2(mr, mul2(c, r.z));
+        v[3] = pbf::add2(mul2(v[0], v[0]), pbf::add2(mul2(v[1], v[1]), mul2(v[2], v[2]), C.one), C.one);
+    }
+#endif
+};
+
+// The boundary's share of the same sums (two-way coupling, no counterpart in
+// the reference): rho0 psi_b W and its gradient psi_b grad W (= (rho0 psi_b /
+// rho0) grad W).  The boundary does not move, so it adds nothing to the sum
+// of the neighbours' squared gradients.
+struct BoundaryDensityTerm {
+    static constexpr int kQuantities = 4, kFactors = 2;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int k) { return k == 0 ? 0 : 1; }
+    __device__ __forceinline__ bool eval(const float4& b, const float4&, float* v, float* f) const {
+        const float rx = xi.x - b.x, ry = xi.y - b.y, rz = xi.z - b.z;
+        const float r_sq = sqn(rx, ry, rz);
+        if (!(r_sq < C.cut)) return false;
+        v[0] = poly6(r_sq, C);
+        const float c = spiky_coeff(r_sq, C);
+        v[1] = c * rx;
+        v[2] = c * ry;
+        v[3] = c * rz;
+        f[0] = C.rho0 * b.w;
+        f[1] = b.w;
+        return true;
+    }
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&,
+                                             const float4&, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.cut;
+        in_b = r.r2.y < C.cut;
+        const float2 psi = make_float2(xa.w, xb.w);
+        v[0] = mul2(mul2(both(C.rho0), psi), poly6_2(r.r2, C));
+        const float2 c = spiky_coeff_2(r.r2, C);
+        v[1] = mul2(psi, mul2(c, r.x));
+        v[2] = mul2(psi, mul2(c, r.y));
+        v[3] = mul2(psi, mul2(c, r.z));
+    }
+#endif
+};
+
+// compute_delta_position (pbf_solver.cpp:181-223).  A zero lambda sum adds an
+// exact zero (no s_corr either); the sum, started at +0, never becomes -0, so
+// skipping it keeps every bit.
+struct DeltaTerm {
+    static constexpr int kQuantities = 3, kFactors = 1;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    __device__ __forceinline__ bool eval(const float4& xj, const float4&, float* v, float* f) const {
+        float rx, ry, rz, lambda_sum;
+        const float r_sq = rel_sq<true>(xi, xj, rx, ry, rz, &lambda_sum);
+        if (!(r_sq < C.cut && lambda_sum != 0.0f)) return false;
+        float s_corr = 0.0f;
+        if (lambda_sum < -1e-10f && C.scorr_on) {
+            float ratio = poly6(r_sq, C) / C.w_dq;
+            ratio = (1.0f < ratio) ? 1.0f : ratio;
+            float rp = ratio * ratio;
+            if (C.corr_n4) rp = rp * rp;
+            s_corr = C.neg_corr_k * rp;
+        }
+        const float c = spiky_coeff(r_sq, C);
+        f[0] = (lambda_sum + s_corr) * C.mass;
+        v[0] = c * rx;
+        v[1] = c * ry;
+        v[2] = c * rz;
+        return true;
+    }
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&,
+                                             const float4&, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        float2 lam = make_float2(xi.w + xa.w, xi.w + xb.w);
+        in_a = r.r2.x < C.cut && lam.x != 0.0f;
+        in_b = r.r2.y < C.cut && lam.y != 0.0f;
+        if (C.scorr_on) {
+            float2 ratio = quotient(poly6_2(r.r2, C), both(C.w_dq), both(C.inv_w_dq));
+            ratio.x = (1.0f < ratio.x) ? 1.0f : ratio.x;
+            ratio.y = (1.0f < ratio.y) ? 1.0f : ratio.y;
+            float2 rp = mul2(ratio, ratio);
+            if (C.corr_n4) rp = mul2(rp, rp);
+            const float2 s = mul2(both(C.neg_corr_k), rp);
+            lam.x = lam.x + (lam.x < -1e-10f ? s.x : 0.0f);
+            lam.y = lam.y + (lam.y < -1e-10f ? s.y : 0.0f);
+        }
+        const float2 a = mul2(lam, both(C.mass));
+        const float2 c = spiky_coeff_2(r.r2, C);
+        v[0] = mul2(a, mul2(c, r.x));
+        v[1] = mul2(a, mul2(c, r.y));
+        v[2] = mul2(a, mul2(c, r.z));
+    }
+#endif
+};
+
+// The boundary's share of the position correction (two-way coupling):
+// lambda_i (rho0 psi_b) grad W.
+struct BoundaryDeltaTerm {
+    static constexpr int kQuantities = 3, kFactors = 1;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    __device__ __forceinline__ bool eval(const float4& b, const float4&, float* v, float* f) const {
+        const float rx = xi.x - b.x, ry = xi.y - b.y, rz = xi.z - b.z;
+        const float r_sq = sqn(rx, ry, rz);
+        if (!(r_sq < C.cut)) return false;
+        const float c = spiky_coeff(r_sq, C);
+        f[0] = xi.w * (C.rho0 * b.w);
+        v[0] = c * rx;
+        v[1] = c * ry;
+        v[2] = c * rz;
+        return true;
+    }
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&,
+                                             const float4&, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.cut;
+        in_b = r.r2.y < C.cut;
+        const float2 c = spiky_coeff_2(r.r2, C);
+        const float2 a = mul2(both(xi.w), mul2(both(C.rho0), make_float2(xa.w, xb.w)));
+        v[0] = mul2(a, mul2(c, r.x));
+        v[1] = mul2(a, mul2(c, r.y));
+        v[2] = mul2(a, mul2(c, r.z));
+    }
+#endif
+};
+
+// apply_xsph_viscosity (pbf_solver.cpp:225-250).
+struct XsphTerm {
+    static constexpr int kQuantities = 3, kFactors = 1;
+    static constexpr bool kExtra = true;
+    const StepConsts& C;
+    const float4 xi, vi;
+    const float4* __restrict__ sv;
+    static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    __device__ __forceinline__ float4 extra(uint32_t q) const { return __ldg(sv + q); }
+    __device__ __forceinline__ bool eval(const float4& xj, const float4& vj, float* v, float* f) const {
+        float rx, ry, rz;
+        const float r_sq = rel_sq(xi, xj, rx, ry, rz);
+        if (!(r_sq < C.h2)) return false;
+        f[0] = poly6(r_sq, C);
+        v[0] = vj.w * (vj.x - vi.x);
+        v[1] = vj.w * (vj.y - vi.y);
+        v[2] = vj.w * (vj.z - vi.z);
+        return true;
+    }
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4& va,
+                                             const float4& vb, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.h2;
+        in_b = r.r2.y < C.h2;
+        const float2 w = poly6_2(r.r2, C), m = make_float2(va.w, vb.w);
+        v[0] = mul2(mul2(m, make_float2(va.x - vi.x, vb.x - vi.x)), w);
+        v[1] = mul2(mul2(m, make_float2(va.y - vi.y, vb.y - vi.y)), w);
+        v[2] = mul2(mul2(m, make_float2(va.z - vi.z, vb.z - vi.z)), w);
+    }
+#endif
+};
+
+// XSPH and the SPH curl of the velocities in one pass (Macklin & Mueller
+// 2013, section 5, with its volume factor):
+//   omega_i = sum_j (m/rho_j') spiky_grad(x*_i - x*_j) x (v_j - v_i).
+struct XsphOmegaTerm {
+    static constexpr int kQuantities = 6, kFactors = 2;
+    static constexpr bool kExtra = true;
+    const StepConsts& C;
+    const float4 xi, vi;
+    const float4* __restrict__ sv;
+    static __host__ __device__ constexpr int factor_of(int k) { return k < 3 ? 0 : 1; }
+    __device__ __forceinline__ float4 extra(uint32_t q) const { return __ldg(sv + q); }
+    __device__ __forceinline__ bool eval(const float4& xj, const float4& vj, float* v, float* f) const {
+        float rx, ry, rz;
+        const float r_sq = rel_sq(xi, xj, rx, ry, rz);
+        if (!(r_sq < C.cut)) return false;
+        const float ux = vj.x - vi.x;
+        const float uy = vj.y - vi.y;
+        const float uz = vj.z - vi.z;
+        f[0] = poly6(r_sq, C);
+        v[0] = vj.w * ux;
+        v[1] = vj.w * uy;
+        v[2] = vj.w * uz;
+        const float c = spiky_coeff(r_sq, C);
+        const float gx = c * rx, gy = c * ry, gz = c * rz;
+        f[1] = vj.w;
+        v[3] = gy * uz - gz * uy;
+        v[4] = gz * ux - gx * uz;
+        v[5] = gx * uy - gy * ux;
+        return true;
+    }
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4& va,
+                                             const float4& vb, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.cut;
+        in_b = r.r2.y < C.cut;
+        const float2 m = make_float2(va.w, vb.w);
+        const float2 ux = make_float2(va.x - vi.x, vb.x - vi.x);
+        const float2 uy = make_float2(va.y - vi.y, vb.y - vi.y);
+        const float2 uz = make_float2(va.z - vi.z, vb.z - vi.z);
+        const float2 w = poly6_2(r.r2, C);
+        v[0] = mul2(mul2(m, ux), w);
+        v[1] = mul2(mul2(m, uy), w);
+        v[2] = mul2(mul2(m, uz), w);
+        const float2 c = spiky_coeff_2(r.r2, C);
+        const float2 gx = mul2(c, r.x), gy = mul2(c, r.y), gz = mul2(c, r.z);
+        // a b - c d with both products rounded: (-c d) + a b, the negation exact.
+        auto cross = [&](float2 p, float2 q, float2 s, float2 t) {
+            return pbf::add2(mul2(p, q), mul2(mul2(s, both(-1.0f)), t), C.one);
+        };
+        v[3] = mul2(m, cross(gy, uz, gz, uy));
+        v[4] = mul2(m, cross(gz, ux, gx, uz));
+        v[5] = mul2(m, cross(gx, uy, gy, ux));
+    }
+#endif
+};
+
+// The gradient of |omega| (vorticity confinement):
+//   eta_i = sum_j (m/rho_j') (|omega_j| - |omega_i|) spiky_grad(x*_i - x*_j).
+// The extras are (m / rho_j', |omega_j|) of the candidate.
+struct VorticityTerm {
+    static constexpr int kQuantities = 3, kFactors = 1;
+    static constexpr bool kExtra = true;
+    const StepConsts& C;
+    const float4 xi;
+    const float wi;
+    const float4* __restrict__ sv;
+    const float4* __restrict__ som;
+    static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    __device__ __forceinline__ float4 extra(uint32_t q) const {
+        return make_float4(__ldg(&sv[q].w), __ldg(&som[q].w), 0.0f, 0.0f);
+    }
+    __device__ __forceinline__ bool eval(const float4& xj, const float4& e, float* v, float* f) const {
+        float rx, ry, rz;
+        const float r_sq = rel_sq(xi, xj, rx, ry, rz);
+        if (!(r_sq < C.cut)) return false;
+        const float c = spiky_coeff(r_sq, C);
+        f[0] = e.x * (e.y - wi);
+        v[0] = c * rx;
+        v[1] = c * ry;
+        v[2] = c * rz;
+        return true;
+    }
+#if !PBF_FAST
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4& ea,
+                                             const float4& eb, float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.cut;
+        in_b = r.r2.y < C.cut;
+        const float2 c = spiky_coeff_2(r.r2, C);
+        const float2 a = mul2(make_float2(ea.x, eb.x), make_float2(ea.y - wi, eb.y - wi));
+        v[0] = mul2(a, mul2(c, r.x));
+        v[1] = mul2(a, mul2(c, r.y));
+        v[2] = mul2(a, mul2(c, r.z));
+    }
+#endif
+};
+
+// ---------------------------------------------------------------------------
+// The passes.  A pass's kernel comes in two forms, over warps of 32 particles
+// and over teams of TP; both find the same sums and share what follows them.
+
+// The sums over the fluid's candidates of every lane that wants: the warp
+// walk, or lane by lane where the warp's particles are scattered.
+template <bool kPersist, bool kLam, class P, class Sums>
+__device__ __forceinline__ void sum_candidates(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
+                                               const int4 cell, bool want, const float4 xi,
+                                               const float4* xin, const StepConsts& C, Sums& sums) {
+    constexpr bool kRuns = std::is_same<P, OneScene>::value;
+    if (warp_walk<kPersist, kLam, kRuns>(sm, G, fluid_index(G), prm, p, cell, want, xi, xin, sums)) return;
+    if (!want) return;
+    for_each_candidate_runs<kRuns>(
+        cell, G, C,
+        [&](uint32_t q) {
+            float4 e{};
+            if constexpr (Sums::kExtra) e = sums.extra(q);
+            sums.add(ld_step<kPersist>(xin + q), e);
+        },
+        [&](uint32_t q, uint32_t L) {
+            float4 e{};
+            if constexpr (Sums::kExtra) e = sums.extra(q);
+            sums.add_run(ld_step<kPersist>(xin + q), e, L);
+        });
+}
+
+// The same over the boundary of a two-way coupled step; `cell` is the
+// particle's cell in the fluid's grid.
+template <class P, class Sums>
+__device__ __forceinline__ void sum_boundary(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
+                                             const int4 cell, bool want, const float4 xi,
+                                             const StepConsts& C, Sums& sums) {
+    const int4 bc = boundary_cell(G, p, cell);
+    if (warp_walk<false, false, false>(sm, G, boundary_index(G), prm, p, bc, want, xi, G.bg.spos, sums))
+        return;
+    if (!want) return;
+    for_each_candidate<4>(bc, G.bg.off, G.bg.kpos, G.bg.bend, G.bg.btab, C,
+                          [&](uint32_t q) { sums.add(__ldg(G.bg.spos + q), float4{}); });
+}
+
+// A thread of a team: its particle in the listing (pl; the same in all four
+// warps) and in the evaluation (pe), and whether it writes pe's results.
+template <int TP>
+struct TeamThread {
+    uint32_t pl, pe;
+    bool al, ae, writer;
+    __device__ __forceinline__ explicit TeamThread(int n) {
+        const uint32_t first = blockIdx.x * (uint32_t)TP;
+        pl = first + (threadIdx.x & 31u) / (32u / TP);
+        pe = first + threadIdx.x / (128u / TP);
+        al = pl < (uint32_t)n;
+        ae = pe < (uint32_t)n;
+        writer = ae && threadIdx.x % (128u / TP) == 0u;
+        if (!al) pl = 0u;
+        if (!ae) pe = 0u;
+    }
+    // Hands a flag of the listing's particles to the evaluation's threads.
+    __device__ __forceinline__ bool hand_over(TeamSmem<TP>& sm, bool v) const {
+        __syncthreads();
+        if (threadIdx.x < 32u && threadIdx.x % (32u / TP) == 0u) sm.flag[threadIdx.x / (32u / TP)] = v;
+        __syncthreads();
+        return sm.flag[threadIdx.x / (128u / TP)] != 0;
+    }
+};
+
+// What the density pass writes for particle p and the rest of its run.
+__device__ __forceinline__ void keep_lambda(uint32_t p, uint32_t rf, const int4 cell, const float4* xin,
+                                            float4* xout, int it, const Grid& G, const StepConsts& C) {
+    // Nothing around moved since the last density pass: keep its rho (srho)
+    // and lambda (x*.w, which the delta pass carried through).
+    const float4 keep = xin[p];
+    xout[p] = keep;
+    for (uint32_t m = p + 1, e = run_end(G, p, rf); m < e; ++m) xout[m] = keep;
+    if (G.lamnz && keep.w != 0.0f) G.lamnz[slot_of(cell.x, cell.y, cell.z, C.grid)] = (uint32_t)it + 1u;
+}
+
+__device__ __forceinline__ void store_lambda(uint32_t p, uint32_t rf, const int4 cell, const float4 xi,
+                                             float density, float Ci, float gix, float giy, float giz,
+                                             float sum_grad_sq, float4* xout, float* __restrict__ srho,
+                                             int it, const Grid& G, const StepConsts& C) {
     sum_grad_sq += sqn(gix, giy, giz);
-    const float Ci = have_ci ? ci_first : density * C.inv_rho0 - 1.0f;
     const float lam = (Ci < 0.0f) ? 0.0f : -Ci / (sum_grad_sq + C.eps);
-    if constexpr (kCoop) {
-        if (coop && G.dhist && it < kWalkHist &&
-            __any_sync(0xffffffffu, !(Ci < 0.0f)) && (threadIdx.x & 31) == 0)
-            atomicAdd(G.dhist + 2 * kWalkHist + it, 1u);
-    }
     if (G.lamnz && lam != 0.0f) G.lamnz[slot_of(cell.x, cell.y, cell.z, C.grid)] = (uint32_t)it + 1u;
     srho[p] = density;
     xout[p] = make_float4(xi.x, xi.y, xi.z, lam);
@@ -1314,15 +2200,143 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
     }
 }
 
-template <int BS, class P, int U = 4>
+// The density pass for sorted particle p.  Reads x* from xin, writes
+// (x*, lambda) to xout and rho to srho.  Scenes whose `iters` are done by
+// iteration `it` are left untouched.  Warp-collective: every lane of the warp
+// calls it, with `active` false past the last particle.
+template <bool kPersist, class P>
+__device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const float4* xin,
+                                                  float4* xout, float* __restrict__ srho, int it,
+                                                  const Grid& G, const P& prm, WalkSmem& sm) {
+    const uint32_t pa = active ? p : 0u;
+    const StepConsts& C = prm.at(G.spid, pa);
+    const int4 cell = cell_at(G, pa);
+    const uint32_t rf = run_flags(G, pa);
+    bool live = active && it < C.iters && !(rf & kCopyBit);
+    if (live && it > 0 && G.moved && cell.w == 0 &&
+        !neighbourhood_stamped<kPersist>(cell, C.grid, G.moved, (uint32_t)it, 0, 3)) {
+        keep_lambda(p, rf, cell, xin, xout, it, G, C);
+        live = false;
+    }
+    if (!__any_sync(0xffffffffu, live)) return;
+    const float4 xi = xin[pa];
+    float density, gix = 0.0f, giy = 0.0f, giz = 0.0f, sum_grad_sq = 0.0f;
+    // Density first: when C_i < 0 lambda_i is 0 whatever the gradient sums,
+    // so a warp can sum the densities alone (poly6 terms, no square root or
+    // division), then walk again, in the same candidate order, for the
+    // gradients of its lanes with C_i >= 0 only.  Each sum sees the same
+    // terms in the same order as the single walk: same bits.  It pays where
+    // most warps have no such lane; which way a warp goes follows the share
+    // of warps that needed gradients in the same iteration of the last step.
+    constexpr bool kHist = std::is_same<P, OneScene>::value;
+    bool dfirst = false;
+    if constexpr (kHist) {
+        if (G.dhist && it < kWalkHist && !G.bg.spos) {
+            const uint32_t need = __ldg(G.dhist + it), ran = __ldg(G.dhist + kWalkHist + it);
+            dfirst = ran > 0 && 3u * need < ran;
+        }
+    }
+    if (kHist && dfirst) {
+        LaneSums<DensityTerm> ds(DensityTerm{C, xi});
+        sum_candidates<kPersist, false>(sm, G, prm, pa, cell, live, xi, xin, C, ds);
+        density = ds.get(0);
+        const bool want = live && !(density * C.inv_rho0 - 1.0f < 0.0f);
+        LaneSums<GradTerm> gs(GradTerm{C, xi});
+        sum_candidates<kPersist, false>(sm, G, prm, pa, cell, want, xi, xin, C, gs);
+        gix = gs.get(0);
+        giy = gs.get(1);
+        giz = gs.get(2);
+        sum_grad_sq = gs.get(3);
+    } else {
+        LaneSums<DensityGradTerm> sums(DensityGradTerm{C, xi});
+        sum_candidates<kPersist, false>(sm, G, prm, pa, cell, live, xi, xin, C, sums);
+        density = sums.get(0);
+        gix = sums.get(1);
+        giy = sums.get(2);
+        giz = sums.get(3);
+        sum_grad_sq = sums.get(4);
+    }
+    if constexpr (kHist) {
+        if (G.bg.spos) {
+            // Two-way coupling: after the fluid terms, the boundary's in the
+            // boundary index's bucket order.
+            LaneSums<BoundaryDensityTerm> bsums(BoundaryDensityTerm{C, xi});
+            const float from[4] = {density, gix, giy, giz};
+            bsums.start(from);
+            sum_boundary(sm, G, prm, pa, cell, live, xi, C, bsums);
+            density = bsums.get(0);
+            gix = bsums.get(1);
+            giy = bsums.get(2);
+            giz = bsums.get(3);
+        }
+    }
+    const float Ci = density * C.inv_rho0 - 1.0f;
+    if constexpr (kHist) {
+        if (G.dhist && it < kWalkHist) {
+            const bool need = __any_sync(0xffffffffu, live && !(Ci < 0.0f));
+            if ((threadIdx.x & 31) == 0) {
+                atomicAdd(G.dhist + 3 * kWalkHist + it, 1u);
+                if (need) atomicAdd(G.dhist + 2 * kWalkHist + it, 1u);
+            }
+        }
+    }
+    if (live) store_lambda(p, rf, cell, xi, density, Ci, gix, giy, giz, sum_grad_sq, xout, srho, it, G, C);
+}
+
+template <int BS, class P>
 __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
 k_density_lambda(const float4* __restrict__ xin, float4* __restrict__ xout, float* __restrict__ srho,
                  int it, int n, const Grid G, const P prm) {
-    using B = CoopBlock<P, BS, false, U>;
-    __shared__ typename B::Smem sm[B::kWarps];
+    __shared__ WalkSmem sm[BS / 32];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    density_lambda_at<false, U>(p, p < (uint32_t)n, xin, xout, srho, it, G, prm,
-                                sm[B::kOn ? threadIdx.x >> 5 : 0]);
+    density_lambda_at<false>(p, p < (uint32_t)n, xin, xout, srho, it, G, prm, sm[threadIdx.x >> 5]);
+}
+
+template <int TP, class P>
+__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+k_density_lambda_team(const float4* __restrict__ xin, float4* __restrict__ xout,
+                      float* __restrict__ srho, int it, int n, const Grid G, const P prm) {
+    __shared__ TeamSmem<TP> sm;
+    const TeamThread<TP> T(n);
+    const int4 cell = cell_at(G, T.pl);
+    bool live;
+    {
+        const StepConsts& C = prm.at(G.spid, T.pl);
+        live = T.al && it < C.iters;
+        if (it > 0 && G.moved) {
+            const bool ask = live && cell.w == 0;
+            const bool near = team_stamped(sm, ask, cell, C.grid, G.moved, (uint32_t)it);
+            if (ask && !near) {
+                if (threadIdx.x < 32u && threadIdx.x % (32u / TP) == 0u)
+                    keep_lambda(T.pl, 0u, cell, xin, xout, it, G, C);
+                live = false;
+            }
+        }
+    }
+    if (!__any_sync(0xffffffffu, live)) return;
+    const bool elive = T.hand_over(sm, live);
+    const StepConsts& C = prm.at(G.spid, T.pe);
+    const float4 xl = xin[T.pl], xi = xin[T.pe];
+    TeamSums<DensityGradTerm, 128 / TP> sums(DensityGradTerm{C, xi});
+    team_walk<TP, false>(sm, G, fluid_index(G), prm, T.pl, cell, live, xl, xin, sums);
+    float density = sums.get(0), gix = sums.get(1), giy = sums.get(2), giz = sums.get(3);
+    const float sum_grad_sq = sums.get(4);
+    if constexpr (std::is_same<P, OneScene>::value) {
+        if (G.bg.spos) {
+            TeamSums<BoundaryDensityTerm, 128 / TP> bsums(BoundaryDensityTerm{C, xi});
+            const float from[4] = {density, gix, giy, giz};
+            bsums.start(from);
+            team_walk<TP, false>(sm, G, boundary_index(G), prm, T.pl, boundary_cell(G, T.pl, cell), live, xl,
+                                 G.bg.spos, bsums);
+            density = bsums.get(0);
+            gix = bsums.get(1);
+            giy = bsums.get(2);
+            giz = bsums.get(3);
+        }
+    }
+    if (elive && T.writer)
+        store_lambda(T.pe, 0u, cell_at(G, T.pe), xi, density, density * C.inv_rho0 - 1.0f, gix, giy, giz,
+                     sum_grad_sq, xout, srho, it, G, C);
 }
 
 // Velocity update with speed clamp (pbf_solver.cpp:81-93) for sorted p; w is
@@ -1343,92 +2357,12 @@ __device__ __forceinline__ float4 update_velocity(float px, float py, float pz, 
     return make_float4(a, b, c, C.mass / rho_j);
 }
 
-// compute_delta_position + apply_delta (pbf_solver.cpp:181-223, :74-76) for
-// sorted particle p.  Reads (x*, lambda) from xin, writes (x* + dp, lambda_i)
-// to xout; on the scene's last iteration also the updated velocity into sv.
-// Warp-collective like density_lambda_at.
-template <bool kPersist, int U, class P, int CH>
-__device__ __forceinline__ void delta_at(uint32_t p, bool active, const float4* xin, float4* xout,
-                                         const float4* __restrict__ sx,
-                                         const float* __restrict__ srho, float4* __restrict__ sv,
-                                         int it, const Grid& G, const P& prm,
-                                         CoopSmem<CH, false>& sm) {
-    constexpr bool kCoop = CoopBlock<P, 32, false, U>::kOn;
-    const uint32_t pa = active ? p : 0u;
-    const StepConsts& C = prm.at(G.spid, pa);
-    const int4 cell = cell_at(G, pa);
-    const uint32_t rf = run_flags(G, pa);
-    const bool live = active && it < C.iters && !(rf & kCopyBit);
-    float4 xi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-    bool walk = live;
-    if (live) {
-        xi = xin[p];
-        // A clean particle with a zero lambda whose 27 cells hold no nonzero
-        // lambda in this iteration has only zero terms: no walk.
-        if (G.lamnz && cell.w == 0 && xi.w == 0.0f &&
-            !neighbourhood_moved<kPersist>(cell, C.grid, G.lamnz, it + 1))
-            walk = false;
-    }
-    // The warp walks cooperatively when every lane is live, even if only
-    // some need the walk: the others have only zero terms, which the walk's
-    // lambda test leaves out, so they list nothing.
-    CoopRow R;
-    bool coop = false;
-    if constexpr (kCoop) coop = coop_row(live, cell, C.grid, R, scene_at(G, pa));
-    if (!live) return;
-    float dx = 0.0f, dy = 0.0f, dz = 0.0f;
-    auto term = [&](const float4& xj, auto L) {
-        float rx, ry, rz, lambda_sum;
-        const float r_sq = rel_sq<true>(xi, xj, rx, ry, rz, &lambda_sum);
-        // A zero lambda sum adds an exact zero (no s_corr either); the sum,
-        // started at +0, never becomes -0, so skipping it keeps every bit.
-        if (r_sq < C.cut && lambda_sum != 0.0f) {
-            float s_corr = 0.0f;
-            if (lambda_sum < -1e-10f && C.scorr_on) {
-                float ratio = poly6(r_sq, C) / C.w_dq;
-                ratio = (1.0f < ratio) ? 1.0f : ratio;
-                float rp = ratio * ratio;
-                if (C.corr_n4) rp = rp * rp;
-                s_corr = C.neg_corr_k * rp;
-            }
-            const float c = spiky_coeff(r_sq, C);
-            const float a = (lambda_sum + s_corr) * C.mass;
-            dx = acc(dx, a * (c * rx), L);
-            dy = acc(dy, a * (c * ry), L);
-            dz = acc(dz, a * (c * rz), L);
-        }
-    };
-    if constexpr (kCoop) {
-        if (coop && __any_sync(0xffffffffu, walk)) {
-            coop_walk<CH, false, kPersist, true, false>(
-                sm, R, cell.x, xi, xin, C.cut, C.grid, G.off,
-                [](uint32_t) { return float4{}; },
-                [&](const float4& xj, const float4&) { term(xj, One{}); },
-                [&](const float4& xj, const float4&, uint32_t L) { term(xj, L); });
-        }
-    }
-    if (walk && !coop)
-        for_each_candidate_runs<U, std::is_same<P, OneScene>::value>(
-            cell, G, C, [&](uint32_t q) { term(ld_step<kPersist>(xin + q), One{}); },
-            [&](uint32_t q, uint32_t L) { term(ld_step<kPersist>(xin + q), Many{L}); });
-    if (G.bg.spos && xi.w != 0.0f) {
-        // Two-way coupling: the boundary's share of the position correction,
-        // lambda_i (rho0 psi_b) grad W, after the fluid terms (zero when
-        // lambda_i is).
-        for_each_candidate<4>(boundary_cell(G, p, cell), G.bg.off, G.bg.kpos, G.bg.bend,
-                              G.bg.btab, C, [&](uint32_t q) {
-                                  const float4 b = __ldg(G.bg.spos + q);
-                                  const float rx = xi.x - b.x, ry = xi.y - b.y, rz = xi.z - b.z;
-                                  const float r_sq = sqn(rx, ry, rz);
-                                  if (r_sq < C.cut) {
-                                      const float c = spiky_coeff(r_sq, C);
-                                      const float a = xi.w * (C.rho0 * b.w);
-                                      dx += a * (c * rx);
-                                      dy += a * (c * ry);
-                                      dz += a * (c * rz);
-                                  }
-                              });
-    }
+// What the delta pass writes for particle p and the rest of its run: (x* + dp,
+// lambda) and, on the scene's last iteration, the updated velocity.
+__device__ __forceinline__ void store_delta(uint32_t p, uint32_t rf, const int4 cell, const float4 xi, float dx,
+                                            float dy, float dz, float4* xout, const float4* __restrict__ sx,
+                                            const float* __restrict__ srho, float4* __restrict__ sv, int it,
+                                            const Grid& G, const StepConsts& C) {
     const float px = xi.x + dx * C.inv_rho0;
     const float py = xi.y + dy * C.inv_rho0;
     const float pz = xi.z + dz * C.inv_rho0;
@@ -1445,16 +2379,96 @@ __device__ __forceinline__ void delta_at(uint32_t p, bool active, const float4* 
     }
 }
 
-template <int BS, class P, int U = 4>
+// compute_delta_position + apply_delta (pbf_solver.cpp:181-223, :74-76) for
+// sorted particle p.  Reads (x*, lambda) from xin, writes (x* + dp, lambda_i)
+// to xout; on the scene's last iteration also the updated velocity into sv.
+// Warp-collective like density_lambda_at.
+template <bool kPersist, class P>
+__device__ __forceinline__ void delta_at(uint32_t p, bool active, const float4* xin, float4* xout,
+                                         const float4* __restrict__ sx,
+                                         const float* __restrict__ srho, float4* __restrict__ sv,
+                                         int it, const Grid& G, const P& prm, WalkSmem& sm) {
+    const uint32_t pa = active ? p : 0u;
+    const StepConsts& C = prm.at(G.spid, pa);
+    const int4 cell = cell_at(G, pa);
+    const uint32_t rf = run_flags(G, pa);
+    const bool live = active && it < C.iters && !(rf & kCopyBit);
+    float4 xi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (live) xi = xin[p];
+    bool walk = live;
+    // A clean particle with a zero lambda whose 27 cells hold no nonzero
+    // lambda in this iteration has only zero terms: no walk.
+    if (live && G.lamnz && cell.w == 0 && xi.w == 0.0f &&
+        !neighbourhood_stamped<kPersist>(cell, C.grid, G.lamnz, (uint32_t)it + 1u, 0, 3))
+        walk = false;
+    LaneSums<DeltaTerm> sums(DeltaTerm{C, xi});
+    sum_candidates<kPersist, true>(sm, G, prm, pa, cell, walk, xi, xin, C, sums);
+    float dx = sums.get(0), dy = sums.get(1), dz = sums.get(2);
+    if constexpr (std::is_same<P, OneScene>::value) {
+        if (G.bg.spos) {
+            // Two-way coupling: the boundary's share after the fluid terms
+            // (zero when lambda_i is).
+            LaneSums<BoundaryDeltaTerm> bsums(BoundaryDeltaTerm{C, xi});
+            const float from[3] = {dx, dy, dz};
+            bsums.start(from);
+            sum_boundary(sm, G, prm, pa, cell, live && xi.w != 0.0f, xi, C, bsums);
+            dx = bsums.get(0);
+            dy = bsums.get(1);
+            dz = bsums.get(2);
+        }
+    }
+    if (live) store_delta(p, rf, cell, xi, dx, dy, dz, xout, sx, srho, sv, it, G, C);
+}
+
+template <int BS, class P>
 __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
 k_delta(const float4* __restrict__ xin, float4* __restrict__ xout, const float4* __restrict__ sx,
         const float* __restrict__ srho, float4* __restrict__ sv, int it, int n, const Grid G,
         const P prm) {
-    using B = CoopBlock<P, BS, false, U>;
-    __shared__ typename B::Smem sm[B::kWarps];
+    __shared__ WalkSmem sm[BS / 32];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    delta_at<false, U>(p, p < (uint32_t)n, xin, xout, sx, srho, sv, it, G, prm,
-                       sm[B::kOn ? threadIdx.x >> 5 : 0]);
+    delta_at<false>(p, p < (uint32_t)n, xin, xout, sx, srho, sv, it, G, prm, sm[threadIdx.x >> 5]);
+}
+
+template <int TP, class P>
+__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+k_delta_team(const float4* __restrict__ xin, float4* __restrict__ xout, const float4* __restrict__ sx,
+             const float* __restrict__ srho, float4* __restrict__ sv, int it, int n, const Grid G,
+             const P prm) {
+    __shared__ TeamSmem<TP> sm;
+    const TeamThread<TP> T(n);
+    const int4 cell = cell_at(G, T.pl);
+    const float4 xl = xin[T.pl];
+    bool live, walk;
+    {
+        const StepConsts& C = prm.at(G.spid, T.pl);
+        live = walk = T.al && it < C.iters;
+        if (G.lamnz) {
+            const bool ask = live && cell.w == 0 && xl.w == 0.0f;
+            const bool near = team_stamped(sm, ask, cell, C.grid, G.lamnz, (uint32_t)it + 1u);
+            if (ask && !near) walk = false;
+        }
+    }
+    const StepConsts& C = prm.at(G.spid, T.pe);
+    const float4 xi = xin[T.pe];
+    TeamSums<DeltaTerm, 128 / TP> sums(DeltaTerm{C, xi});
+    __syncthreads();
+    team_walk<TP, true>(sm, G, fluid_index(G), prm, T.pl, cell, walk, xl, xin, sums);
+    float dx = sums.get(0), dy = sums.get(1), dz = sums.get(2);
+    if constexpr (std::is_same<P, OneScene>::value) {
+        if (G.bg.spos) {
+            TeamSums<BoundaryDeltaTerm, 128 / TP> bsums(BoundaryDeltaTerm{C, xi});
+            const float from[3] = {dx, dy, dz};
+            bsums.start(from);
+            team_walk<TP, false>(sm, G, boundary_index(G), prm, T.pl, boundary_cell(G, T.pl, cell),
+                                 live && xl.w != 0.0f, xl, G.bg.spos, bsums);
+            dx = bsums.get(0);
+            dy = bsums.get(1);
+            dz = bsums.get(2);
+        }
+    }
+    if (T.writer && it < C.iters)
+        store_delta(T.pe, 0u, cell_at(G, T.pe), xi, dx, dy, dz, xout, sx, srho, sv, it, G, C);
 }
 
 // ---------------------------------------------------------------------------
@@ -1511,25 +2525,24 @@ __device__ __forceinline__ bool grid_sync(const GridSync& S) {
 }
 
 template <class P>
-__global__ void __launch_bounds__(kBlock)
+__global__ void __launch_bounds__(kBlock, kPassMinBlocks<kBlock>)
 k_iterate(float4* xa, float4* xb, float* __restrict__ srho, const float4* __restrict__ sx,
           float4* __restrict__ sv, int max_iters, int n, const Grid G, const P prm,
           const GridSync S) {
-    using B = CoopBlock<P, kBlock, false, 4>;
-    __shared__ typename B::Smem sm[B::kWarps];
+    __shared__ WalkSmem sm[kBlock / 32];
     const uint32_t stride = gridDim.x * blockDim.x;
     // The warp strides as a whole, so that its lanes meet in every
     // warp-collective pass call.
     const uint32_t lane = threadIdx.x & 31u;
     const uint32_t w0 = blockIdx.x * blockDim.x + (threadIdx.x & ~31u);
-    auto& my = sm[B::kOn ? threadIdx.x >> 5 : 0];
+    auto& my = sm[threadIdx.x >> 5];
     for (int it = 0; it < max_iters; ++it) {
         for (uint32_t pw = w0; pw < (uint32_t)n; pw += stride)
-            density_lambda_at<true, 4>(pw + lane, pw + lane < (uint32_t)n, xa, xb, srho, it, G,
+            density_lambda_at<true>(pw + lane, pw + lane < (uint32_t)n, xa, xb, srho, it, G,
                                        prm, my);
         if (!grid_sync(S)) return;
         for (uint32_t pw = w0; pw < (uint32_t)n; pw += stride)
-            delta_at<true, 4>(pw + lane, pw + lane < (uint32_t)n, xb, xa, sx, srho, sv, it, G,
+            delta_at<true>(pw + lane, pw + lane < (uint32_t)n, xb, xa, sx, srho, sv, it, G,
                               prm, my);
         if (it + 1 < max_iters && !grid_sync(S)) return;
     }
@@ -1612,56 +2625,13 @@ k_boundary_friction(const float4* __restrict__ xin, float4* __restrict__ sv, int
 
 // apply_xsph_viscosity (pbf_solver.cpp:225-250) + commit, no vorticity.
 // With skip_vort set, scenes with vorticity are left to the vorticity pair.
-template <int BS, class P, int U = 4>
-__global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
-k_xsph_commit(const float4* __restrict__ xin, const float4* __restrict__ sv, const float4* __restrict__ sx,
-              const float* __restrict__ srho, int n, int skip_vort, const Grid G, const P prm) {
-    using B = CoopBlock<P, BS, true, U>;
-    __shared__ typename B::Smem sm[B::kWarps];
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = p < (uint32_t)n;
-    const uint32_t pa = active ? p : 0u;
-    const StepConsts& C = prm.at(G.spid, pa);
-    const int4 cell = cell_at(G, pa);
-    const uint32_t rf = run_flags(G, pa);
-    const bool live = active && !(skip_vort && C.vort_on) && !(rf & kCopyBit);
-    CoopRow R;
-    bool coop = false;
-    if constexpr (B::kOn) coop = coop_row(live && C.xsph_on, cell, C.grid, R, scene_at(G, pa));
-    if (!live) return;
-    const float4 xi = xin[p];
-    const float4 vi = sv[p];
+template <class P>
+__device__ __forceinline__ void store_xsph(uint32_t p, uint32_t rf, const float4 xi, const float4 vi, float cx,
+                                           float cy, float cz, const float4* __restrict__ sx,
+                                           const float* __restrict__ srho, int n, const Grid& G, const P& prm,
+                                           const StepConsts& C) {
     float vx = vi.x, vy = vi.y, vz = vi.z;
     if (C.xsph_on) {
-        float cx = 0.0f, cy = 0.0f, cz = 0.0f;
-        auto term = [&](const float4& xj, const float4& vj, auto L) {
-            float rx, ry, rz;
-            const float r_sq = rel_sq(xi, xj, rx, ry, rz);
-            if (r_sq < C.h2) {
-                const float w = poly6(r_sq, C);
-                cx = acc(cx, vj.w * (vj.x - vi.x) * w, L);
-                cy = acc(cy, vj.w * (vj.y - vi.y) * w, L);
-                cz = acc(cz, vj.w * (vj.z - vi.z) * w, L);
-            }
-        };
-        if constexpr (B::kOn) {
-            if (coop)
-                coop_walk<coop_chunk(BS), true, false, false, true>(
-                    sm[threadIdx.x >> 5], R, cell.x, xi, xin, C.h2, C.grid, G.off,
-                    [&](uint32_t q) { return __ldg(sv + q); },
-                    [&](const float4& xj, const float4& vj) { term(xj, vj, One{}); },
-                    [&](const float4& xj, const float4& vj, uint32_t L) { term(xj, vj, L); });
-        }
-        if (!coop) {
-            auto one = [&](uint32_t q, auto L) {
-                const float4 xj = __ldg(xin + q);
-                float rx, ry, rz;
-                if (rel_sq(xi, xj, rx, ry, rz) < C.h2) term(xj, __ldg(sv + q), L);
-            };
-            for_each_candidate_runs<U, false>(
-                cell, G, C, [&](uint32_t q) { one(q, One{}); },
-                [&](uint32_t q, uint32_t L) { one(q, L); });
-        }
         vx = vi.x + C.xsph_c * cx;
         vy = vi.y + C.xsph_c * cy;
         vz = vi.z + C.xsph_c * cz;
@@ -1670,66 +2640,52 @@ k_xsph_commit(const float4* __restrict__ xin, const float4* __restrict__ sv, con
         commit(m, xi.x, xi.y, xi.z, vx, vy, vz, xi.w, sx, srho, prm.state(G.spid, m), n, C);
 }
 
-// XSPH correction + vorticity omega in one candidate pass (vorticity path).
-// Writes the post-XSPH velocity to sv2 and (omega, |omega|) to som, with
-//   omega_i = sum_j (m/rho_j') spiky_grad(x*_i - x*_j) x (v_j - v_i),
-// the SPH curl (Macklin & Mueller 2013, section 5, with its volume factor).
-template <int BS, class P, int U = 4>
+template <int BS, class P>
 __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
-k_xsph_omega(const float4* __restrict__ xin, const float4* __restrict__ sv, float4* __restrict__ sv2,
-             float4* __restrict__ som, int n, const Grid G, const P prm) {
-    using B = CoopBlock<P, BS, true, U>;
-    __shared__ typename B::Smem sm[B::kWarps];
+k_xsph_commit(const float4* __restrict__ xin, const float4* __restrict__ sv, const float4* __restrict__ sx,
+              const float* __restrict__ srho, int n, int skip_vort, const Grid G, const P prm) {
+    __shared__ WalkSmem sm[BS / 32];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = p < (uint32_t)n;
     const uint32_t pa = active ? p : 0u;
     const StepConsts& C = prm.at(G.spid, pa);
     const int4 cell = cell_at(G, pa);
     const uint32_t rf = run_flags(G, pa);
-    const bool live = active && C.vort_on && !(rf & kCopyBit);
-    CoopRow R;
-    bool coop = false;
-    if constexpr (B::kOn) coop = coop_row(live, cell, C.grid, R, scene_at(G, pa));
-    if (!live) return;
-    const float4 xi = xin[p];
-    const float4 vi = sv[p];
-    float cx = 0.0f, cy = 0.0f, cz = 0.0f, wx = 0.0f, wy = 0.0f, wz = 0.0f;
-    auto term = [&](const float4& xj, const float4& vj, auto L) {
-        float rx, ry, rz;
-        const float r_sq = rel_sq(xi, xj, rx, ry, rz);
-        if (r_sq < C.cut) {
-            const float ux = vj.x - vi.x;
-            const float uy = vj.y - vi.y;
-            const float uz = vj.z - vi.z;
-            const float w = poly6(r_sq, C);
-            cx = acc(cx, vj.w * ux * w, L);
-            cy = acc(cy, vj.w * uy * w, L);
-            cz = acc(cz, vj.w * uz * w, L);
-            const float c = spiky_coeff(r_sq, C);
-            const float gx = c * rx, gy = c * ry, gz = c * rz;
-            wx = acc(wx, vj.w * (gy * uz - gz * uy), L);
-            wy = acc(wy, vj.w * (gz * ux - gx * uz), L);
-            wz = acc(wz, vj.w * (gx * uy - gy * ux), L);
-        }
-    };
-    if constexpr (B::kOn) {
-        if (coop)
-            coop_walk<coop_chunk(BS), true, false, false, true>(
-                sm[threadIdx.x >> 5], R, cell.x, xi, xin, C.cut, C.grid, G.off,
-                [&](uint32_t q) { return __ldg(sv + q); },
-                [&](const float4& xj, const float4& vj) { term(xj, vj, One{}); },
-                [&](const float4& xj, const float4& vj, uint32_t L) { term(xj, vj, L); });
+    const bool live = active && !(skip_vort && C.vort_on) && !(rf & kCopyBit);
+    const float4 xi = xin[pa];
+    const float4 vi = sv[pa];
+    LaneSums<XsphTerm> sums(XsphTerm{C, xi, vi, sv});
+    sum_candidates<false, false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live && C.xsph_on, xi, xin, C, sums);
+    if (live) store_xsph(p, rf, xi, vi, sums.get(0), sums.get(1), sums.get(2), sx, srho, n, G, prm, C);
+}
+
+template <int TP, class P>
+__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+k_xsph_commit_team(const float4* __restrict__ xin, const float4* __restrict__ sv,
+                   const float4* __restrict__ sx, const float* __restrict__ srho, int n, int skip_vort,
+                   const Grid G, const P prm) {
+    __shared__ TeamSmem<TP> sm;
+    const TeamThread<TP> T(n);
+    bool want;
+    {
+        const StepConsts& C = prm.at(G.spid, T.pl);
+        want = T.al && !(skip_vort && C.vort_on) && C.xsph_on;
     }
-    if (!coop) {
-        auto one = [&](uint32_t q, auto L) {
-            const float4 xj = __ldg(xin + q);
-            float rx, ry, rz;
-            if (rel_sq(xi, xj, rx, ry, rz) < C.cut) term(xj, __ldg(sv + q), L);
-        };
-        for_each_candidate_runs<U, false>(
-            cell, G, C, [&](uint32_t q) { one(q, One{}); },
-            [&](uint32_t q, uint32_t L) { one(q, L); });
-    }
+    const StepConsts& C = prm.at(G.spid, T.pe);
+    const float4 xi = xin[T.pe];
+    const float4 vi = sv[T.pe];
+    TeamSums<XsphTerm, 128 / TP> sums(XsphTerm{C, xi, vi, sv});
+    team_walk<TP, false>(sm, G, fluid_index(G), prm, T.pl, cell_at(G, T.pl), want, xin[T.pl], xin, sums);
+    const float cx = sums.get(0), cy = sums.get(1), cz = sums.get(2);
+    if (T.writer && !(skip_vort && C.vort_on))
+        store_xsph(T.pe, 0u, xi, vi, cx, cy, cz, sx, srho, n, G, prm, C);
+}
+
+// XSPH correction + vorticity omega in one candidate pass (vorticity path).
+// Writes the post-XSPH velocity to sv2 and (omega, |omega|) to som.
+__device__ __forceinline__ void store_omega(uint32_t p, uint32_t rf, const float4 vi, float cx, float cy,
+                                            float cz, float wx, float wy, float wz, float4* __restrict__ sv2,
+                                            float4* __restrict__ som, const Grid& G, const StepConsts& C) {
     float vx = vi.x, vy = vi.y, vz = vi.z;
     if (C.xsph_on) {
         vx = vi.x + C.xsph_c * cx;
@@ -1743,17 +2699,11 @@ k_xsph_omega(const float4* __restrict__ xin, const float4* __restrict__ sv, floa
     }
 }
 
-// Vorticity confinement (Macklin & Mueller 2013, section 5) + commit:
-//   eta_i = sum_j (m/rho_j') (|omega_j| - |omega_i|) spiky_grad(x*_i - x*_j),
-//   N = eta / |eta|,  v += dt * eps * (N x omega_i).
-template <int BS, class P, int U = 4>
+template <int BS, class P>
 __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
-k_vorticity_commit(const float4* __restrict__ xin, const float4* __restrict__ sv,
-                   const float4* __restrict__ sv2, const float4* __restrict__ som,
-                   const float4* __restrict__ sx, const float* __restrict__ srho, int n,
-                   const Grid G, const P prm) {
-    using B = CoopBlock<P, BS, true, U>;
-    __shared__ typename B::Smem sm[B::kWarps];
+k_xsph_omega(const float4* __restrict__ xin, const float4* __restrict__ sv, float4* __restrict__ sv2,
+             float4* __restrict__ som, int n, const Grid G, const P prm) {
+    __shared__ WalkSmem sm[BS / 32];
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = p < (uint32_t)n;
     const uint32_t pa = active ? p : 0u;
@@ -1761,46 +2711,41 @@ k_vorticity_commit(const float4* __restrict__ xin, const float4* __restrict__ sv
     const int4 cell = cell_at(G, pa);
     const uint32_t rf = run_flags(G, pa);
     const bool live = active && C.vort_on && !(rf & kCopyBit);
-    CoopRow R;
-    bool coop = false;
-    if constexpr (B::kOn) coop = coop_row(live, cell, C.grid, R, scene_at(G, pa));
-    if (!live) return;
-    const float4 xi = xin[p];
+    const float4 xi = xin[pa];
+    const float4 vi = sv[pa];
+    LaneSums<XsphOmegaTerm> sums(XsphOmegaTerm{C, xi, vi, sv});
+    sum_candidates<false, false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live, xi, xin, C, sums);
+    if (live)
+        store_omega(p, rf, vi, sums.get(0), sums.get(1), sums.get(2), sums.get(3), sums.get(4), sums.get(5),
+                    sv2, som, G, C);
+}
+
+template <int TP, class P>
+__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+k_xsph_omega_team(const float4* __restrict__ xin, const float4* __restrict__ sv, float4* __restrict__ sv2,
+                  float4* __restrict__ som, int n, const Grid G, const P prm) {
+    __shared__ TeamSmem<TP> sm;
+    const TeamThread<TP> T(n);
+    const bool want = T.al && prm.at(G.spid, T.pl).vort_on;
+    const StepConsts& C = prm.at(G.spid, T.pe);
+    const float4 xi = xin[T.pe];
+    const float4 vi = sv[T.pe];
+    TeamSums<XsphOmegaTerm, 128 / TP> sums(XsphOmegaTerm{C, xi, vi, sv});
+    team_walk<TP, false>(sm, G, fluid_index(G), prm, T.pl, cell_at(G, T.pl), want, xin[T.pl], xin, sums);
+    const float cx = sums.get(0), cy = sums.get(1), cz = sums.get(2);
+    const float wx = sums.get(3), wy = sums.get(4), wz = sums.get(5);
+    if (T.writer && C.vort_on) store_omega(T.pe, 0u, vi, cx, cy, cz, wx, wy, wz, sv2, som, G, C);
+}
+
+// Vorticity confinement (Macklin & Mueller 2013, section 5) + commit:
+//   N = eta / |eta|,  v += dt * eps * (N x omega_i).
+template <class P>
+__device__ __forceinline__ void store_vorticity(uint32_t p, uint32_t rf, const float4 xi, float ex, float ey,
+                                                float ez, const float4* __restrict__ sv2,
+                                                const float4* __restrict__ som, const float4* __restrict__ sx,
+                                                const float* __restrict__ srho, int n, const Grid& G,
+                                                const P& prm, const StepConsts& C) {
     const float4 wi = som[p];
-    float ex = 0.0f, ey = 0.0f, ez = 0.0f;
-    // e = (m / rho_j', |omega_j|) of the candidate.
-    auto term = [&](const float4& xj, const float4& e, auto L) {
-        float rx, ry, rz;
-        const float r_sq = rel_sq(xi, xj, rx, ry, rz);
-        if (r_sq < C.cut) {
-            const float c = spiky_coeff(r_sq, C);
-            const float a = e.x * (e.y - wi.w);
-            ex = acc(ex, a * (c * rx), L);
-            ey = acc(ey, a * (c * ry), L);
-            ez = acc(ez, a * (c * rz), L);
-        }
-    };
-    if constexpr (B::kOn) {
-        if (coop)
-            coop_walk<coop_chunk(BS), true, false, false, true>(
-                sm[threadIdx.x >> 5], R, cell.x, xi, xin, C.cut, C.grid, G.off,
-                [&](uint32_t q) {
-                    return make_float4(__ldg(sv + q).w, __ldg(som + q).w, 0.0f, 0.0f);
-                },
-                [&](const float4& xj, const float4& e) { term(xj, e, One{}); },
-                [&](const float4& xj, const float4& e, uint32_t L) { term(xj, e, L); });
-    }
-    if (!coop) {
-        auto one = [&](uint32_t q, auto L) {
-            const float4 xj = __ldg(xin + q);
-            float rx, ry, rz;
-            if (rel_sq(xi, xj, rx, ry, rz) < C.cut)
-                term(xj, make_float4(__ldg(sv + q).w, __ldg(som + q).w, 0.0f, 0.0f), L);
-        };
-        for_each_candidate_runs<U, false>(
-            cell, G, C, [&](uint32_t q) { one(q, One{}); },
-            [&](uint32_t q, uint32_t L) { one(q, L); });
-    }
     const float el = sqrtf(sqn(ex, ey, ez));
     float nx = 0.0f, ny = 0.0f, nz = 0.0f;
     if (el > 1e-9f) {
@@ -1817,6 +2762,45 @@ k_vorticity_commit(const float4* __restrict__ xin, const float4* __restrict__ sv
     const float vz = vb.z + C.vort_scale * fz;
     for (uint32_t m = p, e = run_end(G, p, rf); m < e; ++m)
         commit(m, xi.x, xi.y, xi.z, vx, vy, vz, xi.w, sx, srho, prm.state(G.spid, m), n, C);
+}
+
+template <int BS, class P>
+__global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
+k_vorticity_commit(const float4* __restrict__ xin, const float4* __restrict__ sv,
+                   const float4* __restrict__ sv2, const float4* __restrict__ som,
+                   const float4* __restrict__ sx, const float* __restrict__ srho, int n,
+                   const Grid G, const P prm) {
+    __shared__ WalkSmem sm[BS / 32];
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool active = p < (uint32_t)n;
+    const uint32_t pa = active ? p : 0u;
+    const StepConsts& C = prm.at(G.spid, pa);
+    const int4 cell = cell_at(G, pa);
+    const uint32_t rf = run_flags(G, pa);
+    const bool live = active && C.vort_on && !(rf & kCopyBit);
+    const float4 xi = xin[pa];
+    LaneSums<VorticityTerm> sums(VorticityTerm{C, xi, som[pa].w, sv, som});
+    sum_candidates<false, false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live, xi, xin, C, sums);
+    if (live)
+        store_vorticity(p, rf, xi, sums.get(0), sums.get(1), sums.get(2), sv2, som, sx, srho, n, G, prm, C);
+}
+
+template <int TP, class P>
+__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+k_vorticity_commit_team(const float4* __restrict__ xin, const float4* __restrict__ sv,
+                        const float4* __restrict__ sv2, const float4* __restrict__ som,
+                        const float4* __restrict__ sx, const float* __restrict__ srho, int n, const Grid G,
+                        const P prm) {
+    __shared__ TeamSmem<TP> sm;
+    const TeamThread<TP> T(n);
+    const bool want = T.al && prm.at(G.spid, T.pl).vort_on;
+    const StepConsts& C = prm.at(G.spid, T.pe);
+    const float4 xi = xin[T.pe];
+    TeamSums<VorticityTerm, 128 / TP> sums(VorticityTerm{C, xi, som[T.pe].w, sv, som});
+    team_walk<TP, false>(sm, G, fluid_index(G), prm, T.pl, cell_at(G, T.pl), want, xin[T.pl], xin, sums);
+    const float ex = sums.get(0), ey = sums.get(1), ez = sums.get(2);
+    if (T.writer && C.vort_on)
+        store_vorticity(T.pe, 0u, xi, ex, ey, ez, sv2, som, sx, srho, n, G, prm, C);
 }
 
 // ---------------------------------------------------------------------------
@@ -1923,31 +2907,29 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
 // cell-sorted particles for `max_iters` iterations, with constants from `prm`.
 // Scenes with vorticity take the XSPH+omega / vorticity+commit pair
 // (any_vort), the others XSPH+commit (any_plain).
-// XSPH (+ vorticity) and commit passes with the row loop unrolled U ways.
-template <int BS, int U, class P>
-inline void enqueue_tail(const StepBuffers& B, const Grid& G, const P& prm, int n, int nb,
-                         bool any_vort, bool any_plain, bool xsph_on, cudaStream_t st,
-                         PhaseMarks* pm) {
-    if (any_vort) {
-        k_xsph_omega<BS, P, U><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
-        if (pm) pm->mark(kPhaseXsph, 1, st);
-        k_vorticity_commit<BS, P, U><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho,
-                                                        n, G, prm);
-        if (pm) pm->mark(kPhaseCommit, 1, st);
-    }
-    if (any_plain) {
-        k_xsph_commit<BS, P, U><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n,
-                                                   any_vort ? 1 : 0, G, prm);
-        if (pm) pm->mark(xsph_on ? kPhaseXsph : kPhaseCommit, 1, st);
-    }
+// Particles per team of the neighbour passes, 0 for warp walks, by the number
+// of particles of the launch.  A warp walk of one lane per particle needs
+// some 130,000 particles to keep the chip's 608 schedulers in work; below
+// that its time is that of one warp's chain.  Measured (exact build, times of
+// a whole pass of calls, us, teams of 8 / 16 / 32 / warp walks): 1,000
+// particles at h = 2 r 193 / 238 / 341 / 604; 8,000 at 4 r 365 / 368 / 464 /
+// 992; four steps of 43,993 4,609 / 4,565 / 7,289 / 11,318; 65,565 (fast
+// build) 2,237 / 2,002 / 2,607 / 3,684; a batch of 352,901 5,171 / 3,993 /
+// 4,061 / 3,519.  Teams of 32 were never the fastest and are not built.
+inline int team_size(int n) {
+    if (n < 8192) return 8;
+    if (n < kBigScene) return 16;
+    return 0;
 }
 
-template <int BS, class P>
+// TP: particles per team, 0 for warps of 32 particles in blocks of BS threads.
+template <int BS, int TP, class P>
 inline cudaError_t enqueue_passes_bs(const StepBuffers& B, const Grid& G, int n, int max_iters,
                                      bool any_zero_iters, bool any_vort, bool any_plain,
                                      bool xsph_on, const P prm, cudaStream_t st, PhaseMarks* pm,
                                      int persist_blocks, unsigned int* barrier) {
-    const int nb = grid_of(n, BS);
+    constexpr int T = TP ? TP : 32;
+    const int nb = TP ? grid_of(n, T) : grid_of(n, BS);
     if (persist_blocks > 0 && barrier && max_iters > 0) {
         // The whole Jacobi loop as one cooperative launch.
         cudaError_t e = cudaMemsetAsync(barrier, 0, sizeof(unsigned int), st);
@@ -1967,46 +2949,48 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, const Grid& G, int n,
         if (e != cudaSuccess) return e;
         if (pm) pm->mark(kPhaseDensity, 1, st);
     } else {
-        bool big = false;
-        if constexpr (std::is_same<P, OneScene>::value) big = n >= kBigScene;
         for (int it = 0; it < max_iters; ++it) {
-            if constexpr (std::is_same<P, OneScene>::value) {
-                if (big)
-                    k_density_lambda<BS, P, 8><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
-                else
-                    k_density_lambda<BS, P, 4><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
-            } else {
-                k_density_lambda<BS, P, 4><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
-            }
+            if constexpr (TP != 0)
+                k_density_lambda_team<T><<<nb, 128, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
+            else
+                k_density_lambda<BS><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
             if (pm) pm->mark(kPhaseDensity, 1, st);
-            if constexpr (std::is_same<P, OneScene>::value) {
-                if (big)
-                    k_delta<BS, P, 8><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
-                else
-                    k_delta<BS, P, 4><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
-            } else {
-                k_delta<BS, P, 4><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
-            }
+            if constexpr (TP != 0)
+                k_delta_team<T><<<nb, 128, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
+            else
+                k_delta<BS><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
             if (pm) pm->mark(kPhaseDelta, 1, st);
         }
     }
     if (any_zero_iters) {
-        k_velocity<BS><<<nb, BS, 0, st>>>(B.xa, B.sx, B.srho, B.sv, n, G, prm);
+        k_velocity<BS><<<grid_of(n, BS), BS, 0, st>>>(B.xa, B.sx, B.srho, B.sv, n, G, prm);
         if (pm) pm->mark(kPhaseDelta, 1, st);
     }
     if constexpr (std::is_same<P, OneScene>::value) {
         if (G.bg.spos && prm.C.bfric != 0.0f) {
-            k_boundary_friction<<<nb, BS, 0, st>>>(B.xa, B.sv, n, G, prm.C);
+            k_boundary_friction<<<grid_of(n, BS), BS, 0, st>>>(B.xa, B.sv, n, G, prm.C);
             if (pm) pm->mark(kPhaseXsph, 1, st);
         }
     }
-    if constexpr (std::is_same<P, OneScene>::value) {
-        if (n >= kBigScene)
-            enqueue_tail<BS, 8>(B, G, prm, n, nb, any_vort, any_plain, xsph_on, st, pm);
+    if (any_vort) {
+        if constexpr (TP != 0)
+            k_xsph_omega_team<T><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
         else
-            enqueue_tail<BS, 4>(B, G, prm, n, nb, any_vort, any_plain, xsph_on, st, pm);
-    } else {
-        enqueue_tail<BS, 4>(B, G, prm, n, nb, any_vort, any_plain, xsph_on, st, pm);
+            k_xsph_omega<BS><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
+        if (pm) pm->mark(kPhaseXsph, 1, st);
+        if constexpr (TP != 0)
+            k_vorticity_commit_team<T><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n, G, prm);
+        else
+            k_vorticity_commit<BS><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n, G, prm);
+        if (pm) pm->mark(kPhaseCommit, 1, st);
+    }
+    if (any_plain) {
+        const int skip = any_vort ? 1 : 0;
+        if constexpr (TP != 0)
+            k_xsph_commit_team<T><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
+        else
+            k_xsph_commit<BS><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
+        if (pm) pm->mark(xsph_on ? kPhaseXsph : kPhaseCommit, 1, st);
     }
     return cudaGetLastError();
 }
@@ -2023,16 +3007,22 @@ inline cudaError_t enqueue_passes(const StepBuffers& B, const Grid& G, int n, in
                                   const P prm, cudaStream_t st, PhaseMarks* pm,
                                   int persist_blocks = 0, unsigned int* barrier = nullptr,
                                   int block = kBlock) {
-    if constexpr (std::is_same<P, SceneTable>::value) {
-        if (block == 64)
-            return enqueue_passes_bs<64>(B, G, n, max_iters, any_zero_iters, any_vort, any_plain,
-                                         xsph_on, prm, st, pm, persist_blocks, barrier);
-        if (block == 256)
-            return enqueue_passes_bs<256>(B, G, n, max_iters, any_zero_iters, any_vort, any_plain,
-                                          xsph_on, prm, st, pm, persist_blocks, barrier);
+    auto go = [&](auto bs, auto tp) {
+        return enqueue_passes_bs<decltype(bs)::value, decltype(tp)::value>(
+            B, G, n, max_iters, any_zero_iters, any_vort, any_plain, xsph_on, prm, st, pm,
+            persist_blocks, barrier);
+    };
+    using std::integral_constant;
+    const integral_constant<int, kBlock> bs;
+    switch (team_size(n)) {
+        case 8: return go(bs, integral_constant<int, 8>{});
+        case 16: return go(bs, integral_constant<int, 16>{});
     }
-    return enqueue_passes_bs<kBlock>(B, G, n, max_iters, any_zero_iters, any_vort, any_plain,
-                                     xsph_on, prm, st, pm, persist_blocks, barrier);
+    if constexpr (std::is_same<P, SceneTable>::value) {
+        if (block == 64) return go(integral_constant<int, 64>{}, integral_constant<int, 0>{});
+        if (block == 256) return go(integral_constant<int, 256>{}, integral_constant<int, 0>{});
+    }
+    return go(bs, integral_constant<int, 0>{});
 }
 
 inline cudaError_t enqueue_step(const StepBuffers& B, const StepConsts& C, int iters,

@@ -29,6 +29,7 @@ struct StepConsts {
     float h;         // kernel radius
     float h2;        // h * h                         (sph_kernel.h:25-26)
     float cut;       // smallest r^2 with poly6 == 0 and spiky_grad == 0
+    float r2_min;    // largest r^2 whose square root is <= 1e-7 (spiky_grad == 0, sph_kernel.h:40)
     float inv_cell;  // 1.0f / h                      (neighbor_search.cpp:101)
     float mass;
     float rho0;
@@ -39,6 +40,9 @@ struct StepConsts {
     float k_spiky;   // -(45 / (pi h^6))              (sph_kernel.h:44)
     float w_dq;      // poly6((dq h)^2, h)            (pbf_solver.cpp:188-189)
     float neg_corr_k;
+    float inv_w_dq;  // 1.0f / w_dq
+    float one;       // 1.0f, opaque to the compiler   (exact_pair.cuh)
+    int paired;      // h is in the range of the paired arithmetic (exact_pair.cuh)
     int corr_n4;     // corr_n == 4
     int scorr_on;    // w_dq > 1e-10
     float dt, inv_dt, max_speed, max_speed_sq;  // (pbf_solver.cpp:81-83)
