@@ -28,8 +28,9 @@ __device__ __forceinline__ float2 mul2(float2 a, float2 b) { return __fmul2_rn(a
 __device__ __forceinline__ float2 add2(float2 a, float2 b, float one) {
     return __ffma2_rn(a, both(one), b);
 }
-// a - b (a negation of b and an fma by minus one round alike).
-__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __ffma2_rn(b, both(-1.0f), a); }
+__device__ __forceinline__ float2 neg2(float2 a) { return make_float2(-a.x, -a.y); }
+// a - b, where b is no product.
+__device__ __forceinline__ float2 sub2(float2 a, float2 b) { return __fadd2_rn(a, neg2(b)); }
 
 __device__ __forceinline__ float rsqrt_approx(float x) {
     float y;
@@ -42,14 +43,14 @@ __device__ __forceinline__ float rsqrt_approx(float x) {
 __device__ __forceinline__ void root_and_inverse(float2 x, float2& root, float2& inv) {
     const float2 y = make_float2(rsqrt_approx(x.x), rsqrt_approx(x.y));
     const float2 s = mul2(x, y);
-    const float2 d = __ffma2_rn(mul2(s, both(-1.0f)), s, x);  // x - s s, exact
+    const float2 d = __ffma2_rn(neg2(s), s, x);  // x - s s, exact
     root = __ffma2_rn(d, mul2(y, both(0.5f)), s);
     // 1 / root = u (1 + e + e^2 + ...) with e = 1 - root u.  u lies above the
     // approximation, so that the one root whose inverse is all but halfway
     // between two floats (its significand all ones) rounds to the upper one;
     // with e alone, two other significands get an inverse one ulp off.
     const float2 u = mul2(y, both(1.0000002384185791f));
-    const float2 e = __ffma2_rn(mul2(root, both(-1.0f)), u, both(1.0f));
+    const float2 e = __ffma2_rn(neg2(root), u, both(1.0f));
     inv = __ffma2_rn(__ffma2_rn(e, e, e), u, u);
 }
 
@@ -58,7 +59,7 @@ __device__ __forceinline__ void root_and_inverse(float2 x, float2& root, float2&
 // (or a = 0).
 __device__ __forceinline__ float2 quotient(float2 a, float2 b, float2 inv) {
     const float2 q = mul2(a, inv);
-    const float2 r = __ffma2_rn(mul2(b, both(-1.0f)), q, a);  // a - b q, exact
+    const float2 r = __ffma2_rn(neg2(b), q, a);  // a - b q, exact
     return __ffma2_rn(r, inv, q);
 }
 

@@ -1,6 +1,6 @@
 // C ABI of batched stepping (include/novaphy_pbf.h, "Batches of scenes"):
-// many independent scenes share one cell-key sort, one reference-key sort and
-// one kernel launch per phase.  Each scene keeps its state in place; the
+// many independent scenes share one cell-key sort, one table of reference
+// buckets and one kernel launch per phase.  Each scene keeps its state in place; the
 // kernels reach it through a per-scene table (state pointers, particle range,
 // step constants, slot range) uploaded before every step.
 //
@@ -35,15 +35,13 @@ namespace {
 // The launch sequence of a batch step depends on these; a cached graph is
 // reused (with updated kernel parameters) while they stay the same.
 struct GraphKey {
-    int exact = -1, persist = 0, block = 0, n = 0, nscenes = 0, key_bits = 0, scene_bits = 0,
-        max_iters = 0;
+    int exact = -1, persist = 0, block = 0, n = 0, nscenes = 0, key_bits = 0, max_iters = 0;
     uint32_t nslots = 0;
     bool any_zero = false, any_vort = false, any_plain = false, xsph_on = false;
     bool operator==(const GraphKey& o) const {
         return exact == o.exact && persist == o.persist && block == o.block && n == o.n &&
-               nscenes == o.nscenes &&
-               key_bits == o.key_bits &&
-               scene_bits == o.scene_bits && max_iters == o.max_iters && nslots == o.nslots &&
+               nscenes == o.nscenes && key_bits == o.key_bits && max_iters == o.max_iters &&
+               nslots == o.nslots &&
                any_zero == o.any_zero && any_vort == o.any_vort && any_plain == o.any_plain &&
                xsph_on == o.xsph_on;
     }
@@ -94,12 +92,10 @@ struct pbf_batch {
     int cap = 0;  // particles
     void* wmem = nullptr;  // step scratch (bind_work)
     void* smem = nullptr;  // sort scratch
-    void* xmem = nullptr;  // scene ids, scene-pass temporaries
+    void* xmem = nullptr;  // scene ids
     StepBuffers B{};
     SortScratch sort{};
-    uint32_t *pid = nullptr, *spid = nullptr, *kpid = nullptr, *itmp = nullptr, *perm = nullptr,
-             *stmp = nullptr;
-    unsigned long long* rtmp = nullptr;
+    uint32_t *pid = nullptr, *spid = nullptr;
 
     uint32_t* off = nullptr;  // nslots + 1 offsets, then one alias byte per slot
     uint32_t off_cap = 0;     // entries
@@ -158,7 +154,7 @@ void drop_graph(pbf_batch* b) {
 }
 
 size_t extra_bytes(int c) {
-    return 6 * align_up((size_t)c * 4, 256) + align_up((size_t)c * 8, 256);
+    return 2 * align_up((size_t)c * 4, 256);
 }
 
 int ensure_particles(pbf_batch* b, int n) {
@@ -184,9 +180,8 @@ int ensure_particles(pbf_batch* b, int n) {
     PBF_CUDA(cudaMalloc(&b->xmem, xb));
     char* p = reinterpret_cast<char*>(b->xmem);
     const size_t f1 = align_up((size_t)c * 4, 256);
-    uint32_t** arr[6] = {&b->pid, &b->spid, &b->kpid, &b->itmp, &b->perm, &b->stmp};
-    for (int k = 0; k < 6; ++k) *arr[k] = reinterpret_cast<uint32_t*>(p + k * f1);
-    b->rtmp = reinterpret_cast<unsigned long long*>(p + 6 * f1);
+    b->pid = reinterpret_cast<uint32_t*>(p);
+    b->spid = reinterpret_cast<uint32_t*>(p + f1);
     b->cap = c;
     return PBF_OK;
 }
@@ -206,6 +201,7 @@ int ensure_slots(pbf_batch* b, uint32_t nslots) {
     b->B.slot_alias = reinterpret_cast<unsigned char*>(b->off) + ob;
     b->B.moved = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(b->off) + ob + ab);
     b->B.lamnz = b->B.moved + (c + 1);
+    b->B.slot_bytes = ab + (size_t)(c + 1) * 8;
     return PBF_OK;
 }
 
@@ -371,7 +367,6 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
         int rc = scene_consts(s, dts[k], C);
         if (rc) return rc;
         C.seg_begin = (uint32_t)n_total;
-        C.seg_end = (uint32_t)(n_total + (unsigned long long)s->n);
         C.grid.base = (uint32_t)slots_total;
         n_total += (unsigned long long)s->n;
         slots_total += C.grid.nslots;
@@ -419,7 +414,6 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
     D.nscenes = ns;
     D.nslots = (uint32_t)slots_total;
     D.key_bits = bits_for(slots_total);
-    D.scene_bits = bits_for((unsigned long long)ns);
     D.max_iters = max_iters;
     D.any_zero_iters = any_zero;
     D.any_vort = any_vort;
@@ -431,11 +425,6 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
     D.firsts = reinterpret_cast<const uint32_t*>(t + b->tab_firsts_at);
     D.pid = b->pid;
     D.spid = b->spid;
-    D.kpid = b->kpid;
-    D.rtmp = b->rtmp;
-    D.itmp = b->itmp;
-    D.perm = b->perm;
-    D.stmp = b->stmp;
     D.persist_blocks = 0;
     D.barrier = b->barrier;
     Choice choice;
@@ -476,7 +465,6 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
     key.n = n;
     key.nscenes = ns;
     key.key_bits = D.key_bits;
-    key.scene_bits = D.scene_bits;
     key.max_iters = max_iters;
     key.nslots = D.nslots;
     key.any_zero = any_zero;

@@ -11,23 +11,21 @@
 namespace pbf {
 namespace bnd {
 
-// Cell slot and reference key of points (no prediction).
+// Cell slot of points (no prediction).
 __global__ void __launch_bounds__(kBlock)
-k_ix_keys(const float4* __restrict__ pos, int n, uint32_t* __restrict__ keys,
-          unsigned long long* __restrict__ rkeys, const StepConsts C) {
+k_ix_keys(const float4* __restrict__ pos, int n, uint32_t* __restrict__ keys, const StepConsts C) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     const float4 p = pos[i];
     int cx, cy, cz;
     cell_of(p.x, p.y, p.z, C.inv_cell, cx, cy, cz);
     keys[i] = slot_of(cx, cy, cz, C.grid);
-    rkeys[i] = ref_hash(cx, cy, cz);
 }
 
 __global__ void __launch_bounds__(kBlock)
 k_ix_gather(const uint32_t* __restrict__ sidx, const float4* __restrict__ pos,
             const float* __restrict__ attr, int n, float4* __restrict__ spos,
-            int4* __restrict__ scell, uint32_t* __restrict__ pos_of,
+            int4* __restrict__ scell, uint32_t* __restrict__ link,
             unsigned char* __restrict__ slot_alias, const StepConsts C) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
@@ -38,8 +36,8 @@ k_ix_gather(const uint32_t* __restrict__ sidx, const float4* __restrict__ pos,
     cell_of(q.x, q.y, q.z, C.inv_cell, cx, cy, cz);
     spos[p] = make_float4(q.x, q.y, q.z, attr ? attr[i] : q.w);
     scell[p] = make_int4(cx, cy, cz, 0);
-    pos_of[i] = (uint32_t)p;
-    if (!in_grid(cx, cy, cz, C.grid)) slot_alias[slot_of(cx, cy, cz, C.grid)] = 1;
+    link[p] = kNoBucket;
+    if (!in_grid(cx, cy, cz, C.grid)) slot_alias[slot_of(cx, cy, cz, C.grid)] = kAliasSlot;
 }
 
 __global__ void __launch_bounds__(kBlock)
@@ -60,6 +58,10 @@ k_qcells(const float4* __restrict__ qpos, int nq, int4* __restrict__ qcell, cons
     int cx, cy, cz;
     cell_of(q.x, q.y, q.z, C.inv_cell, cx, cy, cz);
     qcell[i] = make_int4(cx, cy, cz, 0);
+}
+
+__device__ __forceinline__ WalkIndex index_of(const PointIndex& I, const QuerySet& Q) {
+    return WalkIndex{(uint32_t)I.n, I.off, I.bkt.merged, I.bkt.end, Q.btab};
 }
 
 __device__ __forceinline__ int4 query_cell(const QuerySet& Q, int i) {
@@ -109,7 +111,7 @@ k_boundary_density(const float4* __restrict__ x, int n, const QuerySet Q, const 
     if (i >= n) return;
     const float4 xi = x[i];
     float bd = 0.0f;
-    for_each_candidate(query_cell(Q, i), I.off, I.kpos, I.bend, Q.btab, C, [&](uint32_t q) {
+    for_each_candidate(query_cell(Q, i), index_of(I, Q), C, [&](uint32_t q) {
         const float4 b = __ldg(I.spos + q);
         const float r_sq = sqn(xi.x - b.x, xi.y - b.y, xi.z - b.z);
         bd += C.rho0 * b.w * poly6(r_sq, C);
@@ -131,7 +133,7 @@ k_coupling(const float4* __restrict__ bworld, const int* __restrict__ body,
     const float4 xb = bworld[b];
     const float psi_b = xb.w;
     float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-    for_each_candidate(query_cell(Q, b), I.off, I.kpos, I.bend, Q.btab, C, [&](uint32_t q) {
+    for_each_candidate(query_cell(Q, b), index_of(I, Q), C, [&](uint32_t q) {
         const float4 xf = __ldg(I.spos + q);
         const float rx = xb.x - xf.x;
         const float ry = xb.y - xf.y;
@@ -289,7 +291,7 @@ k_volumes(const float4* __restrict__ world, int nb, const QuerySet Q, const Poin
     if (b >= nb) return;
     const float4 xb = world[b];
     float sum_w = 0.0f;
-    for_each_candidate(query_cell(Q, b), I.off, I.kpos, I.bend, Q.btab, C, [&](uint32_t q) {
+    for_each_candidate(query_cell(Q, b), index_of(I, Q), C, [&](uint32_t q) {
         const float4 xj = __ldg(I.spos + q);
         sum_w += poly6(sqn(xb.x - xj.x, xb.y - xj.y, xb.z - xj.z), C);
     });
@@ -306,15 +308,13 @@ cudaError_t index_build(PointIndex& I, const float4* pos, const float* attr, int
     cudaError_t e = cudaMemsetAsync(I.slot_alias, 0, (size_t)C.grid.nslots, st);
     if (e != cudaSuccess) return e;
     const int nb = grid_of(n, kBlock);
-    k_ix_keys<<<nb, kBlock, 0, st>>>(pos, n, I.keys, I.rkeys, C);
+    k_ix_keys<<<nb, kBlock, 0, st>>>(pos, n, I.keys, C);
     e = radix_sort_pairs(I.keys, I.skeys, I.sidx, n, C.grid.key_bits, sort, st);
     if (e != cudaSuccess) return e;
-    e = radix_sort_pairs64(I.rkeys, I.rsorted, I.ridx, n, 64, sort, st);
-    if (e != cudaSuccess) return e;
     k_offsets<<<grid_of((int)C.grid.nslots + 1, 256), 256, 0, st>>>(I.skeys, n, I.off, C.grid.nslots);
-    k_ix_gather<<<nb, kBlock, 0, st>>>(I.sidx, pos, attr, n, I.spos, I.scell, I.pos_of,
+    k_ix_gather<<<nb, kBlock, 0, st>>>(I.sidx, pos, attr, n, I.spos, I.scell, I.bkt.link,
                                        I.slot_alias, C);
-    return enqueue_buckets(I.rsorted, I.ridx, I.pos_of, I.scell, nullptr, I.kpos, I.bend, n, st);
+    return enqueue_buckets(sized_for(I.bkt, n), I.scell, I.sidx, nullptr, I.slot_alias, n, OneScene{C, StateRef{}}, st);
 }
 
 cudaError_t predict_points(const float4* x, const float4* v, int n, float4* out,
@@ -335,12 +335,9 @@ cudaError_t index_classify(const QuerySet& Q, const float4* qpos, int nq, const 
         return cudaMemsetAsync(Q.qown, 0, (size_t)nq * sizeof(int), st);
     }
     StepConsts Cs = C;
-    Cs.seg_begin = 0;
-    Cs.seg_end = (uint32_t)I.n;
     Cs.hash_compat = 1;  // the coupling queries always follow the reference buckets
-    k_classify<<<grid_of(nq, kBlock), kBlock, 0, st>>>(Q.qcell, nq, I.scell, I.rsorted, I.kpos,
-                                                        I.bend, I.slot_alias, Q.btab, Q.qown,
-                                                        nullptr, OneScene{Cs, StateRef{}});
+    k_classify<<<grid_of(nq, kBlock), kBlock, 0, st>>>(Q.qcell, nq, I.scell, nullptr, sized_for(I.bkt, I.n), I.slot_alias,
+                                                        Q.btab, Q.qown, nullptr, OneScene{Cs, StateRef{}});
     return cudaGetLastError();
 }
 

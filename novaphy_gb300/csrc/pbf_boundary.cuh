@@ -15,18 +15,13 @@ namespace pbf {
 
 // The reference's hash grid over one point set, laid out like the step's:
 // dense wrapped cell slots (keys -> skeys/sidx, off, slot_alias) for spatial
-// order, and the reference keys sorted (rsorted/ridx) for exact buckets.
+// order, and the reference buckets over it.
 struct PointIndex {
     int n = 0;
     uint32_t* keys = nullptr;
     uint32_t* skeys = nullptr;
     uint32_t* sidx = nullptr;
-    unsigned long long* rkeys = nullptr;
-    unsigned long long* rsorted = nullptr;
-    uint32_t* ridx = nullptr;
-    uint32_t* pos_of = nullptr;
-    uint32_t* kpos = nullptr;
-    uint32_t* bend = nullptr;
+    BucketTable bkt{};
     float4* spos = nullptr;  // sorted positions, w = per-point attribute
     int4* scell = nullptr;
     uint32_t* off = nullptr;            // nslots + 1

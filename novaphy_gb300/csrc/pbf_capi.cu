@@ -144,6 +144,7 @@ void free_particles(pbf_scene* s) {
         s->B.moved = reinterpret_cast<uint32_t*>(s->B.slot_alias + align_up(s->off_cap, 256));
         s->B.lamnz = s->B.moved + s->off_cap;
         s->B.dhist = s->B.lamnz + s->off_cap;
+        s->B.slot_bytes = align_up(s->off_cap, 256) + (size_t)s->off_cap * 8;
     }
 }
 
@@ -306,6 +307,7 @@ int ensure_offsets(pbf_scene* s, uint32_t nslots) {
     s->B.moved = reinterpret_cast<uint32_t*>(reinterpret_cast<unsigned char*>(s->off) + ob + ab);
     s->B.lamnz = s->B.moved + (nslots + 1);
     s->B.dhist = s->B.lamnz + (nslots + 1);
+    s->B.slot_bytes = ab + (size_t)(nslots + 1) * 8;
     PBF_CUDA(cudaMemsetAsync(s->B.dhist, 0, 4 * kWalkHist * 4, s->stream));
     return PBF_OK;
 }
@@ -399,7 +401,6 @@ int scene_consts(const pbf_scene* s, float dt, StepConsts& C) {
     C.bfric = st.boundary_two_way ? st.boundary_friction : 0.0f;
     C.iters = st.solver_iterations;
     C.seg_begin = 0;
-    C.seg_end = (uint32_t)s->n;
     C.grid = fit_grid(s);
     return PBF_OK;
 }
@@ -1175,8 +1176,8 @@ int alloc_boundary(pbf_scene* s, int nb) {
     b.mem = b.sort_mem = nullptr;
     const int c = nb > 0 ? nb : 1;
     const size_t f4 = align_up((size_t)c * 16, 256), f1 = align_up((size_t)c * 4, 256),
-                 f2 = align_up((size_t)c * 8, 256), f27 = align_up((size_t)c * 27 * 4, 256);
-    const size_t total = 6 * f4 + 9 * f1 + 2 * f2 + f27;
+                 f27 = align_up((size_t)c * 27 * 4, 256);
+    const size_t total = 6 * f4 + 5 * f1 + bucket_bytes(c) + f27;
     PBF_CUDA(cudaMalloc(&b.mem, total));
     char* p = reinterpret_cast<char*>(b.mem);
     auto take = [&](size_t n) { char* r = p; p += n; return r; };
@@ -1190,13 +1191,8 @@ int alloc_boundary(pbf_scene* s, int nb) {
     b.idx.keys = reinterpret_cast<uint32_t*>(take(f1));
     b.idx.skeys = reinterpret_cast<uint32_t*>(take(f1));
     b.idx.sidx = reinterpret_cast<uint32_t*>(take(f1));
-    b.idx.ridx = reinterpret_cast<uint32_t*>(take(f1));
-    b.idx.pos_of = reinterpret_cast<uint32_t*>(take(f1));
-    b.idx.kpos = reinterpret_cast<uint32_t*>(take(f1));
-    b.idx.bend = reinterpret_cast<uint32_t*>(take(f1));
     b.bq.qown = reinterpret_cast<int*>(take(f1));
-    b.idx.rkeys = reinterpret_cast<unsigned long long*>(take(f2));
-    b.idx.rsorted = reinterpret_cast<unsigned long long*>(take(f2));
+    bind_buckets(b.idx.bkt, take(bucket_bytes(c)), c);
     b.bq.btab = reinterpret_cast<uint32_t*>(take(f27));
     PBF_CUDA(cudaMemsetAsync(b.mem, 0, total, s->stream));
     const size_t sb = sort_scratch_bytes(c);
@@ -1394,12 +1390,7 @@ int enqueue_coupling(pbf_scene* s, const StepConsts& C, const float* force_in,
     fidx.keys = s->B.keys;
     fidx.skeys = s->B.skeys;
     fidx.sidx = s->B.sidx;
-    fidx.rkeys = s->B.rkeys;
-    fidx.rsorted = s->B.rsorted;
-    fidx.ridx = s->B.ridx;
-    fidx.pos_of = s->B.pos_of;
-    fidx.kpos = s->B.kpos;
-    fidx.bend = s->B.bend;
+    fidx.bkt = s->B.bkt;
     fidx.spos = s->B.xb;
     fidx.scell = s->B.scell;
     fidx.off = s->B.off;
@@ -1662,8 +1653,9 @@ int two_way_step(pbf_scene* s, const StepConsts& C) {
     BoundaryGrid bg;
     bg.spos = b.idx.spos;
     bg.off = b.idx.off;
-    bg.kpos = b.idx.kpos;
-    bg.bend = b.idx.bend;
+    bg.n = (uint32_t)b.nb;
+    bg.merged = b.idx.bkt.merged;
+    bg.end = b.idx.bkt.end;
     bg.own = b.tw_own;
     bg.btab = b.tw_btab;
     bg.sidx = b.idx.sidx;

@@ -38,7 +38,7 @@ cudaError_t debug_neighbors(const StepBuffers& B, const StepConsts& C, SortScrat
         if (e != cudaSuccess) return e;
     }
     exact::k_debug_neighbors<<<exact::grid_of(C.n, exact::kBlock), exact::kBlock, 0, st>>>(
-        B.xa, B.sx, d_cnt, d_offs, d_out, cap, fill, exact::grid_view(B), C);
+        B.xa, B.sx, d_cnt, d_offs, d_out, cap, fill, exact::grid_view(B, C.n), C);
     return cudaGetLastError();
 }
 

@@ -44,21 +44,35 @@ inline size_t align_up(size_t v, size_t a) { return (v + a - 1) / a * a; }
 // rho, lambda (float) and the float3 staging buffer.
 constexpr size_t kStateBytesPerParticle = 16 + 16 + 4 + 4 + 12;
 
+// Bytes of a BucketTable over c points, and its carving out of [p, p + bytes).
+inline size_t bucket_bytes(int c) {
+    return 6 * align_up((size_t)c * 4, 256) + align_up(((size_t)bucket_slots((uint32_t)c) + 1) * 4, 256);
+}
+
+inline void bind_buckets(BucketTable& T, char* p, int c) {
+    const size_t f1 = align_up((size_t)c * 4, 256);
+    T.end = reinterpret_cast<uint32_t*>(p);
+    T.rep = reinterpret_cast<uint32_t*>(p + 2 * f1);
+    T.link = reinterpret_cast<uint32_t*>(p + 3 * f1);
+    T.start = reinterpret_cast<uint32_t*>(p + 4 * f1);
+    T.merged = reinterpret_cast<uint32_t*>(p + 5 * f1);
+    T.table = reinterpret_cast<uint32_t*>(p + 6 * f1);
+    T.slots = bucket_slots((uint32_t)c);
+}
+
 // Step scratch of c particles, carved from one allocation: the sorted
 // copies (sx, xa, xb, sv, sv2, som, scell: float4/int4), srho, the cell keys
-// and permutation, the reference keys, buckets and classification rows.
+// and permutation, the reference buckets and classification rows.
 inline size_t work_bytes(int c) {
     const size_t f4 = align_up((size_t)c * 16, 256);
     const size_t f1 = align_up((size_t)c * 4, 256);
-    const size_t f2 = align_up((size_t)c * 8, 256);
     const size_t f27 = align_up((size_t)c * 27 * 4, 256);
-    return 7 * f4 + 9 * f1 + 2 * f2 + f27;
+    return 7 * f4 + 5 * f1 + bucket_bytes(c) + f27;
 }
 
 inline void bind_work(StepBuffers& B, void* mem, int c) {
     const size_t f4 = align_up((size_t)c * 16, 256);
     const size_t f1 = align_up((size_t)c * 4, 256);
-    const size_t f2 = align_up((size_t)c * 8, 256);
     char* p = reinterpret_cast<char*>(mem);
     auto take = [&](size_t b) {
         char* r = p;
@@ -76,13 +90,8 @@ inline void bind_work(StepBuffers& B, void* mem, int c) {
     B.keys = reinterpret_cast<uint32_t*>(take(f1));
     B.skeys = reinterpret_cast<uint32_t*>(take(f1));
     B.sidx = reinterpret_cast<uint32_t*>(take(f1));
-    B.ridx = reinterpret_cast<uint32_t*>(take(f1));
-    B.pos_of = reinterpret_cast<uint32_t*>(take(f1));
-    B.kpos = reinterpret_cast<uint32_t*>(take(f1));
-    B.bend = reinterpret_cast<uint32_t*>(take(f1));
     B.sown = reinterpret_cast<int*>(take(f1));
-    B.rkeys = reinterpret_cast<unsigned long long*>(take(f2));
-    B.rsorted = reinterpret_cast<unsigned long long*>(take(f2));
+    bind_buckets(B.bkt, take(bucket_bytes(c)), c);
     B.btab = reinterpret_cast<uint32_t*>(p);
 }
 

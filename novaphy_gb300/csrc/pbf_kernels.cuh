@@ -39,7 +39,6 @@ constexpr int kBigScene = 1 << 17;
 // hundred).
 constexpr uint32_t kRunRow = 1024;
 constexpr uint32_t kNoBucket = 0xffffffffu;
-constexpr uint32_t kImpureBit = 0x80000000u;
 // Flags in a particle's owner word (StepBuffers::sown) for runs of identical
 // particles (k_segments): the particle only copies the results of its run's
 // first particle (kCopyBit), or it is a run's first particle (kLeadBit).  The
@@ -47,9 +46,12 @@ constexpr uint32_t kImpureBit = 0x80000000u;
 constexpr uint32_t kCopyBit = 0x40000000u;
 constexpr uint32_t kLeadBit = 0x80000000u;
 constexpr uint32_t kOwnerMask = 0x3fffffffu;
-// Set in a slot's alias byte (StepBuffers::slot_alias, bit 0: alias) when the
-// slot holds a run's first particle.
+// Bits of a slot's alias byte (StepBuffers::slot_alias): the slot holds a
+// particle from outside the grid box; a run's first particle; particles whose
+// reference bucket holds more than their run of cells.
+constexpr unsigned char kAliasSlot = 1;
 constexpr unsigned char kRunSlot = 2;
+constexpr unsigned char kMergedSlot = 4;
 
 // ---------------------------------------------------------------------------
 // SPH kernels (include/novaphy/fluid/sph_kernel.h:24-46)
@@ -146,16 +148,19 @@ __device__ __forceinline__ unsigned long long ref_hash(int cx, int cy, int cz) {
            ((unsigned long long)(long long)cz * 83492791ULL);
 }
 
-// lower_bound over the sorted reference keys in [a, b).
-__device__ __forceinline__ uint32_t key_lower_bound(const unsigned long long* __restrict__ keys,
-                                                    uint32_t a, uint32_t b, unsigned long long k) {
-    while (a < b) {
-        const uint32_t m = (a + b) >> 1;
-        if (__ldg(keys + m) < k) a = m + 1;
-        else b = m;
+// An index of cell-sorted points that walks visit: cell-order offsets of the
+// slots, and the reference buckets (see BucketTable) of the dirty cells' rows.
+struct WalkIndex {
+    uint32_t n;
+    const uint32_t* __restrict__ off;
+    const uint32_t* __restrict__ merged;
+    const uint32_t* __restrict__ end;
+    const uint32_t* __restrict__ btab;
+    // The cell-order position of bucket position q.
+    __device__ __forceinline__ uint32_t at(uint32_t q) const {
+        return q < n ? q : __ldg(merged + (q - n));
     }
-    return a;
-}
+};
 
 // Visits the candidate sorted positions q of a particle whose step-start cell
 // is `cell`, in the reference's order.  The particle itself is among them:
@@ -167,14 +172,9 @@ __device__ __forceinline__ uint32_t key_lower_bound(const unsigned long long* __
 // that cell, so each (dz, dy) row of three cells is one contiguous range of
 // the cell-sorted order.  cell.w == o + 1 (dirty: a neighbour key is shared
 // with another occupied cell, or a slot holds wrapped aliases): the 27 bucket
-// starts are row o of `btab`; a bucket is the run [start, bend) of the
-// key-sorted order and kpos maps it back to cell-sorted positions.  U is the
-// unroll factor of a row's candidate loop (see kBigScene).
-template <int U = 4, class F>
-__device__ __forceinline__ void for_each_candidate(const int4 cell, const uint32_t* __restrict__ off,
-                                                   const uint32_t* __restrict__ kpos,
-                                                   const uint32_t* __restrict__ bend,
-                                                   const uint32_t* __restrict__ btab,
+// starts are row o of `btab`.
+template <class F>
+__device__ __forceinline__ void for_each_candidate(const int4 cell, const WalkIndex& I,
                                                    const StepConsts& C, F&& f) {
     const GridDesc& G = C.grid;
     if (cell.w == 0) {
@@ -185,25 +185,25 @@ __device__ __forceinline__ void for_each_candidate(const int4 cell, const uint32
                 const uint32_t row = G.base + (uint32_t)G.gx * (wy + (uint32_t)G.gy * wz);
                 const int wx = wrap(cell.x - 1, G.ox, G.gx);
                 if (wx + 2 < G.gx) {
-                    const uint32_t q1 = __ldg(off + row + wx + 3);
-#pragma unroll U
-                    for (uint32_t q = __ldg(off + row + wx); q < q1; ++q) f(q);
+                    const uint32_t q1 = __ldg(I.off + row + wx + 3);
+#pragma unroll 4
+                    for (uint32_t q = __ldg(I.off + row + wx); q < q1; ++q) f(q);
                 } else {
                     for (int d = 0; d < 3; ++d) {
                         const uint32_t s = row + (uint32_t)wrap(cell.x - 1 + d, G.ox, G.gx);
-                        const uint32_t q1 = __ldg(off + s + 1);
-                        for (uint32_t q = __ldg(off + s); q < q1; ++q) f(q);
+                        const uint32_t q1 = __ldg(I.off + s + 1);
+                        for (uint32_t q = __ldg(I.off + s); q < q1; ++q) f(q);
                     }
                 }
             }
         }
     } else {
-        const uint32_t* row = btab + (size_t)(uint32_t)(cell.w - 1) * 27u;
+        const uint32_t* row = I.btab + (size_t)(uint32_t)(cell.w - 1) * 27u;
         for (int k = 0; k < 27; ++k) {
             const uint32_t b0 = __ldg(row + k);
             if (b0 == kNoBucket) continue;
-            const uint32_t b1 = __ldg(bend + b0) & ~kImpureBit;
-            for (uint32_t kq = b0; kq < b1; ++kq) f(__ldg(kpos + kq));
+            const uint32_t b1 = __ldg(I.end + b0);
+            for (uint32_t q = b0; q < b1; ++q) f(I.at(q));
         }
     }
 }
@@ -255,12 +255,19 @@ __device__ __forceinline__ void predict(const float4 xi, const float4 vi, const 
     pz = __fadd_rn(xi.z, __fmul_rn(vz, C.dt));
 }
 
-// Predict + cell slot and reference hash key per particle (particle order).
+// Predict + cell slot per particle (particle order).  Also turns this step's
+// density-pass counts of the last step (dhist, where there are any) into the
+// previous step's.
 template <class P>
 __global__ void __launch_bounds__(kBlock)
-k_predict_key(uint32_t* __restrict__ keys, unsigned long long* __restrict__ rkeys, int n,
-              const SceneIds S, const P prm) {
+k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, int n, const SceneIds S,
+              const P prm) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    static_assert(2 * kWalkHist <= kBlock, "one thread per count");
+    if (dhist && i < 2 * kWalkHist) {
+        dhist[i] = dhist[i + 2 * kWalkHist];
+        dhist[i + 2 * kWalkHist] = 0u;
+    }
     if (i >= n) return;
     const StepConsts& C = prm.at(S.pid, i);
     const StateRef& R = prm.state(S.pid, i);
@@ -270,7 +277,6 @@ k_predict_key(uint32_t* __restrict__ keys, unsigned long long* __restrict__ rkey
     int cx, cy, cz;
     cell_of(px, py, pz, C.inv_cell, cx, cy, cz);
     keys[i] = slot_of(cx, cy, cz, C.grid);
-    rkeys[i] = ref_hash(cx, cy, cz);
 }
 
 // off[s] = lower_bound(skeys, s) for s in [0, nslots].
@@ -288,12 +294,13 @@ k_offsets(const uint32_t* __restrict__ skeys, int n, uint32_t* __restrict__ off,
 }
 
 // Gather particle state into cell-sorted order; recompute x* exactly as
-// predicted.  Records each particle's sorted position (and scene) and flags
-// slots that receive a particle from outside the grid box (wrapped alias).
+// predicted.  Records each particle's scene, empties the bucket chains and
+// flags slots that receive a particle from outside the grid box (wrapped
+// alias).
 template <class P>
 __global__ void __launch_bounds__(kBlock)
 k_gather(const uint32_t* __restrict__ sidx, float4* __restrict__ sx, float4* __restrict__ xa,
-         float* __restrict__ srho, int4* __restrict__ scell, uint32_t* __restrict__ pos_of,
+         float* __restrict__ srho, int4* __restrict__ scell, uint32_t* __restrict__ link,
          unsigned char* __restrict__ slot_alias, uint32_t* __restrict__ err, int n,
          const SceneIds S, const P prm) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
@@ -315,9 +322,9 @@ k_gather(const uint32_t* __restrict__ sidx, float4* __restrict__ sx, float4* __r
     xa[p] = make_float4(px, py, pz, R.lam[l]);
     srho[p] = R.rho[l];
     scell[p] = make_int4(cx, cy, cz, 0);
-    pos_of[i] = (uint32_t)p;
+    link[p] = kNoBucket;
     if (S.spid) S.spid[p] = S.pid[i];
-    if (!in_grid(cx, cy, cz, C.grid)) slot_alias[slot_of(cx, cy, cz, C.grid)] = 1;
+    if (!in_grid(cx, cy, cz, C.grid)) slot_alias[slot_of(cx, cy, cz, C.grid)] = kAliasSlot;
 }
 
 // Runs of particles with bit-identical step state (x, x* and lambda and rho
@@ -394,115 +401,192 @@ k_segments(const StepState S, const int4* __restrict__ scell, const GridDesc Gd,
     if (in) segend[p] = end;
 }
 
-// Reference buckets in key-sorted order: kpos maps key-sorted positions to
-// cell-sorted ones; at each bucket start, bend holds the bucket end with
-// kImpureBit set when the bucket mixes cells (hash collision).  With scene
-// ids (ksid, in key-sorted order) a bucket never crosses a scene boundary:
-// every scene has its own hash grid.  Two launches (enqueue_buckets): the
-// bucket starts find their ends, then members whose cell differs from the
-// previous member's mark their bucket impure.  Both searches gallop, so a
-// bucket of L members costs O(log L) per thread; a serial scan by the start
-// thread took milliseconds on buckets of tens of thousands of particles
-// (fluid piled into a corner cell by the domain clamp).
-struct BucketKeys {
-    const unsigned long long* __restrict__ rsorted;
-    const uint32_t* __restrict__ ksid;
+// Reference buckets over cell-sorted points (see BucketTable), in three
+// launches.  With scene ids (sid, in cell order) a bucket never crosses a
+// scene: every scene has its own hash grid.  This took the place of a radix
+// sort of the points by 64-bit reference key (eight passes) and of binary
+// searches over the sorted keys: a step's neighbour structure has as many runs
+// as occupied cells, a few per cent of its points, and few buckets merge.
+struct CellRuns {
+    const int4* __restrict__ scell;
+    const uint32_t* __restrict__ sid;
     int n;
-    __device__ __forceinline__ bool same(int m, unsigned long long k, uint32_t s0) const {
-        return rsorted[m] == k && (!ksid || ksid[m] == s0);
+    __device__ __forceinline__ bool same(int a, int b) const {
+        const int4 c = scell[a], d = scell[b];
+        return c.x == d.x && c.y == d.y && c.z == d.z && (!sid || sid[a] == sid[b]);
     }
-    // First position after kp outside kp's bucket.
-    __device__ __forceinline__ int end_of(int kp) const {
-        const unsigned long long k = rsorted[kp];
-        const uint32_t s0 = ksid ? ksid[kp] : 0u;
-        int lo = kp, step = 1, hi = kp + 1;
-        while (hi < n && same(hi, k, s0)) {
+    // First position after p outside p's run, and the run's first position.
+    // Both gallop, so a run of L points costs O(log L) per thread: fluid piled
+    // into a corner by the domain clamp makes runs of tens of thousands.
+    // (Positions of one run are contiguous, but a gallop may land in a later
+    // run of the same cell only where its slot holds aliases, whose cells
+    // alternate; there the runs are found one position at a time.)
+    __device__ __forceinline__ int end_of(int p, bool step_by_one) const {
+        int lo = p, step = 1, hi = p + 1;
+        while (hi < n && same(hi, p)) {
             lo = hi;
-            step <<= 1;
-            hi = (n - kp > step) ? kp + step : n;
+            step = step_by_one ? step + 1 : step << 1;
+            hi = (n - p > step) ? p + step : n;
         }
         while (hi - lo > 1) {
             const int mid = lo + ((hi - lo) >> 1);
-            if (same(mid, k, s0)) lo = mid;
+            if (same(mid, p)) lo = mid;
             else hi = mid;
         }
         return hi;
     }
-    // First position of kp's bucket.
-    __device__ __forceinline__ int start_of(int kp) const {
-        const unsigned long long k = rsorted[kp];
-        const uint32_t s0 = ksid ? ksid[kp] : 0u;
-        int hi = kp, step = 1, lo = kp - 1;
-        while (lo >= 0 && same(lo, k, s0)) {
+    __device__ __forceinline__ int start_of(int p, bool step_by_one) const {
+        int hi = p, step = 1, lo = p - 1;
+        while (lo >= 0 && same(lo, p)) {
             hi = lo;
-            step <<= 1;
-            lo = (kp >= step) ? kp - step : -1;
+            step = step_by_one ? step + 1 : step << 1;
+            lo = (p >= step) ? p - step : -1;
         }
         while (hi - lo > 1) {
             const int mid = lo + ((hi - lo) >> 1);
-            if (same(mid, k, s0)) hi = mid;
+            if (same(mid, p)) hi = mid;
             else lo = mid;
         }
         return hi;
     }
+    __device__ __forceinline__ unsigned long long key(int p) const {
+        const int4 c = scell[p];
+        return ref_hash(c.x, c.y, c.z);
+    }
 };
 
-__device__ __forceinline__ uint32_t cell_sorted_pos(const uint32_t* __restrict__ ridx,
-                                                    const uint32_t* __restrict__ pos_of, int kp,
-                                                    int n) {
-    const uint32_t i0 = ridx[kp];
-    uint32_t p0 = pos_of[i0 < (uint32_t)n ? i0 : 0];
-    return p0 < (uint32_t)n ? p0 : 0u;
+__device__ __forceinline__ uint32_t table_slot(unsigned long long key, uint32_t sid, uint32_t slots) {
+    const unsigned long long h = (key ^ (key >> 29)) * 0x9e3779b97f4a7c15ull + (unsigned long long)sid * 0x632be59bd9b4e019ull;
+    return (uint32_t)(h >> 32) & (slots - 1u);
 }
 
+// T with the slots that a build over n of its points uses.
+inline BucketTable sized_for(BucketTable T, int n) {
+    T.slots = bucket_slots((uint32_t)n);
+    return T;
+}
+
+// The first run of the bucket with this key (and scene), kNoBucket if none.
+__device__ __forceinline__ uint32_t find_bucket(const BucketTable& T, const CellRuns& R,
+                                                unsigned long long key, uint32_t sid) {
+    uint32_t h = table_slot(key, sid, T.slots);
+    for (uint32_t k = 0; k < T.slots; ++k) {
+        const uint32_t e = T.table[h];
+        if (e == kNoBucket) return kNoBucket;
+        if (R.key((int)e) == key && (!R.sid || R.sid[e] == sid)) return e;
+        h = (h + 1u) & (T.slots - 1u);
+    }
+    return kNoBucket;
+}
+
+// Every run's end, and its place in the table.
+template <class P>
 __global__ void __launch_bounds__(256)
-k_buckets(const BucketKeys K, const uint32_t* __restrict__ ridx, const uint32_t* __restrict__ pos_of,
-          uint32_t* __restrict__ kpos, uint32_t* __restrict__ bend) {
-    const int kp = blockIdx.x * blockDim.x + threadIdx.x;
-    if (kp >= K.n) return;
-    kpos[kp] = cell_sorted_pos(ridx, pos_of, kp, K.n);
-    if (kp > 0 && K.same(kp - 1, K.rsorted[kp], K.ksid ? K.ksid[kp] : 0u)) return;
-    bend[kp] = (uint32_t)K.end_of(kp);
+k_cell_runs(const BucketTable T, const CellRuns R, const unsigned char* __restrict__ slot_alias, const P prm) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= R.n || (p > 0 && R.same(p, p - 1))) return;
+    const int4 c = R.scell[p];
+    const StepConsts& C = prm.at(R.sid, (uint32_t)p);
+    const bool alias = (slot_alias[slot_of(c.x, c.y, c.z, C.grid)] & kAliasSlot) != 0;
+    T.end[p] = (uint32_t)R.end_of(p, alias);
+    const unsigned long long key = ref_hash(c.x, c.y, c.z);
+    const uint32_t sid = R.sid ? R.sid[p] : 0u;
+    uint32_t rep = (uint32_t)p;
+    uint32_t h = table_slot(key, sid, T.slots);
+    for (uint32_t k = 0; k < T.slots; ++k) {
+        const uint32_t e = atomicCAS(T.table + h, kNoBucket, (uint32_t)p);
+        if (e == kNoBucket) break;
+        if (R.key((int)e) == key && (!R.sid || R.sid[e] == sid)) {
+            rep = e;
+            T.link[p] = atomicExch(T.link + e, (uint32_t)p);
+            break;
+        }
+        h = (h + 1u) & (T.slots - 1u);
+    }
+    T.rep[p] = rep;
+    if (rep == (uint32_t)p) T.start[p] = (uint32_t)p;
 }
 
+// Room for the buckets of more than one run.
+template <class P>
 __global__ void __launch_bounds__(256)
-k_bucket_mix(const BucketKeys K, const uint32_t* __restrict__ ridx,
-             const uint32_t* __restrict__ pos_of, const int4* __restrict__ scell,
-             uint32_t* __restrict__ bend) {
-    const int kp = blockIdx.x * blockDim.x + threadIdx.x;
-    if (kp == 0 || kp >= K.n) return;
-    if (!K.same(kp - 1, K.rsorted[kp], K.ksid ? K.ksid[kp] : 0u)) return;
-    const int4 c = scell[cell_sorted_pos(ridx, pos_of, kp, K.n)];
-    const int4 d = scell[cell_sorted_pos(ridx, pos_of, kp - 1, K.n)];
-    if (c.x != d.x || c.y != d.y || c.z != d.z) atomicOr(bend + K.start_of(kp), kImpureBit);
+k_merge_room(const BucketTable T, const CellRuns R, unsigned char* __restrict__ slot_alias, const P prm) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= R.n || (p > 0 && R.same(p, p - 1))) return;
+    if (T.rep[p] != (uint32_t)p || T.link[p] == kNoBucket) return;
+    uint32_t total = 0u;
+    const StepConsts& C = prm.at(R.sid, (uint32_t)p);
+    for (uint32_t s = (uint32_t)p; s != kNoBucket; s = T.link[s]) {
+        total += T.end[s] - s;
+        const int4 c = R.scell[s];
+        unsigned char* const a = slot_alias + slot_of(c.x, c.y, c.z, C.grid);
+        *a = (unsigned char)(*a | kMergedSlot);
+    }
+    const uint32_t at = (uint32_t)R.n + atomicAdd(T.table + T.slots, total) + 1u;
+    T.start[p] = at;
+    T.end[at] = at + total;
 }
 
-inline cudaError_t enqueue_buckets(const unsigned long long* rsorted, const uint32_t* ridx,
-                                   const uint32_t* pos_of, const int4* scell,
-                                   const uint32_t* ksid, uint32_t* kpos, uint32_t* bend, int n,
+// The members of those buckets, in ascending point index: a point's place is
+// the number of members before it, by a search in each of the other runs.
+template <class P>
+__global__ void __launch_bounds__(256)
+k_merge_runs(const BucketTable T, const CellRuns R, const uint32_t* __restrict__ sidx,
+             const unsigned char* __restrict__ slot_alias, const P prm) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p >= R.n) return;
+    const int4 c = R.scell[p];
+    const StepConsts& C = prm.at(R.sid, (uint32_t)p);
+    const unsigned char a = slot_alias[slot_of(c.x, c.y, c.z, C.grid)];
+    if (!(a & kMergedSlot)) return;
+    const uint32_t own = (uint32_t)R.start_of(p, (a & kAliasSlot) != 0);
+    const uint32_t rep = T.rep[own];
+    if (T.link[rep] == kNoBucket) return;
+    const uint32_t i = sidx[p];
+    uint32_t rank = (uint32_t)p - own;
+    for (uint32_t s = rep; s != kNoBucket; s = T.link[s]) {
+        if (s == own) continue;
+        uint32_t lo = s, hi = T.end[s];
+        while (lo < hi) {
+            const uint32_t m = (lo + hi) >> 1;
+            if (sidx[m] < i) lo = m + 1u;
+            else hi = m;
+        }
+        rank += lo - s;
+    }
+    const uint32_t at = T.start[rep] - (uint32_t)R.n + rank;
+    if (at < (uint32_t)R.n) T.merged[at] = (uint32_t)p;
+}
+
+// T: sized_for n.
+template <class P>
+inline cudaError_t enqueue_buckets(const BucketTable& T, const int4* scell, const uint32_t* sidx,
+                                   const uint32_t* sid, unsigned char* slot_alias, int n, const P& prm,
                                    cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    const BucketKeys K{rsorted, ksid, n};
+    cudaError_t e = cudaMemsetAsync(T.table, 0xff, ((size_t)T.slots + 1) * 4, st);
+    if (e != cudaSuccess) return e;
+    const CellRuns R{scell, sid, n};
     const int nb = (n + 255) / 256;
-    k_buckets<<<nb, 256, 0, st>>>(K, ridx, pos_of, kpos, bend);
-    k_bucket_mix<<<nb, 256, 0, st>>>(K, ridx, pos_of, scell, bend);
+    k_cell_runs<<<nb, 256, 0, st>>>(T, R, slot_alias, prm);
+    k_merge_room<<<nb, 256, 0, st>>>(T, R, slot_alias, prm);
+    k_merge_runs<<<nb, 256, 0, st>>>(T, R, sidx, slot_alias, prm);
     return cudaGetLastError();
 }
 
 // Marks query points whose neighbourhood differs from the reference's
 // buckets over a source point set (qown[p] = owner + 1, else 0) and stores
-// their 27 bucket starts in row `owner` of btab.  Query cells are qcell[0..nq),
-// the source's key-sorted buckets are (rsorted, kpos, bend) with cells scell
-// and slot alias flags of the source's grid; a query of scene s searches the
-// scene's key range [seg_begin, seg_end).  Within a warp, one lane per
-// distinct cell (and scene) does the 27 lookups; the other lanes reuse its row.
+// their 27 bucket starts in row `owner` of btab.  Query cells are qcell[0..nq)
+// (scenes qsid), the source's cells scell (scenes ssid) with buckets T and
+// slot flags of the source's grid.  Within a warp, one lane per distinct cell
+// (and scene) does the 27 lookups; the other lanes reuse its row.
 template <class P>
 __global__ void __launch_bounds__(kBlock)
 k_classify(const int4* __restrict__ qcell, int nq, const int4* __restrict__ scell,
-           const unsigned long long* __restrict__ rsorted, const uint32_t* __restrict__ kpos,
-           const uint32_t* __restrict__ bend, const unsigned char* __restrict__ slot_alias,
-           uint32_t* __restrict__ btab, int* __restrict__ qown, const uint32_t* __restrict__ qsid,
-           const P prm) {
+           const uint32_t* __restrict__ ssid, const BucketTable T,
+           const unsigned char* __restrict__ slot_alias, uint32_t* __restrict__ btab,
+           int* __restrict__ qown, const uint32_t* __restrict__ qsid, const P prm) {
+    const CellRuns R{scell, ssid, 0};
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = p < (uint32_t)nq;
     const int lane = threadIdx.x & 31;
@@ -527,21 +611,20 @@ k_classify(const int4* __restrict__ qcell, int nq, const int4* __restrict__ scel
         const int cy = __shfl_sync(full, cell.y, L);
         const int cz = __shfl_sync(full, cell.z, L);
         const uint32_t grp = __shfl_sync(full, same, L);
+        const uint32_t ls = __shfl_sync(full, sc, L);
         const StepConsts& C = prm.at(qsid, lp);
         int dirty = 0;
         if (C.hash_compat) {
             uint32_t t = kNoBucket;
             if (lane < 27) {
                 const int nx = cx + lane % 3 - 1, ny = cy + (lane / 3) % 3 - 1, nz = cz + lane / 9 - 1;
-                const unsigned long long k = ref_hash(nx, ny, nz);
-                const uint32_t lb = key_lower_bound(rsorted, C.seg_begin, C.seg_end, k);
-                if (lb < C.seg_end && __ldg(rsorted + lb) == k) {
-                    t = lb;
-                    const uint32_t e = __ldg(bend + lb);
-                    const int4 c0 = scell[__ldg(kpos + lb)];
-                    if ((e & kImpureBit) || c0.x != nx || c0.y != ny || c0.z != nz) dirty = 1;
+                const uint32_t e = find_bucket(T, R, ref_hash(nx, ny, nz), ssid ? ls : 0u);
+                if (e != kNoBucket) {
+                    t = T.start[e];
+                    const int4 c0 = scell[e];
+                    if (T.link[e] != kNoBucket || c0.x != nx || c0.y != ny || c0.z != nz) dirty = 1;
                 }
-                if (slot_alias[slot_of(nx, ny, nz, C.grid)]) dirty = 1;
+                if (slot_alias[slot_of(nx, ny, nz, C.grid)] & kAliasSlot) dirty = 1;
             }
             dirty = __any_sync(full, dirty);
             if (dirty && lane < 27) btab[(size_t)lp * 27u + (uint32_t)lane] = t;
@@ -557,10 +640,7 @@ k_classify(const int4* __restrict__ qcell, int nq, const int4* __restrict__ scel
 struct Grid {
     const int4* __restrict__ scell;
     const int* __restrict__ sown;
-    const uint32_t* __restrict__ off;
-    const uint32_t* __restrict__ kpos;
-    const uint32_t* __restrict__ bend;
-    const uint32_t* __restrict__ btab;
+    WalkIndex ix;
     const uint32_t* __restrict__ spid;  // scene of each sorted particle (batches)
     uint32_t* moved;                     // per slot, see StepBuffers::moved
     uint32_t* lamnz;                     // per slot, see StepBuffers::lamnz
@@ -579,11 +659,11 @@ template <bool kRuns, class F, class FR>
 __device__ __forceinline__ void for_each_candidate_runs(const int4 cell, const Grid& G,
                                                         const StepConsts& C, F&& f, FR&& fr) {
     if constexpr (!kRuns) {
-        for_each_candidate(cell, G.off, G.kpos, G.bend, G.btab, C, f);
+        for_each_candidate(cell, G.ix, C, f);
         return;
     }
     if (!G.segend) {
-        for_each_candidate(cell, G.off, G.kpos, G.bend, G.btab, C, f);
+        for_each_candidate(cell, G.ix, C, f);
         return;
     }
     const GridDesc& Gd = C.grid;
@@ -617,43 +697,26 @@ __device__ __forceinline__ void for_each_candidate_runs(const int4 cell, const G
                 const uint32_t row = Gd.base + (uint32_t)Gd.gx * (wy + (uint32_t)Gd.gy * wz);
                 const int wx = wrap(cell.x - 1, Gd.ox, Gd.gx);
                 if (wx + 2 < Gd.gx) {
-                    range(__ldg(G.off + row + wx), __ldg(G.off + row + wx + 3), row + wx, 3);
+                    range(__ldg(G.ix.off + row + wx), __ldg(G.ix.off + row + wx + 3), row + wx, 3);
                 } else {
                     for (int d = 0; d < 3; ++d) {
                         const uint32_t s = row + (uint32_t)wrap(cell.x - 1 + d, Gd.ox, Gd.gx);
-                        range(__ldg(G.off + s), __ldg(G.off + s + 1), s, 1);
+                        range(__ldg(G.ix.off + s), __ldg(G.ix.off + s + 1), s, 1);
                     }
                 }
             }
         }
     } else {
-        const uint32_t* row = G.btab + (size_t)(uint32_t)(cell.w - 1) * 27u;
+        const uint32_t* row = G.ix.btab + (size_t)(uint32_t)(cell.w - 1) * 27u;
         for (int k = 0; k < 27; ++k) {
             const uint32_t b0 = __ldg(row + k);
             if (b0 == kNoBucket) continue;
-            const uint32_t be = __ldg(G.bend + b0);
-            const uint32_t b1 = be & ~kImpureBit;
-            bool any = false;
-            if (!(be & kImpureBit) && b1 - b0 >= kRunRow) {
-                const int4 c = G.scell[__ldg(G.kpos + b0)];
-                any = (__ldg(G.slot_alias + slot_of(c.x, c.y, c.z, Gd)) & kRunSlot) != 0;
-            }
-            if (!any) {
-                for (uint32_t kq = b0; kq < b1; ++kq) f(__ldg(G.kpos + kq));
-                continue;
-            }
-            // One cell's members, in cell order: a run's particles follow its
-            // first one here too.
-            for (uint32_t kq = b0; kq < b1;) {
-                const uint32_t q = __ldg(G.kpos + kq);
-                if ((uint32_t)__ldg(G.sown + q) & kLeadBit) {
-                    const uint32_t L = __ldg(G.segend + q) - q;
-                    fr(q, L);
-                    kq += L;
-                } else {
-                    f(q);
-                    ++kq;
-                }
+            const uint32_t b1 = __ldg(G.ix.end + b0);
+            if (b0 < G.ix.n) {
+                const int4 c = G.scell[b0];
+                range(b0, b1, slot_of(c.x, c.y, c.z, Gd), 1);
+            } else {
+                for (uint32_t q = b0; q < b1; ++q) f(G.ix.at(q));
             }
         }
     }
@@ -786,15 +849,6 @@ struct TeamSmem {
 // (80 registers a thread).
 template <int BS>
 constexpr int kPassMinBlocks = 768 / BS;
-
-// An index of points that a walk visits: cell-order offsets, and the
-// reference buckets of the dirty cells.
-struct WalkIndex {
-    const uint32_t* __restrict__ off;
-    const uint32_t* __restrict__ kpos;
-    const uint32_t* __restrict__ bend;
-    const uint32_t* __restrict__ btab;
-};
 
 // A group: the cells [cx, cx + W - 3] of row (cy, cz), or one dirty cell
 // (own: its bucket row + 1).  split: the row would wrap in x, so its cells
@@ -931,12 +985,11 @@ __device__ __forceinline__ WalkRanges walk_ranges(const WalkGroup& Gr, const Wal
         if (lane < 27) {
             const uint32_t b0 = __ldg(I.btab + (size_t)(Gr.own - 1u) * 27u + (uint32_t)lane);
             if (b0 != kNoBucket) {
-                const uint32_t be = __ldg(I.bend + b0);
                 R.start = b0;
-                R.len = (be & ~kImpureBit) - b0;
+                R.len = __ldg(I.end + b0) - b0;
                 if constexpr (kRuns) {
-                    if (G.segend && R.len >= kRunRow && !(be & kImpureBit)) {
-                        const int4 c = G.scell[__ldg(I.kpos + b0)];
+                    if (G.segend && R.len >= kRunRow && b0 < I.n) {
+                        const int4 c = G.scell[b0];
                         R.runs = (__ldg(G.slot_alias + slot_of(c.x, c.y, c.z, Gd)) & kRunSlot) != 0;
                     }
                 }
@@ -1087,7 +1140,6 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
                 // particle, and the next one begins past the run.
                 uint32_t q = at_q + (uint32_t)lane;
                 const bool ok = (uint32_t)lane < cnt;
-                if (ok && key) q = __ldg(I.kpos + q);
                 const bool first = ok && ((uint32_t)__ldg(G.sown + q) & kLeadBit);
                 const uint32_t m = __ballot_sync(full, first);
                 if (m) {
@@ -1129,7 +1181,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
                 xj[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if ((uint32_t)lane < n) {
                     uint32_t q = sm.base[b + j] + (uint32_t)lane;
-                    if (key) q = __ldg(I.kpos + q);
+                    if (key) q = I.at(q);
                     xj[j] = ld_step<kPersist>(xin + q);
                 }
                 if constexpr (kLam) {
@@ -1192,7 +1244,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
                 uint32_t q = next_q();
                 const uint32_t i = sm.info[w];
                 const bool lead = (i & kLastLeads) && q - bq == (i & 63u) - 1u;
-                if (key) q = __ldg(I.kpos + q);
+                if (key) q = I.at(q);
                 float4 e{};
                 if constexpr (Sums::kExtra) e = sums.extra(q);
                 if (lead) sums.add_run(ld_step<kPersist>(xin + q), e, __ldg(G.segend + q) - q);
@@ -1202,7 +1254,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
             auto load = [&](float4& x, float4& e) {
                 uint32_t q = next_q();
-                if (key) q = __ldg(I.kpos + q);
+                if (key) q = I.at(q);
                 x = ld_step<kPersist>(xin + q);
                 if constexpr (Sums::kExtra) e = sums.extra(q);
             };
@@ -1444,13 +1496,13 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
             const uint32_t two = *reinterpret_cast<const uint32_t*>(my + t);
             if (t < cnt) {
                 uint32_t q = sm.base[(two >> 5) & (kTeamWords - 1)] + (two & 31u);
-                if (key) q = __ldg(I.kpos + q);
+                if (key) q = I.at(q);
                 xa = __ldg(xin + q);
                 if constexpr (Sums::kExtra) ea = sums.extra(q);
             }
             if (t + 1 < cnt) {
                 uint32_t q = sm.base[(two >> 21) & (kTeamWords - 1)] + ((two >> 16) & 31u);
-                if (key) q = __ldg(I.kpos + q);
+                if (key) q = I.at(q);
                 xb = __ldg(xin + q);
                 if constexpr (Sums::kExtra) eb = sums.extra(q);
             }
@@ -1491,7 +1543,7 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
                     xj[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                     if ((uint32_t)lane < n) {
                         uint32_t q = sm.base[b + j] + (uint32_t)lane;
-                        if (key) q = __ldg(I.kpos + q);
+                        if (key) q = I.at(q);
                         xj[j] = __ldg(xin + q);
                     }
                     if constexpr (kLam) {
@@ -1668,11 +1720,11 @@ __device__ __forceinline__ void team_walk(TeamSmem<TP>& sm, const Grid& G, const
 }
 
 __device__ __forceinline__ WalkIndex fluid_index(const Grid& G) {
-    return WalkIndex{G.off, G.kpos, G.bend, G.btab};
+    return G.ix;
 }
 
 __device__ __forceinline__ WalkIndex boundary_index(const Grid& G) {
-    return WalkIndex{G.bg.off, G.bg.kpos, G.bg.bend, G.bg.btab};
+    return WalkIndex{G.bg.n, G.bg.off, G.bg.merged, G.bg.end, G.bg.btab};
 }
 
 // Whether a slot among the 27 around a clean particle's cell holds the stamp
@@ -2145,8 +2197,8 @@ __device__ __forceinline__ void sum_boundary(WalkSmem& sm, const Grid& G, const 
     if (warp_walk<false, false, false>(sm, G, boundary_index(G), prm, p, bc, want, xi, G.bg.spos, sums))
         return;
     if (!want) return;
-    for_each_candidate<4>(bc, G.bg.off, G.bg.kpos, G.bg.bend, G.bg.btab, C,
-                          [&](uint32_t q) { sums.add(__ldg(G.bg.spos + q), float4{}); });
+    for_each_candidate(bc, boundary_index(G), C,
+                       [&](uint32_t q) { sums.add(__ldg(G.bg.spos + q), float4{}); });
 }
 
 // A thread of a team: its particle in the listing (pl; the same in all four
@@ -2598,8 +2650,7 @@ k_boundary_friction(const float4* __restrict__ xin, float4* __restrict__ sv, int
     const float4 xi = xin[p];
     const float4 vi = sv[p];
     float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-    for_each_candidate<4>(boundary_cell(G, p, cell_at(G, p)), G.bg.off, G.bg.kpos, G.bg.bend,
-                          G.bg.btab, C, [&](uint32_t q) {
+    for_each_candidate(boundary_cell(G, p, cell_at(G, p)), boundary_index(G), C, [&](uint32_t q) {
                               const float4 b = __ldg(G.bg.spos + q);
                               const float rx = xi.x - b.x, ry = xi.y - b.y, rz = xi.z - b.z;
                               const float r_sq = sqn(rx, ry, rz);
@@ -2832,7 +2883,7 @@ k_debug_neighbors(const float4* __restrict__ xin, const float4* __restrict__ sx,
     const float4 xi = xin[p];
     const uint32_t i = __float_as_uint(sx[p].w);
     long long k = fill ? offs[i] : 0;
-    for_each_candidate(cell_at(G, p), G.off, G.kpos, G.bend, G.btab, C, [&](uint32_t q) {
+    for_each_candidate(cell_at(G, p), G.ix, C, [&](uint32_t q) {
         if (q == p) return;
         const float4 xj = xin[q];
         if (sqn(xi.x - xj.x, xi.y - xj.y, xi.z - xj.z) < C.h2) {
@@ -2848,10 +2899,10 @@ k_debug_neighbors(const float4* __restrict__ xin, const float4* __restrict__ sx,
 
 inline int grid_of(int n, int b) { return (n + b - 1) / b; }
 
-inline Grid grid_view(const StepBuffers& B, const uint32_t* spid = nullptr,
+inline Grid grid_view(const StepBuffers& B, int n, const uint32_t* spid = nullptr,
                       const BoundaryGrid& bg = BoundaryGrid{}) {
-    return Grid{B.scell, B.sown, B.off, B.kpos, B.bend, B.btab, spid, B.moved, B.lamnz, bg,
-                spid ? nullptr : B.dhist, nullptr, B.slot_alias};
+    return Grid{B.scell, B.sown, WalkIndex{(uint32_t)n, B.off, B.bkt.merged, B.bkt.end, B.btab}, spid,
+                B.moved, B.lamnz, bg, spid ? nullptr : B.dhist, nullptr, B.slot_alias};
 }
 
 // predict, sort by cell and by reference key, cell offsets, gather, reference
@@ -2860,46 +2911,29 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
                                   cudaStream_t st, PhaseMarks* pm = nullptr) {
     const int n = C.n;
     const int nb = grid_of(n, kBlock);
-    StepConsts Cs = C;
-    Cs.seg_begin = 0;
-    Cs.seg_end = (uint32_t)n;
-    const OneScene one{Cs, StateRef{B.x, B.v, B.rho, B.lam, 0u, nullptr}};
+    const OneScene one{C, StateRef{B.x, B.v, B.rho, B.lam, 0u, nullptr}};
     const SceneIds none{nullptr, nullptr};
-    cudaError_t e = cudaMemsetAsync(B.slot_alias, 0, (size_t)C.grid.nslots, st);
-    if (e == cudaSuccess && B.moved) e = cudaMemsetAsync(B.moved, 0, (size_t)C.grid.nslots * 4, st);
-    if (e == cudaSuccess && B.lamnz) e = cudaMemsetAsync(B.lamnz, 0, (size_t)C.grid.nslots * 4, st);
-    if (e == cudaSuccess && B.dhist) {
-        // This step's density-pass counts become the previous step's.
-        e = cudaMemcpyAsync(B.dhist, B.dhist + 2 * kWalkHist, 2 * kWalkHist * 4,
-                            cudaMemcpyDeviceToDevice, st);
-        if (e == cudaSuccess) e = cudaMemsetAsync(B.dhist + 2 * kWalkHist, 0, 2 * kWalkHist * 4, st);
-    }
+    cudaError_t e = cudaMemsetAsync(B.slot_alias, 0, B.slot_bytes, st);
     if (e != cudaSuccess) return e;
     if (pm) pm->mark(-1, 0, st);
-    k_predict_key<<<nb, kBlock, 0, st>>>(B.keys, B.rkeys, n, none, one);
+    k_predict_key<<<nb, kBlock, 0, st>>>(B.keys, B.dhist, n, none, one);
     if (pm) pm->mark(kPhasePredict, 1, st);
     e = radix_sort_pairs(B.keys, B.skeys, B.sidx, n, C.grid.key_bits, sort, st);
     if (e != cudaSuccess) return e;
-    int launches = 2 + (C.grid.key_bits + 7) / 8;
-    if (C.hash_compat) {
-        e = radix_sort_pairs64(B.rkeys, B.rsorted, B.ridx, n, 64, sort, st);
-        if (e != cudaSuccess) return e;
-        launches += 9;
-    }
     k_offsets<<<grid_of((int)C.grid.nslots + 1, 256), 256, 0, st>>>(B.skeys, n, B.off, C.grid.nslots);
-    if (pm) pm->mark(kPhaseGridBuild, launches, st);
-    k_gather<<<nb, kBlock, 0, st>>>(B.sidx, B.sx, B.xa, B.srho, B.scell, B.pos_of, B.slot_alias,
+    if (pm) pm->mark(kPhaseGridBuild, 2 + (C.grid.key_bits + 7) / 8, st);
+    k_gather<<<nb, kBlock, 0, st>>>(B.sidx, B.sx, B.xa, B.srho, B.scell, B.bkt.link, B.slot_alias,
                                     B.err, n, none, one);
     if (C.hash_compat) {
-        e = enqueue_buckets(B.rsorted, B.ridx, B.pos_of, B.scell, nullptr, B.kpos, B.bend, n, st);
+        e = enqueue_buckets(sized_for(B.bkt, n), B.scell, B.sidx, nullptr, B.slot_alias, n, one, st);
         if (e != cudaSuccess) return e;
-        k_classify<<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, B.rsorted, B.kpos, B.bend,
-                                          B.slot_alias, B.btab, B.sown, nullptr, one);
+        k_classify<<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, nullptr, sized_for(B.bkt, n), B.slot_alias, B.btab,
+                                          B.sown, nullptr, one);
     } else {
         e = cudaMemsetAsync(B.sown, 0, (size_t)n * 4, st);
         if (e != cudaSuccess) return e;
     }
-    if (pm) pm->mark(kPhaseNeighborQuery, C.hash_compat ? 4 : 1, st);
+    if (pm) pm->mark(kPhaseNeighborQuery, C.hash_compat ? 5 : 1, st);
     return cudaGetLastError();
 }
 
@@ -3036,7 +3070,7 @@ inline cudaError_t enqueue_step(const StepBuffers& B, const StepConsts& C, int i
     Ci.iters = iters;
     BoundaryGrid bgs = bg ? *bg : BoundaryGrid{};
     if (bg) bgs.sx = B.sx;
-    Grid G = grid_view(B, nullptr, bgs);
+    Grid G = grid_view(B, n, nullptr, bgs);
     if (B.segend && n >= kBigScene) {
         // Runs of identical particles: from here on the owner words of the
         // run's later particles carry kCopyBit, which only the passes below
@@ -3055,20 +3089,6 @@ inline cudaError_t enqueue_step(const StepBuffers& B, const StepConsts& C, int i
 // ---------------------------------------------------------------------------
 // Batches of independent scenes: one sort and one launch per phase for all.
 
-// Reorders the key sort stably by scene: rsorted[p] = rtmp[perm[p]],
-// ridx[p] = itmp[perm[p]].
-__global__ void __launch_bounds__(256)
-k_apply_scene_perm(const unsigned long long* __restrict__ rtmp, const uint32_t* __restrict__ itmp,
-                   const uint32_t* __restrict__ perm, unsigned long long* __restrict__ rsorted,
-                   uint32_t* __restrict__ ridx, int n) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    uint32_t q = perm[p];
-    if (q >= (uint32_t)n) q = 0;
-    rsorted[p] = rtmp[q];
-    ridx[p] = itmp[q];
-}
-
 // pid[i] = the scene whose particle range holds batch particle i.
 __global__ void __launch_bounds__(256)
 k_scene_ids(const uint32_t* __restrict__ firsts, int nscenes, uint32_t* __restrict__ pid, int n) {
@@ -3083,16 +3103,6 @@ k_scene_ids(const uint32_t* __restrict__ firsts, int nscenes, uint32_t* __restri
     pid[i] = (uint32_t)a;
 }
 
-__global__ void __launch_bounds__(256)
-k_scene_of(const uint32_t* __restrict__ itmp, const uint32_t* __restrict__ pid,
-           uint32_t* __restrict__ stmp, int n) {
-    const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= n) return;
-    uint32_t i = itmp[p];
-    if (i >= (uint32_t)n) i = 0;
-    stmp[p] = pid[i];
-}
-
 inline cudaError_t enqueue_batch_step(const StepBuffers& B, const BatchDesc& D, SortScratch& sort,
                                       cudaStream_t st, PhaseMarks* pm = nullptr) {
     const int n = D.n;
@@ -3100,37 +3110,27 @@ inline cudaError_t enqueue_batch_step(const StepBuffers& B, const BatchDesc& D, 
     const int nb = grid_of(n, kBlock);
     const SceneTable tab{D.tab, D.refs};
     const SceneIds ids{D.pid, D.spid};
-    cudaError_t e = cudaMemsetAsync(B.slot_alias, 0, (size_t)D.nslots, st);
-    if (e == cudaSuccess && B.moved) e = cudaMemsetAsync(B.moved, 0, (size_t)D.nslots * 4, st);
-    if (e == cudaSuccess && B.lamnz) e = cudaMemsetAsync(B.lamnz, 0, (size_t)D.nslots * 4, st);
+    cudaError_t e = cudaMemsetAsync(B.slot_alias, 0, B.slot_bytes, st);
     if (e != cudaSuccess) return e;
     if (pm) pm->mark(-1, 0, st);
     k_scene_ids<<<grid_of(n, 256), 256, 0, st>>>(D.firsts, D.nscenes, D.pid, n);
-    k_predict_key<<<nb, kBlock, 0, st>>>(B.keys, B.rkeys, n, ids, tab);
+    k_predict_key<<<nb, kBlock, 0, st>>>(B.keys, nullptr, n, ids, tab);
     if (pm) pm->mark(kPhasePredict, 2, st);
     // Cell order: scene-major because every scene owns a slot range.
     e = radix_sort_pairs(B.keys, B.skeys, B.sidx, n, D.key_bits, sort, st);
     if (e != cudaSuccess) return e;
-    // Reference buckets per scene: sort by key, then stably by scene.
-    e = radix_sort_pairs64(B.rkeys, D.rtmp, D.itmp, n, 64, sort, st);
-    if (e != cudaSuccess) return e;
-    k_scene_of<<<grid_of(n, 256), 256, 0, st>>>(D.itmp, D.pid, D.stmp, n);
-    e = radix_sort_pairs(D.stmp, D.kpid, D.perm, n, D.scene_bits, sort, st);
-    if (e != cudaSuccess) return e;
-    k_apply_scene_perm<<<grid_of(n, 256), 256, 0, st>>>(D.rtmp, D.itmp, D.perm, B.rsorted, B.ridx,
-                                                        n);
     k_offsets<<<grid_of((int)D.nslots + 1, 256), 256, 0, st>>>(B.skeys, n, B.off, D.nslots);
-    if (pm) pm->mark(kPhaseGridBuild, 14 + (D.key_bits + 7) / 8 + (D.scene_bits + 7) / 8, st);
-    k_gather<<<nb, kBlock, 0, st>>>(B.sidx, B.sx, B.xa, B.srho, B.scell, B.pos_of, B.slot_alias,
+    if (pm) pm->mark(kPhaseGridBuild, 2 + (D.key_bits + 7) / 8, st);
+    k_gather<<<nb, kBlock, 0, st>>>(B.sidx, B.sx, B.xa, B.srho, B.scell, B.bkt.link, B.slot_alias,
                                     B.err, n, ids, tab);
-    e = enqueue_buckets(B.rsorted, B.ridx, B.pos_of, B.scell, D.kpid, B.kpos, B.bend, n, st);
+    e = enqueue_buckets(sized_for(B.bkt, n), B.scell, B.sidx, D.spid, B.slot_alias, n, tab, st);
     if (e != cudaSuccess) return e;
-    k_classify<<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, B.rsorted, B.kpos, B.bend, B.slot_alias,
-                                      B.btab, B.sown, D.spid, tab);
-    if (pm) pm->mark(kPhaseNeighborQuery, 4, st);
+    k_classify<<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, D.spid, sized_for(B.bkt, n), B.slot_alias, B.btab, B.sown,
+                                      D.spid, tab);
+    if (pm) pm->mark(kPhaseNeighborQuery, 5, st);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;
-    return enqueue_passes(B, grid_view(B, D.spid), n, D.max_iters, D.any_zero_iters, D.any_vort,
+    return enqueue_passes(B, grid_view(B, n, D.spid), n, D.max_iters, D.any_zero_iters, D.any_vort,
                           D.any_plain, D.xsph_on, tab, st, pm, D.persist_blocks, D.barrier,
                           D.block);
 }

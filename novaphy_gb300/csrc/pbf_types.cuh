@@ -58,8 +58,7 @@ struct StepConsts {
     int two_way;         // the boundary enters the constraint (coupled steps)
     float bfric;         // boundary friction coefficient of two-way steps (0: none)
     int iters;           // Jacobi iterations of this scene
-    uint32_t seg_begin;  // this scene's range in the key-sorted order of a batch
-    uint32_t seg_end;
+    uint32_t seg_begin;  // first particle of this scene in a batch
     GridDesc grid;
 };
 
@@ -70,9 +69,10 @@ struct StepConsts {
 // sorted position to its particle.  All null when the step has none.
 struct BoundaryGrid {
     const float4* spos = nullptr;
+    uint32_t n = 0;  // boundary particles
     const uint32_t* off = nullptr;
-    const uint32_t* kpos = nullptr;
-    const uint32_t* bend = nullptr;
+    const uint32_t* merged = nullptr;
+    const uint32_t* end = nullptr;
     const int* own = nullptr;
     const uint32_t* btab = nullptr;
     const float4* sx = nullptr;
@@ -85,6 +85,33 @@ struct BoundaryGrid {
     const float4* body_lin = nullptr;
     const float4* body_ang = nullptr;
 };
+
+// The reference's hash buckets over cell-sorted points.  A cell's points are
+// next to each other in cell order, in ascending index, as its bucket holds
+// them, so a bucket that only one cell's run hashes to is that run.  The runs
+// (stretches of equal cell; the cells of one slot may alternate where points
+// outside the grid box alias into it) go into a hash table by reference key;
+// the runs of one key are chained, and where there are several, their bucket
+// is written out in ascending point index.
+//
+// A bucket is a range [start, end[start]) of positions: below n, positions of
+// the cell order; from n on, entry position - n of `merged`.
+struct BucketTable {
+    uint32_t* end;     // 2 n: end of the run, or bucket, that starts here
+    uint32_t* rep;     // n: at a run's start, the first run of its bucket
+    uint32_t* link;    // n: at a run's start, the next run of its bucket (kNoBucket: none)
+    uint32_t* start;   // n: at a bucket's first run, the bucket's start
+    uint32_t* merged;  // n: cell-order positions of the merged buckets
+    // slots + 1 words, all ones before a build: runs by reference key (open
+    // addressing), then the merged positions handed out so far, less one.
+    uint32_t* table;
+    uint32_t slots;  // a power of two >= 2 n
+};
+constexpr uint32_t bucket_slots(uint32_t n) {
+    uint32_t s = 1024;
+    while (s < 2u * n && s < 0x80000000u) s <<= 1;
+    return s;
+}
 
 // Device buffers of one step.  Arrays named s* are in sorted (cell) order.
 struct StepBuffers {
@@ -106,15 +133,13 @@ struct StepBuffers {
     int4* scell;    // cell of x* at step start
     // Reference hash buckets (neighbor_search.cpp:14-22) for exact candidate
     // lists where they differ from the plain 27-cell neighbourhood.
-    unsigned long long* rkeys;    // reference key per particle, particle order
-    unsigned long long* rsorted;  // keys sorted (stable)
-    uint32_t* ridx;      // particle of key-sorted position
-    uint32_t* pos_of;    // cell-sorted position of each particle
-    uint32_t* kpos;      // cell-sorted position of each key-sorted position
-    uint32_t* bend;      // at bucket starts: bucket end | impure bit
-    uint32_t* btab;      // 27 bucket starts per dirty owner row
-    int* sown;           // 0 = clean, else owner row + 1
+    BucketTable bkt;
+    uint32_t* btab;  // 27 bucket starts per dirty owner row
+    int* sown;       // 0 = clean, else owner row + 1
     unsigned char* slot_alias;  // slot holds a particle from outside the grid box
+    // Bytes of slot_alias, moved and lamnz together (one range, zeroed by a
+    // step).
+    size_t slot_bytes;
     // Per slot: 1 + the Jacobi iteration whose delta pass last moved a
     // particle of the slot (0: none in this step).
     uint32_t* moved;
@@ -189,7 +214,6 @@ struct BatchDesc {
     int nscenes;
     uint32_t nslots;     // global slot space (sum of the scenes' grids)
     int key_bits;        // bits of a global slot
-    int scene_bits;      // bits of a scene id
     int max_iters;       // largest solver_iterations of the batch
     bool any_zero_iters, any_vort, any_plain, xsph_on;
     const StepConsts* tab;  // device tables, one entry per scene
@@ -197,11 +221,6 @@ struct BatchDesc {
     const uint32_t* firsts;    // nscenes + 1 particle offsets
     uint32_t* pid;             // scene of each particle (particle order)
     uint32_t* spid;            // scene of each cell-sorted particle
-    uint32_t* kpid;            // scene of each key-sorted particle
-    unsigned long long* rtmp;  // key-sorted keys before the scene pass
-    uint32_t* itmp;            // key-sorted particles before the scene pass
-    uint32_t* perm;            // scene-pass permutation
-    uint32_t* stmp;            // scenes of the key-sorted particles before the scene pass
     int persist_blocks;        // > 0: the Jacobi loop as one cooperative launch of this grid
     unsigned int* barrier;     // its grid barrier (count, generation)
     int block;                 // threads per block of the neighbour passes (64, 128, 256)

@@ -53,15 +53,14 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_
     return warp_excl + inc - v;
 }
 
-template <class K>
 __global__ void __launch_bounds__(kSortThreads)
-k_sort_histogram(const K* __restrict__ keys, int n, int passes, uint32_t* __restrict__ hist) {
+k_sort_histogram(const uint32_t* __restrict__ keys, int n, int passes, uint32_t* __restrict__ hist) {
     __shared__ uint32_t sh[kSortMaxPasses][256];
     for (int i = threadIdx.x; i < kSortMaxPasses * 256; i += blockDim.x) (&sh[0][0])[i] = 0u;
     __syncthreads();
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const K k = keys[i];
-        for (int p = 0; p < passes; ++p) atomicAdd(&sh[p][(uint32_t)(k >> (8 * p)) & 255u], 1u);
+        const uint32_t k = keys[i];
+        for (int p = 0; p < passes; ++p) atomicAdd(&sh[p][(k >> (8 * p)) & 255u], 1u);
     }
     __syncthreads();
     for (int i = threadIdx.x; i < passes * 256; i += blockDim.x) {
@@ -71,10 +70,9 @@ k_sort_histogram(const K* __restrict__ keys, int n, int passes, uint32_t* __rest
 }
 
 // One digit pass.  vals_in == nullptr means "values are the input positions".
-template <class K>
 __global__ void __launch_bounds__(kSortThreads)
-k_onesweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
-           K* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n, int shift,
+k_onesweep(const uint32_t* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
+           uint32_t* __restrict__ keys_out, uint32_t* __restrict__ vals_out, int n, int shift,
            const uint32_t* __restrict__ hist, uint32_t* lookback, uint32_t* tile_ctr,
            uint32_t* err) {
     __shared__ uint32_t s_tile;
@@ -82,7 +80,7 @@ k_onesweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     __shared__ uint32_t s_tile_excl[256];
     __shared__ uint32_t s_digit_base[256];
     __shared__ uint32_t s_scan[8];
-    __shared__ K s_keys[kSortTile];
+    __shared__ uint32_t s_keys[kSortTile];
     __shared__ uint32_t s_vals[kSortTile];
 
     const int tid = threadIdx.x;
@@ -98,14 +96,14 @@ k_onesweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
 
     // Load: warp w owns keys [base + 256w, base + 256w + 256), item k of lane l
     // at offset 32k + l, so ranking item by item keeps input order.
-    K key[kSortItems];
+    uint32_t key[kSortItems];
     uint32_t val[kSortItems], rank[kSortItems];
     bool valid[kSortItems];
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
         const long long idx = base + warp * (32 * kSortItems) + k * 32 + lane;
         valid[k] = idx < n;
-        key[k] = valid[k] ? keys_in[idx] : K(0);
+        key[k] = valid[k] ? keys_in[idx] : 0u;
         val[k] = valid[k] ? (vals_in ? vals_in[idx] : (uint32_t)idx) : 0u;
     }
 
@@ -114,7 +112,7 @@ k_onesweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     for (int k = 0; k < kSortItems; ++k) {
         const uint32_t vmask = __ballot_sync(0xffffffffu, valid[k]);
         if (valid[k]) {
-            const uint32_t d = (uint32_t)(key[k] >> shift) & 255u;
+            const uint32_t d = (key[k] >> shift) & 255u;
             const uint32_t peers = __match_any_sync(vmask, d);
             const uint32_t before = s_warp_hist[warp][d];
             rank[k] = before + __popc(peers & lt);
@@ -175,7 +173,7 @@ k_onesweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
 #pragma unroll
     for (int k = 0; k < kSortItems; ++k) {
         if (valid[k]) {
-            const uint32_t d = (uint32_t)(key[k] >> shift) & 255u;
+            const uint32_t d = (key[k] >> shift) & 255u;
             const uint32_t lp = s_tile_excl[d] + s_warp_hist[warp][d] + rank[k];
             if (lp < (uint32_t)kSortTile) {
                 s_keys[lp] = key[k];
@@ -188,8 +186,8 @@ k_onesweep(const K* __restrict__ keys_in, const uint32_t* __restrict__ vals_in,
     const long long rem = (long long)n - base;
     const int tile_n = rem < kSortTile ? (int)rem : kSortTile;
     for (int lp = tid; lp < tile_n; lp += kSortThreads) {
-        const K k = s_keys[lp];
-        const uint32_t d = (uint32_t)(k >> shift) & 255u;
+        const uint32_t k = s_keys[lp];
+        const uint32_t d = (k >> shift) & 255u;
         const uint32_t g = s_digit_base[d] + ((uint32_t)lp - s_tile_excl[d]);
         if (g < (uint32_t)n) {
             keys_out[g] = k;
@@ -205,69 +203,50 @@ void sort_scratch_bind(SortScratch& s, void* base, int capacity) {
     s.capacity = cap;
     s.tiles = (cap + kSortTile - 1) / kSortTile;
     char* p = reinterpret_cast<char*>(base);
-    s.keys_alt = reinterpret_cast<void*>(p);
-    p += sort_scratch_round((size_t)cap * 8);
+    s.keys_alt = reinterpret_cast<uint32_t*>(p);
+    p += sort_scratch_round((size_t)cap * 4);
     s.vals_alt = reinterpret_cast<uint32_t*>(p);
     p += sort_scratch_round((size_t)cap * 4);
-    s.zeroed = reinterpret_cast<uint32_t*>(p);
+    s.err = reinterpret_cast<uint32_t*>(p);
+    p += 64;
     s.hist = reinterpret_cast<uint32_t*>(p);
     p += (size_t)kSortMaxPasses * 256 * 4;
     s.tile_ctr = reinterpret_cast<uint32_t*>(p);
     p += 64;
-    s.err = reinterpret_cast<uint32_t*>(p);
-    p += 64;
     s.lookback = reinterpret_cast<uint32_t*>(p);
-    p += (size_t)kSortMaxPasses * (size_t)s.tiles * 256 * 4;
-    s.zeroed_bytes = (size_t)(p - reinterpret_cast<char*>(s.zeroed));
-}
-
-template <class K>
-static cudaError_t sort_impl(const K* keys_in, K* keys_out, uint32_t* vals_out, int n,
-                             int key_bits, SortScratch& s, cudaStream_t stream) {
-    if (n <= 0) return cudaSuccess;
-    if (n > s.capacity || n > (int)kValueMask) return cudaErrorInvalidValue;
-    int passes = (key_bits + 7) / 8;
-    if (passes < 1) passes = 1;
-    if (passes > (int)(sizeof(K) * 8 / 8) || passes > kSortMaxPasses) return cudaErrorInvalidValue;
-    const int tiles = (n + kSortTile - 1) / kSortTile;
-    // Zero the histograms and tile counters, and the look-back words of the
-    // tiles this sort uses; keep the error word (cleared by its owner).
-    cudaError_t e = cudaMemsetAsync(s.hist, 0, (size_t)kSortMaxPasses * 256 * 4 + 64, stream);
-    if (e != cudaSuccess) return e;
-    for (int p = 0; p < passes; ++p) {
-        e = cudaMemsetAsync(s.lookback + (size_t)p * s.tiles * 256, 0, (size_t)tiles * 256 * 4,
-                            stream);
-        if (e != cudaSuccess) return e;
-    }
-    int hist_blocks = (n + kSortThreads * 16 - 1) / (kSortThreads * 16);
-    if (hist_blocks > 1024) hist_blocks = 1024;
-    k_sort_histogram<K><<<hist_blocks, kSortThreads, 0, stream>>>(keys_in, n, passes, s.hist);
-    // Ping-pong so that the last pass writes keys_out / vals_out.
-    const K* kin = keys_in;
-    const uint32_t* vin = nullptr;
-    K* alt = reinterpret_cast<K*>(s.keys_alt);
-    for (int p = 0; p < passes; ++p) {
-        const bool to_out = ((passes - 1 - p) % 2) == 0;
-        K* kout = to_out ? keys_out : alt;
-        uint32_t* vout = to_out ? vals_out : s.vals_alt;
-        k_onesweep<K><<<tiles, kSortThreads, 0, stream>>>(
-            kin, vin, kout, vout, n, 8 * p, s.hist + p * 256,
-            s.lookback + (size_t)p * s.tiles * 256, s.tile_ctr + p, s.err);
-        kin = kout;
-        vin = vout;
-    }
-    return cudaGetLastError();
 }
 
 cudaError_t radix_sort_pairs(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out,
                              int n, int key_bits, SortScratch& s, cudaStream_t stream) {
-    return sort_impl<uint32_t>(keys_in, keys_out, vals_out, n, key_bits, s, stream);
-}
-
-cudaError_t radix_sort_pairs64(const unsigned long long* keys_in, unsigned long long* keys_out,
-                               uint32_t* vals_out, int n, int key_bits, SortScratch& s,
-                               cudaStream_t stream) {
-    return sort_impl<unsigned long long>(keys_in, keys_out, vals_out, n, key_bits, s, stream);
+    if (n <= 0) return cudaSuccess;
+    if (n > s.capacity || n > (int)kValueMask) return cudaErrorInvalidValue;
+    int passes = (key_bits + 7) / 8;
+    if (passes < 1) passes = 1;
+    if (passes > kSortMaxPasses) return cudaErrorInvalidValue;
+    const int tiles = (n + kSortTile - 1) / kSortTile;
+    // Zero the histograms, the tile counters and the look-back words of this
+    // sort's tiles; the error word is cleared by its owner.
+    cudaError_t e = cudaMemsetAsync(
+        s.hist, 0, (size_t)kSortMaxPasses * 256 * 4 + 64 + (size_t)passes * tiles * 256 * 4, stream);
+    if (e != cudaSuccess) return e;
+    int hist_blocks = (n + kSortThreads * 16 - 1) / (kSortThreads * 16);
+    if (hist_blocks > 1024) hist_blocks = 1024;
+    k_sort_histogram<<<hist_blocks, kSortThreads, 0, stream>>>(keys_in, n, passes, s.hist);
+    // Ping-pong so that the last pass writes keys_out / vals_out.
+    const uint32_t* kin = keys_in;
+    const uint32_t* vin = nullptr;
+    for (int p = 0; p < passes; ++p) {
+        const bool to_out = ((passes - 1 - p) % 2) == 0;
+        uint32_t* kout = to_out ? keys_out : s.keys_alt;
+        uint32_t* vout = to_out ? vals_out : s.vals_alt;
+        k_onesweep<<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, 8 * p,
+                                                       s.hist + p * 256,
+                                                       s.lookback + (size_t)p * tiles * 256,
+                                                       s.tile_ctr + p, s.err);
+        kin = kout;
+        vin = vout;
+    }
+    return cudaGetLastError();
 }
 
 }  // namespace pbf

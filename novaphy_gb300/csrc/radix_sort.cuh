@@ -22,18 +22,17 @@ namespace pbf {
 constexpr int kSortThreads = 256;
 constexpr int kSortItems = 8;
 constexpr int kSortTile = kSortThreads * kSortItems;  // 2048 keys per tile
-constexpr int kSortMaxPasses = 8;
+constexpr int kSortMaxPasses = 4;
 
 // Device scratch of one sorter, sized for `capacity` keys.
 struct SortScratch {
-    void* keys_alt = nullptr;      // ping-pong buffers (room for 64-bit keys)
+    uint32_t* keys_alt = nullptr;  // ping-pong buffers
     uint32_t* vals_alt = nullptr;
-    uint32_t* zeroed = nullptr;    // hist | tile counters | look-back | error word
-    size_t zeroed_bytes = 0;
+    uint32_t* err = nullptr;       // bit 0: look-back wait gave up
+    // One range, zeroed by a sort: hist | tile counters | look-back.
     uint32_t* hist = nullptr;      // [kSortMaxPasses][256]
     uint32_t* tile_ctr = nullptr;  // [kSortMaxPasses]
-    uint32_t* lookback = nullptr;  // [kSortMaxPasses][tiles][256]
-    uint32_t* err = nullptr;       // bit 0: look-back wait gave up
+    uint32_t* lookback = nullptr;  // [passes][tiles of the sort][256]
     int capacity = 0;
     int tiles = 0;
 };
@@ -45,11 +44,10 @@ constexpr size_t sort_scratch_round(size_t b) { return (b + 255) / 256 * 256; }
 constexpr size_t sort_scratch_bytes(int capacity) {
     const size_t cap = capacity > 0 ? (size_t)capacity : 1;
     const size_t tiles = (cap + kSortTile - 1) / kSortTile;
-    return sort_scratch_round(cap * 8)                      // alt keys (room for 64-bit)
-           + sort_scratch_round(cap * 4)                    // alt values
+    return 2 * sort_scratch_round(cap * 4)                  // alt keys and values
+           + 64                                             // error word
            + (size_t)kSortMaxPasses * 256 * 4               // hist
            + 64                                             // tile counters
-           + 64                                             // error word
            + (size_t)kSortMaxPasses * tiles * 256 * 4;      // look-back
 }
 // Carves the scratch out of one device allocation of sort_scratch_bytes().
@@ -60,9 +58,5 @@ void sort_scratch_bind(SortScratch& s, void* base, int capacity);
 // alias the outputs.  Returns a CUDA error code (cudaSuccess on success).
 cudaError_t radix_sort_pairs(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out,
                              int n, int key_bits, SortScratch& s, cudaStream_t stream);
-// Same for 64-bit keys (up to 8 digit passes).
-cudaError_t radix_sort_pairs64(const unsigned long long* keys_in, unsigned long long* keys_out,
-                               uint32_t* vals_out, int n, int key_bits, SortScratch& s,
-                               cudaStream_t stream);
 
 }  // namespace pbf

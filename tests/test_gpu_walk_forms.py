@@ -89,3 +89,28 @@ def test_plain_neighbourhood_away_from_the_axes(port_mt, n):
     w.x = (w.x + shift).astype(np.float32)
     lo, hi = (7.0,) * 3, tuple(7.0 + t for t in w.settings["domain_upper"])
     check(port_mt, w, 1, domain_lower=lo, domain_upper=hi, hash_compat=0)
+
+
+@pytest.mark.parametrize("n", [1, 700, 9000, 140000])
+def test_merged_buckets(port_mt, n):
+    # A block around the origin, where cells on both sides of the axes share reference keys; the scene held
+    # more particles before, and some leave the grid, so that runs of cells alternate within slots.
+    from oracle.oracle import Settings
+
+    big, w = block(n + 5000, seed=19), block(n, seed=17, vorticity=1e-4)
+    w.x = (w.x - w.x.mean(0)).astype(np.float32)
+    out = np.random.default_rng(21).random(n) < 0.03
+    w.v[out] *= np.float32(15.0 * w.settings["kernel_radius"] / w.dt)
+    half = tuple(0.75 * t for t in w.settings["domain_upper"])
+    st = dict(w.settings, domain_lower=tuple(-t for t in half), domain_upper=half)
+    sc = capi.Scene(capi.default_settings(**st, exact_arithmetic=1), big.x, big.v, mass=w.mass)
+    sc.set_gravity(w.gravity)
+    sc.step(w.dt, 1)
+    sc.reset(w.x, w.v)
+    sc.step(w.dt, 2)
+    got = sc.state()
+    sc.close()
+    z = np.zeros(w.n, np.float32)
+    want = port_mt.steps(Settings.make(**st), w.x, w.v, z, z, w.dt, w.gravity, w.mass, 2)
+    for name, a, b in zip("x v rho lam".split(), got, want):
+        assert np.array_equal(a, b), name
