@@ -40,31 +40,30 @@ k_ix_gather(const uint32_t* __restrict__ sidx, const float4* __restrict__ pos,
     if (!in_grid(cx, cy, cz, C.grid)) slot_alias[slot_of(cx, cy, cz, C.grid)] = kAliasSlot;
 }
 
+// Cells of the predicted positions of n particles.
 __global__ void __launch_bounds__(kBlock)
-k_predict_points(const float4* __restrict__ x, const float4* __restrict__ v, int n,
-                 float4* __restrict__ out, const StepConsts C) {
+k_predict_cells(const float4* __restrict__ x, const float4* __restrict__ v, int n,
+                int4* __restrict__ cells, const StepConsts C) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
     float px, py, pz;
     predict(x[i], v[i], C, px, py, pz);
-    out[i] = make_float4(px, py, pz, 0.0f);
-}
-
-__global__ void __launch_bounds__(kBlock)
-k_qcells(const float4* __restrict__ qpos, int nq, int4* __restrict__ qcell, const StepConsts C) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= nq) return;
-    const float4 q = qpos[i];
     int cx, cy, cz;
-    cell_of(q.x, q.y, q.z, C.inv_cell, cx, cy, cz);
-    qcell[i] = make_int4(cx, cy, cz, 0);
+    cell_of(px, py, pz, C.inv_cell, cx, cy, cz);
+    cells[i] = make_int4(cx, cy, cz, 0);
 }
 
 __device__ __forceinline__ WalkIndex index_of(const PointIndex& I, const QuerySet& Q) {
     return WalkIndex{(uint32_t)I.n, I.off, I.bkt.merged, I.bkt.end, Q.btab};
 }
 
-__device__ __forceinline__ int4 query_cell(const QuerySet& Q, int i) {
+// The walks' view of queries against an index: no scenes, stamps or runs.
+__device__ __forceinline__ Grid query_grid(const PointIndex& I, const QuerySet& Q) {
+    return Grid{nullptr, nullptr, index_of(I, Q), nullptr, nullptr, nullptr, BoundaryGrid{}, nullptr, nullptr,
+                nullptr};
+}
+
+__device__ __forceinline__ int4 query_cell(const QuerySet& Q, uint32_t i) {
     int4 c = Q.qcell[i];
     c.w = Q.qown[i];
     return c;
@@ -104,83 +103,220 @@ k_bxform(const float4* __restrict__ local, const int* __restrict__ body, int nb,
     }
 }
 
-__global__ void __launch_bounds__(kBlock)
-k_boundary_density(const float4* __restrict__ x, int n, const QuerySet Q, const PointIndex I,
-                   float* __restrict__ rho, const StepConsts C) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 xi = x[i];
-    float bd = 0.0f;
-    for_each_candidate(query_cell(Q, i), index_of(I, Q), C, [&](uint32_t q) {
-        const float4 b = __ldg(I.spos + q);
+// The coupling's sums run over cell-sorted queries (the fluid index's points
+// against the boundary's, and the other way round), so that a team's 8 or 16
+// queries sit in one cell or two; with one thread per query a few thousand
+// boundary points left most of the chip idle for 600 us.
+
+// Density of the boundary at a fluid point: sum_b rho0 psi_b W.
+struct PsiDensityTerm {
+    static constexpr int kQuantities = 1, kFactors = 1;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    __device__ __forceinline__ bool eval(const float4& b, const float4&, float* v, float* f) const {
         const float r_sq = sqn(xi.x - b.x, xi.y - b.y, xi.z - b.z);
-        bd += C.rho0 * b.w * poly6(r_sq, C);
-    });
-    rho[i] += bd;
-}
-
-__global__ void __launch_bounds__(kBlock)
-k_coupling(const float4* __restrict__ bworld, const int* __restrict__ body,
-           const int* __restrict__ body_dynamic, int nb, int nbodies, const QuerySet Q,
-           const PointIndex I, float4* __restrict__ Fb, const StepConsts C) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const int bi = body[b];
-    if (bi < 0 || bi >= nbodies || !body_dynamic[bi]) {
-        Fb[b] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
-        return;
+        if (!(r_sq < C.h2)) return false;
+        v[0] = poly6(r_sq, C);
+        f[0] = C.rho0 * b.w;
+        return true;
     }
-    const float4 xb = bworld[b];
-    const float psi_b = xb.w;
-    float fx = 0.0f, fy = 0.0f, fz = 0.0f;
-    for_each_candidate(query_cell(Q, b), index_of(I, Q), C, [&](uint32_t q) {
-        const float4 xf = __ldg(I.spos + q);
-        const float rx = xb.x - xf.x;
-        const float ry = xb.y - xf.y;
-        const float rz = xb.z - xf.z;
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&, const float4&,
+                                             float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.h2;
+        in_b = r.r2.y < C.h2;
+        v[0] = mul2(mul2(both(C.rho0), make_float2(xa.w, xb.w)), poly6_2(r.r2, C));
+    }
+};
+
+// Pressure force on a boundary point: sum_f (p_f rho0) psi_b grad W, with
+// p_f rho0 in the fluid point's w (pressure_weight) and psi_b in xi.w.
+struct PressureTerm {
+    static constexpr int kQuantities = 3, kFactors = 1;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    __device__ __forceinline__ bool eval(const float4& xf, const float4&, float* v, float* f) const {
+        const float rx = xi.x - xf.x, ry = xi.y - xf.y, rz = xi.z - xf.z;
         const float r_sq = sqn(rx, ry, rz);
-        if (r_sq >= C.h2) return;
-        const float rho_f = (xf.w < 1.0f) ? 1.0f : xf.w;  // std::max(rho, 1.0f)
-        const float pd = rho_f - C.rho0;
-        const float pressure = (0.0f < pd) ? pd : 0.0f;   // std::max(0.0f, rho - rho0)
-        const float pc = C.mass * pressure / (rho_f * rho_f);
+        if (!(r_sq < C.h2)) return false;
         const float c = spiky_coeff(r_sq, C);
-        const float a = pc * C.rho0 * psi_b;
-        fx += a * (c * rx);
-        fy += a * (c * ry);
-        fz += a * (c * rz);
-    });
-    Fb[b] = make_float4(fx, fy, fz, sqn(fx, fy, fz) > 1e-20f ? 1.0f : 0.0f);
+        f[0] = xf.w * xi.w;
+        v[0] = c * rx;
+        v[1] = c * ry;
+        v[2] = c * rz;
+        return true;
+    }
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&, const float4&,
+                                             float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.h2;
+        in_b = r.r2.y < C.h2;
+        const float2 c = spiky_coeff_2(r.r2, C);
+        const float2 a = mul2(make_float2(xa.w, xb.w), both(xi.w));
+        v[0] = mul2(a, mul2(c, r.x));
+        v[1] = mul2(a, mul2(c, r.y));
+        v[2] = mul2(a, mul2(c, r.z));
+    }
+};
+
+// sum_b W over the boundary itself (Akinci volumes).
+struct VolumeTerm {
+    static constexpr int kQuantities = 1, kFactors = 1;
+    static constexpr bool kExtra = false;
+    const StepConsts& C;
+    const float4 xi;
+    static __host__ __device__ constexpr int factor_of(int) { return -1; }
+    __device__ __forceinline__ bool eval(const float4& b, const float4&, float* v, float* f) const {
+        const float r_sq = sqn(xi.x - b.x, xi.y - b.y, xi.z - b.z);
+        if (!(r_sq < C.h2)) return false;
+        v[0] = poly6(r_sq, C);
+        f[0] = 1.0f;
+        return true;
+    }
+    __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&, const float4&,
+                                             float2* v, bool& in_a, bool& in_b) const {
+        const PairRel r(xi, xa, xb, C.one);
+        in_a = r.r2.x < C.h2;
+        in_b = r.r2.y < C.h2;
+        v[0] = poly6_2(r.r2, C);
+    }
+};
+
+// pc rho0 of a fluid particle of density rho, as the reference's force loop
+// computes it for each pair (fluid_world.cpp:147-155): zero where the fluid is
+// not compressed, so such a particle adds exact zeros and is not listed.
+__device__ __forceinline__ float pressure_weight(float rho, const StepConsts& C) {
+    const float rho_f = (rho < 1.0f) ? 1.0f : rho;   // std::max(rho, 1.0f)
+    const float pd = rho_f - C.rho0;
+    const float pressure = (0.0f < pd) ? pd : 0.0f;  // std::max(0.0f, rho - rho0)
+    const float pc = C.mass * pressure / (rho_f * rho_f);
+    return pc * C.rho0;
 }
 
-__global__ void k_body_reduce(const float4* __restrict__ Fb, const float4* __restrict__ bworld,
-                              const int* __restrict__ list_off, const int* __restrict__ list,
-                              const float4* __restrict__ body_pos, int nbodies,
-                              float* __restrict__ force3, float* __restrict__ torque3) {
-    const int k = blockIdx.x * blockDim.x + threadIdx.x;
-    if (k >= nbodies) return;
-    float f0 = force3[3 * k], f1 = force3[3 * k + 1], f2 = force3[3 * k + 2];
-    float t0 = torque3[3 * k], t1 = torque3[3 * k + 1], t2 = torque3[3 * k + 2];
-    const float4 c = body_pos[k];
-    for (int j = list_off[k]; j < list_off[k + 1]; ++j) {
-        const int b = list[j];
-        const float4 F = Fb[b];
-        if (F.w == 0.0f) continue;
-        f0 += F.x;
-        f1 += F.y;
-        f2 += F.z;
-        const float4 x = bworld[b];
-        const float r0 = x.x - c.x, r1 = x.y - c.y, r2 = x.z - c.z;
-        t0 += r1 * F.z - r2 * F.y;
-        t1 += r2 * F.x - r0 * F.z;
-        t2 += r0 * F.y - r1 * F.x;
+// Boundary density of the fluid index's points: rho += sum, in particle order,
+// and the points' w from the density to the pressure weight.
+template <int TP>
+__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+k_boundary_density(float4* __restrict__ fpos, const uint32_t* __restrict__ fidx, int n, const QuerySet Q,
+                   const PointIndex I, float* __restrict__ rho, const StepConsts C) {
+    __shared__ TeamSmem<TP> sm;
+    const TeamThread<TP> T(n);
+    const Grid G = query_grid(I, Q);
+    const float4 xi = fpos[T.pe];
+    TeamSums<PsiDensityTerm, 128 / TP> sums(PsiDensityTerm{C, xi});
+    team_walk<TP, false>(sm, G, G.ix, OneScene{C, StateRef{}}, T.pl, query_cell(Q, T.pl), T.al, fpos[T.pl], I.spos,
+                         sums);
+    const float bd = sums.get(0);
+    if (T.writer) {
+        const float r = xi.w + bd;
+        const uint32_t i = fidx[T.pe];
+        if (i < (uint32_t)n) rho[i] = r;
+        fpos[T.pe].w = pressure_weight(r, C);
     }
-    force3[3 * k] = f0;
-    force3[3 * k + 1] = f1;
-    force3[3 * k + 2] = f2;
-    torque3[3 * k] = t0;
-    torque3[3 * k + 1] = t1;
-    torque3[3 * k + 2] = t2;
+}
+
+// The same change of w where the densities already hold the boundary's share.
+__global__ void __launch_bounds__(kBlock)
+k_pressure_weights(float4* __restrict__ fpos, int n, const StepConsts C) {
+    const int p = blockIdx.x * blockDim.x + threadIdx.x;
+    if (p < n) fpos[p].w = pressure_weight(fpos[p].w, C);
+}
+
+// Force on each boundary point (bpos, bidx: the boundary index's points and
+// their original numbers) from the fluid index I.
+template <int TP>
+__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+k_coupling(const float4* __restrict__ bpos, const uint32_t* __restrict__ bidx, const int* __restrict__ body,
+           const int* __restrict__ body_dynamic, int nb, int nbodies, const QuerySet Q, const PointIndex I,
+           float4* __restrict__ Fb, const StepConsts C) {
+    __shared__ TeamSmem<TP> sm;
+    const TeamThread<TP> T(nb);
+    const Grid G = query_grid(I, Q);
+    auto feels = [&](uint32_t p) {
+        const uint32_t b = bidx[p];
+        const int bi = b < (uint32_t)nb ? body[b] : -1;
+        return bi >= 0 && bi < nbodies && body_dynamic[bi];
+    };
+    const float4 xi = bpos[T.pe];
+    float4 xl = bpos[T.pl];
+    xl.w = 0.0f;  // lists candidates with a nonzero weight only
+    TeamSums<PressureTerm, 128 / TP> sums(PressureTerm{C, xi});
+    team_walk<TP, true>(sm, G, G.ix, OneScene{C, StateRef{}}, T.pl, query_cell(Q, T.pl), T.al && feels(T.pl), xl,
+                        I.spos, sums);
+    const float fx = sums.get(0), fy = sums.get(1), fz = sums.get(2);
+    if (T.writer) {
+        const uint32_t b = bidx[T.pe];
+        if (b < (uint32_t)nb)
+            Fb[b] = make_float4(fx, fy, fz, feels(T.pe) && sqn(fx, fy, fz) > 1e-20f ? 1.0f : 0.0f);
+    }
+}
+
+// Per body, its boundary points' forces and torques added in boundary order
+// (the reference's): a block per body computes the terms side by side, 256 at
+// a time, and lane k of the first warp adds component k.  One thread per body
+// took 524 us for eight bodies of about 1,000 points, waiting on three
+// dependent loads per point.
+constexpr int kReduceThreads = 256;
+
+__global__ void __launch_bounds__(kReduceThreads)
+k_body_reduce(const float4* __restrict__ Fb, const float4* __restrict__ bworld,
+              const int* __restrict__ list_off, const int* __restrict__ list,
+              const float4* __restrict__ body_pos, int nbodies, float* __restrict__ force3,
+              float* __restrict__ torque3) {
+    __shared__ __align__(16) float term[6][kReduceThreads];
+    __shared__ uint32_t has[kReduceThreads / 32];
+    const int k = blockIdx.x, t = threadIdx.x;
+    if (k >= nbodies) return;
+    const float4 c = body_pos[k];
+    const int j1 = list_off[k + 1];
+    float sum = 0.0f;
+    if (t < 3) sum = force3[3 * k + t];
+    else if (t < 6) sum = torque3[3 * k + t - 3];
+    for (int j0 = list_off[k]; j0 < j1; j0 += kReduceThreads) {
+        const int j = j0 + t;
+        float4 F = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+        if (j < j1) {
+            const int b = __ldg(list + j);
+            F = __ldg(Fb + b);
+            if (F.w != 0.0f) {
+                const float4 x = __ldg(bworld + b);
+                const float r0 = x.x - c.x, r1 = x.y - c.y, r2 = x.z - c.z;
+                term[0][t] = F.x;
+                term[1][t] = F.y;
+                term[2][t] = F.z;
+                term[3][t] = r1 * F.z - r2 * F.y;
+                term[4][t] = r2 * F.x - r0 * F.z;
+                term[5][t] = r0 * F.y - r1 * F.x;
+            }
+        }
+        const uint32_t m = __ballot_sync(0xffffffffu, F.w != 0.0f);
+        if ((t & 31) == 0) has[t >> 5] = m;
+        __syncthreads();
+        if (t < 6) {
+            for (int w = 0; w < kReduceThreads / 32; ++w) {
+                const uint32_t bits = has[w];
+                if (bits == 0xffffffffu) {
+#pragma unroll
+                    for (int i = 0; i < 32; i += 4) {
+                        const float4 v = *reinterpret_cast<const float4*>(&term[t][32 * w + i]);
+                        sum = sum + v.x;
+                        sum = sum + v.y;
+                        sum = sum + v.z;
+                        sum = sum + v.w;
+                    }
+                } else {
+                    for (uint32_t b = bits; b; b &= b - 1u) sum = sum + term[t][32 * w + __ffs(b) - 1];
+                }
+            }
+        }
+        __syncthreads();
+    }
+    if (t < 3) force3[3 * k + t] = sum;
+    else if (t < 6) torque3[3 * k + t - 3] = sum;
 }
 
 // Segmented tree reduction of the same sums: one block per body.  Thread t
@@ -284,19 +420,25 @@ k_rigid_world(pbf_rigid_body* __restrict__ bodies, int nbodies,
     }
 }
 
-__global__ void __launch_bounds__(kBlock)
-k_volumes(const float4* __restrict__ world, int nb, const QuerySet Q, const PointIndex I,
-          float* __restrict__ psi, const StepConsts C) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nb) return;
-    const float4 xb = world[b];
-    float sum_w = 0.0f;
-    for_each_candidate(query_cell(Q, b), index_of(I, Q), C, [&](uint32_t q) {
-        const float4 xj = __ldg(I.spos + q);
-        sum_w += poly6(sqn(xb.x - xj.x, xb.y - xj.y, xb.z - xj.z), C);
-    });
-    psi[b] = (sum_w > 1e-10f) ? 1.0f / sum_w : 0.0f;
+template <int TP>
+__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+k_volumes(int nb, const QuerySet Q, const PointIndex I, float* __restrict__ psi, const StepConsts C) {
+    __shared__ TeamSmem<TP> sm;
+    const TeamThread<TP> T(nb);
+    const Grid G = query_grid(I, Q);
+    const float4 xi = I.spos[T.pe];
+    TeamSums<VolumeTerm, 128 / TP> sums(VolumeTerm{C, xi});
+    team_walk<TP, false>(sm, G, G.ix, OneScene{C, StateRef{}}, T.pl, query_cell(Q, T.pl), T.al, I.spos[T.pl],
+                         I.spos, sums);
+    const float sum_w = sums.get(0);
+    if (T.writer) {
+        const uint32_t b = I.sidx[T.pe];
+        if (b < (uint32_t)nb) psi[b] = (sum_w > 1e-10f) ? 1.0f / sum_w : 0.0f;
+    }
 }
+
+// Queries per team: as the step's passes, with teams at every size.
+inline bool small_teams(int nq) { return team_size(nq) == 8; }
 
 }  // namespace bnd
 
@@ -317,27 +459,27 @@ cudaError_t index_build(PointIndex& I, const float4* pos, const float* attr, int
     return enqueue_buckets(sized_for(I.bkt, n), I.scell, I.sidx, nullptr, I.slot_alias, n, OneScene{C, StateRef{}}, st);
 }
 
-cudaError_t predict_points(const float4* x, const float4* v, int n, float4* out,
-                           const StepConsts& C, cudaStream_t st) {
+cudaError_t predict_cells(const float4* x, const float4* v, int n, int4* cells, const StepConsts& C,
+                          cudaStream_t st) {
     using namespace bnd;
     if (n <= 0) return cudaSuccess;
-    k_predict_points<<<grid_of(n, kBlock), kBlock, 0, st>>>(x, v, n, out, C);
+    k_predict_cells<<<grid_of(n, kBlock), kBlock, 0, st>>>(x, v, n, cells, C);
     return cudaGetLastError();
 }
 
-cudaError_t index_classify(const QuerySet& Q, const float4* qpos, int nq, const PointIndex& I,
-                           const StepConsts& C, cudaStream_t st) {
+cudaError_t index_classify(const QuerySet& Q, int nq, const PointIndex& I, const StepConsts& C,
+                           cudaStream_t st) {
     using namespace bnd;
     if (nq <= 0) return cudaSuccess;
-    k_qcells<<<grid_of(nq, kBlock), kBlock, 0, st>>>(qpos, nq, Q.qcell, C);
     if (I.n <= 0) {
         // Nothing to find: every neighbour bucket is empty.
         return cudaMemsetAsync(Q.qown, 0, (size_t)nq * sizeof(int), st);
     }
     StepConsts Cs = C;
     Cs.hash_compat = 1;  // the coupling queries always follow the reference buckets
-    k_classify<<<grid_of(nq, kBlock), kBlock, 0, st>>>(Q.qcell, nq, I.scell, nullptr, sized_for(I.bkt, I.n), I.slot_alias,
-                                                        Q.btab, Q.qown, nullptr, OneScene{Cs, StateRef{}});
+    k_classify<<<grid_of(nq, kBlock), kBlock, 0, st>>>(Q.qcell, nq, I.scell, nullptr, sized_for(I.bkt, I.n),
+                                                       I.slot_alias, Q.btab, Q.qown, nullptr,
+                                                       OneScene{Cs, StateRef{}});
     return cudaGetLastError();
 }
 
@@ -350,22 +492,33 @@ cudaError_t boundary_xform(const float4* local, const int* body, int nb, const f
     return cudaGetLastError();
 }
 
-cudaError_t boundary_density(const float4* x, int n, const QuerySet& Q, const PointIndex& bidx,
-                             float* rho, const StepConsts& C, cudaStream_t st) {
+cudaError_t boundary_density(const PointIndex& fidx, const QuerySet& Q, const PointIndex& bidx,
+                             float* rho, bool has_boundary, const StepConsts& C, cudaStream_t st) {
     using namespace bnd;
-    if (n <= 0 || bidx.n <= 0) return cudaSuccess;
-    k_boundary_density<<<grid_of(n, kBlock), kBlock, 0, st>>>(x, n, Q, bidx, rho, C);
+    const int n = fidx.n;
+    if (n <= 0) return cudaSuccess;
+    if (has_boundary || bidx.n <= 0)
+        k_pressure_weights<<<grid_of(n, kBlock), kBlock, 0, st>>>(fidx.spos, n, C);
+    else if (small_teams(n))
+        k_boundary_density<8><<<grid_of(n, 8), 128, 0, st>>>(fidx.spos, fidx.sidx, n, Q, bidx, rho, C);
+    else
+        k_boundary_density<16><<<grid_of(n, 16), 128, 0, st>>>(fidx.spos, fidx.sidx, n, Q, bidx, rho, C);
     return cudaGetLastError();
 }
 
-cudaError_t coupling_forces(const float4* bworld, const int* body, const int* body_dynamic,
-                            int nb, int nbodies, const QuerySet& Q, const PointIndex& fidx,
-                            float4* Fb, const StepConsts& C, cudaStream_t st) {
+cudaError_t coupling_forces(const PointIndex& bidx, const int* body, const int* body_dynamic, int nbodies,
+                            const QuerySet& Q, const PointIndex& fidx, float4* Fb, const StepConsts& C,
+                            cudaStream_t st) {
     using namespace bnd;
+    const int nb = bidx.n;
     if (nb <= 0) return cudaSuccess;
     if (fidx.n <= 0) return cudaMemsetAsync(Fb, 0, (size_t)nb * sizeof(float4), st);
-    k_coupling<<<grid_of(nb, kBlock), kBlock, 0, st>>>(bworld, body, body_dynamic, nb, nbodies, Q,
-                                                       fidx, Fb, C);
+    if (small_teams(nb))
+        k_coupling<8><<<grid_of(nb, 8), 128, 0, st>>>(bidx.spos, bidx.sidx, body, body_dynamic, nb, nbodies, Q,
+                                                      fidx, Fb, C);
+    else
+        k_coupling<16><<<grid_of(nb, 16), 128, 0, st>>>(bidx.spos, bidx.sidx, body, body_dynamic, nb, nbodies,
+                                                        Q, fidx, Fb, C);
     return cudaGetLastError();
 }
 
@@ -378,8 +531,8 @@ cudaError_t body_reduce(const float4* Fb, const float4* bworld, const int* list_
         k_body_reduce_tree<<<nbodies, kTreeThreads, 0, st>>>(Fb, bworld, list_off, list, body_pos,
                                                              nbodies, force3, torque3);
     else
-        k_body_reduce<<<grid_of(nbodies, 32), 32, 0, st>>>(Fb, bworld, list_off, list, body_pos,
-                                                           nbodies, force3, torque3);
+        k_body_reduce<<<nbodies, kReduceThreads, 0, st>>>(Fb, bworld, list_off, list, body_pos,
+                                                          nbodies, force3, torque3);
     return cudaGetLastError();
 }
 
@@ -404,11 +557,15 @@ cudaError_t rigid_step(pbf_rigid_body* bodies, int nbodies, const float* force3,
     return cudaGetLastError();
 }
 
-cudaError_t boundary_volumes(const float4* world, int nb, const QuerySet& Q, const PointIndex& I,
-                             float* psi, const StepConsts& C, cudaStream_t st) {
+cudaError_t boundary_volumes(const QuerySet& Q, const PointIndex& I, float* psi, const StepConsts& C,
+                             cudaStream_t st) {
     using namespace bnd;
+    const int nb = I.n;
     if (nb <= 0) return cudaSuccess;
-    k_volumes<<<grid_of(nb, kBlock), kBlock, 0, st>>>(world, nb, Q, I, psi, C);
+    if (small_teams(nb))
+        k_volumes<8><<<grid_of(nb, 8), 128, 0, st>>>(nb, Q, I, psi, C);
+    else
+        k_volumes<16><<<grid_of(nb, 16), 128, 0, st>>>(nb, Q, I, psi, C);
     return cudaGetLastError();
 }
 

@@ -41,34 +41,37 @@ struct QuerySet {
 cudaError_t index_build(PointIndex& I, const float4* pos, const float* attr, int n,
                         const StepConsts& C, SortScratch& sort, cudaStream_t st);
 
-// x* = x + (v + g dt) dt of n particles (w = 0): the positions whose cells
-// a step sorts by (the predict of k_predict_key, the same operations).
-cudaError_t predict_points(const float4* x, const float4* v, int n, float4* out,
-                           const StepConsts& C, cudaStream_t st);
+// Cells of x* = x + (v + g dt) dt of n particles, which a step sorts by (the
+// predict of k_predict_key, the same operations).
+cudaError_t predict_cells(const float4* x, const float4* v, int n, int4* cells, const StepConsts& C,
+                          cudaStream_t st);
 
-// Classifies query points qpos[0..nq) against `I`.
-cudaError_t index_classify(const QuerySet& Q, const float4* qpos, int nq, const PointIndex& I,
-                           const StepConsts& C, cudaStream_t st);
+// Classifies the nq query points in cells Q.qcell against `I`.
+cudaError_t index_classify(const QuerySet& Q, int nq, const PointIndex& I, const StepConsts& C,
+                           cudaStream_t st);
 
 // x_b = T[body] * local (boundary.cpp:178-192); w carries psi.
 cudaError_t boundary_xform(const float4* local, const int* body, int nb, const float4* body_pos,
                            const float4* body_quat, int nbodies, float4* world, cudaStream_t st);
 
 // rho_i += sum_b rho0 psi_b poly6(|x_i - x_b|^2) over boundary buckets
-// (fluid_world.cpp:101-123); x and rho in particle order.
-cudaError_t boundary_density(const float4* x, int n, const QuerySet& Q, const PointIndex& bidx,
-                             float* rho, const StepConsts& C, cudaStream_t st);
+// (fluid_world.cpp:101-123) for the points of the fluid index, whose w is
+// rho_i; Q: those points against `bidx`; rho in particle order.  The points' w
+// becomes their weight in coupling_forces.  has_boundary: the densities
+// already hold the boundary's share, only w changes.
+cudaError_t boundary_density(const PointIndex& fidx, const QuerySet& Q, const PointIndex& bidx,
+                             float* rho, bool has_boundary, const StepConsts& C, cudaStream_t st);
 
 // Per-boundary-particle pressure force from the fluid (fluid_world.cpp:
-// 136-161); fidx indexes final fluid positions with w = density.
-// Fb[b].w = 1 when |F_b|^2 > 1e-20 (the reference's apply threshold).
-cudaError_t coupling_forces(const float4* bworld, const int* body, const int* body_dynamic,
-                            int nb, int nbodies, const QuerySet& Q, const PointIndex& fidx,
-                            float4* Fb, const StepConsts& C, cudaStream_t st);
+// 136-161), in boundary order; Q: the boundary index's points against `fidx`,
+// after boundary_density.  Fb[b].w = 1 when |F_b|^2 > 1e-20 (the reference's
+// apply threshold).
+cudaError_t coupling_forces(const PointIndex& bidx, const int* body, const int* body_dynamic, int nbodies,
+                            const QuerySet& Q, const PointIndex& fidx, float4* Fb, const StepConsts& C,
+                            cudaStream_t st);
 
 // force/torque[k] += F_b, (x_b - p_k) x F_b over body k's boundary particles.
-// tree = false: one thread per body adds them in ascending b, the reference's
-// order (fluid_world.cpp:163-172 + World::apply_force/torque), bit for bit.
+// tree = false: they are added in ascending b, the reference's order (fluid_world.cpp:163-172 + World::apply_force/torque), bit for bit.
 // tree = true: a deterministic segmented tree reduction (one block per body,
 // fixed pairing), within 2 (m - 1) 2^-24 sum_b |term_b| of the serial sum for
 // a body of m terms.
@@ -93,8 +96,9 @@ cudaError_t rigid_world(pbf_rigid_body* bodies, int nbodies, const pbf_rigid_sha
                         const float* torque3, int nforce, float gx, float gy, float gz, float dt,
                         float4* body_pos, float4* body_quat, cudaStream_t st);
 
-// psi_b = 1 / sum_b' poly6 (0 when the sum <= 1e-10), boundary.cpp:152-176.
-cudaError_t boundary_volumes(const float4* world, int nb, const QuerySet& Q, const PointIndex& I,
-                             float* psi, const StepConsts& C, cudaStream_t st);
+// psi_b = 1 / sum_b' poly6 (0 when the sum <= 1e-10), boundary.cpp:152-176, in
+// the order of the indexed points; Q: the index's points against itself.
+cudaError_t boundary_volumes(const QuerySet& Q, const PointIndex& I, float* psi, const StepConsts& C,
+                             cudaStream_t st);
 
 }  // namespace pbf

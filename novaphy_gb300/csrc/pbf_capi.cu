@@ -651,8 +651,7 @@ int pbf_scene_destroy(pbf_scene* s) {
     {
         DeviceGuard dg(s->device);
         if (s->stream) cudaStreamSynchronize(s->stream);
-        for (void* m : {s->bnd.mem, s->bnd.body_mem, s->bnd.sort_mem, s->bnd.fq_mem,
-                        s->bnd.tw_mem, static_cast<void*>(s->bnd.rb),
+        for (void* m : {s->bnd.mem, s->bnd.body_mem, s->bnd.sort_mem, s->bnd.tw_mem, static_cast<void*>(s->bnd.rb),
                         static_cast<void*>(s->bnd.shapes)})
             if (m) cudaFree(m);
         if (s->bnd.idx.off) cudaFree(s->bnd.idx.off);
@@ -1177,7 +1176,7 @@ int alloc_boundary(pbf_scene* s, int nb) {
     const int c = nb > 0 ? nb : 1;
     const size_t f4 = align_up((size_t)c * 16, 256), f1 = align_up((size_t)c * 4, 256),
                  f27 = align_up((size_t)c * 27 * 4, 256);
-    const size_t total = 6 * f4 + 5 * f1 + bucket_bytes(c) + f27;
+    const size_t total = 5 * f4 + 5 * f1 + bucket_bytes(c) + f27;
     PBF_CUDA(cudaMalloc(&b.mem, total));
     char* p = reinterpret_cast<char*>(b.mem);
     auto take = [&](size_t n) { char* r = p; p += n; return r; };
@@ -1186,7 +1185,7 @@ int alloc_boundary(pbf_scene* s, int nb) {
     b.Fb = reinterpret_cast<float4*>(take(f4));
     b.idx.spos = reinterpret_cast<float4*>(take(f4));
     b.idx.scell = reinterpret_cast<int4*>(take(f4));
-    b.bq.qcell = reinterpret_cast<int4*>(take(f4));
+    b.bq.qcell = b.idx.scell;
     b.body = reinterpret_cast<int*>(take(f1));
     b.idx.keys = reinterpret_cast<uint32_t*>(take(f1));
     b.idx.skeys = reinterpret_cast<uint32_t*>(take(f1));
@@ -1213,19 +1212,6 @@ int ensure_boundary_grid(pbf_scene* s, uint32_t nslots) {
     PBF_CUDA(cudaMalloc(&b.idx.off, ob + align_up(nslots, 256)));
     b.idx.slot_alias = reinterpret_cast<unsigned char*>(b.idx.off) + ob;
     b.idx_slots = nslots;
-    return PBF_OK;
-}
-
-int ensure_fluid_queries(pbf_scene* s) {
-    auto& b = s->bnd;
-    if (b.fq_mem && b.fq_cap >= s->n) return PBF_OK;
-    ++s->buf_gen;
-    if (b.fq_mem) cudaFree(b.fq_mem);
-    b.fq_mem = nullptr;
-    const int c = s->n > 0 ? s->n : 1;
-    PBF_CUDA(cudaMalloc(&b.fq_mem, (size_t)c * 16));
-    b.fq_cell = reinterpret_cast<int4*>(b.fq_mem);
-    b.fq_cap = c;
     return PBF_OK;
 }
 
@@ -1369,23 +1355,12 @@ int enqueue_coupling(pbf_scene* s, const StepConsts& C, const float* force_in,
                                    b.world, st);
     if (e == cudaSuccess) e = mark(1);
     if (e != cudaSuccess) return cuda_fail(e, "boundary_xform");
-    // 2. boundary density on the final positions (fluid_world.cpp:101-123)
+    // 2. boundary density on the final positions (fluid_world.cpp:101-123),
+    //    over a fresh fluid index on them; the step's sorted buffers are free
+    //    now.
     int rc = ensure_boundary_grid(s, C.grid.nslots);
     if (rc) return rc;
-    rc = ensure_fluid_queries(s);
-    if (rc) return rc;
     e = index_build(b.idx, b.world, nullptr, b.nb, C, b.sort, st);
-    QuerySet fq{b.fq_cell, s->B.sown, s->B.btab};
-    // A two-way step's densities already hold the boundary's share (from
-    // its last Jacobi iteration).
-    if (!density_has_boundary) {
-        if (e == cudaSuccess) e = index_classify(fq, s->B.x, s->n, b.idx, C, st);
-        if (e == cudaSuccess) e = boundary_density(s->B.x, s->n, fq, b.idx, s->B.rho, C, st);
-    }
-    if (e == cudaSuccess) e = mark(2);
-    if (e != cudaSuccess) return cuda_fail(e, "boundary density");
-    // 3. coupling forces from a fresh fluid grid on the final positions
-    //    (fluid_world.cpp:125-174); the step's sorted buffers are free now.
     PointIndex fidx;
     fidx.keys = s->B.keys;
     fidx.skeys = s->B.skeys;
@@ -1395,10 +1370,17 @@ int enqueue_coupling(pbf_scene* s, const StepConsts& C, const float* force_in,
     fidx.scell = s->B.scell;
     fidx.off = s->B.off;
     fidx.slot_alias = s->B.slot_alias;
-    e = index_build(fidx, s->B.x, s->B.rho, s->n, C, s->sort, st);
-    if (e == cudaSuccess) e = index_classify(b.bq, b.world, b.nb, fidx, C, st);
-    if (e == cudaSuccess)
-        e = coupling_forces(b.world, b.body, b.body_dyn, b.nb, nbodies, b.bq, fidx, b.Fb, C, st);
+    if (e == cudaSuccess) e = index_build(fidx, s->B.x, s->B.rho, s->n, C, s->sort, st);
+    // A two-way step's densities already hold the boundary's share (from
+    // its last Jacobi iteration).
+    const QuerySet fq{fidx.scell, s->B.sown, s->B.btab};
+    if (e == cudaSuccess && !density_has_boundary) e = index_classify(fq, s->n, b.idx, C, st);
+    if (e == cudaSuccess) e = boundary_density(fidx, fq, b.idx, s->B.rho, density_has_boundary, C, st);
+    if (e == cudaSuccess) e = mark(2);
+    if (e != cudaSuccess) return cuda_fail(e, "boundary density");
+    // 3. coupling forces (fluid_world.cpp:125-174)
+    e = index_classify(b.bq, b.nb, fidx, C, st);
+    if (e == cudaSuccess) e = coupling_forces(b.idx, b.body, b.body_dyn, nbodies, b.bq, fidx, b.Fb, C, st);
     if (nbodies > 0) {
         const size_t bytes = (size_t)nbodies * 12;
         if (e == cudaSuccess)
@@ -1546,7 +1528,6 @@ int scene_couple_rigid_locked(pbf_scene* s, float dt, const float g[3]) {
         // Every allocation happens here, before any capture.
         int rc = make_consts(s, dt, key.C);
         if (!rc) rc = ensure_boundary_grid(s, key.C.grid.nslots);
-        if (!rc) rc = ensure_fluid_queries(s);
         if (rc) return rc;
     }
     key.dt = dt;
@@ -1614,7 +1595,7 @@ int scene_couple_rigid_locked(pbf_scene* s, float dt, const float g[3]) {
 
 namespace {
 
-// Buffers of a two-way step: predicted positions, their cells, owner words
+// Buffers of a two-way step: cells of the predicted positions, owner words
 // and bucket rows, per fluid particle.
 int ensure_two_way(pbf_scene* s) {
     auto& b = s->bnd;
@@ -1622,13 +1603,12 @@ int ensure_two_way(pbf_scene* s) {
     if (b.tw_mem) cudaFree(b.tw_mem);
     b.tw_mem = nullptr;
     const size_t c = (size_t)(s->n > 0 ? s->n : 1);
-    const size_t pb = align_up(c * 16, 256), cb = align_up(c * 16, 256), ob = align_up(c * 4, 256);
-    PBF_CUDA(cudaMalloc(&b.tw_mem, pb + cb + ob + c * 27 * 4));
+    const size_t cb = align_up(c * 16, 256), ob = align_up(c * 4, 256);
+    PBF_CUDA(cudaMalloc(&b.tw_mem, cb + ob + c * 27 * 4));
     unsigned char* m = static_cast<unsigned char*>(b.tw_mem);
-    b.tw_pred = reinterpret_cast<float4*>(m);
-    b.tw_cell = reinterpret_cast<int4*>(m + pb);
-    b.tw_own = reinterpret_cast<int*>(m + pb + cb);
-    b.tw_btab = reinterpret_cast<uint32_t*>(m + pb + cb + ob);
+    b.tw_cell = reinterpret_cast<int4*>(m);
+    b.tw_own = reinterpret_cast<int*>(m + cb);
+    b.tw_btab = reinterpret_cast<uint32_t*>(m + cb + ob);
     b.tw_cap = (int)c;
     return PBF_OK;
 }
@@ -1646,9 +1626,9 @@ int two_way_step(pbf_scene* s, const StepConsts& C) {
     cudaError_t e = boundary_xform(b.local, b.body, b.nb, b.body_pos, b.body_quat, b.nbodies,
                                    b.world, st);
     if (e == cudaSuccess) e = index_build(b.idx, b.world, nullptr, b.nb, C, b.sort, st);
-    if (e == cudaSuccess) e = predict_points(s->B.x, s->B.v, s->n, b.tw_pred, C, st);
+    if (e == cudaSuccess) e = predict_cells(s->B.x, s->B.v, s->n, b.tw_cell, C, st);
     QuerySet q{b.tw_cell, b.tw_own, b.tw_btab};
-    if (e == cudaSuccess) e = index_classify(q, b.tw_pred, s->n, b.idx, C, st);
+    if (e == cudaSuccess) e = index_classify(q, s->n, b.idx, C, st);
     if (e != cudaSuccess) return cuda_fail(e, "two-way boundary");
     BoundaryGrid bg;
     bg.spos = b.idx.spos;
@@ -1772,9 +1752,9 @@ int pbf_boundary_volumes(int device, int nb, const float* world3, float kernel_r
                 l[i] = make_float4(world3[3 * i], world3[3 * i + 1], world3[3 * i + 2], 0.0f);
             e = cudaMemcpyAsync(b.world, l.data(), (size_t)nb * 16, cudaMemcpyHostToDevice, s->stream);
             if (e == cudaSuccess) e = index_build(b.idx, b.world, nullptr, nb, C, b.sort, s->stream);
-            if (e == cudaSuccess) e = index_classify(b.bq, b.world, nb, b.idx, C, s->stream);
+            if (e == cudaSuccess) e = index_classify(b.bq, nb, b.idx, C, s->stream);
             float* dpsi = reinterpret_cast<float*>(b.Fb);
-            if (e == cudaSuccess) e = boundary_volumes(b.world, nb, b.bq, b.idx, dpsi, C, s->stream);
+            if (e == cudaSuccess) e = boundary_volumes(b.bq, b.idx, dpsi, C, s->stream);
             if (e == cudaSuccess)
                 e = cudaMemcpyAsync(psi_out, dpsi, (size_t)nb * 4, cudaMemcpyDeviceToHost, s->stream);
             if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);

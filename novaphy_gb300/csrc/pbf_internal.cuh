@@ -152,13 +152,10 @@ struct pbf_scene {
         void* mem = nullptr;       // per-boundary-particle arrays
         void* body_mem = nullptr;  // per-body arrays
         void* sort_mem = nullptr;
-        void* fq_mem = nullptr;    // fluid-query cells (per fluid particle)
-        int fq_cap = 0;
-        // Two-way coupled steps: predicted fluid positions and their
-        // classification against the boundary index (per fluid particle).
+        // Two-way coupled steps: cells of the predicted fluid positions and
+        // their classification against the boundary index (per fluid particle).
         void* tw_mem = nullptr;
         int tw_cap = 0;
-        float4* tw_pred = nullptr;
         int4* tw_cell = nullptr;
         int* tw_own = nullptr;
         uint32_t* tw_btab = nullptr;
@@ -168,7 +165,6 @@ struct pbf_scene {
         float4* Fb = nullptr;
         pbf::PointIndex idx;       // reference buckets over the boundary
         pbf::QuerySet bq;          // boundary queries against the fluid index
-        int4* fq_cell = nullptr;
         float4* body_pos = nullptr;
         float4* body_quat = nullptr;
         float4* body_lin = nullptr;  // body velocities (two-way boundary friction)
