@@ -95,6 +95,7 @@ struct pbf_batch {
     void* xmem = nullptr;  // scene ids
     StepBuffers B{};
     SortScratch sort{};
+    uint32_t* status = nullptr;  // status word of the batch's steps
     uint32_t *pid = nullptr, *spid = nullptr;
 
     uint32_t* off = nullptr;  // nslots + 1 offsets, then one alias byte per slot
@@ -175,6 +176,8 @@ int ensure_particles(pbf_batch* b, int n) {
     PBF_CUDA(cudaMalloc(&b->smem, sb));
     PBF_CUDA(cudaMemsetAsync(b->smem, 0, sb, b->stream));
     sort_scratch_bind(b->sort, b->smem, c);
+    if (!b->status) b->status = take_status_word();
+    if (b->status) b->sort.err = b->status;
     b->B.err = b->sort.err;
     const size_t xb = extra_bytes(c);
     PBF_CUDA(cudaMalloc(&b->xmem, xb));
@@ -637,12 +640,11 @@ int batch_sync(pbf_batch* b) {
     PBF_CUDA(cudaStreamSynchronize(b->stream));
     if (!b->sort.err) return PBF_OK;
     uint32_t err = 0;
-    PBF_CUDA(cudaMemcpy(&err, b->sort.err, 4, cudaMemcpyDeviceToHost));
-    if (err) {
-        PBF_CUDA(cudaMemset(b->sort.err, 0, 4));
+    const int rc = take_status(b->sort.err, b->status, &err);
+    if (rc) return rc;
+    if (err)
         return fail(PBF_ERR_TIMEOUT, "a device-side wait of a batch step gave up (error word " +
                                          std::to_string(err) + ")");
-    }
     return PBF_OK;
 }
 
@@ -756,6 +758,7 @@ int pbf_batch_destroy(pbf_batch* b) {
         for (void* m : {b->wmem, b->smem, b->xmem, static_cast<void*>(b->off),
                         static_cast<void*>(b->d_bad), static_cast<void*>(b->barrier)})
             if (m) cudaFree(m);
+        give_status_word(b->status);
         if (b->done) cudaEventDestroy(b->done);
         if (b->fork) cudaEventDestroy(b->fork);
         if (b->stream) cudaStreamDestroy(b->stream);

@@ -65,6 +65,20 @@ __global__ void k_pack3(const float4* __restrict__ in, float* __restrict__ a3, i
     }
 }
 
+// A scene's state (x, v, rho, lambda) from or to a snapshot's, in one launch.
+__global__ void k_copy_state(const float4* __restrict__ x, const float4* __restrict__ v,
+                             const float* __restrict__ rho, const float* __restrict__ lam,
+                             float4* __restrict__ ox, float4* __restrict__ ov, float* __restrict__ orho,
+                             float* __restrict__ olam, int n) {
+    const int i = blockIdx.x * blockDim.x + threadIdx.x;
+    if (i < n) {
+        ox[i] = x[i];
+        ov[i] = v[i];
+        orho[i] = rho[i];
+        olam[i] = lam[i];
+    }
+}
+
 __global__ void k_finite(const float4* __restrict__ x, const float4* __restrict__ v, int n,
                          uint32_t* __restrict__ flag) {
     const int i = blockIdx.x * blockDim.x + threadIdx.x;
@@ -119,6 +133,61 @@ int pool_alloc(void** p, size_t bytes, int device, cudaStream_t st) {
 
 void pool_free(void* p, cudaStream_t st) {
     if (p) cudaFreeAsync(p, st);
+}
+
+// The words live in one page-locked slab per process, made on first use and
+// kept; a word given back is handed out again.
+static constexpr int kStatusWords = 4096;
+struct StatusWords {
+    std::mutex mu;
+    uint32_t* slab = nullptr;
+    bool tried = false;
+    std::vector<uint32_t*> free;
+};
+static StatusWords& status_words() {
+    static StatusWords* const w = new StatusWords();  // outlives every scene
+    return *w;
+}
+
+uint32_t* take_status_word() {
+    StatusWords& w = status_words();
+    std::lock_guard<std::mutex> lk(w.mu);
+    if (!w.tried) {
+        w.tried = true;
+        void* p = nullptr;
+        if (cudaHostAlloc(&p, kStatusWords * sizeof(uint32_t), cudaHostAllocPortable | cudaHostAllocMapped) ==
+            cudaSuccess) {
+            w.slab = static_cast<uint32_t*>(p);
+            for (int k = kStatusWords; k > 0; --k) w.free.push_back(w.slab + k - 1);
+        } else {
+            cudaGetLastError();
+        }
+    }
+    if (w.free.empty()) return nullptr;
+    uint32_t* const p = w.free.back();
+    w.free.pop_back();
+    *p = 0u;
+    return p;
+}
+
+void give_status_word(uint32_t* p) {
+    if (!p) return;
+    StatusWords& w = status_words();
+    std::lock_guard<std::mutex> lk(w.mu);
+    w.free.push_back(p);
+}
+
+int take_status(uint32_t* device_word, uint32_t* host_word, uint32_t* out) {
+    *out = 0u;
+    if (host_word) {
+        volatile uint32_t* const p = host_word;
+        *out = *p;
+        if (*out) *p = 0u;
+        return PBF_OK;
+    }
+    PBF_CUDA(cudaMemcpy(out, device_word, 4, cudaMemcpyDeviceToHost));
+    if (*out) PBF_CUDA(cudaMemset(device_word, 0, 4));
+    return PBF_OK;
 }
 
 }  // namespace capi
@@ -194,6 +263,8 @@ int ensure_work(pbf_scene* s) {
     if (rc) return rc;
     PBF_CUDA(cudaMemsetAsync(s->smem, 0, sb, s->stream));
     sort_scratch_bind(s->sort, s->smem, c);
+    if (!s->status) s->status = take_status_word();
+    if (s->status) s->sort.err = s->status;
     s->B.err = s->sort.err;
     s->work_cap = c;
     return PBF_OK;
@@ -294,13 +365,16 @@ int ensure_offsets(pbf_scene* s, uint32_t nslots) {
         cudaGraphExecDestroy(s->graph);
         s->graph = nullptr;
     }
-    if (s->off) cudaFree(s->off);
+    pool_free(s->off, s->stream);
     s->off = nullptr;
+    s->off_cap = 0;
     // offsets (nslots + 1 words), one alias byte per slot, a moved word and
     // a lambda word per slot, then the density pass's walk counts
     const size_t ob = align_up((size_t)(nslots + 1) * 4, 256);
     const size_t ab = align_up(nslots + 1, 256);
-    PBF_CUDA(cudaMalloc(&s->off, ob + ab + (size_t)(nslots + 1) * 8 + 4 * kWalkHist * 4));
+    int rc = pool_alloc(reinterpret_cast<void**>(&s->off),
+                        ob + ab + (size_t)(nslots + 1) * 8 + 4 * kWalkHist * 4, s->device, s->stream);
+    if (rc) return rc;
     s->off_cap = nslots + 1;
     s->B.off = s->off;
     s->B.slot_alias = reinterpret_cast<unsigned char*>(s->off) + ob;
@@ -550,12 +624,11 @@ int sync_and_check(pbf_scene* s) {
     PBF_CUDA(cudaStreamSynchronize(s->stream));
     if (!s->sort.err) return PBF_OK;
     uint32_t err = 0;
-    PBF_CUDA(cudaMemcpy(&err, s->sort.err, 4, cudaMemcpyDeviceToHost));
-    if (err) {
-        PBF_CUDA(cudaMemset(s->sort.err, 0, 4));
+    const int rc = take_status(s->sort.err, s->status, &err);
+    if (rc) return rc;
+    if (err)
         return fail(PBF_ERR_TIMEOUT, "device-side wait in the cell sort gave up (error word " +
                                          std::to_string(err) + ")");
-    }
     return PBF_OK;
 }
 
@@ -651,19 +724,22 @@ int pbf_scene_destroy(pbf_scene* s) {
     {
         DeviceGuard dg(s->device);
         if (s->stream) cudaStreamSynchronize(s->stream);
-        for (void* m : {s->bnd.mem, s->bnd.body_mem, s->bnd.sort_mem, s->bnd.tw_mem, static_cast<void*>(s->bnd.rb),
+        for (void* m : {s->bnd.body_mem, s->bnd.tw_mem, static_cast<void*>(s->bnd.rb),
                         static_cast<void*>(s->bnd.shapes)})
             if (m) cudaFree(m);
-        if (s->bnd.idx.off) cudaFree(s->bnd.idx.off);
+        for (void* m : {s->bnd.mem, s->bnd.sort_mem, static_cast<void*>(s->bnd.idx.off),
+                        static_cast<void*>(s->off)})
+            pool_free(m, s->stream);
         if (s->couple_graph) cudaGraphExecDestroy(s->couple_graph);
+        s->off = nullptr;
         free_particles(s);
-        if (s->off) cudaFree(s->off);
         if (s->d_flag) cudaFree(s->d_flag);
         if (s->ev) cudaEventDestroy(s->ev);
         if (s->own_stream) {
             cudaStreamSynchronize(s->own_stream);
             cudaStreamDestroy(s->own_stream);
         }
+        give_status_word(s->status);
     }
     delete s;
     return PBF_OK;
@@ -746,6 +822,17 @@ int pbf_scene_step_timed(pbf_scene* s, float dt, int nsteps, float* ms_out) {
 
 namespace {
 size_t snapshot_bytes(int n) { return (size_t)n * (16 + 16 + 4 + 4); }
+
+struct SnapshotView {
+    float4 *x, *v;
+    float *rho, *lam;
+};
+SnapshotView view_of(const pbf_snapshot* snap) {
+    char* const p = static_cast<char*>(snap->mem);
+    const size_t n = (size_t)snap->n;
+    return SnapshotView{reinterpret_cast<float4*>(p), reinterpret_cast<float4*>(p + n * 16),
+                        reinterpret_cast<float*>(p + n * 32), reinterpret_cast<float*>(p + n * 36)};
+}
 }  // namespace
 
 extern "C" {
@@ -767,15 +854,10 @@ int pbf_snapshot_create(pbf_scene* s, pbf_snapshot** out) {
             delete snap;
             return cuda_fail(e, "pbf_snapshot_create");
         }
-        char* p = reinterpret_cast<char*>(snap->mem);
-        const size_t n = (size_t)s->n;
-        e = cudaMemcpyAsync(p, s->B.x, n * 16, cudaMemcpyDeviceToDevice, s->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(p + n * 16, s->B.v, n * 16, cudaMemcpyDeviceToDevice, s->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(p + n * 32, s->B.rho, n * 4, cudaMemcpyDeviceToDevice, s->stream);
-        if (e == cudaSuccess)
-            e = cudaMemcpyAsync(p + n * 36, s->B.lam, n * 4, cudaMemcpyDeviceToDevice, s->stream);
+        const SnapshotView w = view_of(snap);
+        k_copy_state<<<(s->n + 255) / 256, 256, 0, s->stream>>>(s->B.x, s->B.v, s->B.rho, s->B.lam, w.x, w.v,
+                                                                w.rho, w.lam, s->n);
+        e = cudaGetLastError();
         if (e == cudaSuccess) e = cudaStreamSynchronize(s->stream);
         if (e != cudaSuccess) {
             cudaFree(snap->mem);
@@ -819,12 +901,10 @@ int restore_on(pbf_scene* s, const pbf_snapshot* snap, cudaStream_t st) {
     for (int d = 0; d < 3; ++d) s->gravity[d] = snap->gravity[d];
     s->mass = snap->mass;
     if (snap->n == 0) return PBF_OK;
-    const char* p = reinterpret_cast<const char*>(snap->mem);
-    const size_t n = (size_t)snap->n;
-    PBF_CUDA(cudaMemcpyAsync(s->B.x, p, n * 16, cudaMemcpyDeviceToDevice, st));
-    PBF_CUDA(cudaMemcpyAsync(s->B.v, p + n * 16, n * 16, cudaMemcpyDeviceToDevice, st));
-    PBF_CUDA(cudaMemcpyAsync(s->B.rho, p + n * 32, n * 4, cudaMemcpyDeviceToDevice, st));
-    PBF_CUDA(cudaMemcpyAsync(s->B.lam, p + n * 36, n * 4, cudaMemcpyDeviceToDevice, st));
+    const SnapshotView w = view_of(snap);
+    k_copy_state<<<(snap->n + 255) / 256, 256, 0, st>>>(w.x, w.v, w.rho, w.lam, s->B.x, s->B.v, s->B.rho,
+                                                        s->B.lam, snap->n);
+    PBF_CUDA(cudaGetLastError());
     return PBF_OK;
 }
 
@@ -1171,13 +1251,15 @@ namespace {
 int alloc_boundary(pbf_scene* s, int nb) {
     ++s->buf_gen;
     auto& b = s->bnd;
-    for (void* m : {b.mem, b.sort_mem}) if (m) cudaFree(m);
+    for (void* m : {b.mem, b.sort_mem}) pool_free(m, s->stream);
     b.mem = b.sort_mem = nullptr;
+    b.nb = 0;
     const int c = nb > 0 ? nb : 1;
     const size_t f4 = align_up((size_t)c * 16, 256), f1 = align_up((size_t)c * 4, 256),
                  f27 = align_up((size_t)c * 27 * 4, 256);
     const size_t total = 5 * f4 + 5 * f1 + bucket_bytes(c) + f27;
-    PBF_CUDA(cudaMalloc(&b.mem, total));
+    int rc = pool_alloc(&b.mem, total, s->device, s->stream);
+    if (rc) return rc;
     char* p = reinterpret_cast<char*>(b.mem);
     auto take = [&](size_t n) { char* r = p; p += n; return r; };
     b.local = reinterpret_cast<float4*>(take(f4));
@@ -1195,7 +1277,8 @@ int alloc_boundary(pbf_scene* s, int nb) {
     b.bq.btab = reinterpret_cast<uint32_t*>(take(f27));
     PBF_CUDA(cudaMemsetAsync(b.mem, 0, total, s->stream));
     const size_t sb = sort_scratch_bytes(c);
-    PBF_CUDA(cudaMalloc(&b.sort_mem, sb));
+    rc = pool_alloc(&b.sort_mem, sb, s->device, s->stream);
+    if (rc) return rc;
     PBF_CUDA(cudaMemsetAsync(b.sort_mem, 0, sb, s->stream));
     sort_scratch_bind(b.sort, b.sort_mem, c);
     b.nb = nb;
@@ -1206,10 +1289,13 @@ int ensure_boundary_grid(pbf_scene* s, uint32_t nslots) {
     auto& b = s->bnd;
     if (b.idx.off && b.idx_slots >= nslots) return PBF_OK;
     ++s->buf_gen;
-    if (b.idx.off) cudaFree(b.idx.off);
+    pool_free(b.idx.off, s->stream);
     b.idx.off = nullptr;
+    b.idx_slots = 0;
     const size_t ob = align_up((size_t)(nslots + 1) * 4, 256);
-    PBF_CUDA(cudaMalloc(&b.idx.off, ob + align_up(nslots, 256)));
+    const int rc = pool_alloc(reinterpret_cast<void**>(&b.idx.off), ob + align_up(nslots, 256), s->device,
+                              s->stream);
+    if (rc) return rc;
     b.idx.slot_alias = reinterpret_cast<unsigned char*>(b.idx.off) + ob;
     b.idx_slots = nslots;
     return PBF_OK;
@@ -1739,18 +1825,19 @@ int pbf_boundary_volumes(int device, int nb, const float* world3, float kernel_r
         DeviceGuard dg(s->device);
         update_bbox(s, world3, nb);
         StepConsts C;
-        rc = make_consts(s, 1.0f, C);
-        std::vector<int> bodies(nb, -1);
-        std::vector<float> zero(nb, 0.0f);
+        rc = scene_consts(s, 1.0f, C);
         if (!rc) rc = alloc_boundary(s, nb);
         if (!rc) rc = ensure_boundary_grid(s, C.grid.nslots);
         auto& b = s->bnd;
         cudaError_t e = cudaSuccess;
         if (!rc) {
-            std::vector<float4> l(nb);
-            for (int i = 0; i < nb; ++i)
-                l[i] = make_float4(world3[3 * i], world3[3 * i + 1], world3[3 * i + 2], 0.0f);
-            e = cudaMemcpyAsync(b.world, l.data(), (size_t)nb * 16, cudaMemcpyHostToDevice, s->stream);
+            // The points travel packed, through the (larger) force array.
+            float* const packed = reinterpret_cast<float*>(b.Fb);
+            e = cudaMemcpyAsync(packed, world3, (size_t)nb * 12, cudaMemcpyHostToDevice, s->stream);
+            if (e == cudaSuccess) {
+                k_expand3<<<(nb + 255) / 256, 256, 0, s->stream>>>(packed, b.world, nb);
+                e = cudaGetLastError();
+            }
             if (e == cudaSuccess) e = index_build(b.idx, b.world, nullptr, nb, C, b.sort, s->stream);
             if (e == cudaSuccess) e = index_classify(b.bq, nb, b.idx, C, s->stream);
             float* dpsi = reinterpret_cast<float*>(b.Fb);

@@ -120,6 +120,7 @@ struct pbf_scene {
     uint32_t off_cap = 0;  // entries
     float* staging = nullptr;  // float[3 cap]
     uint32_t* d_flag = nullptr;
+    uint32_t* status = nullptr;  // status word of the scene's steps (take_status_word)
     cudaEvent_t ev = nullptr;  // orders a batch after the scene's own stream
     pbf::SortScratch sort{};
     pbf::StepBuffers B{};
@@ -208,6 +209,13 @@ int scene_consts(const pbf_scene* s, float dt, StepConsts& C);
 // Stream-ordered allocation of scene buffers from the device's scene pool.
 int pool_alloc(void** p, size_t bytes, int device, cudaStream_t st);
 void pool_free(void* p, cudaStream_t st);
+// A status word in page-locked host memory that the device writes to (null
+// when there is none left: the word in the sort scratch then serves), so that
+// a wait for a step ends with a read of it instead of a copy.
+uint32_t* take_status_word();
+void give_status_word(uint32_t* p);
+// Reads and clears a status word after its writers' stream was waited for.
+int take_status(uint32_t* device_word, uint32_t* host_word, uint32_t* out);
 // Copies a snapshot into the scene on stream `st` (asynchronous).
 int restore_on(pbf_scene* s, const pbf_snapshot* snap, cudaStream_t st);
 // Device bytes the scene holds (state, step scratch, offsets table).
