@@ -11,22 +11,29 @@
 namespace pbf {
 namespace bnd {
 
-// Cell slot of points (no prediction).
-__global__ void __launch_bounds__(kBlock)
-k_ix_keys(const float4* __restrict__ pos, int n, uint32_t* __restrict__ keys, const StepConsts C) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    if (i >= n) return;
-    const float4 p = pos[i];
-    int cx, cy, cz;
-    cell_of(p.x, p.y, p.z, C.inv_cell, cx, cy, cz);
-    keys[i] = slot_of(cx, cy, cz, C.grid);
+// Cell slot of points (no prediction), with its digits counted.
+__global__ void __launch_bounds__(kCountThreads)
+k_ix_keys(const float4* __restrict__ pos, int n, uint32_t* __restrict__ keys, const SortCounts counts,
+          const StepConsts C) {
+    __shared__ BlockCounts B;
+    B.begin(counts);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
+        const float4 p = pos[i];
+        int cx, cy, cz;
+        cell_of(p.x, p.y, p.z, C.inv_cell, cx, cy, cz);
+        const uint32_t key = slot_of(cx, cy, cz, C.grid);
+        keys[i] = key;
+        B.count(counts, key);
+    }
+    B.end(counts);
 }
 
 __global__ void __launch_bounds__(kBlock)
 k_ix_gather(const uint32_t* __restrict__ sidx, const float4* __restrict__ pos,
             const float* __restrict__ attr, int n, float4* __restrict__ spos,
             int4* __restrict__ scell, uint32_t* __restrict__ link,
-            unsigned char* __restrict__ slot_alias, const StepConsts C) {
+            unsigned char* __restrict__ slot_alias, const SlotOffsets offsets, const StepConsts C) {
+    if (offsets.block(n)) return;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     uint32_t i = sidx[p];
@@ -447,15 +454,15 @@ cudaError_t index_build(PointIndex& I, const float4* pos, const float* attr, int
     using namespace bnd;
     I.n = n;
     if (n <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(I.slot_alias, 0, (size_t)C.grid.nslots, st);
+    const int bits = C.grid.key_bits, nb = grid_of(n, kBlock);
+    const ClearRange alias{reinterpret_cast<uint32_t*>(I.slot_alias), ((size_t)C.grid.nslots + 3) / 4, 0u};
+    cudaError_t e = clear_ranges(alias, sort_clear(sort, n, bits), bucket_clear(I.bkt, n), st);
     if (e != cudaSuccess) return e;
-    const int nb = grid_of(n, kBlock);
-    k_ix_keys<<<nb, kBlock, 0, st>>>(pos, n, I.keys, C);
-    e = radix_sort_pairs(I.keys, I.skeys, I.sidx, n, C.grid.key_bits, sort, st);
+    k_ix_keys<<<count_blocks(n), kCountThreads, 0, st>>>(pos, n, I.keys, sort_counts(sort, n, bits), C);
+    e = radix_sort_counted(I.keys, I.skeys, I.sidx, n, bits, sort, st);
     if (e != cudaSuccess) return e;
-    k_offsets<<<grid_of((int)C.grid.nslots + 1, 256), 256, 0, st>>>(I.skeys, n, I.off, C.grid.nslots);
-    k_ix_gather<<<nb, kBlock, 0, st>>>(I.sidx, pos, attr, n, I.spos, I.scell, I.bkt.link,
-                                       I.slot_alias, C);
+    k_ix_gather<<<nb + grid_of((int)C.grid.nslots + 1, kBlock), kBlock, 0, st>>>(I.sidx, pos, attr, n, I.spos,
+        I.scell, I.bkt.link, I.slot_alias, SlotOffsets{I.skeys, I.off, C.grid.nslots, nb}, C);
     return enqueue_buckets(sized_for(I.bkt, n), I.scell, I.sidx, nullptr, I.slot_alias, n, OneScene{C, StateRef{}}, st);
 }
 
@@ -477,9 +484,8 @@ cudaError_t index_classify(const QuerySet& Q, int nq, const PointIndex& I, const
     }
     StepConsts Cs = C;
     Cs.hash_compat = 1;  // the coupling queries always follow the reference buckets
-    k_classify<<<grid_of(nq, kBlock), kBlock, 0, st>>>(Q.qcell, nq, I.scell, nullptr, sized_for(I.bkt, I.n),
-                                                       I.slot_alias, Q.btab, Q.qown, nullptr,
-                                                       OneScene{Cs, StateRef{}});
+    k_classify<OneScene><<<grid_of(nq, kBlock), kBlock, 0, st>>>(Q.qcell, nq, I.scell, nullptr,
+        sized_for(I.bkt, I.n), I.slot_alias, Q.btab, Q.qown, nullptr, OneScene{Cs, StateRef{}});
     return cudaGetLastError();
 }
 
@@ -487,8 +493,7 @@ cudaError_t boundary_xform(const float4* local, const int* body, int nb, const f
                            const float4* body_quat, int nbodies, float4* world, cudaStream_t st) {
     using namespace bnd;
     if (nb <= 0) return cudaSuccess;
-    k_bxform<<<grid_of(nb, kBlock), kBlock, 0, st>>>(local, body, nb, body_pos, body_quat, nbodies,
-                                                     world);
+    k_bxform<<<grid_of(nb, kBlock), kBlock, 0, st>>>(local, body, nb, body_pos, body_quat, nbodies, world);
     return cudaGetLastError();
 }
 
@@ -515,10 +520,10 @@ cudaError_t coupling_forces(const PointIndex& bidx, const int* body, const int* 
     if (fidx.n <= 0) return cudaMemsetAsync(Fb, 0, (size_t)nb * sizeof(float4), st);
     if (small_teams(nb))
         k_coupling<8><<<grid_of(nb, 8), 128, 0, st>>>(bidx.spos, bidx.sidx, body, body_dynamic, nb, nbodies, Q,
-                                                      fidx, Fb, C);
+            fidx, Fb, C);
     else
         k_coupling<16><<<grid_of(nb, 16), 128, 0, st>>>(bidx.spos, bidx.sidx, body, body_dynamic, nb, nbodies,
-                                                        Q, fidx, Fb, C);
+            Q, fidx, Fb, C);
     return cudaGetLastError();
 }
 
@@ -528,11 +533,11 @@ cudaError_t body_reduce(const float4* Fb, const float4* bworld, const int* list_
     using namespace bnd;
     if (nbodies <= 0) return cudaSuccess;
     if (tree)
-        k_body_reduce_tree<<<nbodies, kTreeThreads, 0, st>>>(Fb, bworld, list_off, list, body_pos,
-                                                             nbodies, force3, torque3);
+        k_body_reduce_tree<<<nbodies, kTreeThreads, 0, st>>>(Fb, bworld, list_off, list, body_pos, nbodies,
+            force3, torque3);
     else
-        k_body_reduce<<<nbodies, kReduceThreads, 0, st>>>(Fb, bworld, list_off, list, body_pos,
-                                                          nbodies, force3, torque3);
+        k_body_reduce<<<nbodies, kReduceThreads, 0, st>>>(Fb, bworld, list_off, list, body_pos, nbodies,
+            force3, torque3);
     return cudaGetLastError();
 }
 

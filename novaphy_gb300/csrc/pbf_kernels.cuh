@@ -255,43 +255,63 @@ __device__ __forceinline__ void predict(const float4 xi, const float4 vi, const 
     pz = __fadd_rn(xi.z, __fmul_rn(vz, C.dt));
 }
 
-// Predict + cell slot per particle (particle order).  Also turns this step's
-// density-pass counts of the last step (dhist, where there are any) into the
-// previous step's.
+// Predict + cell slot per particle (particle order), with the digits of the
+// slots counted for the sort.  Also turns this step's density-pass counts of
+// the last step (dhist, where there are any) into the previous step's.
 template <class P>
-__global__ void __launch_bounds__(kBlock)
-k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, int n, const SceneIds S,
-              const P prm) {
-    const int i = blockIdx.x * blockDim.x + threadIdx.x;
-    static_assert(2 * kWalkHist <= kBlock, "one thread per count");
-    if (dhist && i < 2 * kWalkHist) {
-        dhist[i] = dhist[i + 2 * kWalkHist];
-        dhist[i + 2 * kWalkHist] = 0u;
+__global__ void __launch_bounds__(kCountThreads)
+k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, int n, const SortCounts counts,
+              const SceneIds S, const P prm) {
+    __shared__ BlockCounts B;
+    const int t = blockIdx.x * blockDim.x + threadIdx.x;
+    static_assert(2 * kWalkHist <= kCountThreads, "one thread per count");
+    if (dhist && t < 2 * kWalkHist) {
+        dhist[t] = dhist[t + 2 * kWalkHist];
+        dhist[t + 2 * kWalkHist] = 0u;
     }
-    if (i >= n) return;
-    const StepConsts& C = prm.at(S.pid, i);
-    const StateRef& R = prm.state(S.pid, i);
-    const uint32_t l = (uint32_t)i - R.first;
-    float px, py, pz;
-    predict(R.x[l], R.v[l], C, px, py, pz);
-    int cx, cy, cz;
-    cell_of(px, py, pz, C.inv_cell, cx, cy, cz);
-    keys[i] = slot_of(cx, cy, cz, C.grid);
+    B.begin(counts);
+    for (int i = t; i < n; i += gridDim.x * blockDim.x) {
+        const StepConsts& C = prm.at(S.pid, i);
+        const StateRef& R = prm.state(S.pid, i);
+        const uint32_t l = (uint32_t)i - R.first;
+        float px, py, pz;
+        predict(R.x[l], R.v[l], C, px, py, pz);
+        int cx, cy, cz;
+        cell_of(px, py, pz, C.inv_cell, cx, cy, cz);
+        const uint32_t key = slot_of(cx, cy, cz, C.grid);
+        keys[i] = key;
+        B.count(counts, key);
+    }
+    B.end(counts);
 }
 
 // off[s] = lower_bound(skeys, s) for s in [0, nslots].
-__global__ void __launch_bounds__(256)
-k_offsets(const uint32_t* __restrict__ skeys, int n, uint32_t* __restrict__ off, uint32_t nslots) {
-    const uint32_t s = blockIdx.x * blockDim.x + threadIdx.x;
+__device__ __forceinline__ void slot_offset(uint32_t s, const uint32_t* __restrict__ skeys, int n,
+                                            uint32_t* __restrict__ off, uint32_t nslots) {
     if (s > nslots) return;
     int a = 0, b = n;
     while (a < b) {
         const int m = (a + b) >> 1;
-        if (__ldg(skeys + m) < s) a = m + 1;
+        if (skeys[m] < s) a = m + 1;
         else b = m;
     }
     off[s] = (uint32_t)a;
 }
+
+// A launch of `points` blocks over the n points and more over the slots: the
+// offsets' searches (a chain of log n loads each) run beside the points' work.
+struct SlotOffsets {
+    const uint32_t* skeys;
+    uint32_t* off;
+    uint32_t nslots;
+    int points;
+    // Whether the block is one of the slots' (and has done its work then).
+    __device__ __forceinline__ bool block(int n) const {
+        if ((int)blockIdx.x < points) return false;
+        slot_offset((blockIdx.x - (uint32_t)points) * blockDim.x + threadIdx.x, skeys, n, off, nslots);
+        return true;
+    }
+};
 
 // Gather particle state into cell-sorted order; recompute x* exactly as
 // predicted.  Records each particle's scene, empties the bucket chains and
@@ -302,7 +322,8 @@ __global__ void __launch_bounds__(kBlock)
 k_gather(const uint32_t* __restrict__ sidx, float4* __restrict__ sx, float4* __restrict__ xa,
          float* __restrict__ srho, int4* __restrict__ scell, uint32_t* __restrict__ link,
          unsigned char* __restrict__ slot_alias, uint32_t* __restrict__ err, int n,
-         const SceneIds S, const P prm) {
+         const SlotOffsets offsets, const SceneIds S, const P prm) {
+    if (offsets.block(n)) return;
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
     if (p >= n) return;
     uint32_t i = sidx[p];
@@ -466,6 +487,11 @@ inline BucketTable sized_for(BucketTable T, int n) {
     return T;
 }
 
+inline ClearRange bucket_clear(const BucketTable& T, int n) {
+    return ClearRange{T.table, (size_t)bucket_slots((uint32_t)n) + 1, 0xffffffffu};
+}
+inline ClearRange slot_clear(const StepBuffers& B) { return ClearRange{reinterpret_cast<uint32_t*>(B.slot_alias), B.slot_bytes / 4, 0u}; }
+
 // The first run of the bucket with this key (and scene), kNoBucket if none.
 __device__ __forceinline__ uint32_t find_bucket(const BucketTable& T, const CellRuns& R,
                                                 unsigned long long key, uint32_t sid) {
@@ -558,19 +584,17 @@ k_merge_runs(const BucketTable T, const CellRuns R, const uint32_t* __restrict__
     if (at < (uint32_t)R.n) T.merged[at] = (uint32_t)p;
 }
 
-// T: sized_for n.
+// T: sized_for n, its table cleared (bucket_clear).
 template <class P>
 inline cudaError_t enqueue_buckets(const BucketTable& T, const int4* scell, const uint32_t* sidx,
                                    const uint32_t* sid, unsigned char* slot_alias, int n, const P& prm,
                                    cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
-    cudaError_t e = cudaMemsetAsync(T.table, 0xff, ((size_t)T.slots + 1) * 4, st);
-    if (e != cudaSuccess) return e;
     const CellRuns R{scell, sid, n};
     const int nb = (n + 255) / 256;
-    k_cell_runs<<<nb, 256, 0, st>>>(T, R, slot_alias, prm);
-    k_merge_room<<<nb, 256, 0, st>>>(T, R, slot_alias, prm);
-    k_merge_runs<<<nb, 256, 0, st>>>(T, R, sidx, slot_alias, prm);
+    k_cell_runs<P><<<nb, 256, 0, st>>>(T, R, slot_alias, prm);
+    k_merge_room<P><<<nb, 256, 0, st>>>(T, R, slot_alias, prm);
+    k_merge_runs<P><<<nb, 256, 0, st>>>(T, R, sidx, slot_alias, prm);
     return cudaGetLastError();
 }
 
@@ -2913,22 +2937,25 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
     const int nb = grid_of(n, kBlock);
     const OneScene one{C, StateRef{B.x, B.v, B.rho, B.lam, 0u, nullptr}};
     const SceneIds none{nullptr, nullptr};
-    cudaError_t e = cudaMemsetAsync(B.slot_alias, 0, B.slot_bytes, st);
-    if (e != cudaSuccess) return e;
     if (pm) pm->mark(-1, 0, st);
-    k_predict_key<<<nb, kBlock, 0, st>>>(B.keys, B.dhist, n, none, one);
-    if (pm) pm->mark(kPhasePredict, 1, st);
-    e = radix_sort_pairs(B.keys, B.skeys, B.sidx, n, C.grid.key_bits, sort, st);
+    const int bits = C.grid.key_bits;
+    cudaError_t e = clear_ranges(slot_clear(B), sort_clear(sort, n, bits),
+                                 C.hash_compat ? bucket_clear(B.bkt, n) : ClearRange{}, st);
     if (e != cudaSuccess) return e;
-    k_offsets<<<grid_of((int)C.grid.nslots + 1, 256), 256, 0, st>>>(B.skeys, n, B.off, C.grid.nslots);
-    if (pm) pm->mark(kPhaseGridBuild, 2 + (C.grid.key_bits + 7) / 8, st);
-    k_gather<<<nb, kBlock, 0, st>>>(B.sidx, B.sx, B.xa, B.srho, B.scell, B.bkt.link, B.slot_alias,
-                                    B.err, n, none, one);
+    k_predict_key<OneScene><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, B.dhist, n, sort_counts(sort, n,
+        bits), none, one);
+    if (pm) pm->mark(kPhasePredict, 2, st);
+    e = radix_sort_counted(B.keys, B.skeys, B.sidx, n, bits, sort, st);
+    if (e != cudaSuccess) return e;
+    if (pm) pm->mark(kPhaseGridBuild, n <= kSmallSort ? 1 : sort_passes(bits), st);
+    k_gather<OneScene><<<nb + grid_of((int)C.grid.nslots + 1, kBlock), kBlock, 0, st>>>(B.sidx, B.sx, B.xa,
+        B.srho, B.scell, B.bkt.link, B.slot_alias, B.err, n, SlotOffsets{B.skeys, B.off, C.grid.nslots, nb},
+        none, one);
     if (C.hash_compat) {
         e = enqueue_buckets(sized_for(B.bkt, n), B.scell, B.sidx, nullptr, B.slot_alias, n, one, st);
         if (e != cudaSuccess) return e;
-        k_classify<<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, nullptr, sized_for(B.bkt, n), B.slot_alias, B.btab,
-                                          B.sown, nullptr, one);
+        k_classify<OneScene><<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, nullptr, sized_for(B.bkt, n),
+            B.slot_alias, B.btab, B.sown, nullptr, one);
     } else {
         e = cudaMemsetAsync(B.sown, 0, (size_t)n * 4, st);
         if (e != cudaSuccess) return e;
@@ -2985,19 +3012,19 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, const Grid& G, int n,
     } else {
         for (int it = 0; it < max_iters; ++it) {
             if constexpr (TP != 0)
-                k_density_lambda_team<T><<<nb, 128, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
+                k_density_lambda_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
             else
-                k_density_lambda<BS><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
+                k_density_lambda<BS, P><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
             if (pm) pm->mark(kPhaseDensity, 1, st);
             if constexpr (TP != 0)
-                k_delta_team<T><<<nb, 128, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
+                k_delta_team<T, P><<<nb, 128, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
             else
-                k_delta<BS><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
+                k_delta<BS, P><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
             if (pm) pm->mark(kPhaseDelta, 1, st);
         }
     }
     if (any_zero_iters) {
-        k_velocity<BS><<<grid_of(n, BS), BS, 0, st>>>(B.xa, B.sx, B.srho, B.sv, n, G, prm);
+        k_velocity<BS, P><<<grid_of(n, BS), BS, 0, st>>>(B.xa, B.sx, B.srho, B.sv, n, G, prm);
         if (pm) pm->mark(kPhaseDelta, 1, st);
     }
     if constexpr (std::is_same<P, OneScene>::value) {
@@ -3008,22 +3035,22 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, const Grid& G, int n,
     }
     if (any_vort) {
         if constexpr (TP != 0)
-            k_xsph_omega_team<T><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
+            k_xsph_omega_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
         else
-            k_xsph_omega<BS><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
+            k_xsph_omega<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
         if (pm) pm->mark(kPhaseXsph, 1, st);
         if constexpr (TP != 0)
-            k_vorticity_commit_team<T><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n, G, prm);
+            k_vorticity_commit_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n, G, prm);
         else
-            k_vorticity_commit<BS><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n, G, prm);
+            k_vorticity_commit<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n, G, prm);
         if (pm) pm->mark(kPhaseCommit, 1, st);
     }
     if (any_plain) {
         const int skip = any_vort ? 1 : 0;
         if constexpr (TP != 0)
-            k_xsph_commit_team<T><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
+            k_xsph_commit_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
         else
-            k_xsph_commit<BS><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
+            k_xsph_commit<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
         if (pm) pm->mark(xsph_on ? kPhaseXsph : kPhaseCommit, 1, st);
     }
     return cudaGetLastError();
@@ -3075,8 +3102,8 @@ inline cudaError_t enqueue_step(const StepBuffers& B, const StepConsts& C, int i
         // Runs of identical particles: from here on the owner words of the
         // run's later particles carry kCopyBit, which only the passes below
         // understand (they skip those particles).
-        k_segments<<<grid_of(n, 256), 256, 0, st>>>(StepState{B.sx, B.xa, B.srho, n}, B.scell,
-                                                    C.grid, B.sown, B.slot_alias, B.segend);
+        k_segments<<<grid_of(n, 256), 256, 0, st>>>(StepState{B.sx, B.xa, B.srho, n}, B.scell, C.grid, B.sown,
+            B.slot_alias, B.segend);
         if (pm) pm->mark(kPhaseNeighborQuery, 1, st);
         G.segend = B.segend;
     }
@@ -3110,23 +3137,24 @@ inline cudaError_t enqueue_batch_step(const StepBuffers& B, const BatchDesc& D, 
     const int nb = grid_of(n, kBlock);
     const SceneTable tab{D.tab, D.refs};
     const SceneIds ids{D.pid, D.spid};
-    cudaError_t e = cudaMemsetAsync(B.slot_alias, 0, B.slot_bytes, st);
-    if (e != cudaSuccess) return e;
     if (pm) pm->mark(-1, 0, st);
-    k_scene_ids<<<grid_of(n, 256), 256, 0, st>>>(D.firsts, D.nscenes, D.pid, n);
-    k_predict_key<<<nb, kBlock, 0, st>>>(B.keys, nullptr, n, ids, tab);
-    if (pm) pm->mark(kPhasePredict, 2, st);
-    // Cell order: scene-major because every scene owns a slot range.
-    e = radix_sort_pairs(B.keys, B.skeys, B.sidx, n, D.key_bits, sort, st);
+    cudaError_t e = clear_ranges(slot_clear(B), sort_clear(sort, n, D.key_bits), bucket_clear(B.bkt, n), st);
     if (e != cudaSuccess) return e;
-    k_offsets<<<grid_of((int)D.nslots + 1, 256), 256, 0, st>>>(B.skeys, n, B.off, D.nslots);
-    if (pm) pm->mark(kPhaseGridBuild, 2 + (D.key_bits + 7) / 8, st);
-    k_gather<<<nb, kBlock, 0, st>>>(B.sidx, B.sx, B.xa, B.srho, B.scell, B.bkt.link, B.slot_alias,
-                                    B.err, n, ids, tab);
+    k_scene_ids<<<grid_of(n, 256), 256, 0, st>>>(D.firsts, D.nscenes, D.pid, n);
+    k_predict_key<SceneTable><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, nullptr, n, sort_counts(sort,
+        n, D.key_bits), ids, tab);
+    if (pm) pm->mark(kPhasePredict, 3, st);
+    // Cell order: scene-major because every scene owns a slot range.
+    e = radix_sort_counted(B.keys, B.skeys, B.sidx, n, D.key_bits, sort, st);
+    if (e != cudaSuccess) return e;
+    if (pm) pm->mark(kPhaseGridBuild, n <= kSmallSort ? 1 : sort_passes(D.key_bits), st);
+    k_gather<SceneTable><<<nb + grid_of((int)D.nslots + 1, kBlock), kBlock, 0, st>>>(B.sidx, B.sx, B.xa,
+        B.srho, B.scell, B.bkt.link, B.slot_alias, B.err, n, SlotOffsets{B.skeys, B.off, D.nslots, nb}, ids,
+        tab);
     e = enqueue_buckets(sized_for(B.bkt, n), B.scell, B.sidx, D.spid, B.slot_alias, n, tab, st);
     if (e != cudaSuccess) return e;
-    k_classify<<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, D.spid, sized_for(B.bkt, n), B.slot_alias, B.btab, B.sown,
-                                      D.spid, tab);
+    k_classify<SceneTable><<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, D.spid, sized_for(B.bkt, n),
+        B.slot_alias, B.btab, B.sown, D.spid, tab);
     if (pm) pm->mark(kPhaseNeighborQuery, 5, st);
     e = cudaGetLastError();
     if (e != cudaSuccess) return e;

@@ -1,6 +1,7 @@
 // Onesweep LSD radix sort (see radix_sort.cuh).
 #include "radix_sort.cuh"
 
+
 namespace pbf {
 
 namespace {
@@ -53,19 +54,126 @@ __device__ __forceinline__ uint32_t block_exclusive_scan_256(uint32_t v, uint32_
     return warp_excl + inc - v;
 }
 
-__global__ void __launch_bounds__(kSortThreads)
-k_sort_histogram(const uint32_t* __restrict__ keys, int n, int passes, uint32_t* __restrict__ hist) {
-    __shared__ uint32_t sh[kSortMaxPasses][256];
-    for (int i = threadIdx.x; i < kSortMaxPasses * 256; i += blockDim.x) (&sh[0][0])[i] = 0u;
-    __syncthreads();
-    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const uint32_t k = keys[i];
-        for (int p = 0; p < passes; ++p) atomicAdd(&sh[p][(k >> (8 * p)) & 255u], 1u);
+__global__ void __launch_bounds__(kCountThreads)
+k_sort_histogram(const uint32_t* __restrict__ keys, int n, const SortCounts S) {
+    __shared__ BlockCounts B;
+    B.begin(S);
+    for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) B.count(S, keys[i]);
+    B.end(S);
+}
+
+__global__ void __launch_bounds__(256)
+k_clear(const ClearRange a, const ClearRange b, const ClearRange c) {
+    const size_t t = (size_t)blockIdx.x * blockDim.x + threadIdx.x, nt = (size_t)gridDim.x * blockDim.x;
+    auto set = [&](const ClearRange& r) {
+        for (size_t i = t; i < r.words / 4; i += nt)
+            reinterpret_cast<uint4*>(r.p)[i] = make_uint4(r.value, r.value, r.value, r.value);
+        if (t < (r.words & 3)) r.p[(r.words & ~(size_t)3) + t] = r.value;
+    };
+    set(a);
+    set(b);
+    set(c);
+}
+
+// All passes of up to kSmallSort keys in one block.  Warp w holds items
+// [256 w, 256 w + 256), item k of lane l at offset 32 k + l, as a tile of
+// k_onesweep does; after each pass the items are read back in sorted order.
+constexpr int kSmallThreads = 1024;
+constexpr int kSmallWarps = kSmallThreads / 32;
+struct SmallSort {
+    uint32_t keys[kSmallSort];
+    unsigned short vals[kSmallSort];
+    unsigned short warp[kSmallWarps][256];  // a digit's keys per warp, then before it
+    uint32_t base[256];
+    uint32_t scan[8];
+};
+
+__global__ void __launch_bounds__(kSmallThreads)
+k_sort_small(const uint32_t* __restrict__ keys_in, uint32_t* __restrict__ keys_out,
+             uint32_t* __restrict__ vals_out, int n, int passes) {
+    extern __shared__ __align__(16) unsigned char raw[];
+    SmallSort& sm = *reinterpret_cast<SmallSort*>(raw);
+    constexpr int kItems = kSmallSort / kSmallThreads;
+    const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    const uint32_t lt = lane_mask_lt();
+    uint32_t key[kItems], val[kItems], rank[kItems];
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int i = warp * (32 * kItems) + k * 32 + lane;
+        key[k] = i < n ? keys_in[i] : 0u;
+        val[k] = (uint32_t)i;
     }
-    __syncthreads();
-    for (int i = threadIdx.x; i < passes * 256; i += blockDim.x) {
-        const uint32_t c = (&sh[0][0])[i];
-        if (c) atomicAdd(&hist[i], c);
+    for (int p = 0; p < passes; ++p) {
+        const int shift = 8 * p;
+        for (int i = tid; i < kSmallWarps * 128; i += kSmallThreads)
+            reinterpret_cast<uint32_t*>(&sm.warp[0][0])[i] = 0u;
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const bool valid = warp * (32 * kItems) + k * 32 + lane < n;
+            const uint32_t vmask = __ballot_sync(0xffffffffu, valid);
+            if (valid) {
+                const uint32_t d = (key[k] >> shift) & 255u;
+                const uint32_t peers = __match_any_sync(vmask, d);
+                const uint32_t before = sm.warp[warp][d];
+                rank[k] = before + __popc(peers & lt);
+                __syncwarp(vmask);
+                if (lane == __ffs(peers) - 1) sm.warp[warp][d] = (unsigned short)(before + __popc(peers));
+            }
+            __syncwarp();
+        }
+        __syncthreads();
+        uint32_t count = 0;
+        if (tid < 256) {
+            for (int w = 0; w < kSmallWarps; ++w) {
+                const uint32_t t = sm.warp[w][tid];
+                sm.warp[w][tid] = (unsigned short)count;
+                count += t;
+            }
+        }
+        // Exclusive prefix of the digits' counts (the first eight warps').
+        uint32_t inc = count;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t t = __shfl_up_sync(0xffffffffu, inc, d);
+            if (lane >= d) inc += t;
+        }
+        if (warp < 8 && lane == 31) sm.scan[warp] = inc;
+        __syncthreads();
+        if (tid < 256) {
+            uint32_t off = 0;
+            for (int w = 0; w < warp; ++w) off += sm.scan[w];
+            sm.base[tid] = off + inc - count;
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            if (warp * (32 * kItems) + k * 32 + lane < n) {
+                const uint32_t d = (key[k] >> shift) & 255u;
+                const uint32_t at = sm.base[d] + sm.warp[warp][d] + rank[k];
+                if (at < (uint32_t)kSmallSort) {
+                    sm.keys[at] = key[k];
+                    sm.vals[at] = (unsigned short)val[k];
+                }
+            }
+        }
+        __syncthreads();
+#pragma unroll
+        for (int k = 0; k < kItems; ++k) {
+            const int i = warp * (32 * kItems) + k * 32 + lane;
+            if (i < n) {
+                key[k] = sm.keys[i];
+                val[k] = sm.vals[i];
+            }
+        }
+    }
+#pragma unroll
+    for (int k = 0; k < kItems; ++k) {
+        const int i = warp * (32 * kItems) + k * 32 + lane;
+        if (i < n) {
+            keys_out[i] = key[k];
+            vals_out[i] = val[k];
+        }
     }
 }
 
@@ -216,22 +324,29 @@ void sort_scratch_bind(SortScratch& s, void* base, int capacity) {
     s.lookback = reinterpret_cast<uint32_t*>(p);
 }
 
-cudaError_t radix_sort_pairs(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out,
-                             int n, int key_bits, SortScratch& s, cudaStream_t stream) {
+cudaError_t clear_ranges(const ClearRange& a, const ClearRange& b, const ClearRange& c, cudaStream_t st) {
+    size_t most = 0;
+    for (const ClearRange* r : {&a, &b, &c}) most = r->words > most ? r->words : most;
+    if (!most) return cudaSuccess;
+    const size_t blocks = (most / 4 + 255) / 256 + 1;
+    k_clear<<<(int)(blocks < 1216 ? blocks : 1216), 256, 0, st>>>(a, b, c);
+    return cudaGetLastError();
+}
+
+cudaError_t radix_sort_counted(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out, int n,
+                               int key_bits, SortScratch& s, cudaStream_t stream) {
     if (n <= 0) return cudaSuccess;
     if (n > s.capacity || n > (int)kValueMask) return cudaErrorInvalidValue;
-    int passes = (key_bits + 7) / 8;
-    if (passes < 1) passes = 1;
+    const int passes = sort_passes(key_bits);
     if (passes > kSortMaxPasses) return cudaErrorInvalidValue;
+    if (n <= kSmallSort) {
+        cudaError_t e = cudaFuncSetAttribute(k_sort_small, cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                             (int)sizeof(SmallSort));
+        if (e != cudaSuccess) return e;
+        k_sort_small<<<1, kSmallThreads, sizeof(SmallSort), stream>>>(keys_in, keys_out, vals_out, n, passes);
+        return cudaGetLastError();
+    }
     const int tiles = (n + kSortTile - 1) / kSortTile;
-    // Zero the histograms, the tile counters and the look-back words of this
-    // sort's tiles; the error word is cleared by its owner.
-    cudaError_t e = cudaMemsetAsync(
-        s.hist, 0, (size_t)kSortMaxPasses * 256 * 4 + 64 + (size_t)passes * tiles * 256 * 4, stream);
-    if (e != cudaSuccess) return e;
-    int hist_blocks = (n + kSortThreads * 16 - 1) / (kSortThreads * 16);
-    if (hist_blocks > 1024) hist_blocks = 1024;
-    k_sort_histogram<<<hist_blocks, kSortThreads, 0, stream>>>(keys_in, n, passes, s.hist);
     // Ping-pong so that the last pass writes keys_out / vals_out.
     const uint32_t* kin = keys_in;
     const uint32_t* vin = nullptr;
@@ -239,14 +354,26 @@ cudaError_t radix_sort_pairs(const uint32_t* keys_in, uint32_t* keys_out, uint32
         const bool to_out = ((passes - 1 - p) % 2) == 0;
         uint32_t* kout = to_out ? keys_out : s.keys_alt;
         uint32_t* vout = to_out ? vals_out : s.vals_alt;
-        k_onesweep<<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, 8 * p,
-                                                       s.hist + p * 256,
-                                                       s.lookback + (size_t)p * tiles * 256,
-                                                       s.tile_ctr + p, s.err);
+        k_onesweep<<<tiles, kSortThreads, 0, stream>>>(kin, vin, kout, vout, n, 8 * p, s.hist + p * 256,
+                                                       s.lookback + (size_t)p * tiles * 256, s.tile_ctr + p,
+                                                       s.err);
         kin = kout;
         vin = vout;
     }
     return cudaGetLastError();
+}
+
+cudaError_t radix_sort_pairs(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out,
+                             int n, int key_bits, SortScratch& s, cudaStream_t stream) {
+    if (n <= 0) return cudaSuccess;
+    if (n > s.capacity || n > (int)kValueMask) return cudaErrorInvalidValue;
+    if (sort_passes(key_bits) > kSortMaxPasses) return cudaErrorInvalidValue;
+    if (n > kSmallSort) {
+        cudaError_t e = clear_ranges(sort_clear(s, n, key_bits), ClearRange{}, ClearRange{}, stream);
+        if (e != cudaSuccess) return e;
+        k_sort_histogram<<<count_blocks(n), kCountThreads, 0, stream>>>(keys_in, n, sort_counts(s, n, key_bits));
+    }
+    return radix_sort_counted(keys_in, keys_out, vals_out, n, key_bits, s, stream);
 }
 
 }  // namespace pbf

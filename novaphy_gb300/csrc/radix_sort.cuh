@@ -53,6 +53,75 @@ constexpr size_t sort_scratch_bytes(int capacity) {
 // Carves the scratch out of one device allocation of sort_scratch_bytes().
 void sort_scratch_bind(SortScratch& s, void* base, int capacity);
 
+inline int sort_passes(int key_bits) { return key_bits <= 8 ? 1 : (key_bits + 7) / 8; }
+
+// Up to this many keys one block does every pass in shared memory (a chain of
+// launches over one to four tiles took 24 us for 8,000 keys).
+constexpr int kSmallSort = 8192;
+
+// A range to be set to `value` before a sort, or another build (k_clear).
+struct ClearRange {
+    uint32_t* p = nullptr;  // 16-byte aligned
+    size_t words = 0;
+    uint32_t value = 0;
+};
+
+// The sort's histograms, tile counters and look-back words (empty for a small
+// sort).  The error word is cleared by its owner.
+inline ClearRange sort_clear(const SortScratch& s, int n, int key_bits) {
+    if (n <= kSmallSort) return ClearRange{};
+    const size_t tiles = ((size_t)n + kSortTile - 1) / kSortTile;
+    return ClearRange{s.hist, (size_t)kSortMaxPasses * 256 + 16 + (size_t)sort_passes(key_bits) * tiles * 256, 0u};
+}
+
+// Sets up to three ranges, in one launch.
+cudaError_t clear_ranges(const ClearRange& a, const ClearRange& b, const ClearRange& c, cudaStream_t st);
+
+// Where a kernel that makes the keys counts their digits (null for a small
+// sort), and the counting: every thread of the block calls count for each of
+// its keys between begin and end.
+struct SortCounts {
+    uint32_t* hist;
+    int passes;
+};
+inline SortCounts sort_counts(const SortScratch& s, int n, int key_bits) {
+    return SortCounts{n <= kSmallSort ? nullptr : s.hist, sort_passes(key_bits)};
+}
+// Blocks of kCountThreads for a kernel over n particles that counts: a few
+// keys per thread at most, so that a block's counts are worth their adding.
+constexpr int kCountThreads = 256;
+inline int count_blocks(int n) {
+    const int b = (n + kCountThreads - 1) / kCountThreads;
+    return b < 152 * 8 ? b : 152 * 8;
+}
+#ifdef __CUDACC__
+struct BlockCounts {
+    uint32_t c[kSortMaxPasses][256];
+    __device__ __forceinline__ void begin(const SortCounts& S) {
+        if (!S.hist) return;
+        for (int i = threadIdx.x; i < S.passes * 256; i += blockDim.x) (&c[0][0])[i] = 0u;
+        __syncthreads();
+    }
+    __device__ __forceinline__ void count(const SortCounts& S, uint32_t key) {
+        if (!S.hist) return;
+        for (int p = 0; p < S.passes; ++p) atomicAdd(&c[p][(key >> (8 * p)) & 255u], 1u);
+    }
+    __device__ __forceinline__ void end(const SortCounts& S) {
+        if (!S.hist) return;
+        __syncthreads();
+        for (int i = threadIdx.x; i < S.passes * 256; i += blockDim.x) {
+            const uint32_t n = (&c[0][0])[i];
+            if (n) atomicAdd(S.hist + i, n);
+        }
+    }
+};
+#endif
+
+// Sorts keys_in[0..n) (each < 2^key_bits) whose scratch was cleared (sort_clear)
+// and whose digits were counted (sort_counts); otherwise as radix_sort_pairs.
+cudaError_t radix_sort_counted(const uint32_t* keys_in, uint32_t* keys_out, uint32_t* vals_out, int n,
+                               int key_bits, SortScratch& s, cudaStream_t stream);
+
 // Sorts keys_in[0..n) (each < 2^key_bits).  Values are the input positions.
 // Results land in keys_out / vals_out.  keys_in is not modified and may not
 // alias the outputs.  Returns a CUDA error code (cudaSuccess on success).
