@@ -207,7 +207,7 @@ __device__ __forceinline__ float pressure_weight(float rho, const StepConsts& C)
 // Boundary density of the fluid index's points: rho += sum, in particle order,
 // and the points' w from the density to the pressure weight.
 template <int TP>
-__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+__global__ void __launch_bounds__(128, kTeamMinBlocks<TP>)
 k_boundary_density(float4* __restrict__ fpos, const uint32_t* __restrict__ fidx, int n, const QuerySet Q,
                    const PointIndex I, float* __restrict__ rho, const StepConsts C) {
     __shared__ TeamSmem<TP> sm;
@@ -236,7 +236,7 @@ k_pressure_weights(float4* __restrict__ fpos, int n, const StepConsts C) {
 // Force on each boundary point (bpos, bidx: the boundary index's points and
 // their original numbers) from the fluid index I.
 template <int TP>
-__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+__global__ void __launch_bounds__(128, kTeamMinBlocks<TP>)
 k_coupling(const float4* __restrict__ bpos, const uint32_t* __restrict__ bidx, const int* __restrict__ body,
            const int* __restrict__ body_dynamic, int nb, int nbodies, const QuerySet Q, const PointIndex I,
            float4* __restrict__ Fb, const StepConsts C) {
@@ -428,7 +428,7 @@ k_rigid_world(pbf_rigid_body* __restrict__ bodies, int nbodies,
 }
 
 template <int TP>
-__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+__global__ void __launch_bounds__(128, kTeamMinBlocks<TP>)
 k_volumes(int nb, const QuerySet Q, const PointIndex I, float* __restrict__ psi, const StepConsts C) {
     __shared__ TeamSmem<TP> sm;
     const TeamThread<TP> T(nb);

@@ -835,8 +835,18 @@ constexpr int kTeamWarps = 4;
 // one-thread walk).
 constexpr int kMaxGroups = 6;
 
+// A group's candidate sequence: ranges [start, start + len) in cell order (key
+// order for a dirty cell), their rows' first slots, and the number of words of
+// the ranges before each.
+struct RangeList {
+    uint32_t start[32], len[32], slot[32];
+    int before[32];
+};
+constexpr uint32_t kRunRange = 0x80000000u;
+
 // Shared memory of a warp walk.
 struct WalkSmem {
+    RangeList ranges;
     // One fp16 row of eight per candidate: x, y, z, |u|^2 (high, low), 1, 1, 0.
     alignas(16) uint32_t stage[128 * 4];
     uint32_t base[kWalkWords];  // first candidate (cell order, or key order in buckets)
@@ -860,6 +870,7 @@ struct TeamSmem {
     static constexpr int kWarpBytes = kTermBytes > 2048 ? kTermBytes : 2048;
     static constexpr int kListRow = kTeamTerms + 2;
     alignas(16) unsigned char warp[kTeamWarps][(kWarpBytes + 15) / 16 * 16];
+    RangeList ranges;
     uint32_t base[kTeamWords];
     uint32_t info[kTeamWords];
     uint32_t mask[kTeamWarps][4 * TP];
@@ -873,6 +884,10 @@ struct TeamSmem {
 // (80 registers a thread).
 template <int BS>
 constexpr int kPassMinBlocks = 768 / BS;
+// The teams' kernels: of 8 particles seven blocks (72 registers), so that up to
+// 8,500 particles run in one wave (8,000: 239 us a step against 258 with six).
+template <int TP>
+constexpr int kTeamMinBlocks = TP == 8 ? 7 : 6;
 
 // A group: the cells [cx, cx + W - 3] of row (cy, cz), or one dirty cell
 // (own: its bucket row + 1).  split: the row would wrap in x, so its cells
@@ -986,35 +1001,28 @@ __device__ __forceinline__ WalkBox walk_box(bool want, const float4 xi, float in
     return B;
 }
 
-// The candidate sequence of a group, one range per lane: [start, start + len)
-// in cell order (key order for a dirty cell), the row's first slot, the
-// number of words before the lane's first one and in total, and with kRuns
-// whether the range holds runs (at least kRunRow candidates in slots with a
-// run's first particle).
-struct WalkRanges {
-    uint32_t start, len, slot;
-    int words, before, total;
-    bool runs;
-};
-
+// Finds the candidate sequence of a group, one range per lane, and writes it to
+// L where `keep` is set (a team's first warp; the caller syncs).  Returns the
+// number of its words, and with kRuns sets `runs` where a range holds runs (at
+// least kRunRow candidates in slots with a run's first particle; kRunRange in
+// its len).
 template <bool kRuns>
-__device__ __forceinline__ WalkRanges walk_ranges(const WalkGroup& Gr, const WalkIndex& I,
-                                                  const GridDesc& Gd, const Grid& G) {
+__device__ __forceinline__ int walk_ranges(RangeList& L, const WalkGroup& Gr, const WalkIndex& I,
+                                           const GridDesc& Gd, const Grid& G, bool keep, bool& runs) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
-    WalkRanges R;
-    R.start = R.len = R.slot = 0u;
-    R.runs = false;
+    uint32_t start = 0u, len = 0u, slot = 0u;
+    bool has_runs = false;
     if (Gr.own) {
         if (lane < 27) {
             const uint32_t b0 = __ldg(I.btab + (size_t)(Gr.own - 1u) * 27u + (uint32_t)lane);
             if (b0 != kNoBucket) {
-                R.start = b0;
-                R.len = __ldg(I.end + b0) - b0;
+                start = b0;
+                len = __ldg(I.end + b0) - b0;
                 if constexpr (kRuns) {
-                    if (G.segend && R.len >= kRunRow && b0 < I.n) {
+                    if (G.segend && len >= kRunRow && b0 < I.n) {
                         const int4 c = G.scell[b0];
-                        R.runs = (__ldg(G.slot_alias + slot_of(c.x, c.y, c.z, Gd)) & kRunSlot) != 0;
+                        has_runs = (__ldg(G.slot_alias + slot_of(c.x, c.y, c.z, Gd)) & kRunSlot) != 0;
                     }
                 }
             }
@@ -1023,35 +1031,42 @@ __device__ __forceinline__ WalkRanges walk_ranges(const WalkGroup& Gr, const Wal
         const int dx = Gr.split ? lane % 3 : 0;
         const int yz = Gr.split ? lane / 3 : lane;
         const int k = Gr.split ? 1 : Gr.W;
-        R.slot = slot_of(Gr.cx - 1 + dx, Gr.cy + yz % 3 - 1, Gr.cz + yz / 3 - 1, Gd);
-        R.start = __ldg(I.off + R.slot);
-        R.len = __ldg(I.off + R.slot + k) - R.start;
+        slot = slot_of(Gr.cx - 1 + dx, Gr.cy + yz % 3 - 1, Gr.cz + yz / 3 - 1, Gd);
+        start = __ldg(I.off + slot);
+        len = __ldg(I.off + slot + k) - start;
         if constexpr (kRuns) {
-            if (G.segend && R.len >= kRunRow)
-                for (int d = 0; d < k; ++d) R.runs |= (__ldg(G.slot_alias + R.slot + d) & kRunSlot) != 0;
+            if (G.segend && len >= kRunRow)
+                for (int d = 0; d < k; ++d) has_runs |= (__ldg(G.slot_alias + slot + d) & kRunSlot) != 0;
         }
     }
-    R.words = (int)((R.len + 31u) >> 5);
-    int sum = R.words;
+    const int words = (int)((len + 31u) >> 5);
+    int sum = words;
 #pragma unroll
     for (int o = 1; o < 32; o <<= 1) {
         const int v = __shfl_up_sync(full, sum, o);
         if (lane >= o) sum += v;
     }
-    R.total = __shfl_sync(full, sum, 31);
-    R.before = sum - R.words;
-    return R;
+    if (keep) {
+        L.start[lane] = start;
+        L.len[lane] = len | (has_runs ? kRunRange : 0u);
+        L.slot[lane] = slot;
+        L.before[lane] = sum - words;
+    }
+    runs = kRuns && __any_sync(full, has_runs);
+    return __shfl_sync(full, sum, 31);
 }
 
-// Lists words [done, done + room) of the sequence; returns how many there are.
-__device__ __forceinline__ int list_words(const WalkRanges& R, int done, int room, uint32_t* base,
-                                          uint32_t* info) {
-    for (int k = max(0, done - R.before); k < R.words && R.before + k < done + room; ++k) {
-        const int w = R.before + k - done;
-        base[w] = R.start + 32u * (uint32_t)k;
-        info[w] = min(32u, R.len - 32u * (uint32_t)k) | ((threadIdx.x & 31u) << 8);
+// Lists words [done, done + room) of a sequence without runs.
+__device__ __forceinline__ void list_words(const RangeList& L, int done, int room, uint32_t* base,
+                                           uint32_t* info) {
+    const int lane = threadIdx.x & 31;
+    const uint32_t start = L.start[lane], len = L.len[lane];
+    const int before = L.before[lane], words = (int)((len + 31u) >> 5);
+    for (int k = max(0, done - before); k < words && before + k < done + room; ++k) {
+        const int w = before + k - done;
+        base[w] = start + 32u * (uint32_t)k;
+        info[w] = min(32u, len - 32u * (uint32_t)k) | ((uint32_t)lane << 8);
     }
-    return min(room, R.total - done);
 }
 
 // Stages four words of candidates and tests them against the 8 NT particles
@@ -1136,33 +1151,36 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
     }
     const bool key = Gr.own != 0u;
     const bool multi = Gr.W > 3;
-    const WalkRanges R = walk_ranges<kRuns>(Gr, I, Gd, G);
-    const bool runs = kRuns && __any_sync(full, R.runs);
+    bool runs;
+    const int total = walk_ranges<kRuns>(sm.ranges, Gr, I, Gd, G, true, runs);
+    __syncwarp();
     // Position of the listing with runs: range and candidate.
     int at_r = 0;
-    uint32_t at_q = __shfl_sync(full, R.start, 0);
+    uint32_t at_q = 0u;
     int done = 0;
     // Lists the next words; returns how many.
     auto fill = [&]() -> int {
         if (!runs) {
-            const int nw = list_words(R, done, kWalkWords, sm.base, sm.info);
+            const int nw = min(kWalkWords, total - done);
+            list_words(sm.ranges, done, kWalkWords, sm.base, sm.info);
             done += nw;
             return nw;
         }
         int nw = 0;
         const int nr = key || Gr.split ? 27 : 9;
         while (nw < kWalkWords && at_r < nr) {
-            const uint32_t e = __shfl_sync(full, R.start + R.len, at_r);
-            if (at_q >= e) {
+            const uint32_t st = sm.ranges.start[at_r], ln = sm.ranges.len[at_r];
+            const uint32_t len_r = ln & ~kRunRange;
+            if (at_q >= len_r) {
                 ++at_r;
-                at_q = __shfl_sync(full, R.start, at_r & 31);
+                at_q = 0u;
                 continue;
             }
-            uint32_t cnt = min(32u, e - at_q), lead = 0u, step = cnt;
-            if (__shfl_sync(full, R.runs ? 1 : 0, at_r)) {
+            uint32_t cnt = min(32u, len_r - at_q), lead = 0u, step = cnt;
+            if (ln & kRunRange) {
                 // A range with runs: the word ends with a run's first
                 // particle, and the next one begins past the run.
-                uint32_t q = at_q + (uint32_t)lane;
+                const uint32_t q = st + at_q + (uint32_t)lane;
                 const bool ok = (uint32_t)lane < cnt;
                 const bool first = ok && ((uint32_t)__ldg(G.sown + q) & kLeadBit);
                 const uint32_t m = __ballot_sync(full, first);
@@ -1176,7 +1194,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
                 }
             }
             if (lane == 0) {
-                sm.base[nw] = at_q;
+                sm.base[nw] = st + at_q;
                 sm.info[nw] = cnt | ((uint32_t)at_r << 8) | lead;
             }
             ++nw;
@@ -1238,8 +1256,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
                     if (lam_zero) m &= nz[j];
                 if (!want) m = 0u;
                 if (multi) {
-                    const uint32_t slot = __shfl_sync(full, R.slot, w < nw ? (sm.info[w] >> 8) & 31u : 0u);
-                    if (m) m &= own_cells(I, slot, ci - Gr.cx, sm.base[w]);
+                    if (m) m &= own_cells(I, sm.ranges.slot[(sm.info[w] >> 8) & 31u], ci - Gr.cx, sm.base[w]);
                 }
                 sm.mask[sm.at(w, lane)] = m;
                 cnt += __popc(m);
@@ -1501,7 +1518,9 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
     }
     const bool key = Gr.own != 0u;
     const bool multi = Gr.W > 3;
-    const WalkRanges R = walk_ranges<false>(Gr, I, Gd, G);
+    bool runs;
+    const int words = walk_ranges<false>(sm.ranges, Gr, I, Gd, G, wid == 0, runs);
+    __syncwarp();
     const bool lam_zero = kLam && xi.w == 0.0f;
     const bool all_zero = kLam && !__any_sync(full, want && xi.w != 0.0f);
     uint32_t run = 0u;  // terms of particle pl listed so far
@@ -1545,10 +1564,9 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
         __syncthreads();
     };
 
-    for (int done = 0; done < R.total;) {
-        const int nw = min(kTeamWords, R.total - done);
-        if (wid == 0) list_words(R, done, kTeamWords, sm.base, sm.info);
-        done += nw;
+    for (int done = 0; done < words; done += kTeamWords) {
+        const int nw = min(kTeamWords, words - done);
+        if (wid == 0) list_words(sm.ranges, done, kTeamWords, sm.base, sm.info);
         __syncthreads();
         for (int b0 = 0; b0 < nw; b0 += 4 * kTeamWarps) {
             // --- phase 1: this warp's four words
@@ -1603,8 +1621,7 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
                     if (!want) v = 0u;
                     if (multi) {
                         const int w = b + j;
-                        const uint32_t slot = __shfl_sync(full, R.slot, w < nw ? (sm.info[w] >> 8) & 31u : 0u);
-                        if (v) v &= own_cells(I, slot, ci - Gr.cx, sm.base[w]);
+                        if (v) v &= own_cells(I, sm.ranges.slot[(sm.info[w] >> 8) & 31u], ci - Gr.cx, sm.base[w]);
                     }
                     m[i] = v;
                 }
@@ -2369,7 +2386,7 @@ k_density_lambda(const float4* __restrict__ xin, float4* __restrict__ xout, floa
 }
 
 template <int TP, class P>
-__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+__global__ void __launch_bounds__(128, kTeamMinBlocks<TP>)
 k_density_lambda_team(const float4* __restrict__ xin, float4* __restrict__ xout,
                       float* __restrict__ srho, int it, int n, const Grid G, const P prm) {
     __shared__ TeamSmem<TP> sm;
@@ -2507,7 +2524,7 @@ k_delta(const float4* __restrict__ xin, float4* __restrict__ xout, const float4*
 }
 
 template <int TP, class P>
-__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+__global__ void __launch_bounds__(128, kTeamMinBlocks<TP>)
 k_delta_team(const float4* __restrict__ xin, float4* __restrict__ xout, const float4* __restrict__ sx,
              const float* __restrict__ srho, float4* __restrict__ sv, int it, int n, const Grid G,
              const P prm) {
@@ -2735,7 +2752,7 @@ k_xsph_commit(const float4* __restrict__ xin, const float4* __restrict__ sv, con
 }
 
 template <int TP, class P>
-__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+__global__ void __launch_bounds__(128, kTeamMinBlocks<TP>)
 k_xsph_commit_team(const float4* __restrict__ xin, const float4* __restrict__ sv,
                    const float4* __restrict__ sx, const float* __restrict__ srho, int n, int skip_vort,
                    const Grid G, const P prm) {
@@ -2796,7 +2813,7 @@ k_xsph_omega(const float4* __restrict__ xin, const float4* __restrict__ sv, floa
 }
 
 template <int TP, class P>
-__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+__global__ void __launch_bounds__(128, kTeamMinBlocks<TP>)
 k_xsph_omega_team(const float4* __restrict__ xin, const float4* __restrict__ sv, float4* __restrict__ sv2,
                   float4* __restrict__ som, int n, const Grid G, const P prm) {
     __shared__ TeamSmem<TP> sm;
@@ -2861,7 +2878,7 @@ k_vorticity_commit(const float4* __restrict__ xin, const float4* __restrict__ sv
 }
 
 template <int TP, class P>
-__global__ void __launch_bounds__(128, kPassMinBlocks<128>)
+__global__ void __launch_bounds__(128, kTeamMinBlocks<TP>)
 k_vorticity_commit_team(const float4* __restrict__ xin, const float4* __restrict__ sv,
                         const float4* __restrict__ sv2, const float4* __restrict__ som,
                         const float4* __restrict__ sx, const float* __restrict__ srho, int n, const Grid G,
