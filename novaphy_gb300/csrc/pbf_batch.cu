@@ -93,6 +93,9 @@ struct pbf_batch {
     void* wmem = nullptr;  // step scratch (bind_work)
     void* smem = nullptr;  // sort scratch
     void* xmem = nullptr;  // scene ids
+    void* lmem = nullptr;  // kept lists (list_bytes(B.list_cap); null: none)
+    int lists_tried = 0;   // the capacity they were last tried for
+    bool lists_off = false;  // a server's batch: its scratch is what batch_reserve took
     StepBuffers B{};
     SortScratch sort{};
     uint32_t* status = nullptr;  // status word of the batch's steps
@@ -187,6 +190,33 @@ int ensure_particles(pbf_batch* b, int n) {
     b->spid = reinterpret_cast<uint32_t*>(p + f1);
     b->cap = c;
     return PBF_OK;
+}
+
+void free_lists(pbf_batch* b) {
+    if (!b->lmem) return;
+    cudaFree(b->lmem);
+    give_list_bytes(list_bytes(b->B.list_cap));
+    b->lmem = nullptr;
+    bind_lists(b->B, nullptr, 0);
+}
+
+// Kept lists for steps of n particles, tried once per size.
+void ensure_lists(pbf_batch* b, int n) {
+    if (b->lists_off || n <= b->B.list_cap || n <= b->lists_tried) return;
+    drop_graph(b);
+    free_lists(b);
+    const int c = std::min(b->cap, n + n / 4);
+    b->lists_tried = c;
+    const size_t lb = list_bytes(c);
+    if (c > kListMaxParticles || !take_list_bytes(lb)) return;
+    void* p = nullptr;
+    if (cudaMalloc(&p, lb) != cudaSuccess) {
+        cudaGetLastError();
+        give_list_bytes(lb);
+        return;
+    }
+    b->lmem = p;
+    bind_lists(b->B, p, c);
 }
 
 int ensure_slots(pbf_batch* b, uint32_t nslots) {
@@ -384,6 +414,7 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
     }
     const int n = (int)n_total;
     int rc = ensure_particles(b, n);
+    if (!rc) ensure_lists(b, n);
     if (!rc) rc = ensure_slots(b, (uint32_t)slots_total);
     if (!rc) rc = ensure_tables(b, ns);
     if (rc) return rc;
@@ -697,6 +728,7 @@ void batch_counters(const pbf_batch* b, long long* captures, long long* updates,
 int batch_reserve(pbf_batch* b, int particles, int scenes) {
     std::lock_guard<std::mutex> lk(b->mu);
     DeviceGuard dg(b->device);
+    b->lists_off = true;
     int rc = ensure_particles(b, particles);
     if (!rc) rc = ensure_tables(b, scenes);
     if (!rc) rc = ensure_bad(b, scenes);
@@ -706,6 +738,7 @@ int batch_reserve(pbf_batch* b, int particles, int scenes) {
 size_t batch_bytes(const pbf_batch* b) {
     size_t t = 0;
     if (b->wmem) t += work_bytes(b->cap) + sort_scratch_bytes(b->cap) + extra_bytes(b->cap);
+    if (b->lmem) t += list_bytes(b->B.list_cap);
     if (b->off)
         t += align_up((size_t)b->off_cap * 4, 256) + align_up(b->off_cap, 256) +
              (size_t)b->off_cap * 8;
@@ -755,6 +788,7 @@ int pbf_batch_destroy(pbf_batch* b) {
             if (kv.second.e0) cudaEventDestroy(kv.second.e0);
             if (kv.second.e1) cudaEventDestroy(kv.second.e1);
         }
+        free_lists(b);
         for (void* m : {b->wmem, b->smem, b->xmem, static_cast<void*>(b->off),
                         static_cast<void*>(b->d_bad), static_cast<void*>(b->barrier)})
             if (m) cudaFree(m);

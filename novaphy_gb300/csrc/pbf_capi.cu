@@ -2,6 +2,7 @@
 // transfer, settings -> per-step constants, and step orchestration with CUDA
 // graph replay.
 #include <algorithm>
+#include <atomic>
 #include <cmath>
 #include <cstdio>
 #include <cstdlib>
@@ -124,6 +125,24 @@ cudaMemPool_t scene_pool(int device) {
     return pools[device];
 }
 
+static std::atomic<size_t> list_bytes_held{0};
+
+bool take_list_bytes(size_t bytes) {
+    size_t free = 0, total = 0;
+    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    if (bytes > free / 4) return false;
+    size_t held = list_bytes_held.load();
+    do {
+        if (held + bytes > kListMaxBytes) return false;
+    } while (!list_bytes_held.compare_exchange_weak(held, held + bytes));
+    return true;
+}
+
+void give_list_bytes(size_t bytes) { list_bytes_held.fetch_sub(bytes); }
+
 int pool_alloc(void** p, size_t bytes, int device, cudaStream_t st) {
     cudaMemPool_t pool = scene_pool(device);
     if (!pool) return fail(PBF_ERR_CUDA, "cudaMemPoolCreate failed");
@@ -195,12 +214,23 @@ int take_status(uint32_t* device_word, uint32_t* host_word, uint32_t* out) {
 
 namespace {
 
+void free_lists(pbf_scene* s) {
+    if (s->lmem) {
+        pool_free(s->lmem, s->stream);
+        give_list_bytes(list_bytes(s->B.list_cap));
+    }
+    s->lmem = nullptr;
+    s->no_lists = false;
+    bind_lists(s->B, nullptr, 0);
+}
+
 void free_particles(pbf_scene* s) {
     ++s->buf_gen;
     if (s->graph) {
         cudaGraphExecDestroy(s->graph);
         s->graph = nullptr;
     }
+    free_lists(s);
     for (void* m : {s->pmem, s->wmem, s->smem}) pool_free(m, s->stream);
     s->pmem = s->wmem = s->smem = nullptr;
     s->cap = s->work_cap = 0;
@@ -247,6 +277,7 @@ int ensure_work(pbf_scene* s) {
         cudaGraphExecDestroy(s->graph);
         s->graph = nullptr;
     }
+    free_lists(s);
     for (void* m : {s->wmem, s->smem}) pool_free(m, s->stream);
     s->wmem = s->smem = nullptr;
     s->work_cap = 0;
@@ -268,6 +299,29 @@ int ensure_work(pbf_scene* s) {
     s->B.err = s->sort.err;
     s->work_cap = c;
     return PBF_OK;
+}
+
+// Kept lists for the scene's own steps, tried once per capacity.
+void ensure_lists(pbf_scene* s) {
+    if (s->lmem || s->no_lists) return;
+    const size_t lb = list_bytes(s->work_cap);
+    s->no_lists = true;
+    if (s->work_cap > kListMaxParticles || !take_list_bytes(lb)) return;
+    cudaMemPool_t pool = scene_pool(s->device);
+    void* p = nullptr;
+    if (!pool || cudaMallocFromPoolAsync(&p, lb, pool, s->stream) != cudaSuccess) {
+        cudaGetLastError();
+        give_list_bytes(lb);
+        return;
+    }
+    ++s->buf_gen;
+    if (s->graph) {
+        cudaGraphExecDestroy(s->graph);
+        s->graph = nullptr;
+    }
+    s->no_lists = false;
+    s->lmem = p;
+    bind_lists(s->B, p, s->work_cap);
 }
 
 }  // namespace
@@ -582,6 +636,7 @@ int run_steps(pbf_scene* s, float dt, int nsteps) {
     StepConsts C;
     int rc = make_consts(s, dt, C);
     if (rc) return rc;
+    ensure_lists(s);
     if (!graphs_enabled()) {
         for (int k = 0; k < nsteps; ++k) {
             rc = enqueue(s, C, s->stream);
@@ -925,6 +980,7 @@ size_t scene_device_bytes(const pbf_scene* s) {
     if (s->wmem)
         b += work_bytes(s->work_cap) + align_up((size_t)s->work_cap * 4, 256) +
              sort_scratch_bytes(s->work_cap);
+    if (s->lmem) b += list_bytes(s->B.list_cap);
     if (s->off)
         b += align_up((size_t)s->off_cap * 4, 256) + align_up(s->off_cap, 256) +
              (size_t)s->off_cap * 8 + 4 * kWalkHist * 4;
@@ -1218,6 +1274,7 @@ int pbf_scene_step_profiled(pbf_scene* s, float dt, float* phase_ms, int* launch
     StepConsts C;
     int rc = make_consts(s, dt, C);
     if (rc) return rc;
+    ensure_lists(s);
     PhaseMarks pm;
     int created = 0;
     cudaError_t e = cudaSuccess;
@@ -1708,6 +1765,7 @@ int two_way_step(pbf_scene* s, const StepConsts& C) {
     int rc = ensure_boundary_grid(s, C.grid.nslots);
     if (!rc) rc = ensure_two_way(s);
     if (rc) return rc;
+    ensure_lists(s);
     cudaStream_t st = s->stream;
     cudaError_t e = boundary_xform(b.local, b.body, b.nb, b.body_pos, b.body_quat, b.nbodies,
                                    b.world, st);

@@ -95,6 +95,31 @@ inline void bind_work(StepBuffers& B, void* mem, int c) {
     B.btab = reinterpret_cast<uint32_t*>(p);
 }
 
+// Kept lists of c particles (StepBuffers::lists): rows, then their numbers.
+// They take seven times the rest of the step scratch, so no scene or batch of
+// more than kListMaxParticles has any, all of a process's together stay below
+// kListMaxBytes, and they are not needed: without them the passes walk.
+constexpr int kListMaxParticles = 4 << 20;
+constexpr size_t kListMaxBytes = (size_t)16 << 30;
+
+inline size_t list_bytes(int c) {
+    const size_t r = align_up((size_t)c, 32);
+    return r * kListRows * sizeof(uint2) + r * 4;
+}
+
+inline void bind_lists(StepBuffers& B, void* mem, int c) {
+    const size_t r = align_up((size_t)c, 32);
+    B.lists = static_cast<uint2*>(mem);
+    B.listed = reinterpret_cast<uint32_t*>(static_cast<char*>(mem) + r * kListRows * sizeof(uint2));
+    B.list_cap = mem ? c : 0;
+    if (!mem) B.listed = nullptr;
+}
+
+// Whether lists of that many bytes may be allocated now (then counted until
+// they are given back).
+bool take_list_bytes(size_t bytes);
+void give_list_bytes(size_t bytes);
+
 }  // namespace capi
 }  // namespace pbf
 
@@ -116,6 +141,8 @@ struct pbf_scene {
     void* pmem = nullptr;  // resident state: x, v, rho, lambda, staging
     void* wmem = nullptr;  // step scratch (sorted copies, keys, buckets)
     void* smem = nullptr;  // sort scratch
+    void* lmem = nullptr;  // kept lists (list_bytes(work_cap); null: none)
+    bool no_lists = false;  // there was no room for them
     uint32_t* off = nullptr;
     uint32_t off_cap = 0;  // entries
     float* staging = nullptr;  // float[3 cap]

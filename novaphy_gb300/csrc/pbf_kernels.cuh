@@ -672,6 +672,8 @@ struct Grid {
     uint32_t* dhist;                     // see StepBuffers::dhist
     const uint32_t* segend;              // see StepBuffers::segend (large single scenes)
     const unsigned char* slot_alias;     // with kRunSlot where segend is set
+    uint2* lists;                        // see StepBuffers::lists (null: none are kept)
+    uint32_t* listed;
 };
 
 // for_each_candidate over a single scene's step with runs of identical
@@ -843,6 +845,27 @@ struct RangeList {
     int before[32];
 };
 constexpr uint32_t kRunRange = 0x80000000u;
+
+// Kept lists.  The density pass keeps each particle's listed candidates, and
+// the delta pass, whose candidates sit where they sat for the density, reads
+// them instead of walking; the XSPH-omega pass keeps them for the vorticity
+// pass.  A row is two candidates (cell-order positions); an odd candidate's
+// partner is the particle itself, whose terms are exact zeros.  A warp walk's
+// particles have their rows side by side (row r of particle p at
+// (p / 32 kListRows + r) 32 + p % 32), a team's particles one after another
+// (p kListRows + r).  StepBuffers::listed holds the number of rows, or kNoList
+// where the walk did not list (lane-by-lane walks, runs) or had no room.
+//
+// What it saves: a walk's listing and scanning are half of its instructions
+// (density of 300,000 particles: 180 of 318 million); a reader has one
+// coalesced 8-byte load per row instead, and a team's warps no longer wait for
+// each other.  The rows of a million particles are 1 GB written and read per
+// iteration, a third of the memory bandwidth while both passes are bound by
+// their instructions.  Measured (us a call, walking / with lists): 1,000
+// particles 105 / 96; 8,000 235 / 204; 4 steps of 43,993 3,989 / 3,332;
+// 65,565 (fast build) 1,862 / 1,603; 3 steps of 395,101 21,180 / 18,450; a
+// million 6,263 / 5,528; a batch of 352,901 3,121 / 2,928.
+__device__ __forceinline__ uint32_t list_at(uint32_t p) { return (p >> 5) * (32u * kListRows) + (p & 31u); }
 
 // Shared memory of a warp walk.
 struct WalkSmem {
@@ -1129,12 +1152,14 @@ __device__ __forceinline__ uint32_t own_cells(const WalkIndex& I, uint32_t slot,
 // started at +0, never are -0, so a lane whose lambda is zero lists
 // candidates with a nonzero one only.  kRuns: in ranges that hold runs of
 // identical particles (k_segments) a run is listed as its first particle,
-// whose term is added as many times as the run is long.
-template <bool kPersist, bool kLam, bool kRuns, class Sums>
+// whose term is added as many times as the run is long.  kKeep: the lane's
+// candidates go to its kept list, from list + list_at(its particle); kept is
+// their number of rows.
+template <bool kPersist, bool kLam, bool kRuns, bool kKeep, class Sums>
 __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bool want, int ci,
                                            const float4 xi, const float4* xin, float inv_h,
                                            const GridDesc& Gd, const WalkIndex& I, const Grid& G,
-                                           Sums& sums) {
+                                           uint32_t p, uint32_t& kept, Sums& sums) {
     const unsigned full = 0xffffffffu;
     const int lane = threadIdx.x & 31;
     const int g = lane >> 2, t4 = lane & 3;
@@ -1281,6 +1306,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             return bq + k;
         };
         if (kRuns && runs) {
+            if (kKeep && want) kept = kNoList;
             for (int t = 0; t < cnt; ++t) {
                 uint32_t q = next_q();
                 const uint32_t i = sm.info[w];
@@ -1293,18 +1319,40 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             }
         } else {
             float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
-            auto load = [&](float4& x, float4& e) {
+            auto load = [&](float4& x, float4& e) -> uint32_t {
                 uint32_t q = next_q();
                 if (key) q = I.at(q);
                 x = ld_step<kPersist>(xin + q);
                 if constexpr (Sums::kExtra) e = sums.extra(q);
+                return q;
             };
-            if (cnt > 0) load(xa, ea);
-            if (cnt > 1) load(xb, eb);
+            // Room for this batch of the lane's list?
+            uint2* to = nullptr;
+            if constexpr (kKeep) {
+                const uint32_t rows = ((uint32_t)cnt + 1u) / 2u;
+                if (kept + rows <= kListRows) {
+                    to = G.lists + list_at(p) + 32u * kept;
+                    kept += rows;
+                } else {
+                    kept = kNoList;
+                }
+            }
+            // The lane's listed candidates t and t + 1 (t < cnt).
+            auto next = [&](int t) {
+                const uint32_t qa = load(xa, ea);
+                uint32_t qb = p;
+                if (t + 1 < cnt) qb = load(xb, eb);
+                if constexpr (kKeep) {
+                    if (to) {
+                        __stcs(to, make_uint2(qa, qb));
+                        to += 32;
+                    }
+                }
+            };
+            if (cnt > 0) next(0);
             for (int t = 0; t < most; t += 2) {
                 const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
-                if (t + 2 < cnt) load(xa, ea);
-                if (t + 3 < cnt) load(xb, eb);
+                if (t + 2 < cnt) next(t + 2);
                 sums.add2(x0, x1, e0, e1, t < cnt, t + 1 < cnt);
             }
         }
@@ -1490,12 +1538,13 @@ struct TeamSums {
 // The team walk of one group (every lane of the team's four warps calls it).
 // In the listing, lane l of each warp stands for the team's particle
 // l / (32 / TP): xi, ci, want as in walk_group.  In the evaluation, thread t
-// stands for particle t / (128 / TP), which is the one that `sums` is about.
-template <int TP, bool kLam, class Sums>
+// stands for particle t / (128 / TP) of the team, sorted position p, which is
+// the one that `sums` and (with kKeep) the kept list are about.
+template <int TP, bool kLam, bool kKeep, class Sums>
 __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr, bool want, int ci,
                                            const float4 xi, const float4* __restrict__ xin, float inv_h,
                                            const GridDesc& Gd, const WalkIndex& I, const Grid& G,
-                                           Sums& sums) {
+                                           uint32_t p, uint32_t& kept, Sums& sums) {
     constexpr int NT = TP / 8;
     constexpr int LPP = 32 / TP;  // listing lanes per particle
     constexpr int WPL = 4 / LPP;  // words of a batch that a lane settles
@@ -1535,22 +1584,34 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
         const unsigned short* const my = sm.list + pe * TeamSmem<TP>::kListRow;
         float2* const rows = reinterpret_cast<float2*>(sm.warp[wid]);
         float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
+        uint2* to = nullptr;
+        if constexpr (kKeep) {
+            const uint32_t rows = ((uint32_t)cnt + 1u) / 2u;
+            if (kept + rows <= kListRows) {
+                to = G.lists + (size_t)p * kListRows + kept;
+                kept += rows;
+            } else {
+                kept = kNoList;
+            }
+        }
+        // Candidates t and t + 1 of the list (t < cnt).
         auto load = [&](int t) {
             const uint32_t two = *reinterpret_cast<const uint32_t*>(my + t);
-            if (t < cnt) {
-                uint32_t q = sm.base[(two >> 5) & (kTeamWords - 1)] + (two & 31u);
-                if (key) q = I.at(q);
-                xa = __ldg(xin + q);
-                if constexpr (Sums::kExtra) ea = sums.extra(q);
-            }
+            uint32_t qa = sm.base[(two >> 5) & (kTeamWords - 1)] + (two & 31u), qb = p;
+            if (key) qa = I.at(qa);
+            xa = __ldg(xin + qa);
+            if constexpr (Sums::kExtra) ea = sums.extra(qa);
             if (t + 1 < cnt) {
-                uint32_t q = sm.base[(two >> 21) & (kTeamWords - 1)] + ((two >> 16) & 31u);
-                if (key) q = I.at(q);
-                xb = __ldg(xin + q);
-                if constexpr (Sums::kExtra) eb = sums.extra(q);
+                qb = sm.base[(two >> 21) & (kTeamWords - 1)] + ((two >> 16) & 31u);
+                if (key) qb = I.at(qb);
+                xb = __ldg(xin + qb);
+                if constexpr (Sums::kExtra) eb = sums.extra(qb);
+            }
+            if constexpr (kKeep) {
+                if (to) to[t >> 1] = make_uint2(qa, qb);
             }
         };
-        load(2 * s < cnt ? 2 * s : 0);
+        if (2 * s < cnt) load(2 * s);
         for (int t0 = 0; t0 < most; t0 += 2 * S) {
             const int t = t0 + 2 * s;
             const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
@@ -1714,10 +1775,10 @@ __device__ __forceinline__ WalkGroup next_group(uint32_t todo, const Grid& G, co
 // `cell` (w = its bucket row + 1, 0 when clean) and x* xi.  Returns false,
 // with nothing summed, when the warp's particles sit in too many cells (the
 // caller walks lane by lane then).
-template <bool kPersist, bool kLam, bool kRuns, class P, class Sums>
+template <bool kPersist, bool kLam, bool kRuns, bool kKeep, class P, class Sums>
 __device__ __forceinline__ bool warp_walk(WalkSmem& sm, const Grid& G, const WalkIndex& I, const P& prm,
                                           uint32_t p, const int4 cell, bool want, const float4 xi,
-                                          const float4* xin, Sums& sums) {
+                                          const float4* xin, uint32_t& kept, Sums& sums) {
     const unsigned full = 0xffffffffu;
     uint32_t todo = __ballot_sync(full, want);
     if (!todo) return true;
@@ -1736,17 +1797,19 @@ __device__ __forceinline__ bool warp_walk(WalkSmem& sm, const Grid& G, const Wal
         GridDesc Gd;
         const WalkGroup Gr = next_group(todo, G, prm, p, sid, cell, mem, inv_h, Gd);
         todo &= ~__ballot_sync(full, mem);
-        walk_group<kPersist, kLam, kRuns>(sm, Gr, mem, cell.x, xi, xin, inv_h, Gd, I, G, sums);
+        walk_group<kPersist, kLam, kRuns, kKeep>(sm, Gr, mem, cell.x, xi, xin, inv_h, Gd, I, G, p, kept, sums);
     }
     return true;
 }
 
 // The team walk (every thread of the team calls it; p, cell, want and xi as
 // in warp_walk, of the listing's particle, the same in all four warps).
-template <int TP, bool kLam, class P, class Sums>
-__device__ __forceinline__ void team_walk(TeamSmem<TP>& sm, const Grid& G, const WalkIndex& I, const P& prm,
-                                          uint32_t p, const int4 cell, bool want, const float4 xi,
-                                          const float4* __restrict__ xin, Sums& sums) {
+// team_walk_keep keeps the lists of the evaluation's particles pe, see team_group.
+template <int TP, bool kLam, bool kKeep, class P, class Sums>
+__device__ __forceinline__ void team_walk_keep(TeamSmem<TP>& sm, const Grid& G, const WalkIndex& I,
+                                               const P& prm, uint32_t p, const int4 cell, bool want,
+                                               const float4 xi, const float4* __restrict__ xin, uint32_t pe,
+                                               uint32_t& kept, Sums& sums) {
     const unsigned full = 0xffffffffu;
     uint32_t todo = __ballot_sync(full, want);
     const uint32_t sid = scene_at(G, p);
@@ -1756,8 +1819,16 @@ __device__ __forceinline__ void team_walk(TeamSmem<TP>& sm, const Grid& G, const
         GridDesc Gd;
         const WalkGroup Gr = next_group(todo, G, prm, p, sid, cell, mem, inv_h, Gd);
         todo &= ~__ballot_sync(full, mem);
-        team_group<TP, kLam>(sm, Gr, mem, cell.x, xi, xin, inv_h, Gd, I, G, sums);
+        team_group<TP, kLam, kKeep>(sm, Gr, mem, cell.x, xi, xin, inv_h, Gd, I, G, pe, kept, sums);
     }
+}
+
+template <int TP, bool kLam, class P, class Sums>
+__device__ __forceinline__ void team_walk(TeamSmem<TP>& sm, const Grid& G, const WalkIndex& I, const P& prm,
+                                          uint32_t p, const int4 cell, bool want, const float4 xi,
+                                          const float4* __restrict__ xin, Sums& sums) {
+    uint32_t kept = 0u;
+    team_walk_keep<TP, kLam, false>(sm, G, I, prm, p, cell, want, xi, xin, 0u, kept, sums);
 }
 
 __device__ __forceinline__ WalkIndex fluid_index(const Grid& G) {
@@ -2207,13 +2278,15 @@ struct VorticityTerm {
 
 // The sums over the fluid's candidates of every lane that wants: the warp
 // walk, or lane by lane where the warp's particles are scattered.
-template <bool kPersist, bool kLam, class P, class Sums>
-__device__ __forceinline__ void sum_candidates(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
-                                               const int4 cell, bool want, const float4 xi,
-                                               const float4* xin, const StepConsts& C, Sums& sums) {
+template <bool kPersist, bool kLam, bool kKeep, class P, class Sums>
+__device__ __forceinline__ void sum_walking(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
+                                            const int4 cell, bool want, const float4 xi, const float4* xin,
+                                            const StepConsts& C, uint32_t& kept, Sums& sums) {
     constexpr bool kRuns = std::is_same<P, OneScene>::value;
-    if (warp_walk<kPersist, kLam, kRuns>(sm, G, fluid_index(G), prm, p, cell, want, xi, xin, sums)) return;
+    if (warp_walk<kPersist, kLam, kRuns, kKeep>(sm, G, fluid_index(G), prm, p, cell, want, xi, xin, kept, sums))
+        return;
     if (!want) return;
+    kept = kNoList;
     for_each_candidate_runs<kRuns>(
         cell, G, C,
         [&](uint32_t q) {
@@ -2228,6 +2301,77 @@ __device__ __forceinline__ void sum_candidates(WalkSmem& sm, const Grid& G, cons
         });
 }
 
+template <bool kPersist, bool kLam, class P, class Sums>
+__device__ __forceinline__ void sum_candidates(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
+                                               const int4 cell, bool want, const float4 xi,
+                                               const float4* xin, const StepConsts& C, Sums& sums) {
+    uint32_t kept = 0u;
+    sum_walking<kPersist, kLam, false>(sm, G, prm, p, cell, want, xi, xin, C, kept, sums);
+}
+
+// The same, keeping the lists (where there is room for any).
+template <bool kPersist, class P, class Sums>
+__device__ __forceinline__ void sum_keeping(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
+                                            const int4 cell, bool want, const float4 xi, const float4* xin,
+                                            const StepConsts& C, Sums& sums) {
+    if constexpr (!kPersist) {
+        if (G.lists) {
+            uint32_t kept = 0u;
+            sum_walking<false, false, true>(sm, G, prm, p, cell, want, xi, xin, C, kept, sums);
+            if (want) G.listed[p] = kept;
+            return;
+        }
+    }
+    sum_candidates<kPersist, false>(sm, G, prm, p, cell, want, xi, xin, C, sums);
+}
+
+// The same from the kept lists, where every lane that wants has one.  kLam: in
+// a warp whose lambdas are all zero, pairs of candidates whose lambdas are
+// zero too are passed over (see walk_group).
+template <bool kPersist, bool kLam, class P, class Sums>
+__device__ __forceinline__ void sum_listed(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
+                                           const int4 cell, bool want, const float4 xi, const float4* xin,
+                                           const StepConsts& C, Sums& sums) {
+    if constexpr (!kPersist) {
+        if (G.lists) {
+            const unsigned full = 0xffffffffu;
+            const uint32_t rows = want ? G.listed[p] : 0u;
+            const uint32_t most = __reduce_max_sync(full, rows);
+            if (most != kNoList) {
+                const bool all_zero = kLam && !__any_sync(full, want && xi.w != 0.0f);
+                const uint2* from = G.lists + list_at(p);
+                float4 xa = xi, xb = xi, ea = make_float4(0.0f, 0.0f, 0.0f, 0.0f), eb = ea;
+                uint2 q = make_uint2(p, p);
+                auto load = [&]() {
+                    xa = __ldg(xin + q.x);
+                    xb = __ldg(xin + q.y);
+                    if constexpr (Sums::kExtra) {
+                        ea = sums.extra(q.x);
+                        eb = sums.extra(q.y);
+                    }
+                };
+                if (rows > 0u) {
+                    q = __ldcs(from);
+                    load();
+                }
+                if (rows > 1u) q = __ldcs(from + 32);
+                from += 64;
+                for (uint32_t r = 0; r < most; ++r) {
+                    const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
+                    if (r + 1u < rows) load();
+                    if (r + 2u < rows) q = __ldcs(from);
+                    from += 32;
+                    const bool has = r < rows;
+                    if (all_zero && !__any_sync(full, has && (x0.w != 0.0f || x1.w != 0.0f))) continue;
+                    sums.add2(x0, x1, e0, e1, has, has);
+                }
+                return;
+            }
+        }
+    }
+    sum_candidates<kPersist, kLam>(sm, G, prm, p, cell, want, xi, xin, C, sums);
+}
+
 // The same over the boundary of a two-way coupled step; `cell` is the
 // particle's cell in the fluid's grid.
 template <class P, class Sums>
@@ -2235,7 +2379,9 @@ __device__ __forceinline__ void sum_boundary(WalkSmem& sm, const Grid& G, const 
                                              const int4 cell, bool want, const float4 xi,
                                              const StepConsts& C, Sums& sums) {
     const int4 bc = boundary_cell(G, p, cell);
-    if (warp_walk<false, false, false>(sm, G, boundary_index(G), prm, p, bc, want, xi, G.bg.spos, sums))
+    uint32_t kept = 0u;
+    if (warp_walk<false, false, false, false>(sm, G, boundary_index(G), prm, p, bc, want, xi, G.bg.spos, kept,
+                                              sums))
         return;
     if (!want) return;
     for_each_candidate(bc, boundary_index(G), C,
@@ -2266,6 +2412,68 @@ struct TeamThread {
         return sm.flag[threadIdx.x / (128u / TP)] != 0;
     }
 };
+
+// The team's sums, keeping the lists (where there is room for any) of the
+// evaluation's particles that want (elive).
+template <int TP, class P, class Sums>
+__device__ __forceinline__ void team_keeping(TeamSmem<TP>& sm, const Grid& G, const P& prm,
+                                             const TeamThread<TP>& T, bool want, bool ewant, const float4 xl,
+                                             const float4* __restrict__ xin, Sums& sums) {
+    const int4 cell = cell_at(G, T.pl);
+    if (G.lists) {
+        uint32_t kept = 0u;
+        team_walk_keep<TP, false, true>(sm, G, fluid_index(G), prm, T.pl, cell, want, xl, xin, T.pe, kept, sums);
+        if (ewant && T.writer) G.listed[T.pe] = kept;
+    } else {
+        team_walk<TP, false>(sm, G, fluid_index(G), prm, T.pl, cell, want, xl, xin, sums);
+    }
+}
+
+// The team's sums from the kept lists, where every particle that wants has
+// one; the warps then need nothing from each other.
+template <int TP, bool kLam, class P, class Sums>
+__device__ __forceinline__ void team_listed(TeamSmem<TP>& sm, const Grid& G, const P& prm,
+                                            const TeamThread<TP>& T, bool want, bool ewant, const float4 xl,
+                                            const float4* __restrict__ xin, Sums& sums) {
+    constexpr int S = 128 / TP;
+    const unsigned full = 0xffffffffu;
+    if (G.lists) {
+        const int rows = ewant ? (int)G.listed[T.pe] : 0;
+        if (!__syncthreads_or(rows == (int)kNoList)) {
+            const int s = threadIdx.x & (S - 1);
+            const int most = (int)__reduce_max_sync(full, (unsigned)rows);
+            const uint2* const from = G.lists + (size_t)T.pe * kListRows;
+            float2* const buf = reinterpret_cast<float2*>(sm.warp[threadIdx.x >> 5]);
+            float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
+            uint2 q = make_uint2(0u, 0u);
+            auto load = [&]() {
+                xa = __ldg(xin + q.x);
+                xb = __ldg(xin + q.y);
+                if constexpr (Sums::kExtra) {
+                    ea = sums.extra(q.x);
+                    eb = sums.extra(q.y);
+                }
+            };
+            if (s < rows) {
+                q = __ldcs(from + s);
+                load();
+            }
+            if (s + S < rows) q = __ldcs(from + s + S);
+            for (int r0 = 0; r0 < most; r0 += S) {
+                const int r = r0 + s;
+                const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
+                if (r + S < rows) load();
+                if (r + 2 * S < rows) q = __ldcs(from + r + 2 * S);
+                sums.put(buf, x0, x1, e0, e1, r < rows, r < rows);
+                __syncwarp();
+                sums.fold(buf);
+                __syncwarp();
+            }
+            return;
+        }
+    }
+    team_walk<TP, kLam>(sm, G, fluid_index(G), prm, T.pl, cell_at(G, T.pl), want, xl, xin, sums);
+}
 
 // What the density pass writes for particle p and the rest of its run.
 __device__ __forceinline__ void keep_lambda(uint32_t p, uint32_t rf, const int4 cell, const float4* xin,
@@ -2331,18 +2539,18 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
     }
     if (kHist && dfirst) {
         LaneSums<DensityTerm> ds(DensityTerm{C, xi});
-        sum_candidates<kPersist, false>(sm, G, prm, pa, cell, live, xi, xin, C, ds);
+        sum_keeping<kPersist>(sm, G, prm, pa, cell, live, xi, xin, C, ds);
         density = ds.get(0);
         const bool want = live && !(density * C.inv_rho0 - 1.0f < 0.0f);
         LaneSums<GradTerm> gs(GradTerm{C, xi});
-        sum_candidates<kPersist, false>(sm, G, prm, pa, cell, want, xi, xin, C, gs);
+        sum_listed<kPersist, false>(sm, G, prm, pa, cell, want, xi, xin, C, gs);
         gix = gs.get(0);
         giy = gs.get(1);
         giz = gs.get(2);
         sum_grad_sq = gs.get(3);
     } else {
         LaneSums<DensityGradTerm> sums(DensityGradTerm{C, xi});
-        sum_candidates<kPersist, false>(sm, G, prm, pa, cell, live, xi, xin, C, sums);
+        sum_keeping<kPersist>(sm, G, prm, pa, cell, live, xi, xin, C, sums);
         density = sums.get(0);
         gix = sums.get(1);
         giy = sums.get(2);
@@ -2411,7 +2619,7 @@ k_density_lambda_team(const float4* __restrict__ xin, float4* __restrict__ xout,
     const StepConsts& C = prm.at(G.spid, T.pe);
     const float4 xl = xin[T.pl], xi = xin[T.pe];
     TeamSums<DensityGradTerm, 128 / TP> sums(DensityGradTerm{C, xi});
-    team_walk<TP, false>(sm, G, fluid_index(G), prm, T.pl, cell, live, xl, xin, sums);
+    team_keeping<TP>(sm, G, prm, T, live, elive, xl, xin, sums);
     float density = sums.get(0), gix = sums.get(1), giy = sums.get(2), giz = sums.get(3);
     const float sum_grad_sq = sums.get(4);
     if constexpr (std::is_same<P, OneScene>::value) {
@@ -2495,7 +2703,7 @@ __device__ __forceinline__ void delta_at(uint32_t p, bool active, const float4* 
         !neighbourhood_stamped<kPersist>(cell, C.grid, G.lamnz, (uint32_t)it + 1u, 0, 3))
         walk = false;
     LaneSums<DeltaTerm> sums(DeltaTerm{C, xi});
-    sum_candidates<kPersist, true>(sm, G, prm, pa, cell, walk, xi, xin, C, sums);
+    sum_listed<kPersist, true>(sm, G, prm, pa, cell, walk, xi, xin, C, sums);
     float dx = sums.get(0), dy = sums.get(1), dz = sums.get(2);
     if constexpr (std::is_same<P, OneScene>::value) {
         if (G.bg.spos) {
@@ -2531,8 +2739,8 @@ k_delta_team(const float4* __restrict__ xin, float4* __restrict__ xout, const fl
     __shared__ TeamSmem<TP> sm;
     const TeamThread<TP> T(n);
     const int4 cell = cell_at(G, T.pl);
-    const float4 xl = xin[T.pl];
-    bool live, walk;
+    const float4 xl = xin[T.pl], xi = xin[T.pe];
+    bool live, walk, ewalk;
     {
         const StepConsts& C = prm.at(G.spid, T.pl);
         live = walk = T.al && it < C.iters;
@@ -2543,10 +2751,12 @@ k_delta_team(const float4* __restrict__ xin, float4* __restrict__ xout, const fl
         }
     }
     const StepConsts& C = prm.at(G.spid, T.pe);
-    const float4 xi = xin[T.pe];
+    // The evaluation's particle: team_stamped left the answers in the flags.
+    ewalk = T.ae && it < C.iters &&
+            !(G.lamnz && cell_at(G, T.pe).w == 0 && xi.w == 0.0f && !sm.flag[threadIdx.x / (128u / TP)]);
     TeamSums<DeltaTerm, 128 / TP> sums(DeltaTerm{C, xi});
     __syncthreads();
-    team_walk<TP, true>(sm, G, fluid_index(G), prm, T.pl, cell, walk, xl, xin, sums);
+    team_listed<TP, true>(sm, G, prm, T, walk, ewalk, xl, xin, sums);
     float dx = sums.get(0), dy = sums.get(1), dz = sums.get(2);
     if constexpr (std::is_same<P, OneScene>::value) {
         if (G.bg.spos) {
@@ -2806,7 +3016,7 @@ k_xsph_omega(const float4* __restrict__ xin, const float4* __restrict__ sv, floa
     const float4 xi = xin[pa];
     const float4 vi = sv[pa];
     LaneSums<XsphOmegaTerm> sums(XsphOmegaTerm{C, xi, vi, sv});
-    sum_candidates<false, false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live, xi, xin, C, sums);
+    sum_keeping<false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live, xi, xin, C, sums);
     if (live)
         store_omega(p, rf, vi, sums.get(0), sums.get(1), sums.get(2), sums.get(3), sums.get(4), sums.get(5),
                     sv2, som, G, C);
@@ -2823,7 +3033,7 @@ k_xsph_omega_team(const float4* __restrict__ xin, const float4* __restrict__ sv,
     const float4 xi = xin[T.pe];
     const float4 vi = sv[T.pe];
     TeamSums<XsphOmegaTerm, 128 / TP> sums(XsphOmegaTerm{C, xi, vi, sv});
-    team_walk<TP, false>(sm, G, fluid_index(G), prm, T.pl, cell_at(G, T.pl), want, xin[T.pl], xin, sums);
+    team_keeping<TP>(sm, G, prm, T, want, T.ae && C.vort_on, xin[T.pl], xin, sums);
     const float cx = sums.get(0), cy = sums.get(1), cz = sums.get(2);
     const float wx = sums.get(3), wy = sums.get(4), wz = sums.get(5);
     if (T.writer && C.vort_on) store_omega(T.pe, 0u, vi, cx, cy, cz, wx, wy, wz, sv2, som, G, C);
@@ -2872,7 +3082,7 @@ k_vorticity_commit(const float4* __restrict__ xin, const float4* __restrict__ sv
     const bool live = active && C.vort_on && !(rf & kCopyBit);
     const float4 xi = xin[pa];
     LaneSums<VorticityTerm> sums(VorticityTerm{C, xi, som[pa].w, sv, som});
-    sum_candidates<false, false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live, xi, xin, C, sums);
+    sum_listed<false, false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live, xi, xin, C, sums);
     if (live)
         store_vorticity(p, rf, xi, sums.get(0), sums.get(1), sums.get(2), sv2, som, sx, srho, n, G, prm, C);
 }
@@ -2889,7 +3099,7 @@ k_vorticity_commit_team(const float4* __restrict__ xin, const float4* __restrict
     const StepConsts& C = prm.at(G.spid, T.pe);
     const float4 xi = xin[T.pe];
     TeamSums<VorticityTerm, 128 / TP> sums(VorticityTerm{C, xi, som[T.pe].w, sv, som});
-    team_walk<TP, false>(sm, G, fluid_index(G), prm, T.pl, cell_at(G, T.pl), want, xin[T.pl], xin, sums);
+    team_listed<TP, false>(sm, G, prm, T, want, T.ae && C.vort_on, xin[T.pl], xin, sums);
     const float ex = sums.get(0), ey = sums.get(1), ez = sums.get(2);
     if (T.writer && C.vort_on)
         store_vorticity(T.pe, 0u, xi, ex, ey, ez, sv2, som, sx, srho, n, G, prm, C);
@@ -2943,7 +3153,8 @@ inline int grid_of(int n, int b) { return (n + b - 1) / b; }
 inline Grid grid_view(const StepBuffers& B, int n, const uint32_t* spid = nullptr,
                       const BoundaryGrid& bg = BoundaryGrid{}) {
     return Grid{B.scell, B.sown, WalkIndex{(uint32_t)n, B.off, B.bkt.merged, B.bkt.end, B.btab}, spid,
-                B.moved, B.lamnz, bg, spid ? nullptr : B.dhist, nullptr, B.slot_alias};
+                B.moved, B.lamnz, bg, spid ? nullptr : B.dhist, nullptr, B.slot_alias,
+                n <= B.list_cap ? B.lists : nullptr, B.listed};
 }
 
 // predict, sort by cell and by reference key, cell offsets, gather, reference

@@ -155,10 +155,20 @@ struct StepBuffers {
     // bit-identical step state in cell order, one past the run's last; 0
     // elsewhere (see k_segments).  Single scenes only (null in batches).
     uint32_t* segend;
+    // Candidate lists kept from one pass of a step for the next, kListRows
+    // rows of two for each of list_cap particles, and the rows of each
+    // (kNoList: no list).  Null where there was no room: the passes walk then.
+    uint2* lists = nullptr;
+    uint32_t* listed = nullptr;
+    int list_cap = 0;
     uint32_t* err;  // device status word
 };
 
 constexpr int kWalkHist = 16;
+// Room for 512 candidates: fluid at rest has 270 in support at h = 4 r, a
+// compressed one up to about 450.
+constexpr uint32_t kListRows = 256;
+constexpr uint32_t kNoList = 0x7fffffffu;
 
 // Phases of one step, named after the reference's PerformanceMonitor scopes
 // (pbf_solver.cpp:29-103).  Fused kernels report under the first scope they
