@@ -104,7 +104,7 @@ constexpr size_t kListMaxBytes = (size_t)16 << 30;
 
 inline size_t list_bytes(int c) {
     const size_t r = align_up((size_t)c, 32);
-    return r * kListRows * sizeof(uint2) + r * 4;
+    return r * kListRows * sizeof(uint2) + r * 4 + 256;
 }
 
 inline void bind_lists(StepBuffers& B, void* mem, int c) {
@@ -113,6 +113,7 @@ inline void bind_lists(StepBuffers& B, void* mem, int c) {
     B.listed = reinterpret_cast<uint32_t*>(static_cast<char*>(mem) + r * kListRows * sizeof(uint2));
     B.list_cap = mem ? c : 0;
     if (!mem) B.listed = nullptr;
+    B.unlisted = mem ? B.listed + r : nullptr;
 }
 
 // Whether lists of that many bytes may be allocated now (then counted until

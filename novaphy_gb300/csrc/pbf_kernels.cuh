@@ -257,11 +257,12 @@ __device__ __forceinline__ void predict(const float4 xi, const float4 vi, const 
 
 // Predict + cell slot per particle (particle order), with the digits of the
 // slots counted for the sort.  Also turns this step's density-pass counts of
-// the last step (dhist, where there are any) into the previous step's.
+// the last step (dhist, where there are any) into the previous step's, and
+// clears the flag of missing lists.
 template <class P>
 __global__ void __launch_bounds__(kCountThreads)
-k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, int n, const SortCounts counts,
-              const SceneIds S, const P prm) {
+k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, uint32_t* __restrict__ unlisted,
+              int n, const SortCounts counts, const SceneIds S, const P prm) {
     __shared__ BlockCounts B;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
     static_assert(2 * kWalkHist <= kCountThreads, "one thread per count");
@@ -269,6 +270,7 @@ k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, int n, 
         dhist[t] = dhist[t + 2 * kWalkHist];
         dhist[t + 2 * kWalkHist] = 0u;
     }
+    if (unlisted && t == 0) *unlisted = 0u;
     B.begin(counts);
     for (int i = t; i < n; i += gridDim.x * blockDim.x) {
         const StepConsts& C = prm.at(S.pid, i);
@@ -674,6 +676,7 @@ struct Grid {
     const unsigned char* slot_alias;     // with kRunSlot where segend is set
     uint2* lists;                        // see StepBuffers::lists (null: none are kept)
     uint32_t* listed;
+    uint32_t* unlisted;
 };
 
 // for_each_candidate over a single scene's step with runs of identical
@@ -825,7 +828,9 @@ __device__ __forceinline__ T ld_step(const T* p) {
 //    leave most of the chip idle, or its warps waiting on one chain each,
 //    with one lane per particle (team_size).
 
-// Words listed before an evaluation, in a warp walk and in a team walk.
+// Words listed before an evaluation, in a warp walk and in a team walk.  With 16
+// the lanes of a warp wait for the longest list twice as often (250,000
+// particles 3,346 us a step against 2,995).
 constexpr int kWalkWords = 32;
 constexpr int kTeamWords = 64;
 // Terms a team lists per particle before an evaluation: room for a round of
@@ -836,6 +841,9 @@ constexpr int kTeamWarps = 4;
 // group's listing costs a warp about as much as a few dozen candidates of a
 // one-thread walk).
 constexpr int kMaxGroups = 6;
+// Warps with more than this many have no lists (as many as 32 measured the
+// same: 14,808 us against 14,790 for three steps of 395,101).
+constexpr int kMaxListGroups = 16;
 
 // A group's candidate sequence: ranges [start, start + len) in cell order (key
 // order for a dirty cell), their rows' first slots, and the number of words of
@@ -846,25 +854,34 @@ struct RangeList {
 };
 constexpr uint32_t kRunRange = 0x80000000u;
 
-// Kept lists.  The density pass keeps each particle's listed candidates, and
-// the delta pass, whose candidates sit where they sat for the density, reads
-// them instead of walking; the XSPH-omega pass keeps them for the vorticity
-// pass.  A row is two candidates (cell-order positions); an odd candidate's
-// partner is the particle itself, whose terms are exact zeros.  A warp walk's
-// particles have their rows side by side (row r of particle p at
-// (p / 32 kListRows + r) 32 + p % 32), a team's particles one after another
-// (p kListRows + r).  StepBuffers::listed holds the number of rows, or kNoList
-// where the walk did not list (lane-by-lane walks, runs) or had no room.
+// Kept lists.  The candidates that a listing finds for a particle, in the
+// reference's order, two to a row (cell-order positions).  The delta pass reads
+// the lists of the density pass, whose candidates sit where they sat; the
+// vorticity pass those of the XSPH-omega pass.
 //
-// What it saves: a walk's listing and scanning are half of its instructions
-// (density of 300,000 particles: 180 of 318 million); a reader has one
-// coalesced 8-byte load per row instead, and a team's warps no longer wait for
-// each other.  The rows of a million particles are 1 GB written and read per
-// iteration, a third of the memory bandwidth while both passes are bound by
-// their instructions.  Measured (us a call, walking / with lists): 1,000
-// particles 105 / 96; 8,000 235 / 204; 4 steps of 43,993 3,989 / 3,332;
-// 65,565 (fast build) 1,862 / 1,603; 3 steps of 395,101 21,180 / 18,450; a
-// million 6,263 / 5,528; a batch of 352,901 3,121 / 2,928.
+// Warps of 32 particles list in a kernel of its own (k_list) and read in every
+// pass (read_lists).  Their rows lie side by side (row r of particle p at
+// (p / 32 kListRows + r) 32 + p % 32), and StepBuffers::listed holds the number
+// of candidates, or kNoList where there were too many, where identical
+// particles count more than once (k_segments) or where the warp had too many
+// groups: those walk.  Teams list and sum in the density and XSPH-omega pass
+// and read in the others; their rows lie one particle after another (p
+// kListRows + r) and are counted, and an odd candidate's partner is the
+// particle itself, whose terms are exact zeros in the passes that read.
+//
+// What it saves: listing and scanning are half of a walk's instructions
+// (density of 300,000 particles: 180 of 318 million), and a warp walks its
+// groups one after another with the lanes of the others idle (1.5 to 2 groups
+// in moving fluid); a reader has one coalesced 8-byte load per row, all lanes
+// busy, no shared memory and 64 registers, so 32 warps an SM instead of 20.
+// The rows of a million particles are 1 GB written and read per iteration, a
+// third of the memory bandwidth while the passes are bound by their
+// instructions.  Measured (us a call; walking / lists kept by a walking
+// density pass / k_list and readers): 1,000 particles 105 / 96 / -; 8,000 235 /
+// 204 / -; 4 steps of 43,993 3,989 / 3,332 / -; 65,565 (fast build) 1,862 /
+// 1,603 / -; 3 steps of 395,101 21,180 / 18,450 / 14,790; a million 6,263 /
+// 5,528 / 4,230; 250,000 with bodies 3,642 / 3,133 / 2,995; a batch of 352,901
+// 3,121 / 2,928 / 2,310.
 __device__ __forceinline__ uint32_t list_at(uint32_t p) { return (p >> 5) * (32u * kListRows) + (p & 31u); }
 
 // Shared memory of a warp walk.
@@ -907,6 +924,12 @@ struct TeamSmem {
 // (80 registers a thread).
 template <int BS>
 constexpr int kPassMinBlocks = 768 / BS;
+// Threads per SM of the kernels that only list (640: 1M step 4,385 us against
+// 4,230) and of those that read lists: 64 registers, or 72 with a batch's
+// tables (16 scenes 2,310 us against 2,360 with 64).
+constexpr int kListThreads = 768;
+template <class P>
+constexpr int kReadThreads = std::is_same<P, OneScene>::value ? 1024 : 896;
 // The teams' kernels: of 8 particles seven blocks (72 registers), so that up to
 // 8,500 particles run in one wave (8,000: 239 us a step against 258 with six).
 template <int TP>
@@ -1152,10 +1175,10 @@ __device__ __forceinline__ uint32_t own_cells(const WalkIndex& I, uint32_t slot,
 // started at +0, never are -0, so a lane whose lambda is zero lists
 // candidates with a nonzero one only.  kRuns: in ranges that hold runs of
 // identical particles (k_segments) a run is listed as its first particle,
-// whose term is added as many times as the run is long.  kKeep: the lane's
-// candidates go to its kept list, from list + list_at(its particle); kept is
-// their number of rows.
-template <bool kPersist, bool kLam, bool kRuns, bool kKeep, class Sums>
+// whose term is added as many times as the run is long.  kList: nothing is
+// summed; the lane's candidates go to the kept list of its particle p, whose
+// rows so far are `kept`.
+template <bool kPersist, bool kLam, bool kRuns, bool kList, class Sums>
 __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bool want, int ci,
                                            const float4 xi, const float4* xin, float inv_h,
                                            const GridDesc& Gd, const WalkIndex& I, const Grid& G,
@@ -1179,6 +1202,10 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
     bool runs;
     const int total = walk_ranges<kRuns>(sm.ranges, Gr, I, Gd, G, true, runs);
     __syncwarp();
+    if (kList && runs) {  // a row has no way to say how often its term counts
+        if (want) kept = kNoList;
+        return;
+    }
     // Position of the listing with runs: range and candidate.
     int at_r = 0;
     uint32_t at_q = 0u;
@@ -1305,8 +1332,29 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             bits &= bits - 1u;
             return bq + k;
         };
-        if (kRuns && runs) {
-            if (kKeep && want) kept = kNoList;
+        if constexpr (kList) {
+            auto take = [&]() {
+                const uint32_t q = next_q();
+                return key ? I.at(q) : q;
+            };
+            if (kept + (uint32_t)cnt <= 2u * kListRows) {
+                uint2* to = G.lists + list_at(p) + 32u * (kept >> 1);
+                int t = 0;
+                if ((kept & 1u) && cnt > 0) {
+                    to->y = take();
+                    to += 32;
+                    t = 1;
+                }
+                for (; t < cnt; t += 2) {
+                    const uint32_t qa = take(), qb = t + 1 < cnt ? take() : p;
+                    __stcs(to, make_uint2(qa, qb));
+                    to += 32;
+                }
+                kept += (uint32_t)cnt;
+            } else {
+                kept = kNoList;
+            }
+        } else if (kRuns && runs) {
             for (int t = 0; t < cnt; ++t) {
                 uint32_t q = next_q();
                 const uint32_t i = sm.info[w];
@@ -1319,40 +1367,18 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             }
         } else {
             float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
-            auto load = [&](float4& x, float4& e) -> uint32_t {
+            auto load = [&](float4& x, float4& e) {
                 uint32_t q = next_q();
                 if (key) q = I.at(q);
                 x = ld_step<kPersist>(xin + q);
                 if constexpr (Sums::kExtra) e = sums.extra(q);
-                return q;
             };
-            // Room for this batch of the lane's list?
-            uint2* to = nullptr;
-            if constexpr (kKeep) {
-                const uint32_t rows = ((uint32_t)cnt + 1u) / 2u;
-                if (kept + rows <= kListRows) {
-                    to = G.lists + list_at(p) + 32u * kept;
-                    kept += rows;
-                } else {
-                    kept = kNoList;
-                }
-            }
-            // The lane's listed candidates t and t + 1 (t < cnt).
-            auto next = [&](int t) {
-                const uint32_t qa = load(xa, ea);
-                uint32_t qb = p;
-                if (t + 1 < cnt) qb = load(xb, eb);
-                if constexpr (kKeep) {
-                    if (to) {
-                        __stcs(to, make_uint2(qa, qb));
-                        to += 32;
-                    }
-                }
-            };
-            if (cnt > 0) next(0);
+            if (cnt > 0) load(xa, ea);
+            if (cnt > 1) load(xb, eb);
             for (int t = 0; t < most; t += 2) {
                 const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
-                if (t + 2 < cnt) next(t + 2);
+                if (t + 2 < cnt) load(xa, ea);
+                if (t + 3 < cnt) load(xb, eb);
                 sums.add2(x0, x1, e0, e1, t < cnt, t + 1 < cnt);
             }
         }
@@ -1369,6 +1395,11 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
 // values and factors of one candidate and whether it is in support; and in the
 // exact build products, the products of two candidates at once.
 //
+// No sums (a walk that only lists).
+struct NoSums {
+    static constexpr bool kExtra = false;
+};
+
 // The sums of one lane (warp walk).
 template <class D>
 struct LaneSums {
@@ -1775,7 +1806,7 @@ __device__ __forceinline__ WalkGroup next_group(uint32_t todo, const Grid& G, co
 // `cell` (w = its bucket row + 1, 0 when clean) and x* xi.  Returns false,
 // with nothing summed, when the warp's particles sit in too many cells (the
 // caller walks lane by lane then).
-template <bool kPersist, bool kLam, bool kRuns, bool kKeep, class P, class Sums>
+template <bool kPersist, bool kLam, bool kRuns, bool kList, class P, class Sums>
 __device__ __forceinline__ bool warp_walk(WalkSmem& sm, const Grid& G, const WalkIndex& I, const P& prm,
                                           uint32_t p, const int4 cell, bool want, const float4 xi,
                                           const float4* xin, uint32_t& kept, Sums& sums) {
@@ -1789,7 +1820,7 @@ __device__ __forceinline__ bool warp_walk(WalkSmem& sm, const Grid& G, const Wal
                             (sid * 2654435761u)) + x * 83492791u;
         const uint32_t same = __match_any_sync(full, want ? k : 0u) & todo;
         const bool first = want && (int)(threadIdx.x & 31) == __ffs(same) - 1;
-        if (__popc(__ballot_sync(full, first)) > kMaxGroups) return false;
+        if (__popc(__ballot_sync(full, first)) > (kList ? kMaxListGroups : kMaxGroups)) return false;
     }
     while (todo) {
         bool mem;
@@ -1797,7 +1828,8 @@ __device__ __forceinline__ bool warp_walk(WalkSmem& sm, const Grid& G, const Wal
         GridDesc Gd;
         const WalkGroup Gr = next_group(todo, G, prm, p, sid, cell, mem, inv_h, Gd);
         todo &= ~__ballot_sync(full, mem);
-        walk_group<kPersist, kLam, kRuns, kKeep>(sm, Gr, mem, cell.x, xi, xin, inv_h, Gd, I, G, p, kept, sums);
+        walk_group<kPersist, kLam, kRuns, kList>(sm, Gr, mem, cell.x, xi, xin, inv_h, Gd, I, G, p, kept,
+                                                 sums);
     }
     return true;
 }
@@ -2278,15 +2310,16 @@ struct VorticityTerm {
 
 // The sums over the fluid's candidates of every lane that wants: the warp
 // walk, or lane by lane where the warp's particles are scattered.
-template <bool kPersist, bool kLam, bool kKeep, class P, class Sums>
-__device__ __forceinline__ void sum_walking(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
-                                            const int4 cell, bool want, const float4 xi, const float4* xin,
-                                            const StepConsts& C, uint32_t& kept, Sums& sums) {
+template <bool kPersist, bool kLam, class P, class Sums>
+__device__ __forceinline__ void sum_candidates(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
+                                               const int4 cell, bool want, const float4 xi,
+                                               const float4* xin, const StepConsts& C, Sums& sums) {
     constexpr bool kRuns = std::is_same<P, OneScene>::value;
-    if (warp_walk<kPersist, kLam, kRuns, kKeep>(sm, G, fluid_index(G), prm, p, cell, want, xi, xin, kept, sums))
+    uint32_t kept = 0u;
+    if (warp_walk<kPersist, kLam, kRuns, false>(sm, G, fluid_index(G), prm, p, cell, want, xi, xin, kept,
+        sums))
         return;
     if (!want) return;
-    kept = kNoList;
     for_each_candidate_runs<kRuns>(
         cell, G, C,
         [&](uint32_t q) {
@@ -2301,75 +2334,46 @@ __device__ __forceinline__ void sum_walking(WalkSmem& sm, const Grid& G, const P
         });
 }
 
-template <bool kPersist, bool kLam, class P, class Sums>
-__device__ __forceinline__ void sum_candidates(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
-                                               const int4 cell, bool want, const float4 xi,
-                                               const float4* xin, const StepConsts& C, Sums& sums) {
-    uint32_t kept = 0u;
-    sum_walking<kPersist, kLam, false>(sm, G, prm, p, cell, want, xi, xin, C, kept, sums);
+// The same sums of a warp from the lanes' kept lists of `cnt` candidates (of
+// lanes that want).  kLam: in a warp whose lambdas are all zero, pairs of candidates
+// whose lambdas are zero too are passed over (see walk_group).
+template <bool kLam, class Sums>
+__device__ __forceinline__ void read_lists(const Grid& G, uint32_t p, bool want, uint32_t cnt,
+                                           const float4 xi, const float4* __restrict__ xin, Sums& sums) {
+    const unsigned full = 0xffffffffu;
+    if (!want) cnt = 0u;
+    const uint32_t most = __reduce_max_sync(full, cnt);
+    const bool all_zero = kLam && !__any_sync(full, want && xi.w != 0.0f);
+    const uint2* from = G.lists + list_at(p);
+    float4 xa = xi, xb = xi, ea = make_float4(0.0f, 0.0f, 0.0f, 0.0f), eb = ea;
+    uint2 q = make_uint2(p, p);
+    auto load = [&]() {
+        xa = __ldg(xin + q.x);
+        xb = __ldg(xin + q.y);
+        if constexpr (Sums::kExtra) {
+            ea = sums.extra(q.x);
+            eb = sums.extra(q.y);
+        }
+    };
+    if (cnt > 0u) {
+        q = __ldcs(from);
+        load();
+    }
+    if (cnt > 2u) q = __ldcs(from + 32);
+    from += 64;
+    for (uint32_t t = 0; t < most; t += 2u) {
+        const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
+        if (t + 2u < cnt) load();
+        if (t + 4u < cnt) q = __ldcs(from);
+        from += 32;
+        if (all_zero && !__any_sync(full, t < cnt && (x0.w != 0.0f || x1.w != 0.0f))) continue;
+        sums.add2(x0, x1, e0, e1, t < cnt, t + 1u < cnt);
+    }
 }
 
-// The same, keeping the lists (where there is room for any).
-template <bool kPersist, class P, class Sums>
-__device__ __forceinline__ void sum_keeping(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
-                                            const int4 cell, bool want, const float4 xi, const float4* xin,
-                                            const StepConsts& C, Sums& sums) {
-    if constexpr (!kPersist) {
-        if (G.lists) {
-            uint32_t kept = 0u;
-            sum_walking<false, false, true>(sm, G, prm, p, cell, want, xi, xin, C, kept, sums);
-            if (want) G.listed[p] = kept;
-            return;
-        }
-    }
-    sum_candidates<kPersist, false>(sm, G, prm, p, cell, want, xi, xin, C, sums);
-}
-
-// The same from the kept lists, where every lane that wants has one.  kLam: in
-// a warp whose lambdas are all zero, pairs of candidates whose lambdas are
-// zero too are passed over (see walk_group).
-template <bool kPersist, bool kLam, class P, class Sums>
-__device__ __forceinline__ void sum_listed(WalkSmem& sm, const Grid& G, const P& prm, uint32_t p,
-                                           const int4 cell, bool want, const float4 xi, const float4* xin,
-                                           const StepConsts& C, Sums& sums) {
-    if constexpr (!kPersist) {
-        if (G.lists) {
-            const unsigned full = 0xffffffffu;
-            const uint32_t rows = want ? G.listed[p] : 0u;
-            const uint32_t most = __reduce_max_sync(full, rows);
-            if (most != kNoList) {
-                const bool all_zero = kLam && !__any_sync(full, want && xi.w != 0.0f);
-                const uint2* from = G.lists + list_at(p);
-                float4 xa = xi, xb = xi, ea = make_float4(0.0f, 0.0f, 0.0f, 0.0f), eb = ea;
-                uint2 q = make_uint2(p, p);
-                auto load = [&]() {
-                    xa = __ldg(xin + q.x);
-                    xb = __ldg(xin + q.y);
-                    if constexpr (Sums::kExtra) {
-                        ea = sums.extra(q.x);
-                        eb = sums.extra(q.y);
-                    }
-                };
-                if (rows > 0u) {
-                    q = __ldcs(from);
-                    load();
-                }
-                if (rows > 1u) q = __ldcs(from + 32);
-                from += 64;
-                for (uint32_t r = 0; r < most; ++r) {
-                    const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
-                    if (r + 1u < rows) load();
-                    if (r + 2u < rows) q = __ldcs(from);
-                    from += 32;
-                    const bool has = r < rows;
-                    if (all_zero && !__any_sync(full, has && (x0.w != 0.0f || x1.w != 0.0f))) continue;
-                    sums.add2(x0, x1, e0, e1, has, has);
-                }
-                return;
-            }
-        }
-    }
-    sum_candidates<kPersist, kLam>(sm, G, prm, p, cell, want, xi, xin, C, sums);
+// Rows of the kept list of a particle that wants, 0 where it does not.
+__device__ __forceinline__ uint32_t list_rows(const Grid& G, uint32_t p, bool want) {
+    return want ? G.listed[p] & kNoList : 0u;
 }
 
 // The same over the boundary of a two-way coupled step; `cell` is the
@@ -2501,26 +2505,41 @@ __device__ __forceinline__ void store_lambda(uint32_t p, uint32_t rf, const int4
     }
 }
 
+// How a pass of a warp finds its sums: by walking; from kept lists; from kept
+// lists and, over a two-way coupled step's boundary, by walking.
+enum PassMode { kWalk, kListed, kListedTwoWay };
+
 // The density pass for sorted particle p.  Reads x* from xin, writes
 // (x*, lambda) to xout and rho to srho.  Scenes whose `iters` are done by
 // iteration `it` are left untouched.  Warp-collective: every lane of the warp
 // calls it, with `active` false past the last particle.
-template <bool kPersist, class P>
+template <bool kPersist, PassMode kMode, class P>
 __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const float4* xin,
                                                   float4* xout, float* __restrict__ srho, int it,
-                                                  const Grid& G, const P& prm, WalkSmem& sm) {
+                                                  const Grid& G, const P& prm, WalkSmem* sm) {
     const uint32_t pa = active ? p : 0u;
     const StepConsts& C = prm.at(G.spid, pa);
     const int4 cell = cell_at(G, pa);
     const uint32_t rf = run_flags(G, pa);
     bool live = active && it < C.iters && !(rf & kCopyBit);
-    if (live && it > 0 && G.moved && cell.w == 0 &&
-        !neighbourhood_stamped<kPersist>(cell, C.grid, G.moved, (uint32_t)it, 0, 3)) {
+    uint32_t rows = 0u;
+    if constexpr (kMode != kWalk) {
+        // k_list has kept lambda where nothing around moved.
+        const uint32_t word = live ? G.listed[pa] : 0u;
+        if (word & kIdle) live = false;
+        rows = live ? word : 0u;
+        if (__reduce_max_sync(0xffffffffu, rows) == kNoList) return;
+    } else if (live && it > 0 && G.moved && cell.w == 0 &&
+               !neighbourhood_stamped<kPersist>(cell, C.grid, G.moved, (uint32_t)it, 0, 3)) {
         keep_lambda(p, rf, cell, xin, xout, it, G, C);
         live = false;
     }
     if (!__any_sync(0xffffffffu, live)) return;
     const float4 xi = xin[pa];
+    auto sum = [&](bool want, auto& sums) {
+        if constexpr (kMode != kWalk) read_lists<false>(G, pa, want, rows, xi, xin, sums);
+        else sum_candidates<kPersist, false>(*sm, G, prm, pa, cell, want, xi, xin, C, sums);
+    };
     float density, gix = 0.0f, giy = 0.0f, giz = 0.0f, sum_grad_sq = 0.0f;
     // Density first: when C_i < 0 lambda_i is 0 whatever the gradient sums,
     // so a warp can sum the densities alone (poly6 terms, no square root or
@@ -2539,32 +2558,32 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
     }
     if (kHist && dfirst) {
         LaneSums<DensityTerm> ds(DensityTerm{C, xi});
-        sum_keeping<kPersist>(sm, G, prm, pa, cell, live, xi, xin, C, ds);
+        sum(live, ds);
         density = ds.get(0);
         const bool want = live && !(density * C.inv_rho0 - 1.0f < 0.0f);
         LaneSums<GradTerm> gs(GradTerm{C, xi});
-        sum_listed<kPersist, false>(sm, G, prm, pa, cell, want, xi, xin, C, gs);
+        sum(want, gs);
         gix = gs.get(0);
         giy = gs.get(1);
         giz = gs.get(2);
         sum_grad_sq = gs.get(3);
     } else {
         LaneSums<DensityGradTerm> sums(DensityGradTerm{C, xi});
-        sum_keeping<kPersist>(sm, G, prm, pa, cell, live, xi, xin, C, sums);
+        sum(live, sums);
         density = sums.get(0);
         gix = sums.get(1);
         giy = sums.get(2);
         giz = sums.get(3);
         sum_grad_sq = sums.get(4);
     }
-    if constexpr (kHist) {
+    if constexpr (kHist && kMode != kListed) {
         if (G.bg.spos) {
             // Two-way coupling: after the fluid terms, the boundary's in the
             // boundary index's bucket order.
             LaneSums<BoundaryDensityTerm> bsums(BoundaryDensityTerm{C, xi});
             const float from[4] = {density, gix, giy, giz};
             bsums.start(from);
-            sum_boundary(sm, G, prm, pa, cell, live, xi, C, bsums);
+            sum_boundary(*sm, G, prm, pa, cell, live, xi, C, bsums);
             density = bsums.get(0);
             gix = bsums.get(1);
             giy = bsums.get(2);
@@ -2584,13 +2603,86 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
     if (live) store_lambda(p, rf, cell, xi, density, Ci, gix, giy, giz, sum_grad_sq, xout, srho, it, G, C);
 }
 
+// The passes' kernels for warps of 32 particles.  Each comes twice: walking,
+// for scenes without kept lists and (rest) for the warps in which some particle
+// has none; and _listed, for the other warps of scenes with lists.  The readers
+// have neither a walk's registers nor its shared memory, so more warps are in
+// flight and the whole L1 holds candidates.
+constexpr int kRestBlocks = 152 * 6;
+
+// Whether the walking launch `rest` leaves this warp out.
+__device__ __forceinline__ bool leave_out(int rest, const Grid& G, uint32_t p, bool want) {
+    return rest && __reduce_max_sync(0xffffffffu, list_rows(G, p, want)) != kNoList;
+}
+
+// Lists the candidates of a pass for its listed kernels.  it >= 0: of Jacobi
+// iteration it's density and delta pass (particles around which nothing moved
+// keep their list and lambda).  it < 0: of the velocity passes; lists of
+// particles around which the last delta pass moved nothing still hold.
+template <int BS, class P>
+__global__ void __launch_bounds__(BS, kListThreads / BS)
+k_list(const float4* __restrict__ xin, float4* __restrict__ xout, int it, int n, const Grid G, const P prm) {
+    __shared__ WalkSmem sm[BS / 32];
+    constexpr bool kRuns = std::is_same<P, OneScene>::value;
+    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+    const bool active = p < (uint32_t)n;
+    const uint32_t pa = active ? p : 0u;
+    const StepConsts& C = prm.at(G.spid, pa);
+    const int4 cell = cell_at(G, pa);
+    const uint32_t rf = run_flags(G, pa);
+    bool live = active && !(rf & kCopyBit);
+    if (it >= 0) {
+        live = live && it < C.iters;
+        if (live && it > 0 && G.moved && cell.w == 0 &&
+            !neighbourhood_stamped<false>(cell, C.grid, G.moved, (uint32_t)it, 0, 3)) {
+            keep_lambda(p, rf, cell, xin, xout, it, G, C);
+            G.listed[p] |= kIdle;
+            live = false;
+        }
+    } else {
+        live = live && (C.vort_on || C.xsph_on);
+        if (live && C.iters > 0 && G.moved && cell.w == 0 &&
+            !neighbourhood_stamped<false>(cell, C.grid, G.moved, (uint32_t)C.iters, 0, 3))
+            live = false;
+    }
+    if (!__any_sync(0xffffffffu, live)) return;
+    uint32_t kept = 0u;
+    NoSums none;
+    if (!warp_walk<false, false, kRuns, true>(sm[threadIdx.x >> 5], G, fluid_index(G), prm, pa, cell, live,
+                                              xin[pa], xin, kept, none))
+        kept = kNoList;
+    if (live) G.listed[p] = kept;
+    if (live && kept == kNoList) *G.unlisted = 1u;
+}
+
 template <int BS, class P>
 __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
 k_density_lambda(const float4* __restrict__ xin, float4* __restrict__ xout, float* __restrict__ srho,
-                 int it, int n, const Grid G, const P prm) {
+                 int it, int n, int rest, const Grid G, const P prm) {
     __shared__ WalkSmem sm[BS / 32];
+    if (rest && *G.unlisted == 0u) return;
+    for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
+        const uint32_t p = b * BS + threadIdx.x;
+        const uint32_t pa = p < (uint32_t)n ? p : 0u;
+        if (!leave_out(rest, G, pa, p < (uint32_t)n && it < prm.at(G.spid, pa).iters &&
+                                           !(run_flags(G,
+                                             pa) & kCopyBit) && !(rest && (G.listed[pa] & kIdle))))
+            density_lambda_at<false, kWalk>(p, p < (uint32_t)n, xin, xout, srho, it, G, prm,
+                                            &sm[threadIdx.x >> 5]);
+    }
+}
+
+template <int BS, PassMode kMode, class P>
+__global__ void __launch_bounds__(BS, kReadThreads<P> / BS)
+k_density_lambda_listed(const float4* __restrict__ xin, float4* __restrict__ xout, float* __restrict__ srho,
+                        int it, int n, const Grid G, const P prm) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    density_lambda_at<false>(p, p < (uint32_t)n, xin, xout, srho, it, G, prm, sm[threadIdx.x >> 5]);
+    WalkSmem* sm = nullptr;
+    if constexpr (kMode == kListedTwoWay) {
+        __shared__ WalkSmem walk[BS / 32];
+        sm = &walk[threadIdx.x >> 5];
+    }
+    density_lambda_at<false, kMode>(p, p < (uint32_t)n, xin, xout, srho, it, G, prm, sm);
 }
 
 template <int TP, class P>
@@ -2684,16 +2776,21 @@ __device__ __forceinline__ void store_delta(uint32_t p, uint32_t rf, const int4 
 // sorted particle p.  Reads (x*, lambda) from xin, writes (x* + dp, lambda_i)
 // to xout; on the scene's last iteration also the updated velocity into sv.
 // Warp-collective like density_lambda_at.
-template <bool kPersist, class P>
+template <bool kPersist, PassMode kMode, class P>
 __device__ __forceinline__ void delta_at(uint32_t p, bool active, const float4* xin, float4* xout,
                                          const float4* __restrict__ sx,
                                          const float* __restrict__ srho, float4* __restrict__ sv,
-                                         int it, const Grid& G, const P& prm, WalkSmem& sm) {
+                                         int it, const Grid& G, const P& prm, WalkSmem* sm) {
     const uint32_t pa = active ? p : 0u;
     const StepConsts& C = prm.at(G.spid, pa);
     const int4 cell = cell_at(G, pa);
     const uint32_t rf = run_flags(G, pa);
     const bool live = active && it < C.iters && !(rf & kCopyBit);
+    uint32_t rows = 0u;
+    if constexpr (kMode != kWalk) {
+        rows = list_rows(G, pa, live);
+        if (__reduce_max_sync(0xffffffffu, rows) == kNoList) return;
+    }
     float4 xi = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
     if (live) xi = xin[p];
     bool walk = live;
@@ -2703,16 +2800,17 @@ __device__ __forceinline__ void delta_at(uint32_t p, bool active, const float4* 
         !neighbourhood_stamped<kPersist>(cell, C.grid, G.lamnz, (uint32_t)it + 1u, 0, 3))
         walk = false;
     LaneSums<DeltaTerm> sums(DeltaTerm{C, xi});
-    sum_listed<kPersist, true>(sm, G, prm, pa, cell, walk, xi, xin, C, sums);
+    if constexpr (kMode != kWalk) read_lists<true>(G, pa, walk, rows, xi, xin, sums);
+    else sum_candidates<kPersist, true>(*sm, G, prm, pa, cell, walk, xi, xin, C, sums);
     float dx = sums.get(0), dy = sums.get(1), dz = sums.get(2);
-    if constexpr (std::is_same<P, OneScene>::value) {
+    if constexpr (std::is_same<P, OneScene>::value && kMode != kListed) {
         if (G.bg.spos) {
             // Two-way coupling: the boundary's share after the fluid terms
             // (zero when lambda_i is).
             LaneSums<BoundaryDeltaTerm> bsums(BoundaryDeltaTerm{C, xi});
             const float from[3] = {dx, dy, dz};
             bsums.start(from);
-            sum_boundary(sm, G, prm, pa, cell, live && xi.w != 0.0f, xi, C, bsums);
+            sum_boundary(*sm, G, prm, pa, cell, live && xi.w != 0.0f, xi, C, bsums);
             dx = bsums.get(0);
             dy = bsums.get(1);
             dz = bsums.get(2);
@@ -2724,11 +2822,32 @@ __device__ __forceinline__ void delta_at(uint32_t p, bool active, const float4* 
 template <int BS, class P>
 __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
 k_delta(const float4* __restrict__ xin, float4* __restrict__ xout, const float4* __restrict__ sx,
-        const float* __restrict__ srho, float4* __restrict__ sv, int it, int n, const Grid G,
+        const float* __restrict__ srho, float4* __restrict__ sv, int it, int n, int rest, const Grid G,
         const P prm) {
     __shared__ WalkSmem sm[BS / 32];
+    if (rest && *G.unlisted == 0u) return;
+    for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
+        const uint32_t p = b * BS + threadIdx.x;
+        const uint32_t pa = p < (uint32_t)n ? p : 0u;
+        if (!leave_out(rest, G, pa, p < (uint32_t)n && it < prm.at(G.spid, pa).iters &&
+                                           !(run_flags(G, pa) & kCopyBit)))
+            delta_at<false, kWalk>(p, p < (uint32_t)n, xin, xout, sx, srho, sv, it, G, prm,
+                                   &sm[threadIdx.x >> 5]);
+    }
+}
+
+template <int BS, PassMode kMode, class P>
+__global__ void __launch_bounds__(BS, kReadThreads<P> / BS)
+k_delta_listed(const float4* __restrict__ xin, float4* __restrict__ xout, const float4* __restrict__ sx,
+               const float* __restrict__ srho, float4* __restrict__ sv, int it, int n, const Grid G,
+               const P prm) {
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    delta_at<false>(p, p < (uint32_t)n, xin, xout, sx, srho, sv, it, G, prm, sm[threadIdx.x >> 5]);
+    WalkSmem* sm = nullptr;
+    if constexpr (kMode == kListedTwoWay) {
+        __shared__ WalkSmem walk[BS / 32];
+        sm = &walk[threadIdx.x >> 5];
+    }
+    delta_at<false, kMode>(p, p < (uint32_t)n, xin, xout, sx, srho, sv, it, G, prm, sm);
 }
 
 template <int TP, class P>
@@ -2841,12 +2960,10 @@ k_iterate(float4* xa, float4* xb, float* __restrict__ srho, const float4* __rest
     auto& my = sm[threadIdx.x >> 5];
     for (int it = 0; it < max_iters; ++it) {
         for (uint32_t pw = w0; pw < (uint32_t)n; pw += stride)
-            density_lambda_at<true>(pw + lane, pw + lane < (uint32_t)n, xa, xb, srho, it, G,
-                                       prm, my);
+            density_lambda_at<true, kWalk>(pw + lane, pw + lane < (uint32_t)n, xa, xb, srho, it, G, prm, &my);
         if (!grid_sync(S)) return;
         for (uint32_t pw = w0; pw < (uint32_t)n; pw += stride)
-            delta_at<true>(pw + lane, pw + lane < (uint32_t)n, xb, xa, sx, srho, sv, it, G,
-                              prm, my);
+            delta_at<true, kWalk>(pw + lane, pw + lane < (uint32_t)n, xb, xa, sx, srho, sv, it, G, prm, &my);
         if (it + 1 < max_iters && !grid_sync(S)) return;
     }
 }
@@ -2942,23 +3059,53 @@ __device__ __forceinline__ void store_xsph(uint32_t p, uint32_t rf, const float4
         commit(m, xi.x, xi.y, xi.z, vx, vy, vz, xi.w, sx, srho, prm.state(G.spid, m), n, C);
 }
 
-template <int BS, class P>
-__global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
-k_xsph_commit(const float4* __restrict__ xin, const float4* __restrict__ sv, const float4* __restrict__ sx,
-              const float* __restrict__ srho, int n, int skip_vort, const Grid G, const P prm) {
-    __shared__ WalkSmem sm[BS / 32];
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+template <PassMode kMode, class P>
+__device__ __forceinline__ void xsph_commit_at(uint32_t p, const float4* __restrict__ xin,
+                                               const float4* __restrict__ sv, const float4* __restrict__ sx,
+                                               const float* __restrict__ srho, int n, int skip_vort,
+                                               const Grid& G, const P& prm, WalkSmem* sm) {
     const bool active = p < (uint32_t)n;
     const uint32_t pa = active ? p : 0u;
     const StepConsts& C = prm.at(G.spid, pa);
-    const int4 cell = cell_at(G, pa);
     const uint32_t rf = run_flags(G, pa);
     const bool live = active && !(skip_vort && C.vort_on) && !(rf & kCopyBit);
+    const bool want = live && C.xsph_on;
+    uint32_t rows = 0u;
+    if constexpr (kMode != kWalk) {
+        rows = list_rows(G, pa, want);
+        if (__reduce_max_sync(0xffffffffu, rows) == kNoList) return;
+    }
     const float4 xi = xin[pa];
     const float4 vi = sv[pa];
     LaneSums<XsphTerm> sums(XsphTerm{C, xi, vi, sv});
-    sum_candidates<false, false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live && C.xsph_on, xi, xin, C, sums);
+    if constexpr (kMode != kWalk) read_lists<false>(G, pa, want, rows, xi, xin, sums);
+    else sum_candidates<false, false>(*sm, G, prm, pa, cell_at(G, pa), want, xi, xin, C, sums);
     if (live) store_xsph(p, rf, xi, vi, sums.get(0), sums.get(1), sums.get(2), sx, srho, n, G, prm, C);
+}
+
+template <int BS, class P>
+__global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
+k_xsph_commit(const float4* __restrict__ xin, const float4* __restrict__ sv, const float4* __restrict__ sx,
+              const float* __restrict__ srho, int n, int skip_vort, int rest, const Grid G, const P prm) {
+    __shared__ WalkSmem sm[BS / 32];
+    if (rest && *G.unlisted == 0u) return;
+    for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
+        const uint32_t p = b * BS + threadIdx.x;
+        const uint32_t pa = p < (uint32_t)n ? p : 0u;
+        const StepConsts& C = prm.at(G.spid, pa);
+        const bool live = p < (uint32_t)n && !(skip_vort && C.vort_on) && !(run_flags(G, pa) & kCopyBit);
+        if (!leave_out(rest, G, pa, live && C.xsph_on)) xsph_commit_at<kWalk>(p, xin, sv, sx, srho, n,
+            skip_vort, G, prm, &sm[threadIdx.x >> 5]);
+    }
+}
+
+template <int BS, class P>
+__global__ void __launch_bounds__(BS, kReadThreads<P> / BS)
+k_xsph_commit_listed(const float4* __restrict__ xin, const float4* __restrict__ sv,
+                     const float4* __restrict__ sx, const float* __restrict__ srho, int n, int skip_vort,
+                     const Grid G, const P prm) {
+    xsph_commit_at<kListed>(blockIdx.x * blockDim.x + threadIdx.x, xin, sv, sx, srho, n, skip_vort, G, prm,
+                            nullptr);
 }
 
 template <int TP, class P>
@@ -3001,25 +3148,53 @@ __device__ __forceinline__ void store_omega(uint32_t p, uint32_t rf, const float
     }
 }
 
-template <int BS, class P>
-__global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
-k_xsph_omega(const float4* __restrict__ xin, const float4* __restrict__ sv, float4* __restrict__ sv2,
-             float4* __restrict__ som, int n, const Grid G, const P prm) {
-    __shared__ WalkSmem sm[BS / 32];
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
+template <PassMode kMode, class P>
+__device__ __forceinline__ void xsph_omega_at(uint32_t p, const float4* __restrict__ xin,
+                                              const float4* __restrict__ sv, float4* __restrict__ sv2,
+                                              float4* __restrict__ som, int n, const Grid& G, const P& prm,
+                                              WalkSmem* sm) {
     const bool active = p < (uint32_t)n;
     const uint32_t pa = active ? p : 0u;
     const StepConsts& C = prm.at(G.spid, pa);
-    const int4 cell = cell_at(G, pa);
     const uint32_t rf = run_flags(G, pa);
     const bool live = active && C.vort_on && !(rf & kCopyBit);
+    const bool want = live;
+    uint32_t rows = 0u;
+    if constexpr (kMode != kWalk) {
+        rows = list_rows(G, pa, want);
+        if (__reduce_max_sync(0xffffffffu, rows) == kNoList) return;
+    }
     const float4 xi = xin[pa];
     const float4 vi = sv[pa];
     LaneSums<XsphOmegaTerm> sums(XsphOmegaTerm{C, xi, vi, sv});
-    sum_keeping<false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live, xi, xin, C, sums);
+    if constexpr (kMode != kWalk) read_lists<false>(G, pa, want, rows, xi, xin, sums);
+    else sum_candidates<false, false>(*sm, G, prm, pa, cell_at(G, pa), want, xi, xin, C, sums);
     if (live)
         store_omega(p, rf, vi, sums.get(0), sums.get(1), sums.get(2), sums.get(3), sums.get(4), sums.get(5),
                     sv2, som, G, C);
+}
+
+template <int BS, class P>
+__global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
+k_xsph_omega(const float4* __restrict__ xin, const float4* __restrict__ sv, float4* __restrict__ sv2,
+             float4* __restrict__ som, int n, int rest, const Grid G, const P prm) {
+    __shared__ WalkSmem sm[BS / 32];
+    if (rest && *G.unlisted == 0u) return;
+    for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
+        const uint32_t p = b * BS + threadIdx.x;
+        const uint32_t pa = p < (uint32_t)n ? p : 0u;
+        const StepConsts& C = prm.at(G.spid, pa);
+        const bool live = p < (uint32_t)n && C.vort_on && !(run_flags(G, pa) & kCopyBit);
+        if (!leave_out(rest, G, pa, live)) xsph_omega_at<kWalk>(p, xin, sv, sv2, som, n, G, prm,
+            &sm[threadIdx.x >> 5]);
+    }
+}
+
+template <int BS, class P>
+__global__ void __launch_bounds__(BS, kReadThreads<P> / BS)
+k_xsph_omega_listed(const float4* __restrict__ xin, const float4* __restrict__ sv, float4* __restrict__ sv2,
+                    float4* __restrict__ som, int n, const Grid G, const P prm) {
+    xsph_omega_at<kListed>(blockIdx.x * blockDim.x + threadIdx.x, xin, sv, sv2, som, n, G, prm, nullptr);
 }
 
 template <int TP, class P>
@@ -3066,25 +3241,56 @@ __device__ __forceinline__ void store_vorticity(uint32_t p, uint32_t rf, const f
         commit(m, xi.x, xi.y, xi.z, vx, vy, vz, xi.w, sx, srho, prm.state(G.spid, m), n, C);
 }
 
+template <PassMode kMode, class P>
+__device__ __forceinline__ void vorticity_commit_at(uint32_t p, const float4* __restrict__ xin,
+    const float4* __restrict__ sv, const float4* __restrict__ sv2, const float4* __restrict__ som,
+    const float4* __restrict__ sx, const float* __restrict__ srho, int n, const Grid& G, const P& prm,
+    WalkSmem* sm) {
+    const bool active = p < (uint32_t)n;
+    const uint32_t pa = active ? p : 0u;
+    const StepConsts& C = prm.at(G.spid, pa);
+    const uint32_t rf = run_flags(G, pa);
+    const bool live = active && C.vort_on && !(rf & kCopyBit);
+    const bool want = live;
+    uint32_t rows = 0u;
+    if constexpr (kMode != kWalk) {
+        rows = list_rows(G, pa, want);
+        if (__reduce_max_sync(0xffffffffu, rows) == kNoList) return;
+    }
+    const float4 xi = xin[pa];
+    LaneSums<VorticityTerm> sums(VorticityTerm{C, xi, som[pa].w, sv, som});
+    if constexpr (kMode != kWalk) read_lists<false>(G, pa, want, rows, xi, xin, sums);
+    else sum_candidates<false, false>(*sm, G, prm, pa, cell_at(G, pa), want, xi, xin, C, sums);
+    if (live)
+        store_vorticity(p, rf, xi, sums.get(0), sums.get(1), sums.get(2), sv2, som, sx, srho, n, G, prm, C);
+}
+
 template <int BS, class P>
 __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
 k_vorticity_commit(const float4* __restrict__ xin, const float4* __restrict__ sv,
                    const float4* __restrict__ sv2, const float4* __restrict__ som,
-                   const float4* __restrict__ sx, const float* __restrict__ srho, int n,
+                   const float4* __restrict__ sx, const float* __restrict__ srho, int n, int rest,
                    const Grid G, const P prm) {
     __shared__ WalkSmem sm[BS / 32];
-    const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
-    const bool active = p < (uint32_t)n;
-    const uint32_t pa = active ? p : 0u;
-    const StepConsts& C = prm.at(G.spid, pa);
-    const int4 cell = cell_at(G, pa);
-    const uint32_t rf = run_flags(G, pa);
-    const bool live = active && C.vort_on && !(rf & kCopyBit);
-    const float4 xi = xin[pa];
-    LaneSums<VorticityTerm> sums(VorticityTerm{C, xi, som[pa].w, sv, som});
-    sum_listed<false, false>(sm[threadIdx.x >> 5], G, prm, pa, cell, live, xi, xin, C, sums);
-    if (live)
-        store_vorticity(p, rf, xi, sums.get(0), sums.get(1), sums.get(2), sv2, som, sx, srho, n, G, prm, C);
+    if (rest && *G.unlisted == 0u) return;
+    for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
+        const uint32_t p = b * BS + threadIdx.x;
+        const uint32_t pa = p < (uint32_t)n ? p : 0u;
+        const StepConsts& C = prm.at(G.spid, pa);
+        const bool live = p < (uint32_t)n && C.vort_on && !(run_flags(G, pa) & kCopyBit);
+        if (!leave_out(rest, G, pa, live)) vorticity_commit_at<kWalk>(p, xin, sv, sv2, som, sx, srho, n, G,
+            prm, &sm[threadIdx.x >> 5]);
+    }
+}
+
+template <int BS, class P>
+__global__ void __launch_bounds__(BS, kReadThreads<P> / BS)
+k_vorticity_commit_listed(const float4* __restrict__ xin, const float4* __restrict__ sv,
+                          const float4* __restrict__ sv2, const float4* __restrict__ som,
+                          const float4* __restrict__ sx, const float* __restrict__ srho, int n,
+                          const Grid G, const P prm) {
+    vorticity_commit_at<kListed>(blockIdx.x * blockDim.x + threadIdx.x, xin, sv, sv2, som, sx, srho, n, G,
+                                 prm, nullptr);
 }
 
 template <int TP, class P>
@@ -3154,7 +3360,7 @@ inline Grid grid_view(const StepBuffers& B, int n, const uint32_t* spid = nullpt
                       const BoundaryGrid& bg = BoundaryGrid{}) {
     return Grid{B.scell, B.sown, WalkIndex{(uint32_t)n, B.off, B.bkt.merged, B.bkt.end, B.btab}, spid,
                 B.moved, B.lamnz, bg, spid ? nullptr : B.dhist, nullptr, B.slot_alias,
-                n <= B.list_cap ? B.lists : nullptr, B.listed};
+                n <= B.list_cap ? B.lists : nullptr, B.listed, B.unlisted};
 }
 
 // predict, sort by cell and by reference key, cell offsets, gather, reference
@@ -3170,7 +3376,8 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
     cudaError_t e = clear_ranges(slot_clear(B), sort_clear(sort, n, bits),
                                  C.hash_compat ? bucket_clear(B.bkt, n) : ClearRange{}, st);
     if (e != cudaSuccess) return e;
-    k_predict_key<OneScene><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, B.dhist, n, sort_counts(sort, n,
+    k_predict_key<OneScene><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, B.dhist, B.unlisted, n,
+                                           sort_counts(sort, n,
         bits), none, one);
     if (pm) pm->mark(kPhasePredict, 2, st);
     e = radix_sort_counted(B.keys, B.skeys, B.sidx, n, bits, sort, st);
@@ -3213,14 +3420,21 @@ inline int team_size(int n) {
 
 // TP: particles per team, 0 for warps of 32 particles in blocks of BS threads.
 template <int BS, int TP, class P>
-inline cudaError_t enqueue_passes_bs(const StepBuffers& B, const Grid& G, int n, int max_iters,
+inline cudaError_t enqueue_passes_bs(const StepBuffers& B, Grid G, int n, int max_iters,
                                      bool any_zero_iters, bool any_vort, bool any_plain,
                                      bool xsph_on, const P prm, cudaStream_t st, PhaseMarks* pm,
                                      int persist_blocks, unsigned int* barrier) {
     constexpr int T = TP ? TP : 32;
     const int nb = TP ? grid_of(n, T) : grid_of(n, BS);
+    // With kept lists a warp pass lists, reads the lists and walks for the rest.
+    const auto rest = [&] { return G.lists ? 1 : 0; };
+    const auto walk_blocks = [&] { return G.lists && nb > kRestBlocks ? kRestBlocks : nb; };
+    const auto list = [&](const float4* xin, float4* xout, int it) {
+        if (G.lists) k_list<BS, P><<<nb, BS, 0, st>>>(xin, xout, it, n, G, prm);
+    };
     if (persist_blocks > 0 && barrier && max_iters > 0) {
-        // The whole Jacobi loop as one cooperative launch.
+        // The whole Jacobi loop as one cooperative launch, which keeps no lists.
+        G.lists = nullptr;
         cudaError_t e = cudaMemsetAsync(barrier, 0, sizeof(unsigned int), st);
         if (e != cudaSuccess) return e;
         cudaLaunchConfig_t cfg = {};
@@ -3241,14 +3455,42 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, const Grid& G, int n,
         for (int it = 0; it < max_iters; ++it) {
             if constexpr (TP != 0)
                 k_density_lambda_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
-            else
-                k_density_lambda<BS, P><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, G, prm);
-            if (pm) pm->mark(kPhaseDensity, 1, st);
+            else {
+                list(B.xa, B.xb, it);
+                if (G.lists) {
+                    if (G.bg.spos) {
+                        if constexpr (std::is_same<P, OneScene>::value)
+                            k_density_lambda_listed<BS, kListedTwoWay, P><<<nb, BS, 0, st>>>(B.xa, B.xb,
+                                B.srho,
+                                it, n, G, prm);
+                    } else {
+                        k_density_lambda_listed<BS, kListed, P><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it,
+                            n, G,
+                            prm);
+                    }
+                }
+                k_density_lambda<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, rest(), G,
+                    prm);
+            }
+            if (pm) pm->mark(kPhaseDensity, TP == 0 && G.lists ? 3 : 1, st);
             if constexpr (TP != 0)
                 k_delta_team<T, P><<<nb, 128, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
-            else
-                k_delta<BS, P><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, G, prm);
-            if (pm) pm->mark(kPhaseDelta, 1, st);
+            else {
+                if (G.lists) {
+                    if (G.bg.spos) {
+                        if constexpr (std::is_same<P, OneScene>::value)
+                            k_delta_listed<BS, kListedTwoWay, P><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho,
+                                B.sv, it, n, G, prm);
+                    } else {
+                        k_delta_listed<BS, kListed, P><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv,
+                            it, n,
+                            G, prm);
+                    }
+                }
+                k_delta<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, rest(),
+                                             G, prm);
+            }
+            if (pm) pm->mark(kPhaseDelta, TP == 0 && G.lists ? 2 : 1, st);
         }
     }
     if (any_zero_iters) {
@@ -3261,25 +3503,41 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, const Grid& G, int n,
             if (pm) pm->mark(kPhaseXsph, 1, st);
         }
     }
+    if constexpr (TP == 0) {
+        list(B.xa, nullptr, -1);
+        if (pm && G.lists) pm->mark(kPhaseXsph, 1, st);
+    }
     if (any_vort) {
         if constexpr (TP != 0)
             k_xsph_omega_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
-        else
-            k_xsph_omega<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
-        if (pm) pm->mark(kPhaseXsph, 1, st);
+        else {
+            if (G.lists) k_xsph_omega_listed<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, G, prm);
+            k_xsph_omega<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, n, rest(), G, prm);
+        }
+        if (pm) pm->mark(kPhaseXsph, TP == 0 && G.lists ? 2 : 1, st);
         if constexpr (TP != 0)
             k_vorticity_commit_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n, G, prm);
-        else
-            k_vorticity_commit<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n, G, prm);
-        if (pm) pm->mark(kPhaseCommit, 1, st);
+        else {
+            if (G.lists)
+                k_vorticity_commit_listed<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho,
+                    n, G,
+                    prm);
+            k_vorticity_commit<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n,
+                rest(), G, prm);
+        }
+        if (pm) pm->mark(kPhaseCommit, TP == 0 && G.lists ? 2 : 1, st);
     }
     if (any_plain) {
         const int skip = any_vort ? 1 : 0;
         if constexpr (TP != 0)
             k_xsph_commit_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
-        else
-            k_xsph_commit<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
-        if (pm) pm->mark(xsph_on ? kPhaseXsph : kPhaseCommit, 1, st);
+        else {
+            if (G.lists) k_xsph_commit_listed<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip,
+                G, prm);
+            k_xsph_commit<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, rest(), G,
+                                               prm);
+        }
+        if (pm) pm->mark(xsph_on ? kPhaseXsph : kPhaseCommit, TP == 0 && G.lists ? 2 : 1, st);
     }
     return cudaGetLastError();
 }
@@ -3369,7 +3627,8 @@ inline cudaError_t enqueue_batch_step(const StepBuffers& B, const BatchDesc& D, 
     cudaError_t e = clear_ranges(slot_clear(B), sort_clear(sort, n, D.key_bits), bucket_clear(B.bkt, n), st);
     if (e != cudaSuccess) return e;
     k_scene_ids<<<grid_of(n, 256), 256, 0, st>>>(D.firsts, D.nscenes, D.pid, n);
-    k_predict_key<SceneTable><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, nullptr, n, sort_counts(sort,
+    k_predict_key<SceneTable><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, nullptr, B.unlisted, n,
+                                             sort_counts(sort,
         n, D.key_bits), ids, tab);
     if (pm) pm->mark(kPhasePredict, 3, st);
     // Cell order: scene-major because every scene owns a slot range.

@@ -160,6 +160,7 @@ struct StepBuffers {
     // (kNoList: no list).  Null where there was no room: the passes walk then.
     uint2* lists = nullptr;
     uint32_t* listed = nullptr;
+    uint32_t* unlisted = nullptr;  // set where a warp pass of the step had no list for a particle
     int list_cap = 0;
     uint32_t* err;  // device status word
 };
@@ -168,7 +169,10 @@ constexpr int kWalkHist = 16;
 // Room for 512 candidates: fluid at rest has 270 in support at h = 4 r, a
 // compressed one up to about 450.
 constexpr uint32_t kListRows = 256;
-constexpr uint32_t kNoList = 0x7fffffffu;
+constexpr uint32_t kNoList = 0x3fffffffu;
+// In a word of StepBuffers::listed (warp passes): nothing around the particle
+// moved, so this iteration's density pass has nothing to do for it.
+constexpr uint32_t kIdle = 0x40000000u;
 
 // Phases of one step, named after the reference's PerformanceMonitor scopes
 // (pbf_solver.cpp:29-103).  Fused kernels report under the first scope they
