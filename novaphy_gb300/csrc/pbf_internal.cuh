@@ -96,11 +96,12 @@ inline void bind_work(StepBuffers& B, void* mem, int c) {
 }
 
 // Kept lists of c particles (StepBuffers::lists): rows, then their numbers.
-// They take seven times the rest of the step scratch, so no scene or batch of
-// more than kListMaxParticles has any, all of a process's together stay below
-// kListMaxBytes, and they are not needed: without them the passes walk.
-constexpr int kListMaxParticles = 4 << 20;
-constexpr size_t kListMaxBytes = (size_t)16 << 30;
+// They take seven times the rest of the step scratch (2 KB a particle), so no
+// scene or batch of more than kListMaxParticles has any, one's stay below a
+// quarter of the free memory, all of a process's together below kListMaxBytes,
+// and they are not needed: without them the passes walk.
+constexpr int kListMaxParticles = 32 << 20;
+constexpr size_t kListMaxBytes = (size_t)64 << 30;
 
 inline size_t list_bytes(int c) {
     const size_t r = align_up((size_t)c, 32);

@@ -820,7 +820,8 @@ __device__ __forceinline__ T ld_step(const T* p) {
 //
 // Two forms:
 //  * the warp walk (walk_group): a warp has 32 particles, one a lane, and a
-//    lane adds its particle's terms itself.  The cheapest per particle;
+//    lane adds its particle's terms itself.  The cheapest per particle.  Scenes
+//    with kept lists (below) only list this way and sum in readers;
 //  * the team walk (team_walk): four warps share TP = 8 or 16 particles.
 //    The warps list different words, then 128 / TP lanes evaluate each
 //    particle's terms side by side and pass them through shared memory to
@@ -882,7 +883,9 @@ constexpr uint32_t kRunRange = 0x80000000u;
 // 1,603 / -; 3 steps of 395,101 21,180 / 18,450 / 14,790; a million 6,263 /
 // 5,528 / 4,230; 250,000 with bodies 3,642 / 3,133 / 2,995; a batch of 352,901
 // 3,121 / 2,928 / 2,310.
-__device__ __forceinline__ uint32_t list_at(uint32_t p) { return (p >> 5) * (32u * kListRows) + (p & 31u); }
+__device__ __forceinline__ size_t list_at(uint32_t p) {
+    return (size_t)(p >> 5) * (32u * kListRows) + (p & 31u);
+}
 
 // Shared memory of a warp walk.
 struct WalkSmem {
@@ -2365,6 +2368,11 @@ __device__ __forceinline__ void read_lists(const Grid& G, uint32_t p, bool want,
         const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
         if (t + 2u < cnt) load();
         if (t + 4u < cnt) q = __ldcs(from);
+        // Lists come from HBM once they outgrow the L2: four rows ahead the
+        // loads found them there (a density pass of 250,000 waited for them
+        // nine cycles in eleven; 1M step 4,230 -> 3,974 us; 8 and 16 rows
+        // ahead 3,987 and 4,013).
+        if (t + 12u < cnt) asm volatile("prefetch.global.L2 [%0];" ::"l"(from + 128));
         from += 32;
         if (all_zero && !__any_sync(full, t < cnt && (x0.w != 0.0f || x1.w != 0.0f))) continue;
         sums.add2(x0, x1, e0, e1, t < cnt, t + 1u < cnt);
@@ -3403,15 +3411,16 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
 // cell-sorted particles for `max_iters` iterations, with constants from `prm`.
 // Scenes with vorticity take the XSPH+omega / vorticity+commit pair
 // (any_vort), the others XSPH+commit (any_plain).
-// Particles per team of the neighbour passes, 0 for warp walks, by the number
-// of particles of the launch.  A warp walk of one lane per particle needs
-// some 130,000 particles to keep the chip's 608 schedulers in work; below
-// that its time is that of one warp's chain.  Measured (exact build, times of
-// a whole pass of calls, us, teams of 8 / 16 / 32 / warp walks): 1,000
-// particles at h = 2 r 193 / 238 / 341 / 604; 8,000 at 4 r 365 / 368 / 464 /
-// 992; four steps of 43,993 4,609 / 4,565 / 7,289 / 11,318; 65,565 (fast
-// build) 2,237 / 2,002 / 2,607 / 3,684; a batch of 352,901 5,171 / 3,993 /
-// 4,061 / 3,519.  Teams of 32 were never the fastest and are not built.
+// Particles per team of the neighbour passes, 0 for warps with one lane per
+// particle, by the number of particles of the launch.  Warps need some 130,000
+// particles to keep the chip's 608 schedulers in work; below that their time
+// is that of one warp's chain.  Measured when both forms walked in every pass
+// (us a call, teams of 8 / 16 / 32 / warps): 1,000 particles at h = 2 r 193 /
+// 238 / 341 / 604; 8,000 at 4 r 365 / 368 / 464 / 992; four steps of 43,993
+// 4,609 / 4,565 / 7,289 / 11,318; 65,565 (fast build) 2,237 / 2,002 / 2,607 /
+// 3,684; a batch of 352,901 5,171 / 3,993 / 4,061 / 3,519.  With kept lists
+// (teams of 16 / warps): 43,993 3,436 / 11,055, 65,565 1,670 / 3,442.  Teams of
+// 32 were never the fastest and are not built.
 inline int team_size(int n) {
     if (n < 8192) return 8;
     if (n < kBigScene) return 16;

@@ -146,7 +146,7 @@ struct StepBuffers {
     // Per slot: 1 + the Jacobi iteration whose density pass last left a
     // particle of the slot with a nonzero lambda (0: none in this step).
     uint32_t* lamnz;
-    // Per Jacobi iteration (kWalkHist of them): how many cooperative warps
+    // Per Jacobi iteration (kWalkHist of them): how many warps
     // of the density pass had a lane with C_i >= 0, and how many ran, in
     // the previous step ([0, 2 kWalkHist)) and in this one (the rest).
     // Single scenes only (null in batches).
