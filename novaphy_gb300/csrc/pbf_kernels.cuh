@@ -843,7 +843,7 @@ constexpr int kTeamWarps = 4;
 // one-thread walk).
 constexpr int kMaxGroups = 6;
 // Warps with more than this many have no lists (as many as 32 measured the
-// same: 14,808 us against 14,790 for three steps of 395,101).
+// same: 14,808 us against 14,790 for three steps of 394,831).
 constexpr int kMaxListGroups = 16;
 
 // A group's candidate sequence: ranges [start, start + len) in cell order (key
@@ -880,9 +880,9 @@ constexpr uint32_t kRunRange = 0x80000000u;
 // instructions.  Measured (us a call; walking / lists kept by a walking
 // density pass / k_list and readers): 1,000 particles 105 / 96 / -; 8,000 235 /
 // 204 / -; 4 steps of 43,993 3,989 / 3,332 / -; 65,565 (fast build) 1,862 /
-// 1,603 / -; 3 steps of 395,101 21,180 / 18,450 / 14,790; a million 6,263 /
-// 5,528 / 4,230; 250,000 with bodies 3,642 / 3,133 / 2,995; a batch of 352,901
-// 3,121 / 2,928 / 2,310.
+// 1,603 / -; 3 steps of 394,831 21,180 / 18,450 / 14,170; a million 6,263 /
+// 5,528 / 3,974; 250,000 with bodies 3,642 / 3,133 / 2,857; a batch of 352,901
+// 3,121 / 2,928 / 2,187.
 __device__ __forceinline__ size_t list_at(uint32_t p) {
     return (size_t)(p >> 5) * (32u * kListRows) + (p & 31u);
 }
