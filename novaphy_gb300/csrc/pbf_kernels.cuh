@@ -2616,6 +2616,8 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
 // has none; and _listed, for the other warps of scenes with lists.  The readers
 // have neither a walk's registers nor its shared memory, so more warps are in
 // flight and the whole L1 holds candidates.
+// Blocks of a walking launch for the rest: one wave, whose blocks go on to the
+// next warps, so that one with nothing to do costs 3 us at any size.
 constexpr int kRestBlocks = 152 * 6;
 
 // Whether the walking launch `rest` leaves this warp out.
