@@ -1357,6 +1357,8 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             } else {
                 kept = kNoList;
             }
+            // A pile whose lists all overflowed is left to the walk at once.
+            if (!__any_sync(full, want && kept != kNoList)) return;
         } else if (kRuns && runs) {
             for (int t = 0; t < cnt; ++t) {
                 uint32_t q = next_q();
