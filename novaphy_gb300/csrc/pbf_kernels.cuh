@@ -2618,9 +2618,11 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
 // has none; and _listed, for the other warps of scenes with lists.  The readers
 // have neither a walk's registers nor its shared memory, so more warps are in
 // flight and the whole L1 holds candidates.
-// Blocks of a walking launch for the rest: one wave, whose blocks go on to the
-// next warps, so that one with nothing to do costs 3 us at any size.
-constexpr int kRestBlocks = 152 * 6;
+// Blocks of a walking launch for the rest, whose blocks go on to the next warps:
+// four waves, so that one with nothing to do costs 5 us at any size and piles
+// spread over the chip (ten steps of the 1M dam break into its corners: 4.74 M
+// particle-steps/s, 4.21 M with one wave, which saved 25 us of a 1M step).
+constexpr int kRestBlocks = 152 * 24;
 
 // Whether the walking launch `rest` leaves this warp out.
 __device__ __forceinline__ bool leave_out(int rest, const Grid& G, uint32_t p, bool want) {
