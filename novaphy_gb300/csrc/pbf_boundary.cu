@@ -114,27 +114,47 @@ k_bxform(const float4* __restrict__ local, const int* __restrict__ body, int nb,
 // against the boundary's, and the other way round), so that a team's 8 or 16
 // queries sit in one cell or two; with one thread per query a few thousand
 // boundary points left most of the chip idle for 600 us.
+//
+// As in the reference, a distance that is not a number is not outside the
+// support, and a factor that is not finite spoils a sum through the zero
+// kernel value of a candidate anywhere in the buckets: such candidates are
+// listed wherever they are (kSpecials, special), and every candidate of such
+// a query.
+
+__device__ __forceinline__ bool finite3(const float4& x) {
+    return isfinite(x.x) && isfinite(x.y) && isfinite(x.z);
+}
+
+// a, or not a number where r^2 is none.
+__device__ __forceinline__ float2 nan_of(float2 r2, float2 a) {
+    return make_float2(isnan(r2.x) ? r2.x : a.x, isnan(r2.y) ? r2.y : a.y);
+}
 
 // Density of the boundary at a fluid point: sum_b rho0 psi_b W.
 struct PsiDensityTerm {
     static constexpr int kQuantities = 1, kFactors = 1;
     static constexpr bool kExtra = false;
+    static constexpr bool kSpecials = true;
     const StepConsts& C;
     const float4 xi;
     static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    static __device__ __forceinline__ bool special(const float4& b, const StepConsts& C) {
+        return !finite3(b) || !isfinite(C.rho0 * b.w);
+    }
     __device__ __forceinline__ bool eval(const float4& b, const float4&, float* v, float* f) const {
         const float r_sq = sqn(xi.x - b.x, xi.y - b.y, xi.z - b.z);
-        if (!(r_sq < C.h2)) return false;
-        v[0] = poly6(r_sq, C);
         f[0] = C.rho0 * b.w;
+        if (r_sq >= C.h2 && isfinite(f[0])) return false;
+        v[0] = poly6(r_sq, C);
         return true;
     }
     __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&, const float4&,
                                              float2* v, bool& in_a, bool& in_b) const {
         const PairRel r(xi, xa, xb, C.one);
-        in_a = r.r2.x < C.h2;
-        in_b = r.r2.y < C.h2;
-        v[0] = mul2(mul2(both(C.rho0), make_float2(xa.w, xb.w)), poly6_2(r.r2, C));
+        const float2 f = mul2(both(C.rho0), make_float2(xa.w, xb.w));
+        in_a = !(r.r2.x >= C.h2) || !isfinite(f.x);
+        in_b = !(r.r2.y >= C.h2) || !isfinite(f.y);
+        v[0] = mul2(f, nan_of(r.r2, poly6_2(r.r2, C)));
     }
 };
 
@@ -143,13 +163,15 @@ struct PsiDensityTerm {
 struct PressureTerm {
     static constexpr int kQuantities = 3, kFactors = 1;
     static constexpr bool kExtra = false;
+    static constexpr bool kSpecials = true;
     const StepConsts& C;
     const float4 xi;
     static __host__ __device__ constexpr int factor_of(int) { return 0; }
+    static __device__ __forceinline__ bool special(const float4& xf, const StepConsts&) { return !finite3(xf); }
     __device__ __forceinline__ bool eval(const float4& xf, const float4&, float* v, float* f) const {
         const float rx = xi.x - xf.x, ry = xi.y - xf.y, rz = xi.z - xf.z;
         const float r_sq = sqn(rx, ry, rz);
-        if (!(r_sq < C.h2)) return false;
+        if (r_sq >= C.h2) return false;
         const float c = spiky_coeff(r_sq, C);
         f[0] = xf.w * xi.w;
         v[0] = c * rx;
@@ -160,9 +182,9 @@ struct PressureTerm {
     __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&, const float4&,
                                              float2* v, bool& in_a, bool& in_b) const {
         const PairRel r(xi, xa, xb, C.one);
-        in_a = r.r2.x < C.h2;
-        in_b = r.r2.y < C.h2;
-        const float2 c = spiky_coeff_2(r.r2, C);
+        in_a = !(r.r2.x >= C.h2);
+        in_b = !(r.r2.y >= C.h2);
+        const float2 c = nan_of(r.r2, spiky_coeff_2(r.r2, C));
         const float2 a = mul2(make_float2(xa.w, xb.w), both(xi.w));
         v[0] = mul2(a, mul2(c, r.x));
         v[1] = mul2(a, mul2(c, r.y));
@@ -174,12 +196,14 @@ struct PressureTerm {
 struct VolumeTerm {
     static constexpr int kQuantities = 1, kFactors = 1;
     static constexpr bool kExtra = false;
+    static constexpr bool kSpecials = true;
     const StepConsts& C;
     const float4 xi;
     static __host__ __device__ constexpr int factor_of(int) { return -1; }
+    static __device__ __forceinline__ bool special(const float4& b, const StepConsts&) { return !finite3(b); }
     __device__ __forceinline__ bool eval(const float4& b, const float4&, float* v, float* f) const {
         const float r_sq = sqn(xi.x - b.x, xi.y - b.y, xi.z - b.z);
-        if (!(r_sq < C.h2)) return false;
+        if (r_sq >= C.h2) return false;
         v[0] = poly6(r_sq, C);
         f[0] = 1.0f;
         return true;
@@ -187,15 +211,16 @@ struct VolumeTerm {
     __device__ __forceinline__ void products(const float4& xa, const float4& xb, const float4&, const float4&,
                                              float2* v, bool& in_a, bool& in_b) const {
         const PairRel r(xi, xa, xb, C.one);
-        in_a = r.r2.x < C.h2;
-        in_b = r.r2.y < C.h2;
-        v[0] = poly6_2(r.r2, C);
+        in_a = !(r.r2.x >= C.h2);
+        in_b = !(r.r2.y >= C.h2);
+        v[0] = nan_of(r.r2, poly6_2(r.r2, C));
     }
 };
 
 // pc rho0 of a fluid particle of density rho, as the reference's force loop
 // computes it for each pair (fluid_world.cpp:147-155): zero where the fluid is
-// not compressed, so such a particle adds exact zeros and is not listed.
+// not compressed, so such a particle adds exact zeros (where psi and the
+// distance are finite) and is not listed.
 __device__ __forceinline__ float pressure_weight(float rho, const StepConsts& C) {
     const float rho_f = (rho < 1.0f) ? 1.0f : rho;   // std::max(rho, 1.0f)
     const float pd = rho_f - C.rho0;
@@ -250,7 +275,7 @@ k_coupling(const float4* __restrict__ bpos, const uint32_t* __restrict__ bidx, c
     };
     const float4 xi = bpos[T.pe];
     float4 xl = bpos[T.pl];
-    xl.w = 0.0f;  // lists candidates with a nonzero weight only
+    xl.w = isfinite(xl.w) ? 0.0f : 1.0f;  // 0: lists candidates with a nonzero weight only
     TeamSums<PressureTerm, 128 / TP> sums(PressureTerm{C, xi});
     team_walk<TP, true>(sm, G, G.ix, OneScene{C, StateRef{}}, T.pl, query_cell(Q, T.pl), T.al && feels(T.pl), xl,
                         I.spos, sums);

@@ -1400,6 +1400,14 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
 // values and factors of one candidate and whether it is in support; and in the
 // exact build products, the products of two candidates at once.
 //
+// Terms whose candidates may have to be evaluated wherever they are (the
+// coupling's, for values that are not finite) set kSpecials and say which:
+// special(x_j).
+template <class D, class = void>
+struct HasSpecials : std::false_type {};
+template <class D>
+struct HasSpecials<D, std::void_t<decltype(D::kSpecials)>> : std::integral_constant<bool, D::kSpecials> {};
+
 // No sums (a walk that only lists).
 struct NoSums {
     static constexpr bool kExtra = false;
@@ -1481,6 +1489,8 @@ struct TeamSums {
     static constexpr int kPairs = (kNq + 1) / 2;
     static constexpr int kRow = 66;
     static constexpr bool kExtra = D::kExtra;
+    static constexpr bool kSpecials = HasSpecials<D>::value;
+    using Term = D;
     static_assert(kPairs <= S, "a lane per pair of quantities");
     float2 sum;
     const D d;
@@ -1606,7 +1616,9 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
     bool runs;
     const int words = walk_ranges<false>(sm.ranges, Gr, I, Gd, G, wid == 0, runs);
     __syncwarp();
-    const bool lam_zero = kLam && xi.w == 0.0f;
+    // A particle all of whose candidates are special.
+    const bool every = Sums::kSpecials && !(isfinite(xi.x) && isfinite(xi.y) && isfinite(xi.z));
+    const bool lam_zero = kLam && xi.w == 0.0f && !every;
     const bool all_zero = kLam && !__any_sync(full, want && xi.w != 0.0f);
     uint32_t run = 0u;  // terms of particle pl listed so far
 
@@ -1672,7 +1684,7 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
 #pragma unroll
             for (int i = 0; i < WPL; ++i) m[i] = 0u;
             if (b < nw) {
-                uint32_t sel[4], nz[4];
+                uint32_t sel[4], nz[4], sp[4];  // words, those with a nonzero w, special ones
                 uint32_t any_nz = 0u;
                 float4 xj[4];
 #pragma unroll
@@ -1689,6 +1701,8 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
                         nz[j] = __ballot_sync(full, xj[j].w != 0.0f);
                         any_nz |= nz[j];
                     }
+                    if constexpr (Sums::kSpecials)
+                        sp[j] = __ballot_sync(full, Sums::Term::special(xj[j], sums.d.C));
                 }
                 const bool test = !B.wide && (!kLam || !all_zero || any_nz != 0u);
                 if (test) {
@@ -1706,15 +1720,16 @@ __device__ __forceinline__ void team_group(TeamSmem<TP>& sm, const WalkGroup& Gr
 #pragma unroll
                 for (int i = 0; i < WPL; ++i) {
                     const int j = j0 + i;
-                    uint32_t in = 0u, innz = 0u;
+                    uint32_t in = 0u, innz = 0u, insp = 0u;
 #pragma unroll
                     for (int c = 0; c < 4; ++c) {
                         if (c == j) in = sel[c];
                         if (kLam && c == j) innz = nz[c];
+                        if (Sums::kSpecials && c == j) insp = sp[c];
                     }
-                    uint32_t v = B.wide ? 0xffffffffu : (test ? sm.mask[wid][j * TP + pl] : 0u);
-                    v &= in;
+                    uint32_t v = B.wide || every ? 0xffffffffu : (test ? sm.mask[wid][j * TP + pl] : 0u);
                     if (kLam && lam_zero) v &= innz;
+                    v = (v | insp) & in;
                     if (!want) v = 0u;
                     if (multi) {
                         const int w = b + j;
