@@ -427,7 +427,7 @@ int ensure_offsets(pbf_scene* s, uint32_t nslots) {
     const size_t ob = align_up((size_t)(nslots + 1) * 4, 256);
     const size_t ab = align_up(nslots + 1, 256);
     int rc = pool_alloc(reinterpret_cast<void**>(&s->off),
-                        ob + ab + (size_t)(nslots + 1) * 8 + 4 * kWalkHist * 4, s->device, s->stream);
+                        ob + ab + (size_t)(nslots + 1) * 8 + kWalkHistWords * 4, s->device, s->stream);
     if (rc) return rc;
     s->off_cap = nslots + 1;
     s->B.off = s->off;
@@ -436,7 +436,7 @@ int ensure_offsets(pbf_scene* s, uint32_t nslots) {
     s->B.lamnz = s->B.moved + (nslots + 1);
     s->B.dhist = s->B.lamnz + (nslots + 1);
     s->B.slot_bytes = ab + (size_t)(nslots + 1) * 8;
-    PBF_CUDA(cudaMemsetAsync(s->B.dhist, 0, 4 * kWalkHist * 4, s->stream));
+    PBF_CUDA(cudaMemsetAsync(s->B.dhist, 0, kWalkHistWords * 4, s->stream));
     return PBF_OK;
 }
 
@@ -983,7 +983,7 @@ size_t scene_device_bytes(const pbf_scene* s) {
     if (s->lmem) b += list_bytes(s->B.list_cap);
     if (s->off)
         b += align_up((size_t)s->off_cap * 4, 256) + align_up(s->off_cap, 256) +
-             (size_t)s->off_cap * 8 + 4 * kWalkHist * 4;
+             (size_t)s->off_cap * 8 + kWalkHistWords * 4;
     return b;
 }
 

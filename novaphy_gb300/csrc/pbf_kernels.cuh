@@ -112,8 +112,23 @@ __device__ __forceinline__ float spiky_coeff(float r_sq, const StepConsts& C) {
 
 // Adding a term to a running sum m times in a row (a run of identical
 // candidates): the float that m single additions of t leave, bit for bit.  A
-// call: inlined, its loop cost the neighbour passes' hot loops registers.
+// call for long runs: inlined, its loop cost the neighbour passes' hot loops
+// registers.
+constexpr uint32_t kAddSingly = 12;
 __device__ __noinline__ float rep_add_call(float s, float t, uint32_t m) { return rep_add(s, t, m); }
+template <int K>
+__device__ __forceinline__ void add_times(float (&s)[K], const float (&t)[K], uint32_t m) {
+    if (m > kAddSingly) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) s[k] = rep_add_call(s[k], t[k], m);
+        return;
+    }
+#pragma unroll 1
+    for (; m; --m) {
+#pragma unroll
+        for (int k = 0; k < K; ++k) s[k] = s[k] + t[k];
+    }
+}
 
 // ---------------------------------------------------------------------------
 // Grid helpers
@@ -265,10 +280,11 @@ k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, uint32_
               int n, const SortCounts counts, const SceneIds S, const P prm) {
     __shared__ BlockCounts B;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
-    static_assert(2 * kWalkHist <= kCountThreads, "one thread per count");
-    if (dhist && t < 2 * kWalkHist) {
-        dhist[t] = dhist[t + 2 * kWalkHist];
-        dhist[t + 2 * kWalkHist] = 0u;
+    static_assert(4 * kWalkHist <= kCountThreads, "one thread per count");
+    if (dhist && t < 4 * kWalkHist) {
+        uint32_t* const d = dhist + (t / (2 * kWalkHist)) * 4 * kWalkHist + t % (2 * kWalkHist);
+        d[0] = d[2 * kWalkHist];
+        d[2 * kWalkHist] = 0u;
     }
     if (unlisted && t == 0) *unlisted = 0u;
     B.begin(counts);
@@ -893,14 +909,15 @@ struct WalkSmem {
     // One fp16 row of eight per candidate: x, y, z, |u|^2 (high, low), 1, 1, 0.
     alignas(16) uint32_t stage[128 * 4];
     uint32_t base[kWalkWords];  // first candidate (cell order, or key order in buckets)
-    uint32_t info[kWalkWords];  // candidates | row << 8 | kLastLeads
+    uint32_t info[kWalkWords];  // candidates | row << 8
     uint32_t mask[kWalkWords * 32];
     // The mask of word w and particle p.  The exclusive-or spreads the four
     // words that a store instruction touches over the banks.
     static __device__ __forceinline__ int at(int w, int p) { return w * 32 + (p ^ ((w & 3) << 3)); }
+    // The candidates of word w that a run's first particle counts
+    // (k_segments), until its masks are there.
+    __device__ __forceinline__ uint32_t& skip(int w) { return mask[at(w, 0)]; }
 };
-// In WalkSmem::info: the word's last candidate leads a run (k_segments).
-constexpr uint32_t kLastLeads = 1u << 16;
 
 // Shared memory of a team walk.  During an evaluation the stage holds the
 // terms on their way to the adding lanes, one row of float2 (two quantities)
@@ -1178,7 +1195,11 @@ __device__ __forceinline__ uint32_t own_cells(const WalkIndex& I, uint32_t slot,
 // started at +0, never are -0, so a lane whose lambda is zero lists
 // candidates with a nonzero one only.  kRuns: in ranges that hold runs of
 // identical particles (k_segments) a run is listed as its first particle,
-// whose term is added as many times as the run is long.  kList: nothing is
+// whose term is added as many times as the run is long (a step of the 1M dam
+// break with a corner cell of 44,000 particles in 27,000 runs takes 213 ms;
+// 434 when a word ended with each run, 255 in the one-thread walks before that,
+// 265 with the runs' particles listed one by one, which costs later steps
+// three times as much).  kList: nothing is
 // summed; the lane's candidates go to the kept list of its particle p, whose
 // rows so far are `kept`.
 template <bool kPersist, bool kLam, bool kRuns, bool kList, class Sums>
@@ -1202,13 +1223,14 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
     }
     const bool key = Gr.own != 0u;
     const bool multi = Gr.W > 3;
-    bool runs;
-    const int total = walk_ranges<kRuns>(sm.ranges, Gr, I, Gd, G, true, runs);
+    bool in_runs;
+    const int total = walk_ranges<kRuns>(sm.ranges, Gr, I, Gd, G, true, in_runs);
     __syncwarp();
-    if (kList && runs) {  // a row has no way to say how often its term counts
+    if (kList && in_runs) {  // a row has no way to say how often its term counts
         if (want) kept = kNoList;
         return;
     }
+    const bool runs = kRuns && !kList && in_runs;
     // Position of the listing with runs: range and candidate.
     int at_r = 0;
     uint32_t at_q = 0u;
@@ -1231,29 +1253,37 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
                 at_q = 0u;
                 continue;
             }
-            uint32_t cnt = min(32u, len_r - at_q), lead = 0u, step = cnt;
-            if (ln & kRunRange) {
-                // A range with runs: the word ends with a run's first
-                // particle, and the next one begins past the run.
-                const uint32_t q = st + at_q + (uint32_t)lane;
-                const bool ok = (uint32_t)lane < cnt;
-                const bool first = ok && ((uint32_t)__ldg(G.sown + q) & kLeadBit);
-                const uint32_t m = __ballot_sync(full, first);
-                if (m) {
-                    const int f = __ffs(m) - 1;
-                    uint32_t len = 0u;
-                    if (lane == f) len = __ldg(G.segend + q) - q;
-                    cnt = (uint32_t)f + 1u;
-                    step = (uint32_t)f + __shfl_sync(full, len, f);
-                    lead = kLastLeads;
+            // A word of up to 32 candidates without those to skip; the next one
+            // begins at `next`.
+            auto word = [&](uint32_t skip, uint32_t next) {
+                if (lane == 0) {
+                    sm.base[nw] = st + at_q;
+                    sm.info[nw] = min(32u, len_r - at_q) | ((uint32_t)at_r << 8);
+                    sm.skip(nw) = skip;
                 }
+                ++nw;
+                at_q = next;
+            };
+            if (!(ln & kRunRange)) {
+                word(0u, at_q + 32u);
+                continue;
             }
-            if (lane == 0) {
-                sm.base[nw] = st + at_q;
-                sm.info[nw] = cnt | ((uint32_t)at_r << 8) | lead;
+            // A range with runs: a word starts past the runs of the words before
+            // it.  The flags of four words at a time, so that their loads overlap.
+            const uint32_t q0 = at_q;
+            uint32_t end[4], copy[4];
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                const uint32_t o = q0 + 32u * (uint32_t)j + (uint32_t)lane;
+                end[j] = o < len_r ? __ldg(G.segend + st + o) : 0u;
+                copy[j] = o < len_r ? (uint32_t)__ldg(G.sown + st + o) & kCopyBit : 0u;
             }
-            ++nw;
-            at_q += step;
+#pragma unroll
+            for (int j = 0; j < 4; ++j) {
+                if (nw >= kWalkWords || at_q != q0 + 32u * (uint32_t)j || at_q >= len_r) break;
+                const uint32_t far = __reduce_max_sync(full, end[j]);
+                word(__ballot_sync(full, copy[j] != 0u), max(at_q + 32u, far > st ? far - st : 0u));
+            }
         }
         return nw;
     };
@@ -1275,6 +1305,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             for (int j = 0; j < 4; ++j) {
                 const uint32_t n = b + j < nw ? sm.info[b + j] & 63u : 0u;
                 sel[j] = bit_range(0u, n);
+                if (kRuns && runs && b + j < nw) sel[j] &= ~sm.skip(b + j);
                 xj[j] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
                 if ((uint32_t)lane < n) {
                     uint32_t q = sm.base[b + j] + (uint32_t)lane;
@@ -1360,15 +1391,26 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             // A pile whose lists all overflowed is left to the walk at once.
             if (!__any_sync(full, want && kept != kNoList)) return;
         } else if (kRuns && runs) {
-            for (int t = 0; t < cnt; ++t) {
-                uint32_t q = next_q();
-                const uint32_t i = sm.info[w];
-                const bool lead = (i & kLastLeads) && q - bq == (i & 63u) - 1u;
+            float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
+            uint32_t la = 0u, lb = 0u;  // ends of the runs they lead, 0 without one
+            uint32_t qa = 0u, qb = 0u;
+            auto load = [&](uint32_t& q, float4& x, float4& e, uint32_t& end) {
+                q = next_q();
                 if (key) q = I.at(q);
-                float4 e{};
+                end = __ldg(G.segend + q);
+                x = ld_step<kPersist>(xin + q);
                 if constexpr (Sums::kExtra) e = sums.extra(q);
-                if (lead) sums.add_run(ld_step<kPersist>(xin + q), e, __ldg(G.segend + q) - q);
-                else sums.add(ld_step<kPersist>(xin + q), e);
+            };
+            if (cnt > 0) load(qa, xa, ea, la);
+            if (cnt > 1) load(qb, xb, eb, lb);
+            for (int t = 0; t < most; t += 2) {
+                const float4 x0 = xa, x1 = xb, e0 = ea, e1 = eb;
+                const uint32_t n0 = t < cnt ? (la ? la - qa : 1u) : 0u;
+                const uint32_t n1 = t + 1 < cnt ? (lb ? lb - qb : 1u) : 0u;
+                if (t + 2 < cnt) load(qa, xa, ea, la);
+                if (t + 3 < cnt) load(qb, xb, eb, lb);
+                if (__any_sync(full, n0 > 1u || n1 > 1u)) sums.add2_times(x0, x1, e0, e1, n0, n1);
+                else sums.add2(x0, x1, e0, e1, n0 != 0u, n1 != 0u);
             }
         } else {
             float4 xa = make_float4(0.0f, 0.0f, 0.0f, 0.0f), xb = xa, ea = xa, eb = xa;
@@ -1446,12 +1488,32 @@ struct LaneSums {
         if (d.eval(xj, ej, v, f)) {
 #pragma unroll
             for (int k = 0; k < kNq; ++k)
-                sum[k] = rep_add_call(sum[k],
-                                      D::factor_of(k) < 0
-                                          ? v[k]
-                                          : f[D::factor_of(k) < 0 ? 0 : D::factor_of(k)] * v[k],
-                                      L);
+                if (D::factor_of(k) >= 0) v[k] = f[D::factor_of(k) < 0 ? 0 : D::factor_of(k)] * v[k];
+            add_times(sum, v, L);
         }
+    }
+    // The terms of two candidates, the first one na times, then the other nb
+    // times.
+    __device__ __forceinline__ void add2_times(const float4& xa, const float4& xb, const float4& ea,
+                                               const float4& eb, uint32_t na, uint32_t nb) {
+#if !PBF_FAST
+        if (d.C.paired) {
+            float2 v[kNq];
+            bool in_a, in_b;
+            d.products(xa, xb, ea, eb, v, in_a, in_b);
+            float a[kNq], b[kNq];
+#pragma unroll
+            for (int k = 0; k < kNq; ++k) {
+                a[k] = v[k].x;
+                b[k] = v[k].y;
+            }
+            add_times(sum, a, in_a ? na : 0u);
+            add_times(sum, b, in_b ? nb : 0u);
+            return;
+        }
+#endif
+        if (na) add_run(xa, ea, na);
+        if (nb) add_run(xb, eb, nb);
     }
     // The terms of two candidates, the first one first, where they are there.
     __device__ __forceinline__ void add2(const float4& xa, const float4& xb, const float4& ea,
@@ -2573,11 +2635,15 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
     // terms in the same order as the single walk: same bits.  It pays where
     // most warps have no such lane; which way a warp goes follows the share
     // of warps that needed gradients in the same iteration of the last step.
+    // Where there are lists, the warps that walk (in piles, or scattered) are
+    // not like the others and follow their own share: with one share for all, a
+    // corner pile of the 1M dam break walked twice (58 ms a pass instead of 25).
     constexpr bool kHist = std::is_same<P, OneScene>::value;
+    uint32_t* const hist = G.dhist && kMode == kWalk && G.lists ? G.dhist + 4 * kWalkHist : G.dhist;
     bool dfirst = false;
     if constexpr (kHist) {
-        if (G.dhist && it < kWalkHist && !G.bg.spos) {
-            const uint32_t need = __ldg(G.dhist + it), ran = __ldg(G.dhist + kWalkHist + it);
+        if (hist && it < kWalkHist && !G.bg.spos) {
+            const uint32_t need = __ldg(hist + it), ran = __ldg(hist + kWalkHist + it);
             dfirst = ran > 0 && 3u * need < ran;
         }
     }
@@ -2617,11 +2683,11 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
     }
     const float Ci = density * C.inv_rho0 - 1.0f;
     if constexpr (kHist) {
-        if (G.dhist && it < kWalkHist) {
+        if (hist && it < kWalkHist) {
             const bool need = __any_sync(0xffffffffu, live && !(Ci < 0.0f));
             if ((threadIdx.x & 31) == 0) {
-                atomicAdd(G.dhist + 3 * kWalkHist + it, 1u);
-                if (need) atomicAdd(G.dhist + 2 * kWalkHist + it, 1u);
+                atomicAdd(hist + 3 * kWalkHist + it, 1u);
+                if (need) atomicAdd(hist + 2 * kWalkHist + it, 1u);
             }
         }
     }

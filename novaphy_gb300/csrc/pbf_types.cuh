@@ -148,7 +148,8 @@ struct StepBuffers {
     uint32_t* lamnz;
     // Per Jacobi iteration (kWalkHist of them): how many warps
     // of the density pass had a lane with C_i >= 0, and how many ran, in
-    // the previous step ([0, 2 kWalkHist)) and in this one (the rest).
+    // the previous step ([0, 2 kWalkHist)) and in this one (the next 2
+    // kWalkHist); then the same of the warps that walk where there are lists.
     // Single scenes only (null in batches).
     uint32_t* dhist;
     // Per sorted position: for the first particle of a run of particles with
@@ -166,6 +167,7 @@ struct StepBuffers {
 };
 
 constexpr int kWalkHist = 16;
+constexpr int kWalkHistWords = 8 * kWalkHist;
 // Room for 512 candidates: fluid at rest has 270 in support at h = 4 r, a
 // compressed one up to about 450.
 constexpr uint32_t kListRows = 256;

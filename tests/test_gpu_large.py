@@ -140,3 +140,47 @@ def test_runs_with_default_scorr(port_mt):
     w = clump_block(2400, seed=10)
     got, want = run_both(port_mt, w, 2, corr_k=0.001, corr_delta_q=0.3)
     assert_equal(got, want, "runs default s_corr")
+
+
+def pile_block(n, lengths, seed, same):
+    """A lattice of 2^18 and more particles and, in one cell of the upper half of its box, n particles: runs of
+    bit-identical ones of the given lengths in turn (same), or all different, in random places of the order."""
+    w = workloads.dam_break((64, 64, 64), 0.02, (3.0, 3.0, 3.0), jitter=1e-4, seed=seed, vorticity=1e-4)
+    rng = np.random.default_rng(seed)
+    h = w.settings["kernel_radius"]
+    at = (2.0 + h * 0.3 + 0.3 * h * rng.random((n, 3))).astype(np.float32)
+    if same:
+        k = 0
+        while k < n:
+            m = min(int(lengths[rng.integers(len(lengths))]), n - k)
+            at[k:k + m] = at[k]
+            k += m
+    w.x = np.concatenate([w.x, at]).astype(np.float32)
+    w.v = np.zeros_like(w.x)
+    return w
+
+
+@pytest.mark.parametrize("lengths", [(1, 2, 3, 5), (1, 31, 33, 63, 64, 65, 97, 200)])
+def test_runs_of_every_length(port_mt, lengths):
+    """Runs too short to be taken as one candidate between longer ones and single particles, in a cell of more
+    candidates than a list holds: the oracle's bits after one and two steps."""
+    for nsteps in (1, 2):
+        w = pile_block(5000, lengths, 21, True)
+        assert_equal(*run_both(port_mt, w, nsteps), ("lengths", lengths, nsteps))
+
+
+def test_a_pile_of_short_runs_costs_no_more_than_one_of_different_particles():
+    """A cell of 20,000 particles, many of them bit-identical in twos to eights, against the same cell with
+    all particles different: the identical ones save work and may not cost any (they cost 2.5 times as much when each
+    run was taken as a candidate of its own)."""
+    ms = []
+    for same in (True, False):
+        w = pile_block(20000, (1, 2, 2, 3, 5, 8), 23, same)
+        sc = capi.Scene(capi.default_settings(**w.settings), w.x, w.v, mass=w.mass)
+        sc.set_gravity(w.gravity)
+        seed = sc.snapshot()
+        sc.replay_timed(seed, w.dt, 1)
+        ms.append(min(sc.replay_timed(seed, w.dt, 1) for _ in range(3)))
+        seed.close()
+        sc.close()
+    assert ms[0] < 1.2 * ms[1], ms
