@@ -345,6 +345,17 @@ int pbf_batch_sync(pbf_batch* batch);
  * the batch).  nscenes must equal the last call's. */
 int pbf_batch_nonfinite(pbf_batch* batch, int nscenes, int* out);
 
+/* Steps keep lists of each particle's neighbours from one pass for the next
+ * where there is room: 2 KB a particle for a scene that steps itself or a batch
+ * of up to 32 million particles, at most a quarter of the device's free memory
+ * and 64 GiB of it in all.  They give way to any other allocation of the
+ * library that would fail.  on == 0: this scene or batch keeps none and frees
+ * those it has.  On by default; the exact build's results are identical either
+ * way.  Without them a step of a million particles takes 6.5 ms instead of 4.0,
+ * one of 44,000 0.73 instead of 0.60. */
+int pbf_scene_set_kept_lists(pbf_scene* scene, int on);
+int pbf_batch_set_kept_lists(pbf_batch* batch, int on);
+
 /* Device bytes held: by a batch's scratch, and by a scene's resident state
  * plus whatever scratch its own steps have allocated. */
 int pbf_batch_device_bytes(const pbf_batch* batch, size_t* out);

@@ -135,6 +135,8 @@ def load() -> C.CDLL:
         "pbf_batch_nonfinite": ([vp, C.c_int, vp], C.c_int),
         "pbf_batch_set_persistent": ([vp, C.c_int], C.c_int),
         "pbf_batch_set_autotune": ([vp, C.c_int], C.c_int),
+        "pbf_batch_set_kept_lists": ([vp, C.c_int], C.c_int),
+        "pbf_scene_set_kept_lists": ([vp, C.c_int], C.c_int),
         "pbf_batch_tuning": ([vp, vp, vp], C.c_int),
         "pbf_server_default_config": ([vp], C.c_int),
         "pbf_server_create": ([C.c_int, vp, vp], C.c_int),
@@ -253,6 +255,9 @@ class Scene:
 
     def set_mass(self, m: float):
         check(self._L.pbf_scene_set_mass(self._h, m))
+
+    def set_kept_lists(self, on: bool = True):
+        check(self._L.pbf_scene_set_kept_lists(self._h, 1 if on else 0))
 
     def reset(self, x, v=None):
         x = _f32(x, (-1, 3))
@@ -544,6 +549,9 @@ class Batch:
 
     def set_autotune(self, on: bool = True):
         check(self._L.pbf_batch_set_autotune(self._h, 1 if on else 0))
+
+    def set_kept_lists(self, on: bool = True):
+        check(self._L.pbf_batch_set_kept_lists(self._h, 1 if on else 0))
 
     def tuning(self) -> tuple[int, int]:
         blk, per = C.c_int(0), C.c_int(0)

@@ -18,6 +18,7 @@
 #include <map>
 #include <memory>
 #include <mutex>
+#include <optional>
 #include <sstream>
 #include <string>
 #include <vector>
@@ -94,8 +95,8 @@ struct pbf_batch {
     void* smem = nullptr;  // sort scratch
     void* xmem = nullptr;  // scene ids
     void* lmem = nullptr;  // kept lists (list_bytes(B.list_cap); null: none)
-    int lists_tried = 0;   // the capacity they were last tried for
-    bool lists_off = false;  // a server's batch: its scratch is what batch_reserve took
+    ListRefusal list_refusal;
+    bool lists_off = false;  // off, or a server's batch: its scratch is what batch_reserve took
     StepBuffers B{};
     SortScratch sort{};
     uint32_t* status = nullptr;  // status word of the batch's steps
@@ -172,18 +173,18 @@ int ensure_particles(pbf_batch* b, int n) {
     // on every step.
     const int c = std::max(n + n / 4, 1024);
     const size_t wb = work_bytes(c);
-    PBF_CUDA(cudaMalloc(&b->wmem, wb));
+    PBF_CUDA(device_malloc(&b->wmem, wb, b->device, b));
     PBF_CUDA(cudaMemsetAsync(b->wmem, 0, wb, b->stream));
     bind_work(b->B, b->wmem, c);
     const size_t sb = sort_scratch_bytes(c);
-    PBF_CUDA(cudaMalloc(&b->smem, sb));
+    PBF_CUDA(device_malloc(&b->smem, sb, b->device, b));
     PBF_CUDA(cudaMemsetAsync(b->smem, 0, sb, b->stream));
     sort_scratch_bind(b->sort, b->smem, c);
     if (!b->status) b->status = take_status_word();
     if (b->status) b->sort.err = b->status;
     b->B.err = b->sort.err;
     const size_t xb = extra_bytes(c);
-    PBF_CUDA(cudaMalloc(&b->xmem, xb));
+    PBF_CUDA(device_malloc(&b->xmem, xb, b->device, b));
     char* p = reinterpret_cast<char*>(b->xmem);
     const size_t f1 = align_up((size_t)c * 4, 256);
     b->pid = reinterpret_cast<uint32_t*>(p);
@@ -193,28 +194,34 @@ int ensure_particles(pbf_batch* b, int n) {
 }
 
 void free_lists(pbf_batch* b) {
-    if (!b->lmem) return;
-    cudaFree(b->lmem);
-    give_list_bytes(list_bytes(b->B.list_cap));
+    if (b->lmem) give_lists(b->lmem, list_bytes(b->B.list_cap), b->device, b->stream);
     b->lmem = nullptr;
     bind_lists(b->B, nullptr, 0);
 }
 
-// Kept lists for steps of n particles, tried once per size.
-void ensure_lists(pbf_batch* b, int n) {
-    if (b->lists_off || n <= b->B.list_cap || n <= b->lists_tried) return;
+bool drop_lists(void* self) {
+    pbf_batch* const b = static_cast<pbf_batch*>(self);
+    if (!b->lmem) return false;
+    cudaStreamSynchronize(b->stream);
     drop_graph(b);
     free_lists(b);
-    const int c = std::min(b->cap, n + n / 4);
-    b->lists_tried = c;
-    const size_t lb = list_bytes(c);
-    if (c > kListMaxParticles || !take_list_bytes(lb)) return;
-    void* p = nullptr;
-    if (cudaMalloc(&p, lb) != cudaSuccess) {
-        cudaGetLastError();
-        give_list_bytes(lb);
+    cudaStreamSynchronize(b->stream);
+    b->list_refusal.set();
+    return true;
+}
+
+// Kept lists for steps of n particles; those of a smaller size stay until the
+// larger ones are there.
+void ensure_lists(pbf_batch* b, int n) {
+    if (b->lists_off || n <= b->B.list_cap || n > kListMaxParticles || b->list_refusal.stands()) return;
+    const int c = std::min({b->cap, n + n / 4, kListMaxParticles});
+    void* const p = take_lists(list_bytes(c), b->device, b->stream);
+    if (!p) {
+        b->list_refusal.set();
         return;
     }
+    drop_graph(b);
+    free_lists(b);
     b->lmem = p;
     bind_lists(b->B, p, c);
 }
@@ -228,7 +235,7 @@ int ensure_slots(pbf_batch* b, uint32_t nslots) {
     const uint32_t c = nslots + nslots / 4 + 1;
     const size_t ob = align_up((size_t)(c + 1) * 4, 256);
     const size_t ab = align_up(c + 1, 256);
-    PBF_CUDA(cudaMalloc(&b->off, ob + ab + (size_t)(c + 1) * 8));
+    PBF_CUDA(device_malloc(&b->off, ob + ab + (size_t)(c + 1) * 8, b->device, b));
     b->off_cap = c + 1;
     b->B.off = b->off;
     b->B.slot_alias = reinterpret_cast<unsigned char*>(b->off) + ob;
@@ -262,7 +269,7 @@ int ensure_tables(pbf_batch* b, int nscenes) {
     b->tab_refs_at = align_up((size_t)c * sizeof(StepConsts), 256);
     b->tab_firsts_at = b->tab_refs_at + align_up((size_t)c * sizeof(StateRef), 256);
     b->tab_bytes = b->tab_firsts_at + align_up((size_t)(c + 1) * 4, 256);
-    PBF_CUDA(cudaMalloc(&b->tmem, b->tab_bytes));
+    PBF_CUDA(device_malloc(&b->tmem, b->tab_bytes, b->device, b));
     b->tab_cap = c;
     return PBF_OK;
 }
@@ -274,7 +281,7 @@ int ensure_bad(pbf_batch* b, int nscenes) {
     b->d_bad = nullptr;
     b->bad_cap = 0;
     const int c = std::max(nscenes + nscenes / 4, 64);
-    PBF_CUDA(cudaMalloc(&b->d_bad, (size_t)c * 4));
+    PBF_CUDA(device_malloc(&b->d_bad, (size_t)c * 4, b->device, b));
     b->bad_cap = c;
     return PBF_OK;
 }
@@ -567,6 +574,7 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
 // overlapping sets cannot deadlock) and checks them.
 struct SceneLocks {
     std::vector<std::unique_lock<std::mutex>> locks;
+    std::optional<HeldLocks> held;
 };
 
 int lock_scenes(const pbf_batch* b, int nscenes, pbf_scene* const* scenes, SceneLocks& L) {
@@ -580,6 +588,9 @@ int lock_scenes(const pbf_batch* b, int nscenes, pbf_scene* const* scenes, Scene
         if (s->device != b->device) return fail(PBF_ERR_INVALID_ARG, "a scene is on another device");
     L.locks.reserve(sorted.size());
     for (pbf_scene* s : sorted) L.locks.emplace_back(s->mu);
+    std::vector<const void*> held(sorted.begin(), sorted.end());
+    held.push_back(b);
+    L.held.emplace(std::move(held));
     return PBF_OK;
 }
 
@@ -773,6 +784,7 @@ int pbf_batch_create(int device, pbf_batch** out) {
         cudaStreamDestroy(b->stream);
         return cuda_fail(ce, "pbf_batch_create");
     }
+    add_list_owner(b.get(), device, &b->mu, drop_lists);
     *out = b.release();
     return PBF_OK;
 }
@@ -781,6 +793,7 @@ int pbf_batch_destroy(pbf_batch* b) {
     if (!b) return PBF_OK;
     {
         DeviceGuard dg(b->device);
+        remove_list_owner(b);
         if (b->stream) cudaStreamSynchronize(b->stream);
         drop_graph(b);
         free_tables(b);
@@ -795,9 +808,23 @@ int pbf_batch_destroy(pbf_batch* b) {
         give_status_word(b->status);
         if (b->done) cudaEventDestroy(b->done);
         if (b->fork) cudaEventDestroy(b->fork);
-        if (b->stream) cudaStreamDestroy(b->stream);
+        if (b->stream) {
+            cudaStreamSynchronize(b->stream);
+            cudaStreamDestroy(b->stream);
+        }
     }
     delete b;
+    memory_given_back();
+    return PBF_OK;
+}
+
+int pbf_batch_set_kept_lists(pbf_batch* b, int on) {
+    if (!b) return fail(PBF_ERR_INVALID_ARG, "batch is NULL");
+    std::lock_guard<std::mutex> lk(b->mu);
+    DeviceGuard dg(b->device);
+    b->lists_off = on == 0;
+    b->list_refusal = ListRefusal{};
+    if (b->lists_off && drop_lists(b)) memory_given_back();
     return PBF_OK;
 }
 

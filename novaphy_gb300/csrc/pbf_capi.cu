@@ -102,6 +102,20 @@ void set_last_error(const std::string& msg) { g_last_error = msg; }
 namespace pbf {
 namespace capi {
 
+static cudaMemPool_t make_pool(int device, unsigned long long keep) {
+    cudaMemPoolProps props{};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = device;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+    return pool;
+}
+
 // One stream-ordered memory pool per device for scene state and scratch.
 // Freed blocks stay in the pool (release threshold: never), so opening and
 // closing scenes neither synchronizes the device, as cudaMalloc/cudaFree
@@ -111,42 +125,157 @@ cudaMemPool_t scene_pool(int device) {
     static std::vector<cudaMemPool_t> pools;
     std::lock_guard<std::mutex> lk(mu);
     if ((int)pools.size() <= device) pools.resize((size_t)device + 1, nullptr);
-    if (!pools[device]) {
-        cudaMemPoolProps props{};
-        props.allocType = cudaMemAllocationTypePinned;
-        props.location.type = cudaMemLocationTypeDevice;
-        props.location.id = device;
-        cudaMemPool_t pool = nullptr;
-        if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) return nullptr;
-        unsigned long long keep = ~0ull;
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
-        pools[device] = pool;
-    }
+    if (!pools[device]) pools[device] = make_pool(device, ~0ull);
     return pools[device];
 }
 
-static std::atomic<size_t> list_bytes_held{0};
+// The lists' own pool per device, which holds on to kListKeepBytes at most.
+static cudaMemPool_t list_pool(int device) {
+    static std::mutex mu;
+    static std::vector<cudaMemPool_t> pools;
+    std::lock_guard<std::mutex> lk(mu);
+    if ((int)pools.size() <= device) pools.resize((size_t)device + 1, nullptr);
+    if (!pools[device]) pools[device] = make_pool(device, kListKeepBytes);
+    return pools[device];
+}
 
-bool take_list_bytes(size_t bytes) {
-    size_t free = 0, total = 0;
-    if (cudaMemGetInfo(&free, &total) != cudaSuccess) {
+// Bytes that the pool has taken from the device and nobody uses.
+static size_t pool_unused(cudaMemPool_t pool) {
+    unsigned long long reserved = 0, used = 0;
+    if (!pool || cudaMemPoolGetAttribute(pool, cudaMemPoolAttrReservedMemCurrent, &reserved) != cudaSuccess ||
+        cudaMemPoolGetAttribute(pool, cudaMemPoolAttrUsedMemCurrent, &used) != cudaSuccess) {
         cudaGetLastError();
-        return false;
+        return 0;
     }
-    if (bytes > free / 4) return false;
-    size_t held = list_bytes_held.load();
-    do {
-        if (held + bytes > kListMaxBytes) return false;
-    } while (!list_bytes_held.compare_exchange_weak(held, held + bytes));
+    return reserved > used ? (size_t)(reserved - used) : 0;
+}
+
+// What the lists of each device hold, and the objects that may hold some.
+struct ListOwner {
+    void* self;
+    int device;
+    std::mutex* mu;
+    bool (*drop)(void*);
+};
+struct ListBook {
+    std::mutex mu;
+    std::vector<size_t> held;  // by device
+    std::vector<ListOwner> owners;
+    std::atomic<unsigned> epoch{0};
+};
+static ListBook& list_book() {
+    static ListBook* const b = new ListBook();  // outlives every scene
+    return *b;
+}
+static thread_local std::vector<const void*> t_held;
+
+void memory_given_back() { ++list_book().epoch; }
+
+bool ListRefusal::stands() {
+    if (refused && (epoch != list_book().epoch || ++calls >= kListRetry)) refused = false;
+    return refused;
+}
+void ListRefusal::set() {
+    refused = true;
+    epoch = list_book().epoch;
+    calls = 0;
+}
+
+static bool count_lists(int device, size_t bytes, bool take) {
+    static std::mutex mu;
+    std::lock_guard<std::mutex> lk(mu);
+    std::vector<size_t>& held = list_book().held;
+    if ((int)held.size() <= device) held.resize((size_t)device + 1, 0);
+    if (take && held[device] + bytes > kListMaxBytes) return false;
+    held[device] = take ? held[device] + bytes : held[device] - bytes;
     return true;
 }
 
-void give_list_bytes(size_t bytes) { list_bytes_held.fetch_sub(bytes); }
+void* take_lists(size_t bytes, int device, cudaStream_t st) {
+    cudaMemPool_t pool = list_pool(device);
+    size_t free = 0, total = 0;
+    if (!pool || cudaMemGetInfo(&free, &total) != cudaSuccess) {
+        cudaGetLastError();
+        return nullptr;
+    }
+    free += pool_unused(pool) + pool_unused(scene_pool(device));
+    if (bytes > free / 4 || !count_lists(device, bytes, true)) return nullptr;
+    void* p = nullptr;
+    if (cudaMallocFromPoolAsync(&p, bytes, pool, st) != cudaSuccess) {
+        cudaGetLastError();
+        count_lists(device, bytes, false);
+        return nullptr;
+    }
+    return p;
+}
 
-int pool_alloc(void** p, size_t bytes, int device, cudaStream_t st) {
-    cudaMemPool_t pool = scene_pool(device);
+void give_lists(void* p, size_t bytes, int device, cudaStream_t st) {
+    if (!p) return;
+    cudaFreeAsync(p, st);
+    count_lists(device, bytes, false);
+}
+
+void add_list_owner(void* self, int device, std::mutex* mu, bool (*drop)(void*)) {
+    ListBook& B = list_book();
+    std::lock_guard<std::mutex> lk(B.mu);
+    B.owners.push_back(ListOwner{self, device, mu, drop});
+}
+
+void remove_list_owner(void* self) {
+    ListBook& B = list_book();
+    std::lock_guard<std::mutex> lk(B.mu);
+    for (size_t k = 0; k < B.owners.size(); ++k)
+        if (B.owners[k].self == self) {
+            B.owners[k] = B.owners.back();
+            B.owners.pop_back();
+            break;
+        }
+}
+
+// Only one thread reclaims at a time, and it waits for no object's lock, so
+// two that run out of room together cannot wait for each other.
+bool reclaim_lists(int device, void* self) {
+    ListBook& B = list_book();
+    std::lock_guard<std::mutex> lk(B.mu);
+    bool any = false;
+    for (const ListOwner& o : B.owners) {
+        if (o.device != device) continue;
+        if (o.self == self) {
+            any |= o.drop(o.self);
+            continue;
+        }
+        if (std::find(t_held.begin(), t_held.end(), o.self) != t_held.end()) continue;
+        std::unique_lock<std::mutex> ol(*o.mu, std::try_to_lock);
+        if (ol.owns_lock()) any |= o.drop(o.self);
+    }
+    for (cudaMemPool_t pool : {list_pool(device), scene_pool(device)})
+        if (pool) cudaMemPoolTrimTo(pool, 0);
+    return any;
+}
+
+HeldLocks::HeldLocks(std::vector<const void*> objects) { t_held = std::move(objects); }
+HeldLocks::~HeldLocks() { t_held.clear(); }
+
+cudaError_t device_malloc(void** p, size_t bytes, int device, void* self) {
+    cudaError_t e = cudaMalloc(p, bytes);
+    if (e != cudaErrorMemoryAllocation) return e;
+    cudaGetLastError();
+    reclaim_lists(device, self);
+    e = cudaMalloc(p, bytes);
+    if (e != cudaSuccess) cudaGetLastError();
+    return e;
+}
+
+int pool_alloc(void** p, size_t bytes, pbf_scene* s) {
+    cudaMemPool_t pool = scene_pool(s->device);
     if (!pool) return fail(PBF_ERR_CUDA, "cudaMemPoolCreate failed");
-    PBF_CUDA(cudaMallocFromPoolAsync(p, bytes, pool, st));
+    cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s->stream);
+    if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        reclaim_lists(s->device, s);
+        e = cudaMallocFromPoolAsync(p, bytes, pool, s->stream);
+    }
+    if (e != cudaSuccess) return cuda_fail(e, "cudaMallocFromPoolAsync");
     return PBF_OK;
 }
 
@@ -215,13 +344,25 @@ int take_status(uint32_t* device_word, uint32_t* host_word, uint32_t* out) {
 namespace {
 
 void free_lists(pbf_scene* s) {
-    if (s->lmem) {
-        pool_free(s->lmem, s->stream);
-        give_list_bytes(list_bytes(s->B.list_cap));
-    }
+    if (s->lmem) give_lists(s->lmem, list_bytes(s->B.list_cap), s->device, s->stream);
     s->lmem = nullptr;
-    s->no_lists = false;
+    s->list_refusal = ListRefusal{};
     bind_lists(s->B, nullptr, 0);
+}
+
+bool drop_lists(void* self) {
+    pbf_scene* const s = static_cast<pbf_scene*>(self);
+    if (!s->lmem) return false;
+    cudaStreamSynchronize(s->stream);
+    ++s->buf_gen;
+    if (s->graph) {
+        cudaGraphExecDestroy(s->graph);
+        s->graph = nullptr;
+    }
+    free_lists(s);
+    cudaStreamSynchronize(s->stream);
+    s->list_refusal.set();
+    return true;
 }
 
 void free_particles(pbf_scene* s) {
@@ -256,7 +397,7 @@ int alloc_particles(pbf_scene* s, int cap) {
     const size_t f1 = align_up((size_t)c * 4, 256);
     const size_t f3 = align_up((size_t)c * 12, 256);
     const size_t total = 2 * f4 + 2 * f1 + f3;
-    int rc = pool_alloc(&s->pmem, total, s->device, s->stream);
+    int rc = pool_alloc(&s->pmem, total, s);
     if (rc) return rc;
     char* p = reinterpret_cast<char*>(s->pmem);
     s->B.x = reinterpret_cast<float4*>(p);
@@ -284,13 +425,13 @@ int ensure_work(pbf_scene* s) {
     const int c = s->cap > 0 ? s->cap : 1;
     // The step scratch batches share, then the scene's run ends.
     const size_t wb = work_bytes(c) + align_up((size_t)c * 4, 256);
-    int rc = pool_alloc(&s->wmem, wb, s->device, s->stream);
+    int rc = pool_alloc(&s->wmem, wb, s);
     if (rc) return rc;
     PBF_CUDA(cudaMemsetAsync(s->wmem, 0, wb, s->stream));
     bind_work(s->B, s->wmem, c);
     s->B.segend = reinterpret_cast<uint32_t*>(static_cast<char*>(s->wmem) + work_bytes(c));
     const size_t sb = sort_scratch_bytes(c);
-    rc = pool_alloc(&s->smem, sb, s->device, s->stream);
+    rc = pool_alloc(&s->smem, sb, s);
     if (rc) return rc;
     PBF_CUDA(cudaMemsetAsync(s->smem, 0, sb, s->stream));
     sort_scratch_bind(s->sort, s->smem, c);
@@ -301,17 +442,12 @@ int ensure_work(pbf_scene* s) {
     return PBF_OK;
 }
 
-// Kept lists for the scene's own steps, tried once per capacity.
+// Kept lists for the scene's own steps.
 void ensure_lists(pbf_scene* s) {
-    if (s->lmem || s->no_lists) return;
-    const size_t lb = list_bytes(s->work_cap);
-    s->no_lists = true;
-    if (s->work_cap > kListMaxParticles || !take_list_bytes(lb)) return;
-    cudaMemPool_t pool = scene_pool(s->device);
-    void* p = nullptr;
-    if (!pool || cudaMallocFromPoolAsync(&p, lb, pool, s->stream) != cudaSuccess) {
-        cudaGetLastError();
-        give_list_bytes(lb);
+    if (s->lmem || !s->lists_on || s->work_cap > kListMaxParticles || s->list_refusal.stands()) return;
+    void* const p = take_lists(list_bytes(s->work_cap), s->device, s->stream);
+    if (!p) {
+        s->list_refusal.set();
         return;
     }
     ++s->buf_gen;
@@ -319,7 +455,6 @@ void ensure_lists(pbf_scene* s) {
         cudaGraphExecDestroy(s->graph);
         s->graph = nullptr;
     }
-    s->no_lists = false;
     s->lmem = p;
     bind_lists(s->B, p, s->work_cap);
 }
@@ -426,8 +561,7 @@ int ensure_offsets(pbf_scene* s, uint32_t nslots) {
     // a lambda word per slot, then the density pass's walk counts
     const size_t ob = align_up((size_t)(nslots + 1) * 4, 256);
     const size_t ab = align_up(nslots + 1, 256);
-    int rc = pool_alloc(reinterpret_cast<void**>(&s->off),
-                        ob + ab + (size_t)(nslots + 1) * 8 + kWalkHistWords * 4, s->device, s->stream);
+    int rc = pool_alloc(reinterpret_cast<void**>(&s->off), ob + ab + (size_t)(nslots + 1) * 8 + kWalkHistWords * 4, s);
     if (rc) return rc;
     s->off_cap = nslots + 1;
     s->B.off = s->off;
@@ -761,6 +895,7 @@ int pbf_scene_create(int device, const pbf_settings* settings, int n, const floa
         return cuda_fail(ce, "cudaStreamCreate");
     }
     s->stream = s->own_stream;
+    add_list_owner(s, device, &s->mu, drop_lists);
     rc = set_state(s, n, x3, v3);
     if (rc == PBF_OK) {
         ce = cudaStreamSynchronize(s->stream);
@@ -778,6 +913,7 @@ int pbf_scene_destroy(pbf_scene* s) {
     if (!s) return PBF_OK;
     {
         DeviceGuard dg(s->device);
+        remove_list_owner(s);
         if (s->stream) cudaStreamSynchronize(s->stream);
         for (void* m : {s->bnd.body_mem, s->bnd.tw_mem, static_cast<void*>(s->bnd.rb),
                         static_cast<void*>(s->bnd.shapes)})
@@ -797,6 +933,17 @@ int pbf_scene_destroy(pbf_scene* s) {
         give_status_word(s->status);
     }
     delete s;
+    memory_given_back();
+    return PBF_OK;
+}
+
+int pbf_scene_set_kept_lists(pbf_scene* s, int on) {
+    if (!s) return fail(PBF_ERR_INVALID_ARG, "scene is NULL");
+    std::lock_guard<std::mutex> lk(s->mu);
+    DeviceGuard dg(s->device);
+    s->lists_on = on != 0;
+    s->list_refusal = ListRefusal{};
+    if (!s->lists_on && drop_lists(s)) memory_given_back();
     return PBF_OK;
 }
 
@@ -904,7 +1051,7 @@ int pbf_snapshot_create(pbf_scene* s, pbf_snapshot** out) {
     for (int d = 0; d < 3; ++d) snap->gravity[d] = s->gravity[d];
     snap->mass = s->mass;
     if (s->n > 0) {
-        cudaError_t e = cudaMalloc(&snap->mem, snapshot_bytes(s->n));
+        cudaError_t e = device_malloc(&snap->mem, snapshot_bytes(s->n), s->device, s);
         if (e != cudaSuccess) {
             delete snap;
             return cuda_fail(e, "pbf_snapshot_create");
@@ -929,6 +1076,7 @@ int pbf_snapshot_destroy(pbf_snapshot* snap) {
     if (snap->mem) {
         DeviceGuard dg(snap->device);
         cudaFree(snap->mem);
+        memory_given_back();
     }
     delete snap;
     return PBF_OK;
@@ -1177,7 +1325,7 @@ int pbf_scene_debug_cells(pbf_scene* s, float dt, int* cells3) {
     int rc = make_consts(s, dt, C);
     if (rc) return rc;
     int* d = nullptr;
-    PBF_CUDA(cudaMalloc(&d, (size_t)s->n * 12));
+    PBF_CUDA(device_malloc(&d, (size_t)s->n * 12, s->device, s));
     cudaError_t e = debug_cells(s->B, C, d, s->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(cells3, d, (size_t)s->n * 12, cudaMemcpyDeviceToHost, s->stream);
@@ -1203,7 +1351,7 @@ int pbf_scene_debug_neighbors(pbf_scene* s, float dt, long long* offsets, int* o
     long long* d_offs = nullptr;
     int* d_out = nullptr;
     std::vector<long long> cnt(n);
-    cudaError_t e = cudaMalloc(&d_cnt, (size_t)n * 8);
+    cudaError_t e = device_malloc(&d_cnt, (size_t)n * 8, s->device, s);
     if (e == cudaSuccess) e = debug_neighbors(s->B, C, s->sort, d_cnt, nullptr, nullptr, 0, 0, s->stream);
     if (e == cudaSuccess)
         e = cudaMemcpyAsync(cnt.data(), d_cnt, (size_t)n * 8, cudaMemcpyDeviceToHost, s->stream);
@@ -1216,8 +1364,8 @@ int pbf_scene_debug_neighbors(pbf_scene* s, float dt, long long* offsets, int* o
     offsets[n] = tot;
     *total = tot;
     if (e == cudaSuccess && out_idx && cap > 0) {
-        e = cudaMalloc(&d_offs, (size_t)(n + 1) * 8);
-        if (e == cudaSuccess) e = cudaMalloc(&d_out, (size_t)std::max<long long>(cap, 1) * 4);
+        e = device_malloc(&d_offs, (size_t)(n + 1) * 8, s->device, s);
+        if (e == cudaSuccess) e = device_malloc(&d_out, (size_t)std::max<long long>(cap, 1) * 4, s->device, s);
         if (e == cudaSuccess)
             e = cudaMemcpyAsync(d_offs, offsets, (size_t)(n + 1) * 8, cudaMemcpyHostToDevice, s->stream);
         if (e == cudaSuccess)
@@ -1315,7 +1463,7 @@ int alloc_boundary(pbf_scene* s, int nb) {
     const size_t f4 = align_up((size_t)c * 16, 256), f1 = align_up((size_t)c * 4, 256),
                  f27 = align_up((size_t)c * 27 * 4, 256);
     const size_t total = 5 * f4 + 5 * f1 + bucket_bytes(c) + f27;
-    int rc = pool_alloc(&b.mem, total, s->device, s->stream);
+    int rc = pool_alloc(&b.mem, total, s);
     if (rc) return rc;
     char* p = reinterpret_cast<char*>(b.mem);
     auto take = [&](size_t n) { char* r = p; p += n; return r; };
@@ -1334,7 +1482,7 @@ int alloc_boundary(pbf_scene* s, int nb) {
     b.bq.btab = reinterpret_cast<uint32_t*>(take(f27));
     PBF_CUDA(cudaMemsetAsync(b.mem, 0, total, s->stream));
     const size_t sb = sort_scratch_bytes(c);
-    rc = pool_alloc(&b.sort_mem, sb, s->device, s->stream);
+    rc = pool_alloc(&b.sort_mem, sb, s);
     if (rc) return rc;
     PBF_CUDA(cudaMemsetAsync(b.sort_mem, 0, sb, s->stream));
     sort_scratch_bind(b.sort, b.sort_mem, c);
@@ -1350,8 +1498,7 @@ int ensure_boundary_grid(pbf_scene* s, uint32_t nslots) {
     b.idx.off = nullptr;
     b.idx_slots = 0;
     const size_t ob = align_up((size_t)(nslots + 1) * 4, 256);
-    const int rc = pool_alloc(reinterpret_cast<void**>(&b.idx.off), ob + align_up(nslots, 256), s->device,
-                              s->stream);
+    const int rc = pool_alloc(reinterpret_cast<void**>(&b.idx.off), ob + align_up(nslots, 256), s);
     if (rc) return rc;
     b.idx.slot_alias = reinterpret_cast<unsigned char*>(b.idx.off) + ob;
     b.idx_slots = nslots;
@@ -1401,7 +1548,7 @@ int pbf_scene_set_boundary(pbf_scene* s, int nb, const float* local3, const int*
                  sl = align_up(std::max<size_t>(lst.size(), 1) * 4, 256),
                  s12 = align_up((size_t)cap * 12, 256);
     const size_t need = 4 * s16 + 2 * s4 + sl + 2 * s12;
-    PBF_CUDA(cudaMalloc(&b.body_mem, need));
+    PBF_CUDA(device_malloc(&b.body_mem, need, s->device, s));
     char* p = reinterpret_cast<char*>(b.body_mem);
     auto take = [&](size_t n) { char* r = p; p += n; return r; };
     b.body_pos = reinterpret_cast<float4*>(take(s16));
@@ -1747,7 +1894,7 @@ int ensure_two_way(pbf_scene* s) {
     b.tw_mem = nullptr;
     const size_t c = (size_t)(s->n > 0 ? s->n : 1);
     const size_t cb = align_up(c * 16, 256), ob = align_up(c * 4, 256);
-    PBF_CUDA(cudaMalloc(&b.tw_mem, cb + ob + c * 27 * 4));
+    PBF_CUDA(device_malloc(&b.tw_mem, cb + ob + c * 27 * 4, s->device, s));
     unsigned char* m = static_cast<unsigned char*>(b.tw_mem);
     b.tw_cell = reinterpret_cast<int4*>(m);
     b.tw_own = reinterpret_cast<int*>(m + cb);
@@ -1921,10 +2068,10 @@ int pbf_sort_pairs_host(int device, int n, const unsigned* keys, int key_bits, u
     uint32_t *dk = nullptr, *dko = nullptr, *dvo = nullptr;
     void* scratch = nullptr;
     SortScratch ss;
-    cudaError_t e = cudaMalloc(&dk, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&dko, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&dvo, (size_t)n * 4);
-    if (e == cudaSuccess) e = cudaMalloc(&scratch, sort_scratch_bytes(n));
+    cudaError_t e = device_malloc(&dk, (size_t)n * 4, device, nullptr);
+    if (e == cudaSuccess) e = device_malloc(&dko, (size_t)n * 4, device, nullptr);
+    if (e == cudaSuccess) e = device_malloc(&dvo, (size_t)n * 4, device, nullptr);
+    if (e == cudaSuccess) e = device_malloc(&scratch, sort_scratch_bytes(n), device, nullptr);
     if (e == cudaSuccess) e = cudaMemset(scratch, 0, sort_scratch_bytes(n));
     if (e == cudaSuccess) {
         sort_scratch_bind(ss, scratch, n);

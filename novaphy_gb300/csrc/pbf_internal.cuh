@@ -5,6 +5,7 @@
 #include <cstddef>
 #include <mutex>
 #include <string>
+#include <vector>
 
 #include "novaphy_pbf.h"
 #include "pbf_boundary.cuh"
@@ -96,12 +97,16 @@ inline void bind_work(StepBuffers& B, void* mem, int c) {
 }
 
 // Kept lists of c particles (StepBuffers::lists): rows, then their numbers.
-// They take seven times the rest of the step scratch (2 KB a particle), so no
-// scene or batch of more than kListMaxParticles has any, one's stay below a
-// quarter of the free memory, all of a process's together below kListMaxBytes,
-// and they are not needed: without them the passes walk.
+// They take seven times the rest of the step scratch (2 KB a particle) and are
+// not needed (without them the passes walk).  So no scene or batch of more than
+// kListMaxParticles has any, one's stay below a quarter of the free memory and
+// all of a device's together below kListMaxBytes, and an allocation that finds
+// no room gets theirs (reclaim_lists).  Freed ones stay in their pool up to
+// kListKeepBytes, those of two million particles: mapping those of a million
+// anew takes 1.7 ms of a new scene's first step.
 constexpr int kListMaxParticles = 32 << 20;
 constexpr size_t kListMaxBytes = (size_t)64 << 30;
+constexpr size_t kListKeepBytes = (size_t)4 << 30;
 
 inline size_t list_bytes(int c) {
     const size_t r = align_up((size_t)c, 32);
@@ -117,10 +122,43 @@ inline void bind_lists(StepBuffers& B, void* mem, int c) {
     B.unlisted = mem ? B.listed + r : nullptr;
 }
 
-// Whether lists of that many bytes may be allocated now (then counted until
-// they are given back).
-bool take_list_bytes(size_t bytes);
-void give_list_bytes(size_t bytes);
+// Lists of that many bytes on stream `st`, null where they may not be taken now.
+void* take_lists(size_t bytes, int device, cudaStream_t st);
+void give_lists(void* p, size_t bytes, int device, cudaStream_t st);
+// After a refusal, lists are tried again once memory was given back
+// (memory_given_back) and every kListRetry calls.
+struct ListRefusal {
+    bool refused = false;
+    unsigned epoch = 0, calls = 0;
+    bool stands();
+    void set();
+};
+constexpr unsigned kListRetry = 64;
+void memory_given_back();
+
+// Objects that may hold lists, and how to free them: drop(self) is called with
+// the object's lock held, waits for the work that reads them, and returns
+// whether there were any.
+void add_list_owner(void* self, int device, std::mutex* mu, bool (*drop)(void* self));
+void remove_list_owner(void* self);
+// Frees the lists of every object of the device whose lock is free, and those
+// of `self`, whose lock the caller holds.  HeldLocks names the other objects
+// whose locks the calling thread holds.
+bool reclaim_lists(int device, void* self);
+struct HeldLocks {
+    explicit HeldLocks(std::vector<const void*> objects);
+    ~HeldLocks();
+    HeldLocks(const HeldLocks&) = delete;
+    HeldLocks& operator=(const HeldLocks&) = delete;
+};
+
+// cudaMalloc for the object `self`, once more after reclaim_lists where there
+// is no room.
+cudaError_t device_malloc(void** p, size_t bytes, int device, void* self);
+template <class T>
+cudaError_t device_malloc(T** p, size_t bytes, int device, void* self) {
+    return device_malloc(reinterpret_cast<void**>(p), bytes, device, self);
+}
 
 }  // namespace capi
 }  // namespace pbf
@@ -144,7 +182,8 @@ struct pbf_scene {
     void* wmem = nullptr;  // step scratch (sorted copies, keys, buckets)
     void* smem = nullptr;  // sort scratch
     void* lmem = nullptr;  // kept lists (list_bytes(work_cap); null: none)
-    bool no_lists = false;  // there was no room for them
+    bool lists_on = true;  // the scene may have kept lists
+    pbf::capi::ListRefusal list_refusal;  // of lists for work_cap particles
     uint32_t* off = nullptr;
     uint32_t off_cap = 0;  // entries
     float* staging = nullptr;  // float[3 cap]
@@ -235,8 +274,9 @@ int check_settings(const pbf_settings* st);
 GridDesc fit_grid(const pbf_scene* s);
 // Per-step constants of the scene with time step dt (no allocation).
 int scene_consts(const pbf_scene* s, float dt, StepConsts& C);
-// Stream-ordered allocation of scene buffers from the device's scene pool.
-int pool_alloc(void** p, size_t bytes, int device, cudaStream_t st);
+// Stream-ordered allocation of scene buffers from the device's scene pool, on
+// the scene's stream (its lock held).
+int pool_alloc(void** p, size_t bytes, pbf_scene* s);
 void pool_free(void* p, cudaStream_t st);
 // A status word in page-locked host memory that the device writes to (null
 // when there is none left: the word in the sort scratch then serves), so that
