@@ -909,7 +909,7 @@ struct WalkSmem {
     // One fp16 row of eight per candidate: x, y, z, |u|^2 (high, low), 1, 1, 0.
     alignas(16) uint32_t stage[128 * 4];
     uint32_t base[kWalkWords];  // first candidate (cell order, or key order in buckets)
-    uint32_t info[kWalkWords];  // candidates | row << 8
+    uint32_t info[kWalkWords];  // candidates | row << 8 | kRunWord
     uint32_t mask[kWalkWords * 32];
     // The mask of word w and particle p.  The exclusive-or spreads the four
     // words that a store instruction touches over the banks.
@@ -918,6 +918,10 @@ struct WalkSmem {
     // (k_segments), until its masks are there.
     __device__ __forceinline__ uint32_t& skip(int w) { return mask[at(w, 0)]; }
 };
+
+// In WalkSmem::info: a word of a range with runs, whose first particles stand
+// for them; in the other ranges every candidate counts once.
+constexpr uint32_t kRunWord = 1u << 16;
 
 // Shared memory of a team walk.  During an evaluation the stage holds the
 // terms on their way to the adding lanes, one row of float2 (two quantities)
@@ -1196,7 +1200,7 @@ __device__ __forceinline__ uint32_t own_cells(const WalkIndex& I, uint32_t slot,
 // candidates with a nonzero one only.  kRuns: in ranges that hold runs of
 // identical particles (k_segments) a run is listed as its first particle,
 // whose term is added as many times as the run is long (a step of the 1M dam
-// break with a corner cell of 44,000 particles in 27,000 runs takes 213 ms;
+// break with a corner cell of 44,000 particles in 27,000 runs takes 229 ms;
 // 434 when a word ended with each run, 255 in the one-thread walks before that,
 // 265 with the runs' particles listed one by one, which costs later steps
 // three times as much).  kList: nothing is
@@ -1258,7 +1262,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             auto word = [&](uint32_t skip, uint32_t next) {
                 if (lane == 0) {
                     sm.base[nw] = st + at_q;
-                    sm.info[nw] = min(32u, len_r - at_q) | ((uint32_t)at_r << 8);
+                    sm.info[nw] = min(32u, len_r - at_q) | ((uint32_t)at_r << 8) | (ln & kRunRange ? kRunWord : 0u);
                     sm.skip(nw) = skip;
                 }
                 ++nw;
@@ -1317,6 +1321,7 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
                     any_nz |= nz[j];
                 }
             }
+            if (kRuns && runs) __syncwarp();  // the masks take the place of skip
             const bool test = !B.wide && (!kLam || !all_zero || any_nz != 0u);
             if (test) {
                 uint32_t h0[4], h1[4];
@@ -1396,8 +1401,8 @@ __device__ __forceinline__ void walk_group(WalkSmem& sm, const WalkGroup& Gr, bo
             uint32_t qa = 0u, qb = 0u;
             auto load = [&](uint32_t& q, float4& x, float4& e, uint32_t& end) {
                 q = next_q();
+                end = sm.info[w] & kRunWord ? __ldg(G.segend + q) : 0u;
                 if (key) q = I.at(q);
-                end = __ldg(G.segend + q);
                 x = ld_step<kPersist>(xin + q);
                 if constexpr (Sums::kExtra) e = sums.extra(q);
             };
