@@ -488,7 +488,8 @@ cudaError_t index_build(PointIndex& I, const float4* pos, const float* attr, int
     if (e != cudaSuccess) return e;
     k_ix_gather<<<nb + grid_of((int)C.grid.nslots + 1, kBlock), kBlock, 0, st>>>(I.sidx, pos, attr, n, I.spos,
         I.scell, I.bkt.link, I.slot_alias, SlotOffsets{I.skeys, I.off, C.grid.nslots, nb}, C);
-    return enqueue_buckets(sized_for(I.bkt, n), I.scell, I.sidx, nullptr, I.slot_alias, n, OneScene{C, StateRef{}}, st);
+    return enqueue_buckets(sized_for(I.bkt, n), I.scell, I.sidx, nullptr, I.off, I.slot_alias, n,
+                           OneScene{C, StateRef{}}, st);
 }
 
 cudaError_t predict_cells(const float4* x, const float4* v, int n, int4* cells, const StepConsts& C,

@@ -47,17 +47,17 @@ constexpr size_t kStateBytesPerParticle = 16 + 16 + 4 + 4 + 12;
 
 // Bytes of a BucketTable over c points, and its carving out of [p, p + bytes).
 inline size_t bucket_bytes(int c) {
-    return 6 * align_up((size_t)c * 4, 256) + align_up(((size_t)bucket_slots((uint32_t)c) + 1) * 4, 256);
+    return 8 * align_up((size_t)c * 4, 256) + align_up(((size_t)bucket_slots((uint32_t)c) + 1) * 4, 256);
 }
 
 inline void bind_buckets(BucketTable& T, char* p, int c) {
     const size_t f1 = align_up((size_t)c * 4, 256);
     T.end = reinterpret_cast<uint32_t*>(p);
-    T.rep = reinterpret_cast<uint32_t*>(p + 2 * f1);
-    T.link = reinterpret_cast<uint32_t*>(p + 3 * f1);
-    T.start = reinterpret_cast<uint32_t*>(p + 4 * f1);
-    T.merged = reinterpret_cast<uint32_t*>(p + 5 * f1);
-    T.table = reinterpret_cast<uint32_t*>(p + 6 * f1);
+    T.rep = reinterpret_cast<uint32_t*>(p + 3 * f1);
+    T.link = reinterpret_cast<uint32_t*>(p + 4 * f1);
+    T.start = reinterpret_cast<uint32_t*>(p + 5 * f1);
+    T.merged = reinterpret_cast<uint32_t*>(p + 6 * f1);
+    T.table = reinterpret_cast<uint32_t*>(p + 8 * f1);
     T.slots = bucket_slots((uint32_t)c);
 }
 

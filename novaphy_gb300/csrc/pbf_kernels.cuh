@@ -454,17 +454,15 @@ struct CellRuns {
         const int4 c = scell[a], d = scell[b];
         return c.x == d.x && c.y == d.y && c.z == d.z && (!sid || sid[a] == sid[b]);
     }
-    // First position after p outside p's run, and the run's first position.
-    // Both gallop, so a run of L points costs O(log L) per thread: fluid piled
-    // into a corner by the domain clamp makes runs of tens of thousands.
-    // (Positions of one run are contiguous, but a gallop may land in a later
-    // run of the same cell only where its slot holds aliases, whose cells
-    // alternate; there the runs are found one position at a time.)
-    __device__ __forceinline__ int end_of(int p, bool step_by_one) const {
+    // First position after p outside p's run, and the run's first position, in
+    // a slot without aliases (where a cell has one run).  Both gallop, so a run
+    // of L points costs O(log L) per thread: fluid piled into a corner by the
+    // domain clamp makes runs of tens of thousands.
+    __device__ __forceinline__ int end_of(int p) const {
         int lo = p, step = 1, hi = p + 1;
         while (hi < n && same(hi, p)) {
             lo = hi;
-            step = step_by_one ? step + 1 : step << 1;
+            step <<= 1;
             hi = (n - p > step) ? p + step : n;
         }
         while (hi - lo > 1) {
@@ -474,11 +472,11 @@ struct CellRuns {
         }
         return hi;
     }
-    __device__ __forceinline__ int start_of(int p, bool step_by_one) const {
+    __device__ __forceinline__ int start_of(int p) const {
         int hi = p, step = 1, lo = p - 1;
         while (lo >= 0 && same(lo, p)) {
             hi = lo;
-            step = step_by_one ? step + 1 : step << 1;
+            step <<= 1;
             lo = (p >= step) ? p - step : -1;
         }
         while (hi - lo > 1) {
@@ -523,16 +521,93 @@ __device__ __forceinline__ uint32_t find_bucket(const BucketTable& T, const Cell
     return kNoBucket;
 }
 
-// Every run's end, and its place in the table.
+// The points of a cell in a slot that holds aliases, where the cells' runs
+// may alternate: positions [b0, b1) of the cell order, run start p.  Called by
+// a warp together, 128 positions a round.  Returns whether p is the first of
+// its cell; then the cell's other points get kMember | p, and T.end[p] is the
+// end of its only run, or kListed | at where `merged` holds several (with
+// their end in T.end[n + at]).  A pile of L points among aliases takes L / 128
+// rounds for each cell in its slot.  One thread per run stepping through it,
+// and every point of a merged bucket stepping back to its run's start and
+// searching all runs of the bucket, took 17.5 ms for 60,000 points of two
+// cells in turn (2.5 ms now).
+__device__ __forceinline__ bool alias_cell(const BucketTable& T, const CellRuns& R, int p, int b0, int b1) {
+    const unsigned full = 0xffffffffu;
+    const int lane = threadIdx.x & 31;
+    b1 = min(b1, R.n);
+    for (int b = p; b > b0; b -= 128) {
+        bool found = false;
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int q = b - 1 - 32 * j - lane;
+            found |= q >= b0 && R.same(q, p);
+        }
+        if (__any_sync(full, found)) return false;
+    }
+    int count = 0, last = p;
+    for (int b = p; b < b1; b += 128) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int q = b + 32 * j + lane;
+            const bool in = q < b1 && R.same(q, p);
+            if (in && q != p) T.rep[q] = kMember | (uint32_t)p;
+            const uint32_t m = __ballot_sync(full, in);
+            if (m) last = b + 32 * j + 31 - __clz(m);
+            count += __popc(m);
+        }
+    }
+    uint32_t at = 0u;
+    const bool listed = count != last - p + 1;
+    if (listed && lane == 0) at = atomicAdd(T.table + T.slots, (uint32_t)count) + 1u;
+    at = __shfl_sync(full, at, 0);
+    // (No room only after a failed sort; keep every access in range.)
+    if (!listed || at + (uint32_t)count > 2u * (uint32_t)R.n) {
+        if (lane == 0) T.end[p] = (uint32_t)(listed ? p + 1 : last + 1);
+        return true;
+    }
+    if (lane == 0) {
+        T.end[p] = kListed | at;
+        T.end[(uint32_t)R.n + at] = (uint32_t)R.n + at + (uint32_t)count;
+    }
+    for (int b = p; b <= last; b += 128) {
+#pragma unroll
+        for (int j = 0; j < 4; ++j) {
+            const int q = b + 32 * j + lane;
+            const bool in = q <= last && R.same(q, p);
+            const uint32_t m = __ballot_sync(full, in);
+            if (in) T.merged[at + (uint32_t)__popc(m & ((1u << lane) - 1u))] = (uint32_t)q;
+            at += (uint32_t)__popc(m);
+        }
+    }
+    return true;
+}
+
+// Every cell's points (T.end at the first one), and its place in the table.
 template <class P>
-__global__ void __launch_bounds__(256)
-k_cell_runs(const BucketTable T, const CellRuns R, const unsigned char* __restrict__ slot_alias, const P prm) {
+__global__ void __launch_bounds__(256, 6)
+k_cell_runs(const BucketTable T, const CellRuns R, const uint32_t* __restrict__ off,
+            const unsigned char* __restrict__ slot_alias, const P prm) {
     const int p = blockIdx.x * blockDim.x + threadIdx.x;
-    if (p >= R.n || (p > 0 && R.same(p, p - 1))) return;
-    const int4 c = R.scell[p];
-    const StepConsts& C = prm.at(R.sid, (uint32_t)p);
-    const bool alias = (slot_alias[slot_of(c.x, c.y, c.z, C.grid)] & kAliasSlot) != 0;
-    T.end[p] = (uint32_t)R.end_of(p, alias);
+    bool first = p < R.n && !(p > 0 && R.same(p, p - 1));
+    int4 c = make_int4(0, 0, 0, 0);
+    uint32_t slot = 0u;
+    bool alias = false;
+    if (first) {
+        c = R.scell[p];
+        const StepConsts& C = prm.at(R.sid, (uint32_t)p);
+        slot = slot_of(c.x, c.y, c.z, C.grid);
+        alias = (slot_alias[slot] & kAliasSlot) != 0;
+        if (!alias) T.end[p] = (uint32_t)R.end_of(p);
+    }
+    uint32_t todo = __ballot_sync(0xffffffffu, alias);
+    while (todo) {
+        const int l = __ffs(todo) - 1;
+        todo &= todo - 1u;
+        const uint32_t s = __shfl_sync(0xffffffffu, slot, l);
+        const bool leads = alias_cell(T, R, __shfl_sync(0xffffffffu, p, l), (int)off[s], (int)off[s + 1]);
+        if ((int)(threadIdx.x & 31) == l) first = leads;
+    }
+    if (!first) return;
     const unsigned long long key = ref_hash(c.x, c.y, c.z);
     const uint32_t sid = R.sid ? R.sid[p] : 0u;
     uint32_t rep = (uint32_t)p;
@@ -548,10 +623,13 @@ k_cell_runs(const BucketTable T, const CellRuns R, const unsigned char* __restri
         h = (h + 1u) & (T.slots - 1u);
     }
     T.rep[p] = rep;
-    if (rep == (uint32_t)p) T.start[p] = (uint32_t)p;
+    if (rep != (uint32_t)p) return;
+    uint32_t lo = (uint32_t)p, hi;
+    if (alias) T.points(lo, (uint32_t)R.n, lo, hi);
+    T.start[p] = lo;
 }
 
-// Room for the buckets of more than one run.
+// Room for the buckets of more than one cell.
 template <class P>
 __global__ void __launch_bounds__(256)
 k_merge_room(const BucketTable T, const CellRuns R, unsigned char* __restrict__ slot_alias, const P prm) {
@@ -561,7 +639,9 @@ k_merge_room(const BucketTable T, const CellRuns R, unsigned char* __restrict__ 
     uint32_t total = 0u;
     const StepConsts& C = prm.at(R.sid, (uint32_t)p);
     for (uint32_t s = (uint32_t)p; s != kNoBucket; s = T.link[s]) {
-        total += T.end[s] - s;
+        uint32_t lo, hi;
+        T.points(s, (uint32_t)R.n, lo, hi);
+        total += hi - lo;
         const int4 c = R.scell[s];
         unsigned char* const a = slot_alias + slot_of(c.x, c.y, c.z, C.grid);
         *a = (unsigned char)(*a | kMergedSlot);
@@ -572,7 +652,7 @@ k_merge_room(const BucketTable T, const CellRuns R, unsigned char* __restrict__ 
 }
 
 // The members of those buckets, in ascending point index: a point's place is
-// the number of members before it, by a search in each of the other runs.
+// the number of members before it, by a search in each of the cells.
 template <class P>
 __global__ void __launch_bounds__(256)
 k_merge_runs(const BucketTable T, const CellRuns R, const uint32_t* __restrict__ sidx,
@@ -583,34 +663,38 @@ k_merge_runs(const BucketTable T, const CellRuns R, const uint32_t* __restrict__
     const StepConsts& C = prm.at(R.sid, (uint32_t)p);
     const unsigned char a = slot_alias[slot_of(c.x, c.y, c.z, C.grid)];
     if (!(a & kMergedSlot)) return;
-    const uint32_t own = (uint32_t)R.start_of(p, (a & kAliasSlot) != 0);
+    const uint32_t n = (uint32_t)R.n;
+    uint32_t own = (uint32_t)p;
+    if (!(a & kAliasSlot)) own = (uint32_t)R.start_of(p);
+    else if (T.rep[p] & kMember) own = T.rep[p] & ~kMember;
     const uint32_t rep = T.rep[own];
     if (T.link[rep] == kNoBucket) return;
     const uint32_t i = sidx[p];
-    uint32_t rank = (uint32_t)p - own;
+    uint32_t rank = 0u;
     for (uint32_t s = rep; s != kNoBucket; s = T.link[s]) {
-        if (s == own) continue;
-        uint32_t lo = s, hi = T.end[s];
+        uint32_t first, lo, hi;
+        T.points(s, n, first, hi);
+        lo = first;
         while (lo < hi) {
-            const uint32_t m = (lo + hi) >> 1;
-            if (sidx[m] < i) lo = m + 1u;
+            const uint32_t m = lo + ((hi - lo) >> 1);
+            if (sidx[m < n ? m : T.merged[m - n]] < i) lo = m + 1u;
             else hi = m;
         }
-        rank += lo - s;
+        rank += lo - first;
     }
-    const uint32_t at = T.start[rep] - (uint32_t)R.n + rank;
-    if (at < (uint32_t)R.n) T.merged[at] = (uint32_t)p;
+    const uint32_t at = T.start[rep] - n + rank;
+    if (at < 2u * n) T.merged[at] = (uint32_t)p;
 }
 
 // T: sized_for n, its table cleared (bucket_clear).
 template <class P>
 inline cudaError_t enqueue_buckets(const BucketTable& T, const int4* scell, const uint32_t* sidx,
-                                   const uint32_t* sid, unsigned char* slot_alias, int n, const P& prm,
-                                   cudaStream_t st) {
+                                   const uint32_t* sid, const uint32_t* off, unsigned char* slot_alias, int n,
+                                   const P& prm, cudaStream_t st) {
     if (n <= 0) return cudaSuccess;
     const CellRuns R{scell, sid, n};
     const int nb = (n + 255) / 256;
-    k_cell_runs<P><<<nb, 256, 0, st>>>(T, R, slot_alias, prm);
+    k_cell_runs<P><<<nb, 256, 0, st>>>(T, R, off, slot_alias, prm);
     k_merge_room<P><<<nb, 256, 0, st>>>(T, R, slot_alias, prm);
     k_merge_runs<P><<<nb, 256, 0, st>>>(T, R, sidx, slot_alias, prm);
     return cudaGetLastError();
@@ -3487,7 +3571,7 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
         B.srho, B.scell, B.bkt.link, B.slot_alias, B.err, n, SlotOffsets{B.skeys, B.off, C.grid.nslots, nb},
         none, one);
     if (C.hash_compat) {
-        e = enqueue_buckets(sized_for(B.bkt, n), B.scell, B.sidx, nullptr, B.slot_alias, n, one, st);
+        e = enqueue_buckets(sized_for(B.bkt, n), B.scell, B.sidx, nullptr, B.off, B.slot_alias, n, one, st);
         if (e != cudaSuccess) return e;
         k_classify<OneScene><<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, nullptr, sized_for(B.bkt, n),
             B.slot_alias, B.btab, B.sown, nullptr, one);
@@ -3739,7 +3823,7 @@ inline cudaError_t enqueue_batch_step(const StepBuffers& B, const BatchDesc& D, 
     k_gather<SceneTable><<<nb + grid_of((int)D.nslots + 1, kBlock), kBlock, 0, st>>>(B.sidx, B.sx, B.xa,
         B.srho, B.scell, B.bkt.link, B.slot_alias, B.err, n, SlotOffsets{B.skeys, B.off, D.nslots, nb}, ids,
         tab);
-    e = enqueue_buckets(sized_for(B.bkt, n), B.scell, B.sidx, D.spid, B.slot_alias, n, tab, st);
+    e = enqueue_buckets(sized_for(B.bkt, n), B.scell, B.sidx, D.spid, B.off, B.slot_alias, n, tab, st);
     if (e != cudaSuccess) return e;
     k_classify<SceneTable><<<nb, kBlock, 0, st>>>(B.scell, n, B.scell, D.spid, sized_for(B.bkt, n),
         B.slot_alias, B.btab, B.sown, D.spid, tab);

@@ -88,24 +88,39 @@ struct BoundaryGrid {
 
 // The reference's hash buckets over cell-sorted points.  A cell's points are
 // next to each other in cell order, in ascending index, as its bucket holds
-// them, so a bucket that only one cell's run hashes to is that run.  The runs
-// (stretches of equal cell; the cells of one slot may alternate where points
-// outside the grid box alias into it) go into a hash table by reference key;
-// the runs of one key are chained, and where there are several, their bucket
-// is written out in ascending point index.
+// them, so a bucket that only one cell hashes to is that run.  Only in slots
+// that points outside the grid box alias into may the runs of several cells
+// alternate; the points of a cell with several runs are written out
+// (alias_cell).  The cells go into a hash table by reference key; the cells of
+// one key are chained, and where there are several, their bucket is written
+// out in ascending point index.
 //
-// A bucket is a range [start, end[start]) of positions: below n, positions of
-// the cell order; from n on, entry position - n of `merged`.
+// A bucket, and a cell's points, is a range [start, end[start]) of positions:
+// below n, positions of the cell order; from n on, entry position - n of
+// `merged`.
+constexpr uint32_t kListed = 0x80000000u, kMember = 0x80000000u;
 struct BucketTable {
-    uint32_t* end;     // 2 n: end of the run, or bucket, that starts here
-    uint32_t* rep;     // n: at a run's start, the first run of its bucket
-    uint32_t* link;    // n: at a run's start, the next run of its bucket (kNoBucket: none)
-    uint32_t* start;   // n: at a bucket's first run, the bucket's start
-    uint32_t* merged;  // n: cell-order positions of the merged buckets
-    // slots + 1 words, all ones before a build: runs by reference key (open
-    // addressing), then the merged positions handed out so far, less one.
+    // 3 n: end of the cell's run, or of the bucket, that starts here; kListed |
+    // at for a cell whose points are the range from n + at on.
+    uint32_t* end;
+    // n: at a cell's first point, the first cell of its bucket; in slots with
+    // aliases, kMember | the first point at the cell's others.
+    uint32_t* rep;
+    uint32_t* link;    // n: at a cell's first point, the next cell of its bucket (kNoBucket: none)
+    uint32_t* start;   // n: at a bucket's first cell, the bucket's start
+    uint32_t* merged;  // 2 n: cell-order positions of written-out cells and buckets
+    // slots + 1 words, all ones before a build: cells by reference key (open
+    // addressing), then the positions handed out in `merged` so far, less one.
     uint32_t* table;
     uint32_t slots;  // a power of two >= 2 n
+#if defined(__CUDACC__)
+    // The points [lo, hi) of the cell whose first point is s.
+    __device__ __forceinline__ void points(uint32_t s, uint32_t n, uint32_t& lo, uint32_t& hi) const {
+        const uint32_t e = end[s];
+        lo = e & kListed ? n + (e & ~kListed) : s;
+        hi = e & kListed ? end[lo] : e;
+    }
+#endif
 };
 constexpr uint32_t bucket_slots(uint32_t n) {
     uint32_t s = 1024;
