@@ -14,6 +14,7 @@ float constants round like the reference's on x86 and on Arm.
 from __future__ import annotations
 
 import concurrent.futures as cf
+import hashlib
 import os
 import shutil
 import subprocess
@@ -76,9 +77,23 @@ def _run(cmd: list[str], verbose: bool) -> None:
         print(r.stdout + r.stderr, flush=True)
 
 
+def kernel_id() -> str:
+    """Names this build's kernels (their sources and flags), for what is measured with them and kept on disk."""
+    h = hashlib.sha256(repr((NVCC_COMMON[:-4], sorted(CU_FLAGS.items()))).encode())
+    for f in sorted(os.listdir(CSRC)):
+        if f.endswith((".cu", ".cuh", ".h")):
+            with open(os.path.join(CSRC, f), "rb") as src:
+                h.update(f.encode() + src.read())
+    return h.hexdigest()[:16]
+
+
 def _compile_cu(src: str, verbose: bool, extra: list[str]) -> str:
     obj = os.path.join(BUILD, os.path.basename(src) + ".o")
-    if _stale(obj, _deps(os.path.join(CSRC, src))):
+    deps = _deps(os.path.join(CSRC, src))
+    if src == "pbf_batch.cu":  # holds kernel_id
+        deps += [os.path.join(CSRC, s) for s in CU_SOURCES]
+        extra = [*extra, f'-DPBF_KERNEL_ID="{kernel_id()}"']
+    if _stale(obj, deps):
         _run([nvcc(), *NVCC_COMMON, *CU_FLAGS.get(src, []), *extra, "-c",
               os.path.join(CSRC, src), "-o", obj], verbose)
     return obj

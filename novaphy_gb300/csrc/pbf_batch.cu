@@ -292,7 +292,14 @@ bool graphs_enabled() {
 }
 
 // Where tuning decisions are kept: $PBF_AUTOTUNE_CACHE, else
-// ~/.cache/novaphy_gb300/autotune.jsonl.  One JSON object per line.
+// ~/.cache/novaphy_gb300/autotune.jsonl.  One JSON object per line.  A decision
+// holds for the kernels that it was measured with (kKernelId, a hash of the
+// sources): the persistent loop, once the faster one for some shapes, is not
+// with the kept lists and the teams, which it has none of.
+#ifndef PBF_KERNEL_ID
+#define PBF_KERNEL_ID __DATE__ " " __TIME__
+#endif
+const char* const kKernelId = PBF_KERNEL_ID;
 std::string cache_file() {
     if (const char* p = std::getenv("PBF_AUTOTUNE_CACHE")) return p;
     const char* home = std::getenv("HOME");
@@ -317,7 +324,7 @@ void load_tuning(pbf_batch* b) {
     std::ifstream in(b->cache_path);
     std::string line;
     while (std::getline(in, line)) {
-        if (json_field(line, "gpu") != b->gpu) continue;
+        if (json_field(line, "gpu") != b->gpu || json_field(line, "kernels") != kKernelId) continue;
         const std::string cls = json_field(line, "class");
         const std::string block = json_field(line, "block"), persist = json_field(line, "persistent");
         if (cls.empty() || block.empty() || persist.empty()) continue;
@@ -340,17 +347,17 @@ void save_tuning(const pbf_batch* b, const std::string& cls, const TuneState& t)
     }
     std::ofstream out(path, std::ios::app);
     if (!out) return;  // a cache that cannot be written only costs re-tuning
-    out << "{\"gpu\": \"" << b->gpu << "\", \"class\": \"" << cls << "\", \"block\": "
-        << t.best.block << ", \"persistent\": " << t.best.persist << ", \"ms\": " << t.best_ms
+    out << "{\"gpu\": \"" << b->gpu << "\", \"kernels\": \"" << kKernelId << "\", \"class\": \"" << cls
+        << "\", \"block\": " << t.best.block << ", \"persistent\": " << t.best.persist << ", \"ms\": " << t.best_ms
         << "}\n";
 }
 
 // Class of a batch shape: arithmetic build, particle-count octave, largest
-// iteration count, vorticity on any scene.
-std::string tune_class(int exact, int n, int max_iters, bool any_vort) {
+// iteration count, vorticity on any scene, whether there are kept lists.
+std::string tune_class(int exact, int n, int max_iters, bool any_vort, bool lists) {
     std::ostringstream o;
     o << (exact ? "exact" : "fast") << " n2^" << bits_for((unsigned long long)n) << " it"
-      << max_iters << (any_vort ? " vort" : "");
+      << max_iters << (any_vort ? " vort" : "") << (lists ? " lists" : "");
     return o.str();
 }
 
@@ -473,7 +480,7 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
     int trial = -1;
     std::string cls;
     if (b->autotune && !pm) {
-        cls = tune_class(exact, n, max_iters, any_vort);
+        cls = tune_class(exact, n, max_iters, any_vort, b->lmem && n <= b->B.list_cap);
         choice = pick_choice(b, cls, &trial);
     }
     D.block = choice.block;
