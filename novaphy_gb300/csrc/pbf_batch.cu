@@ -211,8 +211,8 @@ bool drop_lists(void* self) {
 }
 
 // Kept lists for steps of n particles; those of a smaller size stay until the
-// larger ones are there.
-void ensure_lists(pbf_batch* b, int n) {
+// larger ones are there.  off: whether the first steps list nothing.
+void ensure_lists(pbf_batch* b, int n, bool off) {
     if (b->lists_off || n <= b->B.list_cap || n > kListMaxParticles || b->list_refusal.stands()) return;
     const int c = std::min({b->cap, n + n / 4, kListMaxParticles});
     void* const p = take_lists(list_bytes(c), b->device, b->stream);
@@ -224,6 +224,10 @@ void ensure_lists(pbf_batch* b, int n) {
     free_lists(b);
     b->lmem = p;
     bind_lists(b->B, p, c);
+    if (begin_lists(b->B, off, b->stream) != cudaSuccess) {
+        cudaGetLastError();
+        free_lists(b);
+    }
 }
 
 int ensure_slots(pbf_batch* b, uint32_t nslots) {
@@ -404,7 +408,7 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
                const std::vector<int>& orig, int exact, PhaseMarks* pm) {
     const int ns = (int)list.size();
     if (ns == 0) return PBF_OK;
-    unsigned long long n_total = 0, slots_total = 0;
+    unsigned long long n_total = 0, n_over = 0, slots_total = 0;
     int max_iters = 0;
     bool any_zero = false, any_vort = false, any_plain = false, xsph_on = false;
     std::vector<StepConsts> consts((size_t)ns);
@@ -416,6 +420,7 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
         C.seg_begin = (uint32_t)n_total;
         C.grid.base = (uint32_t)slots_total;
         n_total += (unsigned long long)s->n;
+        if (rest_neighbors(C.h, C.rho0, C.mass) > kListRestMax) n_over += (unsigned long long)s->n;
         slots_total += C.grid.nslots;
         if (n_total > (1ull << 30)) return fail(PBF_ERR_CAPACITY, "at most 2^30 particles per batch");
         if (slots_total > (1ull << 30))
@@ -428,7 +433,7 @@ int step_group(pbf_batch* b, const std::vector<pbf_scene*>& list, const std::vec
     }
     const int n = (int)n_total;
     int rc = ensure_particles(b, n);
-    if (!rc) ensure_lists(b, n);
+    if (!rc) ensure_lists(b, n, 2 * n_over > n_total);
     if (!rc) rc = ensure_slots(b, (uint32_t)slots_total);
     if (!rc) rc = ensure_tables(b, ns);
     if (rc) return rc;

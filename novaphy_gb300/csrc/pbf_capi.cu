@@ -457,6 +457,12 @@ void ensure_lists(pbf_scene* s) {
     }
     s->lmem = p;
     bind_lists(s->B, p, s->work_cap);
+    const pbf_settings& t = s->settings;
+    const bool off = rest_neighbors(t.kernel_radius, t.rest_density, s->mass) > kListRestMax;
+    if (begin_lists(s->B, off, s->stream) != cudaSuccess) {
+        cudaGetLastError();
+        free_lists(s);
+    }
 }
 
 }  // namespace

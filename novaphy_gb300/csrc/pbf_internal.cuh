@@ -119,7 +119,23 @@ inline void bind_lists(StepBuffers& B, void* mem, int c) {
     B.listed = reinterpret_cast<uint32_t*>(static_cast<char*>(mem) + r * kListRows * sizeof(uint2));
     B.list_cap = mem ? c : 0;
     if (!mem) B.listed = nullptr;
-    B.unlisted = mem ? B.listed + r : nullptr;
+    B.missing = mem ? reinterpret_cast<ListRecord*>(B.listed + r) : nullptr;
+}
+
+// Begins the record of lists just taken.  Fluid at rest has `rest` neighbours
+// in support: above kListRestMax the first steps try no lists (h = 5 r, 523:
+// 1M step 20.0 ms with lists that partly overflow, 22.1 without; 5.2 r, 589:
+// 27.7 and 25.5; 6 r: 54.1 and 40.7; 262,144 particles at 5 r 6.5 and 6.7, at
+// 5.1 r, 556, 7.9 and 7.1).
+constexpr double kListRestMax = 540.0;
+inline double rest_neighbors(float h, float rho0, float mass) {
+    return (double)rho0 * (4.0 / 3.0) * 3.14159265358979 * (double)h * h * h / (double)mass;
+}
+inline cudaError_t begin_lists(const StepBuffers& B, bool off, cudaStream_t st) {
+    cudaError_t e = cudaMemsetAsync(B.missing, 0, sizeof(ListRecord), st);
+    // (kListsOff fits the lowest byte.)
+    if (e == cudaSuccess && off) e = cudaMemsetAsync(&B.missing->off, (int)kListsOff, 1, st);
+    return e;
 }
 
 // Lists of that many bytes on stream `st`, null where they may not be taken now.

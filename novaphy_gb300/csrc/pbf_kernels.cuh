@@ -273,10 +273,10 @@ __device__ __forceinline__ void predict(const float4 xi, const float4 vi, const 
 // Predict + cell slot per particle (particle order), with the digits of the
 // slots counted for the sort.  Also turns this step's density-pass counts of
 // the last step (dhist, where there are any) into the previous step's, and
-// clears the flag of missing lists.
+// begins the step's record of missing lists (ListRecord).
 template <class P>
 __global__ void __launch_bounds__(kCountThreads)
-k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, uint32_t* __restrict__ unlisted,
+k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, ListRecord* __restrict__ missing,
               int n, const SortCounts counts, const SceneIds S, const P prm) {
     __shared__ BlockCounts B;
     const int t = blockIdx.x * blockDim.x + threadIdx.x;
@@ -286,7 +286,11 @@ k_predict_key(uint32_t* __restrict__ keys, uint32_t* __restrict__ dhist, uint32_
         d[0] = d[2 * kWalkHist];
         d[2 * kWalkHist] = 0u;
     }
-    if (unlisted && t == 0) *unlisted = 0u;
+    if (missing && t == 0) {
+        const uint32_t off = missing->off;
+        missing->off = off ? off - 1u : (2u * missing->failed > missing->tried ? kListsOff : 0u);
+        missing->any = missing->tried = missing->failed = 0u;
+    }
     B.begin(counts);
     for (int i = t; i < n; i += gridDim.x * blockDim.x) {
         const StepConsts& C = prm.at(S.pid, i);
@@ -776,7 +780,7 @@ struct Grid {
     const unsigned char* slot_alias;     // with kRunSlot where segend is set
     uint2* lists;                        // see StepBuffers::lists (null: none are kept)
     uint32_t* listed;
-    uint32_t* unlisted;
+    ListRecord* missing;
 };
 
 // for_each_candidate over a single scene's step with runs of identical
@@ -2811,10 +2815,16 @@ k_list(const float4* __restrict__ xin, float4* __restrict__ xout, int it, int n,
     const uint32_t p = blockIdx.x * blockDim.x + threadIdx.x;
     const bool active = p < (uint32_t)n;
     const uint32_t pa = active ? p : 0u;
+    const uint32_t off = G.missing->off;  // (waited for with the loads that follow)
     const StepConsts& C = prm.at(G.spid, pa);
     const int4 cell = cell_at(G, pa);
     const uint32_t rf = run_flags(G, pa);
     bool live = active && !(rf & kCopyBit);
+    if (off) {
+        if (active) G.listed[p] = kNoList;
+        if (threadIdx.x == 0) G.missing->any = 1u;
+        return;
+    }
     if (it >= 0) {
         live = live && it < C.iters;
         if (live && it > 0 && G.moved && cell.w == 0 &&
@@ -2836,7 +2846,7 @@ k_list(const float4* __restrict__ xin, float4* __restrict__ xout, int it, int n,
                                               xin[pa], xin, kept, none))
         kept = kNoList;
     if (live) G.listed[p] = kept;
-    if (live && kept == kNoList) *G.unlisted = 1u;
+    if (live && kept == kNoList) G.missing->any = 1u;
 }
 
 template <int BS, class P>
@@ -2844,13 +2854,18 @@ __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
 k_density_lambda(const float4* __restrict__ xin, float4* __restrict__ xout, float* __restrict__ srho,
                  int it, int n, int rest, const Grid G, const P prm) {
     __shared__ WalkSmem sm[BS / 32];
-    if (rest && *G.unlisted == 0u) return;
+    if (rest && G.missing->any == 0u) return;
     for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
         const uint32_t p = b * BS + threadIdx.x;
         const uint32_t pa = p < (uint32_t)n ? p : 0u;
-        if (!leave_out(rest, G, pa, p < (uint32_t)n && it < prm.at(G.spid, pa).iters &&
-                                           !(run_flags(G,
-                                             pa) & kCopyBit) && !(rest && (G.listed[pa] & kIdle))))
+        const bool out = leave_out(rest, G, pa, p < (uint32_t)n && it < prm.at(G.spid, pa).iters &&
+                                                    !(run_flags(G, pa) & kCopyBit) &&
+                                                    !(rest && (G.listed[pa] & kIdle)));
+        if (rest && (p & (32u * kListSample - 1u)) == 0u) {
+            atomicAdd(&G.missing->tried, 1u);
+            if (!out) atomicAdd(&G.missing->failed, 1u);
+        }
+        if (!out)
             density_lambda_at<false, kWalk>(p, p < (uint32_t)n, xin, xout, srho, it, G, prm,
                                             &sm[threadIdx.x >> 5]);
     }
@@ -3009,7 +3024,7 @@ k_delta(const float4* __restrict__ xin, float4* __restrict__ xout, const float4*
         const float* __restrict__ srho, float4* __restrict__ sv, int it, int n, int rest, const Grid G,
         const P prm) {
     __shared__ WalkSmem sm[BS / 32];
-    if (rest && *G.unlisted == 0u) return;
+    if (rest && G.missing->any == 0u) return;
     for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
         const uint32_t p = b * BS + threadIdx.x;
         const uint32_t pa = p < (uint32_t)n ? p : 0u;
@@ -3272,7 +3287,7 @@ __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
 k_xsph_commit(const float4* __restrict__ xin, const float4* __restrict__ sv, const float4* __restrict__ sx,
               const float* __restrict__ srho, int n, int skip_vort, int rest, const Grid G, const P prm) {
     __shared__ WalkSmem sm[BS / 32];
-    if (rest && *G.unlisted == 0u) return;
+    if (rest && G.missing->any == 0u) return;
     for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
         const uint32_t p = b * BS + threadIdx.x;
         const uint32_t pa = p < (uint32_t)n ? p : 0u;
@@ -3363,7 +3378,7 @@ __global__ void __launch_bounds__(BS, kPassMinBlocks<BS>)
 k_xsph_omega(const float4* __restrict__ xin, const float4* __restrict__ sv, float4* __restrict__ sv2,
              float4* __restrict__ som, int n, int rest, const Grid G, const P prm) {
     __shared__ WalkSmem sm[BS / 32];
-    if (rest && *G.unlisted == 0u) return;
+    if (rest && G.missing->any == 0u) return;
     for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
         const uint32_t p = b * BS + threadIdx.x;
         const uint32_t pa = p < (uint32_t)n ? p : 0u;
@@ -3456,7 +3471,7 @@ k_vorticity_commit(const float4* __restrict__ xin, const float4* __restrict__ sv
                    const float4* __restrict__ sx, const float* __restrict__ srho, int n, int rest,
                    const Grid G, const P prm) {
     __shared__ WalkSmem sm[BS / 32];
-    if (rest && *G.unlisted == 0u) return;
+    if (rest && G.missing->any == 0u) return;
     for (uint32_t b = blockIdx.x; b * BS < (uint32_t)n; b += gridDim.x) {
         const uint32_t p = b * BS + threadIdx.x;
         const uint32_t pa = p < (uint32_t)n ? p : 0u;
@@ -3544,7 +3559,7 @@ inline Grid grid_view(const StepBuffers& B, int n, const uint32_t* spid = nullpt
                       const BoundaryGrid& bg = BoundaryGrid{}) {
     return Grid{B.scell, B.sown, WalkIndex{(uint32_t)n, B.off, B.bkt.merged, B.bkt.end, B.btab}, spid,
                 B.moved, B.lamnz, bg, spid ? nullptr : B.dhist, nullptr, B.slot_alias,
-                n <= B.list_cap ? B.lists : nullptr, B.listed, B.unlisted};
+                n <= B.list_cap ? B.lists : nullptr, B.listed, B.missing};
 }
 
 // predict, sort by cell and by reference key, cell offsets, gather, reference
@@ -3560,7 +3575,7 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
     cudaError_t e = clear_ranges(slot_clear(B), sort_clear(sort, n, bits),
                                  C.hash_compat ? bucket_clear(B.bkt, n) : ClearRange{}, st);
     if (e != cudaSuccess) return e;
-    k_predict_key<OneScene><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, B.dhist, B.unlisted, n,
+    k_predict_key<OneScene><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, B.dhist, B.missing, n,
                                            sort_counts(sort, n,
         bits), none, one);
     if (pm) pm->mark(kPhasePredict, 2, st);
@@ -3812,7 +3827,7 @@ inline cudaError_t enqueue_batch_step(const StepBuffers& B, const BatchDesc& D, 
     cudaError_t e = clear_ranges(slot_clear(B), sort_clear(sort, n, D.key_bits), bucket_clear(B.bkt, n), st);
     if (e != cudaSuccess) return e;
     k_scene_ids<<<grid_of(n, 256), 256, 0, st>>>(D.firsts, D.nscenes, D.pid, n);
-    k_predict_key<SceneTable><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, nullptr, B.unlisted, n,
+    k_predict_key<SceneTable><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, nullptr, B.missing, n,
                                              sort_counts(sort,
         n, D.key_bits), ids, tab);
     if (pm) pm->mark(kPhasePredict, 3, st);

@@ -128,6 +128,18 @@ constexpr uint32_t bucket_slots(uint32_t n) {
     return s;
 }
 
+// What the warp passes of the steps had no kept lists for.  Where most warps
+// fail to list (fluid whose particles have more neighbours than a list holds),
+// listing in vain takes a quarter of a step, so steps without any follow.
+struct ListRecord {
+    uint32_t any;     // a particle of this step has no list
+    uint32_t tried;   // every kListSample-th warp of the density passes that walk for the rest,
+    uint32_t failed;  // and those of them that walk
+    uint32_t off;     // steps to come (with this one) that list nothing
+};
+constexpr uint32_t kListSample = 32;
+constexpr uint32_t kListsOff = 31;
+
 // Device buffers of one step.  Arrays named s* are in sorted (cell) order.
 struct StepBuffers {
     float4* x;      // positions, particle order (w unused)
@@ -176,7 +188,7 @@ struct StepBuffers {
     // (kNoList: no list).  Null where there was no room: the passes walk then.
     uint2* lists = nullptr;
     uint32_t* listed = nullptr;
-    uint32_t* unlisted = nullptr;  // set where a warp pass of the step had no list for a particle
+    ListRecord* missing = nullptr;
     int list_cap = 0;
     uint32_t* err;  // device status word
 };
