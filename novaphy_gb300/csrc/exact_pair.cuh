@@ -10,11 +10,12 @@
 //    (P. Markstein, "Computation of elementary functions on the IBM RISC
 //    System/6000 processor", IBM J. R&D 34, 1990): an approximation, its
 //    exact residual by fma, and one correction, which rounds correctly.
-//    They share one reciprocal square root.  Checked on the GPU: the root
-//    against sqrtf for every float in [1e-14, 1.1e4]; the quotient against
-//    IEEE division for every pair of significands where the inverse is the
-//    correctly rounded one, and for every dividend with each of the 449
-//    roots of that range whose inverse is not.
+//    They share one reciprocal square root.  tests/test_gpu_exact_pair.py
+//    checks the root against sqrtf for every float in [1e-14, 1.1e4], and the
+//    quotient against IEEE division for every significand of the dividend, at
+//    three exponents, with 4,096 roots and with each of the 449 of that range
+//    whose inverse is not the correctly rounded one.  (With the correctly
+//    rounded inverse the last correction rounds correctly: Markstein's theorem.)
 #pragma once
 
 #include <cuda_runtime.h>
