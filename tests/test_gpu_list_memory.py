@@ -101,16 +101,19 @@ def test_lists_give_way(ballast):
 
 def test_a_refusal_does_not_last(ballast):
     w = lattice(160)
-    ballast.take(5 * GB // 2)
     sc = scene(w)
+    snap = sc.snapshot()
+    ballast.take(5 * GB // 2)
     sc.step(w.dt)
     without = capi.scene_device_bytes(sc)
     assert without < list_bytes(w.n)
     ballast.free()
     for _ in range(80):
-        sc.step(1e-6, sync=False)
+        sc.restore(snap)  # the same step each time, not a pile's
+        sc.step(w.dt, sync=False)
     sc.sync()
     assert capi.scene_device_bytes(sc) > list_bytes(w.n)
+    snap.close()
     sc.close()
 
 
