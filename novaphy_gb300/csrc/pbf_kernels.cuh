@@ -765,7 +765,7 @@ k_classify(const int4* __restrict__ qcell, int nq, const int4* __restrict__ scel
 }
 
 // ---------------------------------------------------------------------------
-// Constraint and velocity kernels (one thread per cell-sorted particle)
+// Constraint and velocity kernels (a lane or part of a team per cell-sorted particle)
 
 struct Grid {
     const int4* __restrict__ scell;
@@ -2551,7 +2551,8 @@ __device__ __forceinline__ void read_lists(const Grid& G, uint32_t p, bool want,
     }
 }
 
-// Rows of the kept list of a particle that wants, 0 where it does not.
+// Candidates of the kept list of a particle that wants (kNoList: no list), 0
+// where it does not.
 __device__ __forceinline__ uint32_t list_rows(const Grid& G, uint32_t p, bool want) {
     return want ? G.listed[p] & kNoList : 0u;
 }
@@ -2794,8 +2795,9 @@ __device__ __forceinline__ void density_lambda_at(uint32_t p, bool active, const
 // flight and the whole L1 holds candidates.
 // Blocks of a walking launch for the rest, whose blocks go on to the next warps:
 // four waves, so that one with nothing to do costs 5 us at any size and piles
-// spread over the chip (ten steps of the 1M dam break into its corners: 4.74 M
-// particle-steps/s, 4.21 M with one wave, which saved 25 us of a 1M step).
+// spread over the chip (ten steps of the 1M dam break into its corners, before a
+// word held runs: 4.74 M particle-steps/s, 4.21 M with one wave, which saved 25
+// us of a 1M step).
 constexpr int kRestBlocks = 152 * 24;
 
 // Whether the walking launch `rest` leaves this warp out.
@@ -3562,8 +3564,8 @@ inline Grid grid_view(const StepBuffers& B, int n, const uint32_t* spid = nullpt
                 n <= B.list_cap ? B.lists : nullptr, B.listed, B.missing};
 }
 
-// predict, sort by cell and by reference key, cell offsets, gather, reference
-// buckets, classification: the neighbour structure of one scene's step.
+// predict, sort by cell, cell offsets and gather, reference buckets,
+// classification: the neighbour structure of one scene's step.
 inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, SortScratch& sort,
                                   cudaStream_t st, PhaseMarks* pm = nullptr) {
     const int n = C.n;
@@ -3576,8 +3578,7 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
                                  C.hash_compat ? bucket_clear(B.bkt, n) : ClearRange{}, st);
     if (e != cudaSuccess) return e;
     k_predict_key<OneScene><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, B.dhist, B.missing, n,
-                                           sort_counts(sort, n,
-        bits), none, one);
+        sort_counts(sort, n, bits), none, one);
     if (pm) pm->mark(kPhasePredict, 2, st);
     e = radix_sort_counted(B.keys, B.skeys, B.sidx, n, bits, sort, st);
     if (e != cudaSuccess) return e;
@@ -3598,20 +3599,20 @@ inline cudaError_t enqueue_prefix(const StepBuffers& B, const StepConsts& C, Sor
     return cudaGetLastError();
 }
 
-// The constraint, velocity, XSPH, vorticity and commit passes over n
-// cell-sorted particles for `max_iters` iterations, with constants from `prm`.
-// Scenes with vorticity take the XSPH+omega / vorticity+commit pair
-// (any_vort), the others XSPH+commit (any_plain).
 // Particles per team of the neighbour passes, 0 for warps with one lane per
 // particle, by the number of particles of the launch.  Warps need some 130,000
 // particles to keep the chip's 608 schedulers in work; below that their time
 // is that of one warp's chain.  Measured when both forms walked in every pass
 // (us a call, teams of 8 / 16 / 32 / warps): 1,000 particles at h = 2 r 193 /
-// 238 / 341 / 604; 8,000 at 4 r 365 / 368 / 464 / 992; four steps of 43,993
-// 4,609 / 4,565 / 7,289 / 11,318; 65,565 (fast build) 2,237 / 2,002 / 2,607 /
-// 3,684; a batch of 352,901 5,171 / 3,993 / 4,061 / 3,519.  With kept lists
-// (teams of 16 / warps): 43,993 3,436 / 11,055, 65,565 1,670 / 3,442.  Teams of
-// 32 were never the fastest and are not built.
+// 238 / 341 / 604; 8,000 at 4 r 365 / 368 / 464 / 992; a batch of 352,901 5,171
+// / 3,993 / 4,061 / 3,519.  Teams of 32 were never the fastest and are not built.
+// With kept lists (teams of 16 / warps), one step of a lattice at 4 r: 32,768
+// particles 446 / 666, 64,000 774 / 766, 97,336 1,066 / 944, 132,651 1,518 /
+// 1,239, 216,000 2,324 / 1,543; coupled, 250,000 4,075 / 2,895.  The line lies
+// above the lattice's, because fluid in motion scatters: of four steps of 43,993
+// particles (3,349 / 12,403) the first two take warps 0.9 ms each, and in the
+// others a few warps over scattered cells, which keep no lists, walk for 0.3 to
+// 0.7 ms in every pass; 65,565 in the fast build 1,671 / 2,503.
 inline int team_size(int n) {
     if (n < 8192) return 8;
     if (n < kBigScene) return 16;
@@ -3661,16 +3662,14 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, Grid G, int n, int ma
                     if (G.bg.spos) {
                         if constexpr (std::is_same<P, OneScene>::value)
                             k_density_lambda_listed<BS, kListedTwoWay, P><<<nb, BS, 0, st>>>(B.xa, B.xb,
-                                B.srho,
-                                it, n, G, prm);
+                                B.srho, it, n, G, prm);
                     } else {
                         k_density_lambda_listed<BS, kListed, P><<<nb, BS, 0, st>>>(B.xa, B.xb, B.srho, it,
-                            n, G,
-                            prm);
+                            n, G, prm);
                     }
                 }
-                k_density_lambda<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, rest(), G,
-                    prm);
+                k_density_lambda<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.xb, B.srho, it, n, rest(),
+                    G, prm);
             }
             if (pm) pm->mark(kPhaseDensity, TP == 0 && G.lists ? 3 : 1, st);
             if constexpr (TP != 0)
@@ -3683,12 +3682,11 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, Grid G, int n, int ma
                                 B.sv, it, n, G, prm);
                     } else {
                         k_delta_listed<BS, kListed, P><<<nb, BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv,
-                            it, n,
-                            G, prm);
+                            it, n, G, prm);
                     }
                 }
-                k_delta<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n, rest(),
-                                             G, prm);
+                k_delta<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xb, B.xa, B.sx, B.srho, B.sv, it, n,
+                    rest(), G, prm);
             }
             if (pm) pm->mark(kPhaseDelta, TP == 0 && G.lists ? 2 : 1, st);
         }
@@ -3720,8 +3718,7 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, Grid G, int n, int ma
         else {
             if (G.lists)
                 k_vorticity_commit_listed<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho,
-                    n, G,
-                    prm);
+                    n, G, prm);
             k_vorticity_commit<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.sv, B.sv2, B.som, B.sx, B.srho, n,
                 rest(), G, prm);
         }
@@ -3732,10 +3729,10 @@ inline cudaError_t enqueue_passes_bs(const StepBuffers& B, Grid G, int n, int ma
         if constexpr (TP != 0)
             k_xsph_commit_team<T, P><<<nb, 128, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
         else {
-            if (G.lists) k_xsph_commit_listed<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip,
+            if (G.lists)
+                k_xsph_commit_listed<BS, P><<<nb, BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, G, prm);
+            k_xsph_commit<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, rest(),
                 G, prm);
-            k_xsph_commit<BS, P><<<walk_blocks(), BS, 0, st>>>(B.xa, B.sv, B.sx, B.srho, n, skip, rest(), G,
-                                               prm);
         }
         if (pm) pm->mark(xsph_on ? kPhaseXsph : kPhaseCommit, TP == 0 && G.lists ? 2 : 1, st);
     }
@@ -3828,8 +3825,7 @@ inline cudaError_t enqueue_batch_step(const StepBuffers& B, const BatchDesc& D, 
     if (e != cudaSuccess) return e;
     k_scene_ids<<<grid_of(n, 256), 256, 0, st>>>(D.firsts, D.nscenes, D.pid, n);
     k_predict_key<SceneTable><<<count_blocks(n), kCountThreads, 0, st>>>(B.keys, nullptr, B.missing, n,
-                                             sort_counts(sort,
-        n, D.key_bits), ids, tab);
+        sort_counts(sort, n, D.key_bits), ids, tab);
     if (pm) pm->mark(kPhasePredict, 3, st);
     // Cell order: scene-major because every scene owns a slot range.
     e = radix_sort_counted(B.keys, B.skeys, B.sidx, n, D.key_bits, sort, st);
